@@ -93,11 +93,291 @@ __device__ void affine_scan(T* al, T* be, int n, Aff<T>* wsum) {
   __syncthreads();
 }
 
+// ------------------------------------------------------------------ n <= 4096: state in registers
+// One instance per CTA of 256 threads, P = ceil(n / 256) <= 16 contiguous nodes per thread.
+// The time loop is serial, so a step's latency is the run time.  The recurrence coefficients do
+// not change with time, so every product of them that the affine scan needs (per thread, per
+// shuffle level, per warp) is formed once before the loop and a step scans only the additive
+// parts: P dependent FMAs, five shuffles, the totals of the preceding warps, P FMAs.  The
+// composition order is that of affine_scan, so the values are the same.  The two sweeps cut the
+// nodes into chunks from opposite ends, so the intermediate values and the new state cross
+// through one padded shared-memory row (one pad word per chunk of even length: neighbouring
+// threads then start on different banks).  P is a template argument: the chunk loops have no
+// branches and constant offsets, without which a step takes twice as long.
+// Measured at n = 4096: FP32 4.5 us -> 0.9-1.2 us a step, factorisation 2.1 ms -> 0.1-0.27 ms;
+// 48 instances of 64..4096 nodes 16.0 -> 2.15 ms; FP64, 16 instances, 36.6 -> 19.5 ms.
+// What bounds it: the dependent chains of one CTA (FP32), FP64 issue of one SM (FP64, nine
+// operations a node and step at 1.7 lanes a clock).
+enum { RMAXP = 16 };
+
+// a product that no neighbouring addition is contracted with (the shared-memory form rounds it)
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+
+// b of x_k = a_k x_{k-1} + b_k composed over the preceding threads (affine_scan's order)
+template <typename T>
+__device__ __forceinline__ T scan_carry(T acc, const T (&la)[5], T ea, const Aff<T>* wt, int lane, int w) {
+#pragma unroll
+  for (int l = 0; l < 5; ++l) {
+    const T up = __shfl_up_sync(0xffffffffu, acc, 1 << l);
+    if (lane >= (1 << l)) acc = fma(la[l], up, acc);
+  }
+  T ex = __shfl_up_sync(0xffffffffu, acc, 1);
+  if (lane == 0) ex = (T)0;
+  if (lane == 31) const_cast<Aff<T>*>(wt)[w].b = acc;
+  __syncthreads();
+  T run = (T)0;
+#pragma unroll
+  for (int q = 0; q < 7; ++q) {
+    const Aff<T> t = wt[q];
+    if (q < w) run = fma(t.a, run, t.b);
+  }
+  return w > 0 ? fma(ea, run, ex) : ex;
+}
+
+// the time-invariant factors of scan_carry for one sweep: per shuffle level, the exclusive
+// product of the warp's preceding threads, and the warp totals' factors in wt
+template <typename T>
+__device__ __forceinline__ void scan_factors(T prod, T (&la)[5], T& ea, Aff<T>* wt, int lane, int w) {
+  T a = prod;
+#pragma unroll
+  for (int l = 0; l < 5; ++l) {
+    la[l] = a;
+    const T up = __shfl_up_sync(0xffffffffu, a, 1 << l);
+    if (lane >= (1 << l)) a = a * up;
+  }
+  ea = __shfl_up_sync(0xffffffffu, a, 1);
+  if (lane == 0) ea = (T)1;
+  if (lane == 31) wt[w].a = a;
+}
+
+// The roundings are those of reactor_kernel: its contraction of Ls c_{i-1} + Ld c_i + Lp c_{i+1}
+// is written out, since the last digits of a long FP32 run follow it.
+template <typename T, int P>
+__device__ void reactor_steps(const mjx_reactor_instance& I, T* row, const double* piv, Aff<T>* wt,
+                              const double* tri, T* out) {
+  const int n = I.n, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const bool dk = I.variant == MJX_REACTOR_DANCKWERTS, dkcn = I.variant == MJX_REACTOR_DANCKWERTS_CN;
+  constexpr int pad = (P & 1) ? 0 : 1;
+  const int lo = tid * P;                         // forward chunk: nodes lo .. lo + nf - 1
+  const int hi = n - 1 - lo;                      // backward chunk: nodes hi .. hi - nb + 1
+  const int nf = max(0, min(P, n - lo)), nb = max(0, min(P, hi + 1));
+  const int fph = lo + pad * tid;                 // row index of node lo
+  const int bq = hi >= 0 ? hi / P : 1, bph = hi >= 0 ? hi + pad * bq : P, brem = (n - 1) % P;
+  // tri: sub, dia, sup of the interior rows, sub and dia of the last, sup of row 0.  Places
+  // beyond a chunk's nodes get the identity (factor 1, value 0), so that the loops below run
+  // without branches; their row reads stay inside the row's slack and are not used.
+  T al[P], mi[P], ng[P];
+  T pf = (T)1, pb = (T)1;
+#pragma unroll
+  for (int k = 0; k < P; ++k) {
+    const int i = lo + k;
+    al[k] = (T)1; mi[k] = (T)0;
+    if (k < nf) {
+      const double m = piv[i];
+      const double sub = i == 0 ? (dk ? tri[0] : 0.0) : (i == n - 1 ? tri[3] : tri[0]);
+      mi[k] = (T)m;
+      al[k] = (T)(-sub * m);
+    }
+    pf = al[k] * pf;
+    const int j = hi - k;
+    ng[k] = (T)1;
+    if (k < nb) {
+      const double sup = j == n - 1 ? 0.0 : (j == 0 ? tri[5] : tri[2]);
+      ng[k] = -(T)(sup * piv[j]);
+    }
+    pb = ng[k] * pb;
+  }
+  Aff<T>* wf = wt;
+  Aff<T>* wb = wt + 8;
+  T laf[5], lab[5], eaf, eab;
+  scan_factors<T>(pf, laf, eaf, wf, lane, w);
+  scan_factors<T>(pb, lab, eab, wb, lane, w);
+  // rhs coefficients: r = c + dt/2 (Ls c_{i-1} + Ld c_i + Lp c_{i+1}) and the source of row 0
+  const double* L = tri + 6;
+  const T Ls = (T)L[0], Ld = (T)L[1], Lp = (T)L[2], Lsl = (T)L[3], Ldl = (T)L[4];
+  const T idz = (T)L[5], kp = (T)L[6], Dat = (T)I.Da, dtt = (T)I.dt, half_dt = (T)(0.5 * I.dt);
+  const T cin = (T)I.c_inlet;
+#pragma unroll
+  for (int k = 0; k < P; ++k)
+    if (k < nf) row[fph + k] = (!dk && !dkcn && lo + k == 0) ? cin : (T)I.c_init;
+  __syncthreads();
+  // Warps whose chunks are whole and hold no end row take loops without masks; the other one or
+  // two compute the same loops and then put in the end rows' values and the zeros beyond.
+  const bool full = __all_sync(0xffffffffu, lo + P <= n);
+  const bool inner = full && __all_sync(0xffffffffu, lo > 0 && lo + P < n);
+  const int kl = n - 1 - lo;  // the chunk place of the last node, if it is here
+  T d[P];
+  for (int step = 0; step < I.n_steps; ++step) {
+    T cv[P + 2];  // c at nodes lo - 1 .. lo + P
+    cv[0] = row[max(fph - 1 - pad, 0)];
+#pragma unroll
+    for (int k = 0; k <= P; ++k) cv[k + 1] = row[fph + k + (k >= P ? pad : 0)];
+    if (dk) {
+      if (lo == 0) cv[0] = (T)0;
+#pragma unroll
+      for (int k = 0; k < P; ++k) {
+        const T cl = cv[k], ci = cv[k + 1], cr = cv[k + 2];
+        const T lap = k == kl ? (T)2 * cl - (T)2 * ci : cl - (T)2 * ci + cr;
+        const T adv = k == 0 && lo == 0 ? -(ci - (T)1) * idz : -(ci - cl) * idz;
+        const T r = ci + kp * lap + dtt * (adv - Dat * ci);
+        d[k] = k < nf ? mul_rn(r, mi[k]) : (T)0;
+      }
+    } else {
+      T d0 = (T)0, dl = (T)0;
+      if (!inner) {  // rows 0 and n - 1
+        const T r0 = fma(half_dt, fma(Ld, cv[1], mul_rn(Lp, cv[2])), cv[1]);
+        d0 = mul_rn(dkcn ? r0 + mul_rn(dtt, idz) : cin, mi[0]);
+        const int last = n - 1 + pad * ((n - 1) / P), prev = n - 2 + pad * ((n - 2) / P);
+        const T cn = row[last], cm = row[max(prev, 0)];
+        dl = fma(half_dt, fma(Ldl, cn, mul_rn(Lsl, cm)), cn);
+      }
+#pragma unroll
+      for (int k = 0; k < P; ++k) {
+        const T Mc = fma(Lp, cv[k + 2], fma(Ld, cv[k + 1], mul_rn(Ls, cv[k])));
+        d[k] = mul_rn(fma(half_dt, Mc, cv[k + 1]), mi[k]);
+      }
+      if (!inner) {
+#pragma unroll
+        for (int k = 0; k < P; ++k) {
+          if (k >= kl) d[k] = k == kl ? mul_rn(dl, mi[k]) : (T)0;
+        }
+        if (lo == 0) d[0] = d0;
+      }
+    }
+    T acc = (T)0;
+#pragma unroll
+    for (int k = 0; k < P; ++k) acc = fma(al[k], acc, d[k]);
+    T y = scan_carry<T>(acc, laf, eaf, wf, lane, w);  // its barrier also ends the reads of the row
+    if (full) {
+#pragma unroll
+      for (int k = 0; k < P; ++k) {
+        y = fma(al[k], y, d[k]);
+        row[fph + k] = y;
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < P; ++k) {
+        y = fma(al[k], y, d[k]);
+        row[k < nf ? fph + k : -RMAXP - 2] = y;  // the slack's first word takes what is beyond
+      }
+    }
+    __syncthreads();
+    acc = (T)0;
+#pragma unroll
+    for (int k = 0; k < P; ++k) d[k] = row[bph - k - (k > brem ? pad : 0)];
+    if (!full) {
+#pragma unroll
+      for (int k = 0; k < P; ++k)
+        if (k >= nb) d[k] = (T)0;
+    }
+#pragma unroll
+    for (int k = 0; k < P; ++k) acc = fma(ng[k], acc, d[k]);
+    y = scan_carry<T>(acc, lab, eab, wb, lane, w);
+    if (full) {
+#pragma unroll
+      for (int k = 0; k < P; ++k) {
+        y = fma(ng[k], y, d[k]);
+        row[bph - k - (k > brem ? pad : 0)] = y;
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < P; ++k) {
+        y = fma(ng[k], y, d[k]);
+        row[k < nb ? bph - k - (k > brem ? pad : 0) : -RMAXP - 2] = y;
+      }
+    }
+    __syncthreads();
+  }
+  for (int i = tid; i < n; i += blockDim.x) out[i] = row[i + pad * (i / P)];
+}
+
+// Tridiagonal entries of the implicit matrix (tri[0..5]: sub, dia, sup of the interior rows,
+// sub and dia of the last row, sup of row 0; the returned dia0) and of the explicit operator
+// (tri[6..]: Ls, Ld, Lp, Lsl, Ldl, 1/dz, kappa), as reactor_kernel builds them.
+__device__ __forceinline__ double reactor_entries(const mjx_reactor_instance& I, double* tri) {
+  const int n = I.n;
+  const double Pe = I.Pe, Da = I.Da, dt = I.dt;
+  const bool dk = I.variant == MJX_REACTOR_DANCKWERTS, dkcn = I.variant == MJX_REACTOR_DANCKWERTS_CN;
+  const double dz = (dk || dkcn) ? 1.0 / n : 1.0 / (n - 1);
+  const double q = (1.0 / Pe) / (dz * dz);
+  const double kap = 0.5 * dt / (Pe * dz * dz);
+  const double Ls = q + 1.0 / dz, Ld = -2.0 * q - 1.0 / dz - Da, Lp = q;
+  const double Lsl = dkcn ? 2.0 * q + 1.0 / dz : q, Ldl = dkcn ? Ld : -q - 1.0 / dz - Da;
+  tri[0] = dk ? -kap : -0.5 * dt * Ls;
+  tri[1] = dk ? 1.0 + 2.0 * kap : 1.0 - 0.5 * dt * Ld;
+  tri[2] = dk ? -kap : -0.5 * dt * Lp;
+  tri[3] = dk ? -2.0 * kap : -0.5 * dt * Lsl;
+  tri[4] = dk ? 1.0 + 2.0 * kap : 1.0 - 0.5 * dt * Ldl;
+  tri[5] = (dk || dkcn) ? tri[2] : 0.0;
+  tri[6] = Ls; tri[7] = Ld; tri[8] = Lp; tri[9] = Lsl; tri[10] = Ldl; tri[11] = 1.0 / dz; tri[12] = kap;
+  return (dk || dkcn) ? tri[1] : 1.0;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) reactor_reg_kernel(ReactorArgs A) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ double tri[13];
+  __shared__ Aff<T> wt[16];
+  __shared__ int filled;
+  const mjx_reactor_instance I = A.inst[blockIdx.x];
+  const int n = I.n, tid = threadIdx.x;
+  T* out = reinterpret_cast<T*>(A.out) + I.offset;
+  if (n > 256 * RMAXP) return;  // reactor_kernel's
+  if (I.variant < MJX_REACTOR_DANCKWERTS || I.variant > MJX_REACTOR_DANCKWERTS_CN) {  // an RK4 instance
+    for (int i = tid; i < n; i += blockDim.x) out[i] = (T)NAN;
+    return;
+  }
+  const int per = (n + 255) / 256;
+  double* piv = reinterpret_cast<double*>(smem_raw);  // pivots 1/(b_i - a_i c'_{i-1})
+  T* row = reinterpret_cast<T*>(piv + n) + RMAXP + 2;  // slack on both sides
+  // Thomas factorisation, sequential in FP64 (each dependent FP64 instruction takes ~64
+  // cycles): the interior rows are equal, so once a pivot repeats exactly all later ones do;
+  // near that point the reciprocal is two Newton steps from the last pivot.
+  if (tid == 0) {
+    const double dia0 = reactor_entries(I, tri);
+    const double sub = tri[0], dia = tri[1], sup = tri[2];
+    double m = 1.0 / dia0;
+    double c = (n > 1 ? tri[5] : 0.0) * m;
+    piv[0] = m;
+    int i = 1;
+    for (; i < n - 1; ++i) {
+      const double x = dia - sub * c;
+      const double last = m;
+      const double e = 1.0 - x * m;
+      if (fabs(e) < 1e-4) {
+        m = m + m * e;
+        m = m + m * (1.0 - x * m);
+      } else {
+        m = 1.0 / x;
+      }
+      c = sup * m;
+      piv[i] = m;
+      if (m == last && i > 1) { ++i; break; }
+    }
+    filled = i;
+    if (n > 1) piv[n - 1] = 1.0 / (tri[4] - tri[3] * c);
+  }
+  __syncthreads();
+  const double mlast = piv[filled - 1];
+  for (int i = filled + tid; i < n - 1; i += blockDim.x) piv[i] = mlast;
+  __syncthreads();
+#define MJX_RSTEPS(PP) \
+  case PP: reactor_steps<T, PP>(I, row, piv, wt, tri, out); break;
+  switch (per) {
+    MJX_RSTEPS(1) MJX_RSTEPS(2) MJX_RSTEPS(3) MJX_RSTEPS(4) MJX_RSTEPS(5) MJX_RSTEPS(6) MJX_RSTEPS(7) MJX_RSTEPS(8)
+    MJX_RSTEPS(9) MJX_RSTEPS(10) MJX_RSTEPS(11) MJX_RSTEPS(12) MJX_RSTEPS(13) MJX_RSTEPS(14) MJX_RSTEPS(15)
+    MJX_RSTEPS(16)
+  }
+#undef MJX_RSTEPS
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256) reactor_kernel(ReactorArgs A) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const mjx_reactor_instance I = A.inst[blockIdx.x];
   const int n = I.n;
+  if (n <= 256 * RMAXP) return;  // reactor_reg_kernel's
   if (I.variant < MJX_REACTOR_DANCKWERTS || I.variant > MJX_REACTOR_DANCKWERTS_CN) {  // an RK4 instance
     T* o = reinterpret_cast<T*>(A.out) + I.offset;
     for (int i = threadIdx.x; i < n; i += blockDim.x) o[i] = (T)NAN;
@@ -293,6 +573,13 @@ __global__ void __launch_bounds__(32 * RW) reactor_rk4_kernel(ReactorArgs A) {
     if (i0 + q < n) out[i0 + q] = c[q];
 }
 
+// dynamic shared memory of reactor_reg_kernel: pivots and one padded row of 256 chunks with
+// slack on both sides (per grows with n, so the longest instance needs the most)
+static size_t reactor_reg_smem(int max_n, int elem) {
+  const int n = max_n < 256 * RMAXP ? max_n : 256 * RMAXP, per = (n + 255) / 256;
+  return (size_t)n * 8 + (size_t)(256 * (per + 1) + 2 * RMAXP + 6) * elem;
+}
+
 }  // namespace mjx
 
 using namespace mjx;
@@ -319,14 +606,26 @@ mjx_status mjx_reactor_cn_batch(const mjx_reactor_instance* inst_dev, int n_inst
     MJX_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     MJX_CUDA_TRY(cudaFuncSetAttribute(reactor_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
     MJX_CUDA_TRY(cudaFuncSetAttribute(reactor_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+    const int reg = (int)reactor_reg_smem(256 * RMAXP, 8);
+    MJX_CUDA_TRY(cudaFuncSetAttribute(reactor_reg_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, reg));
+    MJX_CUDA_TRY(cudaFuncSetAttribute(reactor_reg_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, reg));
     return MJX_OK;
   }));
   if (smem > 227 * 1024) return MJX_BAD_SHAPE;
   ReactorArgs A;
   A.inst = inst_dev; A.out = out; A.n_inst = n_inst;
   cudaStream_t s = (cudaStream_t)stream;
-  if (e == 4) reactor_kernel<float><<<n_inst, 256, smem, s>>>(A);
-  else reactor_kernel<double><<<n_inst, 256, smem, s>>>(A);
+  // instances of up to 4096 nodes run in registers, longer ones (FP32 up to 10 900, FP64 up to
+  // 5 400, whose state does not fit 256 threads) in shared memory; each kernel leaves the
+  // other's instances alone, so an instance's result does not depend on the batch
+  const size_t rsm = reactor_reg_smem(max_n, e);
+  if (e == 4) reactor_reg_kernel<float><<<n_inst, 256, rsm, s>>>(A);
+  else reactor_reg_kernel<double><<<n_inst, 256, rsm, s>>>(A);
+  MJX_CUDA_TRY(cudaGetLastError());
+  if (max_n > 256 * RMAXP) {
+    if (e == 4) reactor_kernel<float><<<n_inst, 256, smem, s>>>(A);
+    else reactor_kernel<double><<<n_inst, 256, smem, s>>>(A);
+  }
   return cuda_status(cudaGetLastError());
 }
 

@@ -108,3 +108,22 @@ def test_tubular_rk4_sweep_published(cuda):
         for c, o, ref in zip([cases[i] for i in sel], outs, [refs[i] for i in sel]):
             err = float(np.max(np.abs(o.double().cpu().numpy() - ref)))
             assert err < tol * max(1.0, float(np.max(np.abs(ref)))), (c.n, c.variant, dtype, err)
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float64, 1e-11), (torch.float32, 1e-4)])
+@pytest.mark.parametrize("variant", ["danckwerts", "dirichlet", "danckwerts_cn"])
+def test_reactor_chunk_edges_vs_oracle(cuda, variant, dtype, tol):
+    # the register kernel gives each of 256 threads ceil(n / 256) nodes, cut from both ends:
+    # lengths around the chunk edges, its last length (4096) and the shared-memory kernel's first
+    from moljax_gb300.core import reactor as R
+    kind = {"danckwerts": R.DANCKWERTS, "dirichlet": R.DIRICHLET, "danckwerts_cn": R.DANCKWERTS_CN}[variant]
+    fn = {"danckwerts": OR.danckwerts_cn, "danckwerts_cn": OR.danckwerts_full_cn,
+          "dirichlet": lambda *a: OR.dirichlet_cn(*a[:5], 1.0, a[5])}[variant]
+    cases = []
+    for i, n in enumerate((3, 33, 255, 256, 257, 511, 513, 1025, 2049, 4095, 4097)):
+        dt = 0.5 / n if variant == "danckwerts" else R.served_dt(n)[0]
+        cases.append(R.ReactorCase(n, 15.0 + 17 * i, 0.5 + 0.4 * i, dt, 8, kind, 0.25))
+    for c, o in zip(cases, R.solve_batch(cases, dtype)):
+        ref = fn(c.n, c.Pe, c.Da, c.dt, c.n_steps, c.c_init)
+        err = np.linalg.norm(o.double().cpu().numpy() - ref) / np.linalg.norm(ref)
+        assert err < tol, (c.n, err)
