@@ -147,7 +147,7 @@ size_t mjx_dftn_plan_bytes(int n, int dtype);
 mjx_status mjx_dftn_plan_init(void* plan, int n, int dtype, void* stream);
 size_t mjx_spectral_general2d_ws_bytes(int ny, int nx, int nfields, int dtype);
 /* out_f = real(IFFT2( m FFT2(in_f) )) for ny x nx interiors of any supported size, on the
- * full complex spectrum (row DFTs, transpose, column DFTs, multiplier, and back).  mult:
+ * half spectrum (row pairs r2c, column DFTs with the multiplier, c2r).  mult:
  * MJX_MULT_SCALE/HELMHOLTZ/CN/EXP/LAP with lam the FD or spectral symbol and D_f, the
  * advection forms MJX_MULT_ADV_* with vx_f, vy_f (may be NULL: zero), or MJX_MULT_TABLE with
  * table [ny][nx].  The same operations as mjx_spectral_apply2d / mjx_advdiff_op2d /
@@ -155,6 +155,13 @@ size_t mjx_spectral_general2d_ws_bytes(int ny, int nx, int nfields, int dtype);
 mjx_status mjx_spectral_apply_general2d(const void* plan_y, const void* plan_x, const mjx_grid2d* grid, int symbol,
                                         int dtype, int nfields, const double* D, const double* vx,
                                         const double* vy, double h, int mult, const void* table,
+                                        const void* in, void* out, void* ws, size_t ws_bytes, void* stream);
+
+/* n_steps times u_f <- real(IFFT2( m(h, D_f, lam) FFT2(u_f) )), each a full transform pair, by
+ * the general form above (the FFT-CN loop of fft_cn_step on grids of any supported size).
+ * mult: SCALE/HELMHOLTZ/CN/EXP/LAP.  Same workspace. */
+mjx_status mjx_spectral_steps_general2d(const void* plan_y, const void* plan_x, const mjx_grid2d* grid, int symbol,
+                                        int dtype, int nfields, const double* D, double h, int mult, int n_steps,
                                         const void* in, void* out, void* ws, size_t ws_bytes, void* stream);
 
 size_t mjx_spectral_general3d_ws_bytes(int nz, int ny, int nx, int dtype);

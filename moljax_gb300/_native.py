@@ -196,6 +196,8 @@ SIGNATURES = {
     "mjx_spectral_apply_general2d": (_i, [_vp, _vp, C.POINTER(Grid2DC), _i, _i, _i, C.POINTER(C.c_double),
                                           C.POINTER(C.c_double), C.POINTER(C.c_double), _d, _i, _vp, _vp, _vp,
                                           _vp, _sz, _vp]),
+    "mjx_spectral_steps_general2d": (_i, [_vp, _vp, C.POINTER(Grid2DC), _i, _i, _i, C.POINTER(C.c_double),
+                                          _d, _i, _i, _vp, _vp, _vp, _sz, _vp]),
     "mjx_spectral_general3d_ws_bytes": (_sz, [_i, _i, _i, _i]),
     "mjx_spectral_apply_general3d": (_i, [_vp, _vp, _vp, C.POINTER(Grid3DC), _i, _i, _d, _d, _i, _i, _vp, _vp,
                                           _vp, _sz, _vp]),

@@ -1,26 +1,32 @@
-// Spectral multipliers on periodic 2D grids of any size (numpy/jnp.fft accept any n; the
-// fused row/column passes of spectral.cu take powers of two).
+// Spectral multipliers on periodic 2D grids and 3D boxes of any size (numpy/jnp.fft accept any
+// n; the fused row/column passes of spectral.cu take powers of two).
 //
-// out_f = real(IFFT2( m(kx, ky) FFT2(in_f) )) on the full complex spectrum:
-//   R   real -> complex, row DFTs of length nx          [f][y][x]
-//   T   transpose                                        [f][x][y]
-//   C   row DFTs of length ny, multiplier, inverse DFTs  [f][x][y]
-//   T   transpose back, inverse row DFTs of length nx, real part
-// A DFT of length n is the shared-memory Stockham FFT when n is a power of two, a
-// mixed-radix (2, 3, 4, 5) Stockham FFT when n has no other prime factor, and
-// Bluestein's chirp-z form otherwise: with c[j] = exp(-i pi j^2 / n),
+// out_f = real(IFFT2( m(kx, ky) FFT2(in_f) )) on the half spectrum kx = 0..nx/2:
+//   R   r2c of row pairs (two real rows ride one complex DFT)   spec[f][y][ld]
+//   C   forward DFT along y, multiplier, inverse DFT, in place
+//   R'  c2r of row pairs
+// and on a box R, C along y per plane, C along z with the multiplier, C along y back, R'.
+// Several applications in a row fuse R' with the next R (rows go from spectrum to spectrum)
+// and read the multiplier from a table formed once.  A DFT of length n is the shared-memory
+// Stockham FFT when n is a power of two, a mixed-radix (2, 3, 4, 5) Stockham FFT when n has no
+// other prime factor, and Bluestein's chirp-z form otherwise: with c[j] = exp(-i pi j^2 / n),
 //   DFT_n(z)[k] = c[k] * IFFT_L( FFT_L(z c) * FFT_L(b) )[k],  b[j] = conj(c[|j|]),
 // a circular convolution of length L = 2^ceil(log2(2n - 1)) <= 4096 (n <= 2048).
-// Inverse DFTs use IDFT(z) = conj(DFT(conj(z))) / n.  The multiplier of the full
-// spectrum needs no Hermitian averaging: the real part is taken at the end, as the
-// reference's real(ifft2(.)) does.
+// Inverse DFTs use IDFT(z) = conj(DFT(conj(z))) / n.  The reference keeps real(ifft2(.)); on
+// the half spectrum that is the multiplier (m(k) + conj(m(-k))) / 2, which equals m(k) but on
+// the Nyquist lines of the advection forms and for tables without that symmetry.
+//
+// The full-spectrum form that this replaces (real to complex, row DFTs, transpose, column
+// DFTs, a multiplier pass with FP64 cosines per point, and back: nine launches in 2D, fourteen
+// in 3D) took 127 us a step at 450 x 600 FP32 and 626 us at 100^3 FP64; this one 24 us and
+// 235 us.  What bounds it: launch and barrier latency on L2-resident grids, FP64 issue.
 #include <math.h>
 #include <string.h>
 
 #include <vector>
 
-#include "fft.cuh"
 #include "autotune.cuh"
+#include "tfft.cuh"
 
 namespace mjx {
 
@@ -33,7 +39,7 @@ static inline size_t g256(size_t b) { return (b + 255) & ~size_t(255); }
 struct DftGeom {
   int n, L, log2L, bluestein, mixed, nrad;
   int rad[16];
-  size_t tw, chirp, bhat, total;
+  size_t tw, chirp, bhat, sym, total;
 };
 
 // radices 4, 2, 3, 5 covering n, or 0 if n has another prime factor
@@ -69,6 +75,7 @@ static DftGeom dft_geom(int n, int elem) {
   g.tw = o; o += g256(g.L * c);
   g.chirp = o; o += g256(n * c);
   g.bhat = o; o += g256(g.L * c);
+  g.sym = o; o += g256((size_t)2 * n * sizeof(double));  // d^2 lambda: FD, then spectral
   g.total = o;
   return g;
 }
@@ -102,410 +109,488 @@ static void host_fft2(std::vector<double>& re, std::vector<double>& im) {
 }
 
 template <typename T>
-struct DftArgs {
-  cx<T>* data;        // rows of n complex values, row stride ld
-  long long nrows, ld;
-  const cx<T>* tw;    // length-L twiddles (mixed radix: exp(-2 pi i m / n), m < n)
+struct Dft {
+  const cx<T>* tw;    // length-L twiddles in the form of tile_dft
   const cx<T>* chirp; // length n
   const cx<T>* bhat;  // length L, FFT_L(b) / L
-  int n, L, log2L, bluestein, nseq, inverse;
-  int mixed, nrad, tpsm;  // mixed radix: passes and threads per sequence
-  int rad[16];
-  T scale;
+  int n, L, bluestein;
+  int odd;            // an odd number of passes: the buffers swap
+  int tps;            // threads per sequence
+  int staged;         // the tables are copied to shared memory first
+  unsigned long long rad;
 };
 
-// small forward DFTs in registers (w = exp(-2 pi i / r)); the constants are cos/sin of
-// 2 pi/3, 2 pi/5, 4 pi/5
-template <typename C>
-__device__ __forceinline__ void sdft(C* v, int r) {
-  typedef decltype(C::x) R;
-  if (r == 2) {
-    const C a = v[0], b = v[1];
-    v[0] = cadd(a, b); v[1] = csub(a, b);
-  } else if (r == 3) {
-    const R h = (R)0.86602540378443864676;  // sin(2 pi / 3)
-    const C a = v[0], t = cadd(v[1], v[2]), d = csub(v[1], v[2]);
-    const C m = mk<C>(a.x - (R)0.5 * t.x, a.y - (R)0.5 * t.y);
-    const C q = mk<C>(h * d.y, -h * d.x);  // -i h d
-    v[0] = cadd(a, t); v[1] = cadd(m, q); v[2] = csub(m, q);
-  } else if (r == 4) {
-    const C a = v[0], b = v[1], c = v[2], d = v[3];
-    const C s0 = cadd(a, c), s1 = csub(a, c), t0 = cadd(b, d), t1 = csub(b, d);
-    const C jt1 = mk<C>(t1.y, -t1.x);  // -i (b - d)
-    v[0] = cadd(s0, t0); v[2] = csub(s0, t0); v[1] = cadd(s1, jt1); v[3] = csub(s1, jt1);
-  } else {  // r == 5
-    const R c1 = (R)0.30901699437494742410, c2 = (R)-0.80901699437494742410;
-    const R s1 = (R)0.95105651629515357212, s2 = (R)0.58778525229247312917;
-    const C a = v[0];
-    const C t1 = cadd(v[1], v[4]), t2 = cadd(v[2], v[3]), t3 = csub(v[1], v[4]), t4 = csub(v[2], v[3]);
-    const C m1 = mk<C>(a.x + c1 * t1.x + c2 * t2.x, a.y + c1 * t1.y + c2 * t2.y);
-    const C m2 = mk<C>(a.x + c2 * t1.x + c1 * t2.x, a.y + c2 * t1.y + c1 * t2.y);
-    const C n1 = mk<C>(s1 * t3.x + s2 * t4.x, s1 * t3.y + s2 * t4.y);
-    const C n2 = mk<C>(s2 * t3.x - s1 * t4.x, s2 * t3.y - s1 * t4.y);
-    v[0] = mk<C>(a.x + t1.x + t2.x, a.y + t1.y + t2.y);
-    v[1] = mk<C>(m1.x + n1.y, m1.y - n1.x);  // m1 - i n1
-    v[4] = mk<C>(m1.x - n1.y, m1.y + n1.x);  // m1 + i n1
-    v[2] = mk<C>(m2.x + n2.y, m2.y - n2.x);
-    v[3] = mk<C>(m2.x - n2.y, m2.y + n2.x);
+// A tile's two buffers and its tables.  Small tiles copy the tables to shared memory while
+// their data loads are in flight: a pass whose twiddles come from a cold L1 waits ~700 cycles
+// for L2, several times the pass itself.
+template <typename T>
+struct Tile {
+  cx<T>* cur;
+  cx<T>* alt;
+  const cx<T>* tw;
+  const cx<T>* chirp;
+  const cx<T>* bhat;
+  int lS, tid, nth;
+};
+
+template <typename T>
+__device__ __forceinline__ Tile<T> tile_begin(const Dft<T>& d, unsigned char* smem, int lS) {
+  typedef cx<T> C;
+  Tile<T> t;
+  const int m = sp_size(d.L << lS);
+  t.cur = reinterpret_cast<C*>(smem);
+  t.alt = t.cur + m;
+  t.lS = lS; t.tid = threadIdx.x; t.nth = blockDim.x;
+  t.tw = d.tw; t.chirp = d.chirp; t.bhat = d.bhat;
+  if (d.staged) {
+    C* w = t.alt + m;
+    for (int i = t.tid; i < d.L; i += t.nth) w[i] = __ldg(&d.tw[i]);
+    t.tw = w;
+    if (d.bluestein) {
+      C* b = w + d.L;
+      C* c = b + d.L;
+      for (int i = t.tid; i < d.L; i += t.nth) b[i] = __ldg(&d.bhat[i]);
+      for (int i = t.tid; i < d.n; i += t.nth) c[i] = __ldg(&d.chirp[i]);
+      t.bhat = b; t.chirp = c;
+    }
   }
+  return t;
 }
 
-// Mixed-radix Stockham DFT of lengths n = 2^a 3^b 5^c: pass (r, p) maps butterfly j
-// (k = j mod p) from src[j + t n/r] to dst[(j - k) r + k + t p] after the twiddles
-// w^(k t), w = exp(-2 pi i / (p r)); two shared buffers alternate between passes.
+// Forward DFT of the tile's sequences (elements 0 .. n - 1 of each), left in t.cur.  The caller
+// has synchronised.
 template <typename T>
-__global__ void __launch_bounds__(256) dft_mixed_kernel(const __grid_constant__ DftArgs<T> a) {
+__device__ __forceinline__ void dft_tile(const Dft<T>& d, Tile<T>& t) {
+  typedef cx<T> C;
+  const int lS = t.lS, L = d.L, n = d.n;
+  if (d.bluestein) {
+    for (int e = t.tid; e < (L << lS); e += t.nth) {
+      const int j = e >> lS;
+      t.cur[sp(e)] = j < n ? cmul(t.cur[sp(e)], t.chirp[j]) : mk<C>((T)0, (T)0);
+    }
+    __syncthreads();
+  }
+  tile_dft<T>(t.cur, t.alt, L, d.rad, lS, t.tw, t.tid, t.nth);
+  if (d.odd) { C* x = t.cur; t.cur = t.alt; t.alt = x; }
+  if (!d.bluestein) return;
+  // the inverse transform of the product by conjugation
+  for (int e = t.tid; e < (L << lS); e += t.nth) t.cur[sp(e)] = cconj(cmul(t.cur[sp(e)], t.bhat[e >> lS]));
+  __syncthreads();
+  tile_dft<T>(t.cur, t.alt, L, d.rad, lS, t.tw, t.tid, t.nth);
+  if (d.odd) { C* x = t.cur; t.cur = t.alt; t.alt = x; }
+  for (int e = t.tid; e < (n << lS); e += t.nth) t.cur[sp(e)] = cmul(cconj(t.cur[sp(e)]), t.chirp[e >> lS]);
+  __syncthreads();
+}
+
+// ------------------------------------------------------------------ row pass
+enum { GROW_LOAD_SPEC = 1, GROW_STORE_REAL = 2, GROW_STORE_SPEC = 4 };
+
+template <typename T>
+struct GRowArgs {
+  Dft<T> d;
+  const T* in;        // real rows of n values
+  T* out;
+  cx<T>* spec;        // half-spectrum rows, stride ld
+  long long nrows;    // real rows; pair q holds rows 2q and 2q + 1
+  int ld, lS, flags;
+};
+
+// S = 2^lS row pairs per CTA.
+template <typename T>
+__global__ void __launch_bounds__(512) grow_kernel(const __grid_constant__ GRowArgs<T> a) {
   typedef cx<T> C;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int n = a.n, T_ = a.tpsm, tid = threadIdx.x;
-  C* b0 = reinterpret_cast<C*>(smem_raw);
-  C* b1 = b0 + (long long)a.nseq * n;
-  const int s = tid / T_, lt = tid - s * T_;
-  const long long row = (long long)blockIdx.x * a.nseq + s;
-  const bool active = s < a.nseq && row < a.nrows;
-  C* x = a.data + row * a.ld;
-  C* src = b0 + s * n;
-  C* dst = b1 + s * n;
-  if (active)
-    for (int j = lt; j < n; j += T_) {
-      C v = x[j];
-      if (a.inverse) v.y = -v.y;
-      src[j] = v;
+  const int n = a.d.n, hx = n / 2 + 1, lS = a.lS, S = 1 << lS, tid = threadIdx.x, nth = blockDim.x;
+  Tile<T> t = tile_begin<T>(a.d, smem_raw, lS);
+  const long long r0 = ((long long)blockIdx.x << lS) * 2;  // first row of this CTA
+  const float rn = 1.0f / (float)n, rh = 1.0f / (float)hx;
+  if (a.flags & GROW_LOAD_SPEC) {
+    // conj of Z_k = A_k + i B_k and Z_{n-k} = conj(A_k) + i conj(B_k)
+    for (int e = tid; e < S * hx; e += nth) {
+      const int s = fdiv(e, rh), k = e - s * hx;
+      const long long ra = r0 + 2 * s, rb = ra + 1;
+      C A = mk<C>((T)0, (T)0), B = A;
+      if (ra < a.nrows) A = a.spec[ra * a.ld + k];
+      if (rb < a.nrows) B = a.spec[rb * a.ld + k];
+      t.cur[sp((k << lS) + s)] = mk<C>(A.x - B.y, -(A.y + B.x));
+      if (k > 0 && 2 * k < n) t.cur[sp(((n - k) << lS) + s)] = mk<C>(A.x + B.y, A.y - B.x);
     }
-  __syncthreads();
-  int p = 1;
-  for (int q = 0; q < a.nrad; ++q) {
-    const int r = a.rad[q], nb = n / r, step = n / (p * r);
-    if (active)
-      for (int j = lt; j < nb; j += T_) {
-        const int k = j % p;
-        C v[5];
-        for (int t = 0; t < r; ++t) v[t] = src[j + t * nb];
-        if (p > 1)
-          for (int t = 1; t < r; ++t) v[t] = cmul(v[t], __ldg(&a.tw[k * t * step]));
-        sdft(v, r);
-        const int base = (j - k) * r + k;
-        for (int t = 0; t < r; ++t) dst[base + t * p] = v[t];
+    __syncthreads();
+    dft_tile<T>(a.d, t);
+    if (a.flags & GROW_STORE_REAL) {
+      for (int e = tid; e < S * n; e += nth) {
+        const int s = fdiv(e, rn), x = e - s * n;
+        const long long ra = r0 + 2 * s, rb = ra + 1;
+        const C v = t.cur[sp((x << lS) + s)];
+        if (ra < a.nrows) a.out[ra * n + x] = v.x;
+        if (rb < a.nrows) a.out[rb * n + x] = -v.y;
       }
-    __syncthreads();
-    C* tmp = src; src = dst; dst = tmp;
-    p *= r;
+      return;
+    }
+    for (int e = tid; e < S * n; e += nth) {  // the real rows a + i b, never stored
+      const C v = t.cur[sp(e)];
+      t.cur[sp(e)] = mk<C>(v.x, -v.y);
+    }
+  } else {
+    for (int e = tid; e < S * n; e += nth) {
+      const int s = fdiv(e, rn), x = e - s * n;
+      const long long ra = r0 + 2 * s, rb = ra + 1;
+      const T va = ra < a.nrows ? a.in[ra * n + x] : (T)0, vb = rb < a.nrows ? a.in[rb * n + x] : (T)0;
+      t.cur[sp((x << lS) + s)] = mk<C>(va, vb);
+    }
   }
-  if (active)
-    for (int j = lt; j < n; j += T_) {
-      C v = src[j];
-      if (a.inverse) v.y = -v.y;
-      x[j] = mk<C>(v.x * a.scale, v.y * a.scale);
-    }
-}
-
-// nseq rows per CTA, each in its own shared-memory segment of length L
-template <typename T>
-__global__ void __launch_bounds__(256) dft_rows_kernel(const __grid_constant__ DftArgs<T> a) {
-  typedef cx<T> C;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* buf = reinterpret_cast<C*>(smem_raw);
-  const int L = a.L, tps = L >= 16 ? L / 16 : 1, tid = threadIdx.x;
-  const int s = tid / tps, lt = tid - s * tps;
-  const long long row = (long long)blockIdx.x * a.nseq + s;
-  const bool active = s < a.nseq && row < a.nrows;
-  const int base = s * L;
-  C* x = a.data + row * a.ld;
-  if (active)
-    for (int j = lt; j < L; j += tps) {
-      C v = mk<C>((T)0, (T)0);
-      if (j < a.n) {
-        v = x[j];
-        if (a.inverse) v.y = -v.y;
-        if (a.bluestein) v = cmul(v, __ldg(&a.chirp[j]));
-      }
-      buf[sp(base + j)] = v;
-    }
   __syncthreads();
-  fft_smem<T, false, false>(buf, L, a.log2L, a.nseq, L, 1, a.tw, tid);
-  if (a.bluestein) {
-    if (active)
-      for (int j = lt; j < L; j += tps) buf[sp(base + j)] = cmul(buf[sp(base + j)], __ldg(&a.bhat[j]));
-    __syncthreads();
-    fft_smem<T, true, false>(buf, L, a.log2L, a.nseq, L, 1, a.tw, tid);
-    if (active)
-      for (int j = lt; j < a.n; j += tps) buf[sp(base + j)] = cmul(buf[sp(base + j)], __ldg(&a.chirp[j]));
-    __syncthreads();
-  }
-  if (active)
-    for (int j = lt; j < a.n; j += tps) {
-      C v = buf[sp(base + j)];
-      if (a.inverse) v.y = -v.y;
-      x[j] = mk<C>(v.x * a.scale, v.y * a.scale);
-    }
-}
-
-// out[b][c][r] = in[b][r][c] for rows x cols matrices, 32 x 32 tiles
-template <typename T>
-__global__ void transpose_kernel(const cx<T>* __restrict__ in, cx<T>* __restrict__ out, int rows, int cols) {
-  __shared__ cx<T> tile[32][33];
-  const long long b = blockIdx.z;
-  const cx<T>* src = in + b * (long long)rows * cols;
-  cx<T>* dst = out + b * (long long)rows * cols;
-  const int c0 = blockIdx.x * 32;
-  // row tiles in a grid-stride loop (gridDim.y is capped at 65535)
-  for (int r0 = blockIdx.y * 32; r0 < rows; r0 += gridDim.y * 32) {
-    for (int i = threadIdx.y; i < 32; i += 8) {
-      const int r = r0 + i, c = c0 + threadIdx.x;
-      if (r < rows && c < cols) tile[i][threadIdx.x] = src[(long long)r * cols + c];
-    }
-    __syncthreads();
-    for (int i = threadIdx.y; i < 32; i += 8) {
-      const int c = c0 + i, r = r0 + threadIdx.x;
-      if (r < rows && c < cols) dst[(long long)c * rows + r] = tile[threadIdx.x][i];
-    }
-    __syncthreads();
+  dft_tile<T>(a.d, t);
+  for (int e = tid; e < S * hx; e += nth) {
+    const int s = fdiv(e, rh), k = e - s * hx;
+    const long long ra = r0 + 2 * s, rb = ra + 1;
+    const C Zk = t.cur[sp((k << lS) + s)], Zm = t.cur[sp(((k == 0 ? 0 : n - k) << lS) + s)];
+    if (ra < a.nrows) a.spec[ra * a.ld + k] = mk<C>((T)0.5 * (Zk.x + Zm.x), (T)0.5 * (Zk.y - Zm.y));
+    if (rb < a.nrows) a.spec[rb * a.ld + k] = mk<C>((T)0.5 * (Zk.y + Zm.y), (T)0.5 * (Zm.x - Zk.x));
   }
 }
 
-template <typename T>
-__global__ void real_to_complex_kernel(const T* __restrict__ in, cx<T>* __restrict__ out, long long n) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    out[i] = mk<cx<T>>(in[i], (T)0);
-}
-
-template <typename T>
-__global__ void complex_real_kernel(const cx<T>* __restrict__ in, T* __restrict__ out, long long n) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    out[i] = in[i].x;
-}
-
-struct GenMul {
-  int nx, ny, symbol, mult, nf;
-  double dx, dy, h;
+// ------------------------------------------------------------------ multipliers
+struct GMul {
+  int mult, nx, nb, ny;     // sizes along x, the batch axis of a box (0 in 2D), the column
+  int symbol;
+  const double* sx;         // d^2 lambda along x, the batch axis and the column
+  const double* sb;
+  const double* sy;
+  double ix, ib, iy;        // 1 / d^2 of each
+  double kxs, kys;          // 2 pi / (n d) along x and the column (advection forms)
+  double h, scale;
   double D[4], vx[4], vy[4];
 };
 
-// multiplier on the transposed spectrum [f][kx][ky]
+// The multiplier of half-spectrum point (ky, kx) of field f (box: ky along z, kb along y),
+// times the normalisation, as a complex number; FP64 throughout.
+__device__ __forceinline__ double2 gmul_value(const GMul& m, int f, int ky, int kb, int kx) {
+  double lam = m.sx[kx] * m.ix + m.sy[ky] * m.iy;
+  if (m.nb) lam += m.sb[kb] * m.ib;
+  const double zr = m.h * m.D[f] * lam;
+  double fr, fi = 0.0;
+  if (m.mult < MJX_MULT_ADV_SOLVE) {
+    if (m.mult == MJX_MULT_HELMHOLTZ) {
+      double den = 1.0 - zr;
+      if (fabs(den) < 1e-14) den = 1e-14;
+      fr = 1.0 / den;
+    } else if (m.mult == MJX_MULT_CN) {
+      fr = (1.0 + 0.5 * zr) / (1.0 - 0.5 * zr);
+    } else if (m.mult == MJX_MULT_LAP) {
+      fr = zr;
+    } else if (m.mult == MJX_MULT_EXP) {
+      fr = exp(zr);
+    } else {
+      fr = 1.0;
+    }
+    return make_double2(fr * m.scale, 0.0);
+  }
+  // z = h (D lam - i (vx kx + vy ky)) with fftfreq indices (the Nyquist index of an even
+  // length negative), averaged with the conjugate at -k
+  const int mx = kx < (m.nx + 1) / 2 ? kx : kx - m.nx, my = ky < (m.ny + 1) / 2 ? ky : ky - m.ny;
+  double mre = 0.0, mim = 0.0;
+#pragma unroll 1
+  for (int side = 0; side < 2; ++side) {
+    const int qx = side ? (2 * mx == -m.nx ? mx : -mx) : mx, qy = side ? (2 * my == -m.ny ? my : -my) : my;
+    const double zi = -m.h * (m.vx[f] * m.kxs * qx + m.vy[f] * m.kys * qy);
+    if (m.mult == MJX_MULT_ADV_SOLVE) {
+      double dr = 1.0 - zr, di = -zi;
+      if (sqrt(dr * dr + di * di) < 1e-14) { dr = 1e-14; di = 0.0; }
+      const double den = dr * dr + di * di;
+      fr = dr / den; fi = -di / den;
+    } else if (m.mult == MJX_MULT_ADV_LAP) {
+      fr = zr; fi = zi;
+    } else if (m.mult == MJX_MULT_ADV_CN) {
+      const double nr = 1.0 + 0.5 * zr, ni = 0.5 * zi, dr = 1.0 - 0.5 * zr, di = -0.5 * zi;
+      const double den = dr * dr + di * di;
+      fr = (nr * dr + ni * di) / den; fi = (ni * dr - nr * di) / den;
+    } else {
+      double sn, cs;
+      sincos(zi, &sn, &cs);
+      const double ez = exp(zr);
+      fr = ez * cs; fi = ez * sn;
+    }
+    mre += 0.5 * fr;
+    mim += side ? -0.5 * fi : 0.5 * fi;
+  }
+  return make_double2(mre * m.scale, mim * m.scale);
+}
+
+// ------------------------------------------------------------------ column pass
+enum { GCOL_NONE = 0, GCOL_VALUE = 1, GCOL_TABLE = 2, GCOL_USER = 3 };
+
 template <typename T>
-__global__ void general_mult_kernel(cx<T>* __restrict__ s, const T* __restrict__ table, const GenMul m) {
-  const long long per = (long long)m.nx * m.ny, total = per * m.nf;
-  const double twopi = 6.283185307179586476925286766559;
+struct GColArgs {
+  Dft<T> d;
+  cx<T>* spec;
+  const T* tab;        // GCOL_TABLE: formed multipliers [batch][n][ld]; GCOL_USER: the caller's [ny][nx]
+  long long bstride;   // complex elements between batch entries (fields or planes)
+  int ld, ncols, hx;   // row stride, columns; columns with (col mod ldx) >= hx are padding
+  int ldx;             // row length of a z-pass column index (ld in 2D)
+  int lC, dirs, mode;
+  GMul m;
+};
+
+// C = 2^lC columns per CTA; blockIdx.y is the batch entry.
+template <typename T>
+__global__ void __launch_bounds__(512) gcol_kernel(const __grid_constant__ GColArgs<T> a) {
+  typedef cx<T> C;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int n = a.d.n, lC = a.lC, Cn = 1 << lC, tid = threadIdx.x, nth = blockDim.x;
+  Tile<T> t = tile_begin<T>(a.d, smem_raw, lC);
+  const int c0 = blockIdx.x << lC, b = blockIdx.y;
+  C* g = a.spec + (long long)b * a.bstride + c0;
+  const bool inv_first = (a.dirs & 1) == 0;
+  for (int e = tid; e < (n << lC); e += nth) {
+    const int j = e >> lC, c = e & (Cn - 1);
+    C v = c0 + c < a.ncols ? g[(long long)j * a.ld + c] : mk<C>((T)0, (T)0);
+    if (inv_first) v.y = -v.y;
+    t.cur[sp(e)] = v;
+  }
+  __syncthreads();
+  dft_tile<T>(a.d, t);
+  if (a.dirs == 3) {
+    for (int e = tid; e < (n << lC); e += nth) {
+      const int j = e >> lC, c = e & (Cn - 1), col = c0 + c;
+      const C v = t.cur[sp(e)];
+      T mr = (T)0, mi = (T)0;
+      if (col < a.ncols) {
+        if (a.mode == GCOL_TABLE) {
+          mr = a.tab[((long long)b * n + j) * a.ld + col];
+        } else {
+          const int kb = a.m.nb ? col / a.ldx : 0, kx = col - kb * a.ldx;
+          if (kx < a.hx) {
+            if (a.mode == GCOL_USER) {  // the real kernel's Hermitian part
+              const int jm = j == 0 ? 0 : n - j, xm = kx == 0 ? 0 : a.m.nx - kx;
+              mr = (T)(0.5 * a.m.scale * ((double)a.tab[(long long)j * a.m.nx + kx] + (double)a.tab[(long long)jm * a.m.nx + xm]));
+            } else {
+              const double2 f = gmul_value(a.m, b, j, kb, kx);
+              mr = (T)f.x; mi = (T)f.y;
+            }
+          }
+        }
+      }
+      // conj(m v), for the inverse by conjugation
+      t.cur[sp(e)] = mk<C>(v.x * mr - v.y * mi, -(v.x * mi + v.y * mr));
+    }
+    __syncthreads();
+    dft_tile<T>(a.d, t);
+  }
+  const bool neg = (a.dirs & 2) != 0;
+  for (int e = tid; e < (n << lC); e += nth) {
+    const int j = e >> lC, c = e & (Cn - 1);
+    C v = t.cur[sp(e)];
+    if (neg) v.y = -v.y;
+    if (c0 + c < a.ncols) g[(long long)j * a.ld + c] = v;
+  }
+}
+
+// the formed multipliers of a real symbol, [batch][n][ld]
+template <typename T>
+__global__ void gtab_kernel(T* tab, const __grid_constant__ GMul m, int nf, int n, int ld, int ldx, int hx) {
+  const long long per = (long long)n * ld, total = per * nf;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
     const int f = (int)(i / per);
     const long long r = i - f * per;
-    const int kx = (int)(r / m.ny), ky = (int)(r - (long long)kx * m.ny);
-    const cx<T> v = s[i];
-    if (m.mult == MJX_MULT_TABLE) {
-      const T t = table[(long long)ky * m.nx + kx];
-      s[i] = mk<cx<T>>(v.x * t, v.y * t);
-      continue;
-    }
-    // fftfreq indices (the Nyquist index of an even length negative)
-    const int mx = kx < (m.nx + 1) / 2 ? kx : kx - m.nx, my = ky < (m.ny + 1) / 2 ? ky : ky - m.ny;
-    double lam;
-    if (m.symbol == MJX_SYMBOL_FD) {
-      lam = (2.0 * cospi(2.0 * kx / m.nx) - 2.0) / (m.dx * m.dx) + (2.0 * cospi(2.0 * ky / m.ny) - 2.0) / (m.dy * m.dy);
-    } else {
-      const double ax = twopi * mx / (m.nx * m.dx), ay = twopi * my / (m.ny * m.dy);
-      lam = -(ax * ax + ay * ay);
-    }
-    const double zr = m.h * m.D[f] * lam;
-    const double zi = -m.h * (m.vx[f] * twopi * mx / (m.nx * m.dx) + m.vy[f] * twopi * my / (m.ny * m.dy));
-    double fr, fi;
-    switch (m.mult) {
-      case MJX_MULT_SCALE: fr = 1.0; fi = 0.0; break;
-      case MJX_MULT_HELMHOLTZ:
-      case MJX_MULT_ADV_SOLVE: {
-        double dr = 1.0 - zr, di = -zi;
-        if (sqrt(dr * dr + di * di) < 1e-14) { dr = 1e-14; di = 0.0; }
-        const double den = dr * dr + di * di;
-        fr = dr / den; fi = -di / den;
-        break;
-      }
-      case MJX_MULT_CN:
-      case MJX_MULT_ADV_CN: {
-        const double nr = 1.0 + 0.5 * zr, ni = 0.5 * zi, dr = 1.0 - 0.5 * zr, di = -0.5 * zi;
-        const double den = dr * dr + di * di;
-        fr = (nr * dr + ni * di) / den; fi = (ni * dr - nr * di) / den;
-        break;
-      }
-      case MJX_MULT_LAP:
-      case MJX_MULT_ADV_LAP: fr = zr; fi = zi; break;
-      default: {  // exp
-        double sn, cs;
-        sincos(zi, &sn, &cs);
-        const double ez = exp(zr);
-        fr = ez * cs; fi = ez * sn;
-      }
-    }
-    const T Fr = (T)fr, Fi = (T)fi;
-    s[i] = mk<cx<T>>(v.x * Fr - v.y * Fi, v.x * Fi + v.y * Fr);
+    const int j = (int)(r / ld), col = (int)(r - (long long)j * ld);
+    const int kb = m.nb ? col / ldx : 0, kx = col - kb * ldx;
+    tab[i] = kx < hx ? (T)gmul_value(m, f, j, kb, kx).x : (T)0;
   }
 }
 
-// threads per sequence tp in [1, 256] (default n/8); sequences per CTA within 256
-// threads and 96 KB of shared memory
-template <typename T>
-static void mixed_launch(DftArgs<T>& a, int tp) {
-  int T_ = tp;
-  if (T_ < 1) T_ = 1;
-  if (T_ > 256) T_ = 256;
-  a.tpsm = T_;
-  int ns = 256 / T_;
-  const int cap = (int)((96 * 1024) / (2 * (size_t)a.n * sizeof(cx<T>)));
-  if (ns > cap) ns = cap;
-  a.nseq = ns < 1 ? 1 : ns;
+// ------------------------------------------------------------------ launch geometry
+// half-spectrum row length, whole 32-byte sectors
+static int gen_ld(int nx, int elem) {
+  const int q = 32 / (2 * elem);
+  return (nx / 2 + 1 + q - 1) / q * q;
+}
+
+// radices (at most 16 of them, each below 16) as tile_dft takes them
+static unsigned long long pack_radices(int k, const int* rad) {
+  unsigned long long r = 0;
+  for (int i = 0; i < k; ++i) r |= (unsigned long long)rad[i] << (4 * i);
+  return r;
 }
 
 template <typename T>
-static DftArgs<T> dft_args(const void* plan, int n, cx<T>* data, long long nrows, long long ld, int inverse) {
+static Dft<T> dft_desc(const void* plan, int n) {
   const DftGeom g = dft_geom(n, sizeof(T));
   const char* p = (const char*)plan;
-  DftArgs<T> a;
-  memset(&a, 0, sizeof(a));
-  a.data = data; a.nrows = nrows; a.ld = ld;
-  a.tw = (const cx<T>*)(p + g.tw); a.chirp = (const cx<T>*)(p + g.chirp); a.bhat = (const cx<T>*)(p + g.bhat);
-  a.n = n; a.L = g.L; a.log2L = g.log2L; a.bluestein = g.bluestein; a.inverse = inverse;
-  a.mixed = g.mixed; a.nrad = g.nrad;
-  for (int i = 0; i < 16; ++i) a.rad[i] = g.rad[i];
+  Dft<T> d;
+  memset(&d, 0, sizeof(d));
+  d.tw = (const cx<T>*)(p + g.tw); d.chirp = (const cx<T>*)(p + g.chirp); d.bhat = (const cx<T>*)(p + g.bhat);
+  d.n = n; d.L = g.L; d.bluestein = g.bluestein;
   if (g.mixed) {
+    d.rad = pack_radices(g.nrad, g.rad);
+    d.odd = g.nrad & 1;
     DftTune t;
-    const int tp = (tune_dft_get(n, (int)sizeof(T), &t) && t.tpsm > 0) ? t.tpsm : n / 8;
-    mixed_launch(a, tp);
+    d.tps = (tune_dft_get(n, (int)sizeof(T), &t) && t.tpsm > 0) ? t.tpsm : n / 8;
   } else {
-    const int tps = g.L >= 16 ? g.L / 16 : 1;
-    a.nseq = tps >= 256 ? 1 : 256 / tps;
+    int passes = 0;
+    d.rad = tile_pow2_radices(g.log2L, &passes);
+    d.odd = passes & 1;
+    d.tps = g.L / 8;
   }
-  a.scale = (T)(inverse ? 1.0 / n : 1.0);
-  return a;
+  if (d.tps < 1) d.tps = 1;
+  if (d.tps > 256) d.tps = 256;
+  return d;
 }
 
 template <typename T>
-static cudaError_t dft_rows(const DftArgs<T>& a, cudaStream_t s) {
-  if (a.mixed) {
-    const long long grid = (a.nrows + a.nseq - 1) / a.nseq;
-    const size_t smem = (size_t)2 * a.nseq * a.n * sizeof(cx<T>);
-    dft_mixed_kernel<T><<<(unsigned)grid, a.nseq * a.tpsm, smem, s>>>(a);
-    return cudaGetLastError();
-  }
-  const int tps = a.L >= 16 ? a.L / 16 : 1;
-  const long long grid = (a.nrows + a.nseq - 1) / a.nseq;
-  const size_t smem = (size_t)sp_size(a.nseq * a.L) * sizeof(cx<T>);
-  dft_rows_kernel<T><<<(unsigned)grid, a.nseq * tps, smem, s>>>(a);
+static size_t tile_smem(const Dft<T>& d, int l) {
+  size_t e = 2 * (size_t)sp_size(d.L << l);
+  if (d.staged) e += (size_t)d.L + (d.bluestein ? (size_t)d.L + d.n : 0);
+  return e * sizeof(cx<T>);
+}
+
+// Sequences per CTA (log2) for `total` sequences: up to `want`, within 512 threads and 96 KB of
+// shared memory (one sequence may take more), halved until the pass has about one CTA per SM;
+// tables in shared memory where the whole stays under 96 KB.  A pass with few sequences doubles
+// the threads of each (n/4 instead of n/8): its time is a chain of passes, not throughput.
+template <typename T>
+static int tile_log(Dft<T>& d, long long total, int want) {
+  const size_t cap = 96 * 1024;
+  int l = 0;
+  while ((2 << l) <= want && (2 << l) * d.tps <= 512 && tile_smem<T>(d, l + 1) <= cap) ++l;
+  while (l > 0 && (total + (1 << l) - 1) >> l < 128) --l;
+  if (((d.tps << l) + 31) / 32 * ((total + (1 << l) - 1) >> l) < 152 * 8 && (2 * d.tps << l) <= 512) d.tps *= 2;
+  d.staged = 1;
+  if (tile_smem<T>(d, l) > cap) d.staged = 0;
+  return l;
+}
+
+template <typename T>
+static int tile_threads(const Dft<T>& d, int l) {
+  const int t = ((d.tps << l) + 31) & ~31;
+  return t < 64 ? 64 : (t > 512 ? 512 : t);
+}
+
+template <typename T>
+static cudaError_t grow(const Dft<T>& d0, const T* in, T* out, cx<T>* spec, long long nrows, int ld, int flags,
+                        cudaStream_t s) {
+  GRowArgs<T> a;
+  memset(&a, 0, sizeof(a));
+  a.d = d0; a.in = in; a.out = out; a.spec = spec; a.nrows = nrows; a.ld = ld; a.flags = flags;
+  const long long pairs = (nrows + 1) / 2;
+  a.lS = tile_log<T>(a.d, pairs, 8);
+  const long long grid = (pairs + (1 << a.lS) - 1) >> a.lS;
+  grow_kernel<T><<<(unsigned)grid, tile_threads<T>(a.d, a.lS), tile_smem<T>(a.d, a.lS), s>>>(a);
   return cudaGetLastError();
 }
 
 template <typename T>
-static cudaError_t transpose(const cx<T>* in, cx<T>* out, int rows, int cols, int batch, cudaStream_t s) {
-  const int ty = (rows + 31) / 32;
-  dim3 grid((cols + 31) / 32, ty < 65535 ? ty : 65535, batch), block(32, 8);
-  transpose_kernel<T><<<grid, block, 0, s>>>(in, out, rows, cols);
+static cudaError_t gcol(GColArgs<T> a, int batch, cudaStream_t s) {
+  // 4 FP32 or 2 FP64 columns fill a 32-byte sector of each row; twice that where the grid is large
+  a.lC = tile_log<T>(a.d, (long long)a.ncols * batch, sizeof(T) == 4 ? 8 : 4);
+  dim3 grid((a.ncols + (1 << a.lC) - 1) >> a.lC, batch);
+  gcol_kernel<T><<<grid, tile_threads<T>(a.d, a.lC), tile_smem<T>(a.d, a.lC), s>>>(a);
   return cudaGetLastError();
+}
+
+static const double* plan_symbol(const void* plan, int n, int elem, int symbol) {
+  const DftGeom g = dft_geom(n, elem);
+  return (const double*)((const char*)plan + g.sym) + (symbol == MJX_SYMBOL_FD ? 0 : n);
+}
+
+static void symbol_axis(const void* plan, int n, int elem, int symbol, double d, const double** s, double* inv) {
+  *s = plan_symbol(plan, n, elem, symbol);
+  *inv = 1.0 / (d * d);
 }
 
 template <typename T>
 static mjx_status general_apply(const void* plan_y, const void* plan_x, const mjx_grid2d* g, int symbol, int nf,
                                 const double* D, const double* vx, const double* vy, double h, int mult,
-                                const T* table, const T* in, T* out, void* ws, cudaStream_t s) {
-  const int ny = g->ny, nx = g->nx;
-  const long long per = (long long)ny * nx, n = per * nf;
-  cx<T>* A = (cx<T>*)ws;
-  cx<T>* B = A + n;
-  const int threads = 256, blocks = 152 * 8;
-  real_to_complex_kernel<T><<<blocks, threads, 0, s>>>(in, A, n);
-  MJX_CUDA_TRY(cudaGetLastError());
-  MJX_CUDA_TRY(dft_rows<T>(dft_args<T>(plan_x, nx, A, (long long)nf * ny, nx, 0), s));
-  MJX_CUDA_TRY(transpose<T>(A, B, ny, nx, nf, s));
-  MJX_CUDA_TRY(dft_rows<T>(dft_args<T>(plan_y, ny, B, (long long)nf * nx, ny, 0), s));
-  GenMul m;
-  memset(&m, 0, sizeof(m));
-  m.nx = nx; m.ny = ny; m.symbol = symbol; m.mult = mult; m.nf = nf; m.dx = g->dx; m.dy = g->dy; m.h = h;
+                                const T* table, int n_steps, const T* in, T* out, void* ws, cudaStream_t s) {
+  const int ny = g->ny, nx = g->nx, ld = gen_ld(nx, sizeof(T)), hx = nx / 2 + 1;
+  const double twopi = 6.283185307179586476925286766559;
+  cx<T>* spec = (cx<T>*)ws;
+  T* tab = (T*)(spec + (size_t)nf * ny * ld);
+  const Dft<T> dx = dft_desc<T>(plan_x, nx);
+  GColArgs<T> c;
+  memset(&c, 0, sizeof(c));
+  c.d = dft_desc<T>(plan_y, ny);
+  c.spec = spec; c.bstride = (long long)ny * ld; c.ld = c.ldx = ld; c.ncols = c.hx = hx; c.dirs = 3;
+  GMul& m = c.m;
+  m.mult = mult; m.nx = nx; m.nb = 0; m.ny = ny; m.symbol = symbol; m.h = h;
+  symbol_axis(plan_x, nx, sizeof(T), symbol, g->dx, &m.sx, &m.ix);
+  symbol_axis(plan_y, ny, sizeof(T), symbol, g->dy, &m.sy, &m.iy);
+  m.kxs = twopi / (nx * g->dx);
+  m.kys = twopi / (ny * g->dy);
+  m.scale = 1.0 / ((double)nx * (double)ny);
   for (int f = 0; f < nf; ++f) {
     m.D[f] = D ? D[f] : 0.0;
     m.vx[f] = vx ? vx[f] : 0.0;
     m.vy[f] = vy ? vy[f] : 0.0;
   }
-  general_mult_kernel<T><<<blocks, threads, 0, s>>>(B, table, m);
-  MJX_CUDA_TRY(cudaGetLastError());
-  MJX_CUDA_TRY(dft_rows<T>(dft_args<T>(plan_y, ny, B, (long long)nf * nx, ny, 1), s));
-  MJX_CUDA_TRY(transpose<T>(B, A, nx, ny, nf, s));
-  MJX_CUDA_TRY(dft_rows<T>(dft_args<T>(plan_x, nx, A, (long long)nf * ny, nx, 1), s));
-  complex_real_kernel<T><<<blocks, threads, 0, s>>>(A, out, n);
-  MJX_CUDA_TRY(cudaGetLastError());
+  c.mode = mult == MJX_MULT_TABLE ? GCOL_USER : GCOL_VALUE;
+  c.tab = table;
+  const long long rows = (long long)nf * ny;
+  MJX_CUDA_TRY(grow<T>(dx, in, nullptr, spec, rows, ld, GROW_STORE_SPEC, s));
+  if (n_steps > 1 && mult < MJX_MULT_ADV_SOLVE) {
+    gtab_kernel<T><<<152 * 4, 256, 0, s>>>(tab, m, nf, ny, ld, ld, hx);
+    MJX_CUDA_TRY(cudaGetLastError());
+    c.mode = GCOL_TABLE;
+    c.tab = tab;
+  }
+  for (int i = 0; i < n_steps; ++i) {
+    MJX_CUDA_TRY(gcol<T>(c, nf, s));
+    const bool last = i == n_steps - 1;
+    MJX_CUDA_TRY(grow<T>(dx, nullptr, out, spec, rows, ld,
+                         GROW_LOAD_SPEC | (last ? GROW_STORE_REAL : GROW_STORE_SPEC), s));
+  }
   return MJX_OK;
 }
 
-struct GenMul3 {
-  int nx, ny, nz, symbol, mult;
-  double dx, dy, dz, h, D;
-};
-
-// multiplier on the spectrum laid out [kx][ky][kz]
-template <typename T>
-__global__ void general_mult3_kernel(cx<T>* __restrict__ s, const GenMul3 m) {
-  const long long total = (long long)m.nx * m.ny * m.nz;
-  const double twopi = 6.283185307179586476925286766559;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    const int kz = (int)(i % m.nz);
-    const long long r = i / m.nz;
-    const int ky = (int)(r % m.ny), kx = (int)(r / m.ny);
-    double lam;
-    if (m.symbol == MJX_SYMBOL_FD) {
-      lam = (2.0 * cospi(2.0 * kx / m.nx) - 2.0) / (m.dx * m.dx) + (2.0 * cospi(2.0 * ky / m.ny) - 2.0) / (m.dy * m.dy) +
-            (2.0 * cospi(2.0 * kz / m.nz) - 2.0) / (m.dz * m.dz);
-    } else {
-      const int mx = kx < (m.nx + 1) / 2 ? kx : kx - m.nx, my = ky < (m.ny + 1) / 2 ? ky : ky - m.ny;
-      const int mz = kz < (m.nz + 1) / 2 ? kz : kz - m.nz;
-      const double ax = twopi * mx / (m.nx * m.dx), ay = twopi * my / (m.ny * m.dy), az = twopi * mz / (m.nz * m.dz);
-      lam = -(ax * ax + ay * ay + az * az);
-    }
-    const double z = m.h * m.D * lam;
-    double f;
-    switch (m.mult) {
-      case MJX_MULT_SCALE: f = 1.0; break;
-      case MJX_MULT_HELMHOLTZ: {
-        double den = 1.0 - z;
-        if (fabs(den) < 1e-14) den = 1e-14;
-        f = 1.0 / den;
-        break;
-      }
-      case MJX_MULT_CN: f = (1.0 + 0.5 * z) / (1.0 - 0.5 * z); break;
-      case MJX_MULT_LAP: f = z; break;
-      default: f = exp(z);
-    }
-    const cx<T> v = s[i];
-    s[i] = mk<cx<T>>(v.x * (T)f, v.y * (T)f);
-  }
-}
-
-// one application on [nz][ny][nx]: x DFTs, per-plane transpose -> [z][x][y], y DFTs,
-// transpose (nz x nx ny) -> [x][y][z], z DFTs, multiplier, and back
+// n_steps applications on [nz][ny][nx]
 template <typename T>
 static mjx_status general_apply3(const void* pz, const void* py, const void* px, const mjx_grid3d* g, int symbol,
-                                 double D, double h, int mult, const T* in, T* out, void* ws, cudaStream_t s) {
-  const int nz = g->nz, ny = g->ny, nx = g->nx;
-  const long long n = (long long)nz * ny * nx;
-  cx<T>* A = (cx<T>*)ws;
-  cx<T>* B = A + n;
-  const int threads = 256, blocks = 152 * 8;
-  real_to_complex_kernel<T><<<blocks, threads, 0, s>>>(in, A, n);
-  MJX_CUDA_TRY(cudaGetLastError());
-  MJX_CUDA_TRY(dft_rows<T>(dft_args<T>(px, nx, A, (long long)nz * ny, nx, 0), s));
-  MJX_CUDA_TRY(transpose<T>(A, B, ny, nx, nz, s));                     // [z][x][y]
-  MJX_CUDA_TRY(dft_rows<T>(dft_args<T>(py, ny, B, (long long)nz * nx, ny, 0), s));
-  MJX_CUDA_TRY(transpose<T>(B, A, nz, nx * ny, 1, s));                 // [x][y][z]
-  MJX_CUDA_TRY(dft_rows<T>(dft_args<T>(pz, nz, A, (long long)nx * ny, nz, 0), s));
-  GenMul3 m;
-  m.nx = nx; m.ny = ny; m.nz = nz; m.symbol = symbol; m.mult = mult;
-  m.dx = g->dx; m.dy = g->dy; m.dz = g->dz; m.h = h; m.D = D;
-  general_mult3_kernel<T><<<blocks, threads, 0, s>>>(A, m);
-  MJX_CUDA_TRY(cudaGetLastError());
-  MJX_CUDA_TRY(dft_rows<T>(dft_args<T>(pz, nz, A, (long long)nx * ny, nz, 1), s));
-  MJX_CUDA_TRY(transpose<T>(A, B, nx * ny, nz, 1, s));                 // [z][x][y]
-  MJX_CUDA_TRY(dft_rows<T>(dft_args<T>(py, ny, B, (long long)nz * nx, ny, 1), s));
-  MJX_CUDA_TRY(transpose<T>(B, A, nx, ny, nz, s));                     // [z][y][x]
-  MJX_CUDA_TRY(dft_rows<T>(dft_args<T>(px, nx, A, (long long)nz * ny, nx, 1), s));
-  complex_real_kernel<T><<<blocks, threads, 0, s>>>(A, out, n);
-  MJX_CUDA_TRY(cudaGetLastError());
+                                 double D, double h, int mult, int n_steps, const T* in, T* out, void* ws,
+                                 cudaStream_t s) {
+  const int nz = g->nz, ny = g->ny, nx = g->nx, ld = gen_ld(nx, sizeof(T)), hx = nx / 2 + 1;
+  cx<T>* spec = (cx<T>*)ws;
+  T* tab = (T*)(spec + (size_t)nz * ny * ld);
+  const Dft<T> dx = dft_desc<T>(px, nx);
+  GColArgs<T> y;
+  memset(&y, 0, sizeof(y));
+  y.d = dft_desc<T>(py, ny);
+  y.spec = spec; y.bstride = (long long)ny * ld; y.ld = y.ldx = ld; y.ncols = y.hx = hx;
+  GColArgs<T> z = y, yb = y;
+  y.dirs = 1;
+  yb.dirs = 2;
+  z.d = dft_desc<T>(pz, nz);
+  z.bstride = 0; z.ld = z.ncols = ny * ld; z.dirs = 3; z.mode = GCOL_VALUE;
+  GMul& m = z.m;
+  m.mult = mult; m.nx = nx; m.nb = ny; m.ny = nz; m.symbol = symbol; m.h = h; m.D[0] = D;
+  symbol_axis(px, nx, sizeof(T), symbol, g->dx, &m.sx, &m.ix);
+  symbol_axis(py, ny, sizeof(T), symbol, g->dy, &m.sb, &m.ib);
+  symbol_axis(pz, nz, sizeof(T), symbol, g->dz, &m.sy, &m.iy);
+  m.scale = 1.0 / ((double)nx * (double)ny * (double)nz);
+  if (n_steps > 1) {
+    gtab_kernel<T><<<152 * 4, 256, 0, s>>>(tab, m, 1, nz, ny * ld, ld, hx);
+    MJX_CUDA_TRY(cudaGetLastError());
+    z.mode = GCOL_TABLE;
+    z.tab = tab;
+  }
+  const long long rows = (long long)nz * ny;
+  MJX_CUDA_TRY(grow<T>(dx, in, nullptr, spec, rows, ld, GROW_STORE_SPEC, s));
+  for (int i = 0; i < n_steps; ++i) {
+    MJX_CUDA_TRY(gcol<T>(y, nz, s));
+    MJX_CUDA_TRY(gcol<T>(z, 1, s));
+    MJX_CUDA_TRY(gcol<T>(yb, nz, s));
+    const bool last = i == n_steps - 1;
+    MJX_CUDA_TRY(grow<T>(dx, nullptr, out, spec, rows, ld,
+                         GROW_LOAD_SPEC | (last ? GROW_STORE_REAL : GROW_STORE_SPEC), s));
+  }
   return MJX_OK;
+}
+
+// workspace: the half spectra and the formed multipliers (at least the four reals per point of
+// a full complex spectrum and its transpose, which the query has always asked for)
+static size_t general_ws(size_t rows, int nx, int elem) {
+  const size_t need = rows * gen_ld(nx, elem) * 3 * elem, old = rows * nx * 4 * elem;
+  return need > old ? need : old;
 }
 
 static mjx_status set_dft_attrs() {
@@ -514,10 +599,10 @@ static mjx_status set_dft_attrs() {
     int dev = 0, optin = 0;
     MJX_CUDA_TRY(cudaGetDevice(&dev));
     MJX_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    MJX_CUDA_TRY(cudaFuncSetAttribute(dft_rows_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
-    MJX_CUDA_TRY(cudaFuncSetAttribute(dft_rows_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
-    MJX_CUDA_TRY(cudaFuncSetAttribute(dft_mixed_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
-    MJX_CUDA_TRY(cudaFuncSetAttribute(dft_mixed_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+    MJX_CUDA_TRY(cudaFuncSetAttribute(grow_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+    MJX_CUDA_TRY(cudaFuncSetAttribute(grow_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+    MJX_CUDA_TRY(cudaFuncSetAttribute(gcol_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+    MJX_CUDA_TRY(cudaFuncSetAttribute(gcol_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
     return MJX_OK;
   });
 }
@@ -545,7 +630,11 @@ mjx_status mjx_dftn_plan_init(void* plan, int n, int dtype, void* stream) {
     else { double* q = (double*)(host.data() + off); q[2 * i] = re; q[2 * i + 1] = im; }
   };
   const double twopi = 6.283185307179586476925286766559, pi = 0.5 * twopi;
-  for (int j = 0; j < g.L; ++j) put(g.tw, j, cos(twopi * j / g.L), -sin(twopi * j / g.L));  // L = n when mixed
+  for (int j = 0; j < g.L; ++j) {  // L = n unless Bluestein
+    double re, im;
+    tile_twiddle(j, g.L, e, &re, &im);
+    put(g.tw, j, re, im);
+  }
   if (g.bluestein) {
     std::vector<double> cre(n), cim(n);
     for (int j = 0; j < n; ++j) {  // exp(-i pi j^2 / n), j^2 reduced mod 2n to keep the angle exact
@@ -562,6 +651,12 @@ mjx_status mjx_dftn_plan_init(void* plan, int n, int dtype, void* stream) {
     host_fft2(bre, bim);
     for (int j = 0; j < g.L; ++j) put(g.bhat, j, bre[j] / g.L, bim[j] / g.L);
   }
+  double* sym = (double*)(host.data() + g.sym);
+  for (int j = 0; j < n; ++j) {
+    const int m = j < (n + 1) / 2 ? j : j - n;  // fftfreq index
+    sym[j] = 2.0 * cos(twopi * j / n) - 2.0;
+    sym[n + j] = -(twopi * m / n) * (twopi * m / n);
+  }
   cudaStream_t s = (cudaStream_t)stream;
   MJX_CUDA_TRY(cudaMemcpyAsync(plan, host.data(), g.total, cudaMemcpyHostToDevice, s));
   MJX_CUDA_TRY(cudaStreamSynchronize(s));
@@ -571,13 +666,13 @@ mjx_status mjx_dftn_plan_init(void* plan, int n, int dtype, void* stream) {
 size_t mjx_spectral_general2d_ws_bytes(int ny, int nx, int nfields, int dtype) {
   const int e = elem_size(dtype);
   if (!e || !dft_len_ok(ny) || !dft_len_ok(nx) || nfields < 1 || nfields > 4) return 0;
-  return (size_t)2 * nfields * ny * nx * 2 * e;
+  return general_ws((size_t)nfields * ny, nx, e);
 }
 
-mjx_status mjx_spectral_apply_general2d(const void* plan_y, const void* plan_x, const mjx_grid2d* g, int symbol,
-                                        int dtype, int nfields, const double* D, const double* vx,
-                                        const double* vy, double h, int mult, const void* table,
-                                        const void* in, void* out, void* ws, size_t ws_bytes, void* stream) {
+static mjx_status general2d(const void* plan_y, const void* plan_x, const mjx_grid2d* g, int symbol, int dtype,
+                            int nfields, const double* D, const double* vx, const double* vy, double h, int mult,
+                            const void* table, int n_steps, const void* in, void* out, void* ws, size_t ws_bytes,
+                            void* stream) {
   const int e = elem_size(dtype);
   if (!e) return MJX_BAD_DTYPE;
   if (!g || !plan_y || !plan_x || !in || !out || nfields < 1 || nfields > 4) return MJX_BAD_ARG;
@@ -594,15 +689,34 @@ mjx_status mjx_spectral_apply_general2d(const void* plan_y, const void* plan_x, 
   cudaStream_t s = (cudaStream_t)stream;
   if (e == 4)
     return general_apply<float>(plan_y, plan_x, g, symbol, nfields, D, vx, vy, h, mult, (const float*)table,
-                                (const float*)in, (float*)out, ws, s);
+                                n_steps, (const float*)in, (float*)out, ws, s);
   return general_apply<double>(plan_y, plan_x, g, symbol, nfields, D, vx, vy, h, mult, (const double*)table,
-                               (const double*)in, (double*)out, ws, s);
+                               n_steps, (const double*)in, (double*)out, ws, s);
+}
+
+mjx_status mjx_spectral_apply_general2d(const void* plan_y, const void* plan_x, const mjx_grid2d* g, int symbol,
+                                        int dtype, int nfields, const double* D, const double* vx,
+                                        const double* vy, double h, int mult, const void* table,
+                                        const void* in, void* out, void* ws, size_t ws_bytes, void* stream) {
+  return general2d(plan_y, plan_x, g, symbol, dtype, nfields, D, vx, vy, h, mult, table, 1, in, out, ws, ws_bytes,
+                   stream);
+}
+
+mjx_status mjx_spectral_steps_general2d(const void* plan_y, const void* plan_x, const mjx_grid2d* g, int symbol,
+                                        int dtype, int nfields, const double* D, double h, int mult, int n_steps,
+                                        const void* in, void* out, void* ws, size_t ws_bytes, void* stream) {
+  if (!D || n_steps < 1) return MJX_BAD_ARG;
+  if (mult != MJX_MULT_SCALE && mult != MJX_MULT_HELMHOLTZ && mult != MJX_MULT_CN && mult != MJX_MULT_EXP &&
+      mult != MJX_MULT_LAP)
+    return MJX_BAD_ARG;
+  return general2d(plan_y, plan_x, g, symbol, dtype, nfields, D, nullptr, nullptr, h, mult, nullptr, n_steps, in, out,
+                   ws, ws_bytes, stream);
 }
 
 size_t mjx_spectral_general3d_ws_bytes(int nz, int ny, int nx, int dtype) {
   const int e = elem_size(dtype);
   if (!e || !dft_len_ok(nz) || !dft_len_ok(ny) || !dft_len_ok(nx)) return 0;
-  return (size_t)2 * nz * ny * nx * 2 * e;
+  return general_ws((size_t)nz * ny, nx, e);
 }
 
 mjx_status mjx_spectral_apply_general3d(const void* plan_z, const void* plan_y, const void* plan_x,
@@ -621,23 +735,20 @@ mjx_status mjx_spectral_apply_general3d(const void* plan_z, const void* plan_y, 
   if (!ws || ws_bytes < mjx_spectral_general3d_ws_bytes(g->nz, g->ny, g->nx, dtype)) return MJX_WORKSPACE;
   MJX_TRY(set_dft_attrs());
   cudaStream_t s = (cudaStream_t)stream;
-  for (int i = 0; i < n_steps; ++i) {  // each application a full transform pair
-    const void* src = i == 0 ? in : out;
-    mjx_status st = e == 4 ? general_apply3<float>(plan_z, plan_y, plan_x, g, symbol, D, h, mult, (const float*)src,
-                                                   (float*)out, ws, s)
-                           : general_apply3<double>(plan_z, plan_y, plan_x, g, symbol, D, h, mult,
-                                                    (const double*)src, (double*)out, ws, s);
-    if (st != MJX_OK) return st;
-  }
-  return MJX_OK;
+  if (e == 4)
+    return general_apply3<float>(plan_z, plan_y, plan_x, g, symbol, D, h, mult, n_steps, (const float*)in,
+                                 (float*)out, ws, s);
+  return general_apply3<double>(plan_z, plan_y, plan_x, g, symbol, D, h, mult, n_steps, (const double*)in,
+                                (double*)out, ws, s);
 }
 
 }  // extern "C"
 
-// Autotuner of the mixed-radix row DFT of length n: every candidate schedule
-// (dft_schedules) with threads per sequence n/4, n/8 and n/16 is timed on nrows rows of
-// scratch (one warm-up launch, then reps launches between CUDA events); the fastest is
-// installed in the registry for n and this element size.
+// Autotuner of the mixed-radix DFT of length n: every candidate schedule (dft_schedules) with
+// threads per sequence n/4, n/8 and n/16 is timed in the spectrum-to-spectrum row pass (an
+// inverse and a forward DFT of every row pair) on nrows rows of scratch (one warm-up launch,
+// then reps launches between CUDA events); the fastest is installed in the registry for n and
+// this element size.
 template <typename T>
 static mjx_status tune_dft(const void* plan, int n, long long nrows, cx<T>* data, int reps, double* times,
                            int max_times, int* n_cand, int* best, cudaStream_t s) {
@@ -653,7 +764,11 @@ static mjx_status tune_dft(const void* plan, int n, long long nrows, cx<T>* data
     if (!dup) uniq[ntp++] = v;
   }
   tune_dft_clear(n, (int)sizeof(T));
-  DftArgs<T> a = dft_args<T>(plan, n, data, nrows, n, 0);
+  Dft<T> d = dft_desc<T>(plan, n);
+  const int ld = gen_ld(n, sizeof(T));
+  long long rows = nrows * n / ld;  // half-spectrum rows that fit the scratch
+  if (rows > nrows) rows = nrows;
+  if (rows < 1) return MJX_WORKSPACE;
   cudaEvent_t e0, e1;
   MJX_CUDA_TRY(cudaEventCreate(&e0));
   MJX_CUDA_TRY(cudaEventCreate(&e1));
@@ -662,12 +777,15 @@ static mjx_status tune_dft(const void* plan, int n, long long nrows, cx<T>* data
   mjx_status st = MJX_OK;
   for (int i = 0; i < ns && st == MJX_OK; ++i) {
     for (int j = 0; j < ntp && st == MJX_OK; ++j, ++k) {
-      a.nrad = sched[17 * i];
-      for (int q = 0; q < 16; ++q) a.rad[q] = sched[17 * i + 1 + q];
-      mixed_launch(a, uniq[j]);
-      cudaError_t ce = dft_rows<T>(a, s);
+      d.rad = pack_radices(sched[17 * i], sched + 17 * i + 1);
+      d.odd = sched[17 * i] & 1;
+      d.tps = uniq[j];
+      auto pass = [&]() {
+        return grow<T>(d, nullptr, nullptr, data, rows, ld, GROW_LOAD_SPEC | GROW_STORE_SPEC, s);
+      };
+      cudaError_t ce = pass();
       if (ce == cudaSuccess) ce = cudaEventRecord(e0, s);
-      for (int r = 0; r < reps && ce == cudaSuccess; ++r) ce = dft_rows<T>(a, s);
+      for (int r = 0; r < reps && ce == cudaSuccess; ++r) ce = pass();
       if (ce == cudaSuccess) ce = cudaEventRecord(e1, s);
       if (ce == cudaSuccess) ce = cudaEventSynchronize(e1);
       float ms = 0.f;

@@ -1,0 +1,225 @@
+// Tile DFT in shared memory: S = 2^lS interleaved sequences (element j of sequence s at
+// sp(j S + s)), mixed radices 2, 3, 4, 5, 8, Stockham autosort between two buffers.
+//
+// All butterflies of a pass (n / R of them for each sequence) are one flat list over which any
+// number of threads strides, neighbouring threads on neighbouring words: every warp but the
+// last of a pass is full, whatever n and R are.  That matters most in FP64, where a warp's
+// instruction takes 64 cycles of its sub-partition with any number of active lanes.  Two
+// buffers cost shared memory and save a barrier a pass.
+//
+// FP64 twiddles are stored as (cos, tan) of their angle: with w = e^{-i theta} = c (1 - i t),
+//   a +- w b = (a.x +- c u, a.y +- c v),  u = b.x + t b.y,  v = b.y - t b.x,
+// six fused multiply-adds instead of the ten operations of a complex product and two sums, and
+// two roundings a component instead of three (the scheme of Linzer and Feig, 1993).  Radix 4
+// takes 24 FP64 instructions instead of 34, radix 8 72 instead of 84.  At theta = pi/2 and
+// 3 pi/2 the pair is (2^-60, +-2^60).  FP32 keeps (cos, -sin): it is not bound by its
+// arithmetic, and the large tangents would shorten its range.
+#pragma once
+
+#include <math.h>
+
+#include "fft.cuh"
+
+namespace mjx {
+
+// host: entry j of n of a twiddle table in the form that tile_dft reads
+inline void tile_twiddle(int j, int n, int elem, double* re, double* im) {
+  if (elem == 4) {
+    const double ang = 6.283185307179586476925286766559 * (double)j / (double)n;
+    *re = cos(ang);
+    *im = -sin(ang);
+  } else if (4LL * j == n || 4LL * j == 3LL * n) {
+    *re = 0x1p-60;
+    *im = 4LL * j == n ? 0x1p60 : -0x1p60;
+  } else {  // the tangent belongs to the rounded cosine, so that their product is the sine
+    const long double a = 6.283185307179586476925286766559005768L * (long double)j / (long double)n;
+    *re = (double)cosl(a);
+    *im = (double)(sinl(a) / (long double)*re);
+  }
+}
+
+// w b
+__device__ __forceinline__ float2 tw_mul(float2 b, float2 w) { return cmul(b, w); }
+__device__ __forceinline__ double2 tw_mul(double2 b, double2 w) {
+  return mk<double2>(w.x * fma(w.y, b.y, b.x), w.x * fma(-w.y, b.x, b.y));
+}
+// (a, b) <- (a + w b, a - w b)
+__device__ __forceinline__ void tw_bf(float2& a, float2& b, float2 w) {
+  const float2 t = cmul(b, w);
+  b = csub(a, t);
+  a = cadd(a, t);
+}
+__device__ __forceinline__ void tw_bf(double2& a, double2& b, double2 w) {
+  const double u = fma(w.y, b.y, b.x), v = fma(-w.y, b.x, b.y);
+  b = mk<double2>(fma(-w.x, u, a.x), fma(-w.x, v, a.y));
+  a = mk<double2>(fma(w.x, u, a.x), fma(w.x, v, a.y));
+}
+// (a, b) <- (a - i w b, a + i w b)
+__device__ __forceinline__ void tw_bfr(float2& a, float2& b, float2 w) {
+  const float2 t = rot<false>(cmul(b, w));
+  b = csub(a, t);
+  a = cadd(a, t);
+}
+__device__ __forceinline__ void tw_bfr(double2& a, double2& b, double2 w) {
+  const double u = fma(w.y, b.y, b.x), v = fma(-w.y, b.x, b.y);
+  b = mk<double2>(fma(-w.x, v, a.x), fma(w.x, u, a.y));
+  a = mk<double2>(fma(w.x, v, a.x), fma(-w.x, u, a.y));
+}
+
+// v <- DFT_R(v_t w^t) in natural order, w^t the table entry at t * i; ne = n / 8 (radix 8)
+template <typename T, int R, bool FIRST>
+__device__ __forceinline__ void tile_bf(cx<T>* v, const cx<T>* tw, int i, int ne) {
+  typedef cx<T> C;
+  if constexpr (R == 2) {
+    if (FIRST) dft2<false>(v[0], v[1]);
+    else tw_bf(v[0], v[1], tw[i]);
+  } else if constexpr (R == 3) {
+    const T h = (T)0.86602540378443864676;  // sin(2 pi / 3)
+    C t, d = v[2];
+    if (FIRST) {
+      t = cadd(v[1], v[2]); d = csub(v[1], v[2]);
+    } else {
+      t = tw_mul(v[1], tw[i]);
+      tw_bf(t, d, tw[2 * i]);
+    }
+    const C a = v[0], m = mk<C>(a.x - (T)0.5 * t.x, a.y - (T)0.5 * t.y);
+    v[0] = cadd(a, t);
+    v[1] = mk<C>(m.x + h * d.y, m.y - h * d.x);
+    v[2] = mk<C>(m.x - h * d.y, m.y + h * d.x);
+  } else if constexpr (R == 4) {
+    if (FIRST) {
+      dft4<false>(v[0], v[1], v[2], v[3]);
+    } else {
+      const C w1 = tw[i], w2 = tw[2 * i];
+      tw_bf(v[0], v[2], w2);
+      tw_bf(v[1], v[3], w2);
+      tw_bf(v[0], v[1], w1);
+      tw_bfr(v[2], v[3], w1);
+      const C t = v[1];  // X0, X2, X1, X3 -> natural order
+      v[1] = v[2]; v[2] = t;
+    }
+  } else if constexpr (R == 5) {
+    // cos / sin of 2 pi/5 and 4 pi/5
+    const T c1 = (T)0.30901699437494742410, c2 = (T)-0.80901699437494742410;
+    const T s1 = (T)0.95105651629515357212, s2 = (T)0.58778525229247312917;
+    C t1, t2, t3 = v[4], t4 = v[3];
+    if (FIRST) {
+      t1 = cadd(v[1], v[4]); t3 = csub(v[1], v[4]);
+      t2 = cadd(v[2], v[3]); t4 = csub(v[2], v[3]);
+    } else {
+      t1 = tw_mul(v[1], tw[i]);
+      tw_bf(t1, t3, tw[4 * i]);
+      t2 = tw_mul(v[2], tw[2 * i]);
+      tw_bf(t2, t4, tw[3 * i]);
+    }
+    const C a = v[0];
+    const C m1 = mk<C>(a.x + c1 * t1.x + c2 * t2.x, a.y + c1 * t1.y + c2 * t2.y);
+    const C m2 = mk<C>(a.x + c2 * t1.x + c1 * t2.x, a.y + c2 * t1.y + c1 * t2.y);
+    const C n1 = mk<C>(s1 * t3.x + s2 * t4.x, s1 * t3.y + s2 * t4.y);
+    const C n2 = mk<C>(s2 * t3.x - s1 * t4.x, s2 * t3.y - s1 * t4.y);
+    v[0] = mk<C>(a.x + t1.x + t2.x, a.y + t1.y + t2.y);
+    v[1] = mk<C>(m1.x + n1.y, m1.y - n1.x);  // m1 - i n1
+    v[4] = mk<C>(m1.x - n1.y, m1.y + n1.x);  // m1 + i n1
+    v[2] = mk<C>(m2.x + n2.y, m2.y - n2.x);
+    v[3] = mk<C>(m2.x - n2.y, m2.y + n2.x);
+  } else {
+    if (FIRST) {
+      dft8<false>(v);
+    } else {
+      // even and odd samples as radix 4 with w^2, then the odd half with w and w e^{-i pi/4}
+      const C w1 = tw[i], w2 = tw[2 * i], w4 = tw[4 * i], we = tw[i + ne];
+      tw_bf(v[0], v[4], w4);
+      tw_bf(v[2], v[6], w4);
+      tw_bf(v[1], v[5], w4);
+      tw_bf(v[3], v[7], w4);
+      tw_bf(v[0], v[2], w2);   // E0, E2
+      tw_bfr(v[4], v[6], w2);  // E1, E3
+      tw_bf(v[1], v[3], w2);   // O0, O2
+      tw_bfr(v[5], v[7], w2);  // O1, O3
+      tw_bf(v[0], v[1], w1);   // X0, X4
+      tw_bf(v[4], v[5], we);   // X1, X5
+      tw_bfr(v[2], v[3], w1);  // X2, X6
+      tw_bfr(v[6], v[7], we);  // X3, X7
+      const C x1 = v[4], x2 = v[2], x3 = v[6], x4 = v[1], x6 = v[3];
+      v[1] = x1; v[2] = x2; v[3] = x3; v[4] = x4; v[6] = x6;
+    }
+  }
+}
+
+// a / b for 0 <= a < 2^20, b >= 1, given 1.0f / b: exact, since the half keeps the quotient
+// away from integers by 1/(2b), more than the roundings can move it
+__device__ __forceinline__ int fdiv(int a, float rb) { return (int)(((float)a + 0.5f) * rb); }
+
+// One pass: butterfly j (k = j mod p) of each sequence from src[j + t n/R] to
+// dst[(j - k) R + k + t p], after the twiddles w^(k t), w = exp(-2 pi i / (p R)).
+template <typename T, int R>
+__device__ __forceinline__ void tile_pass(const cx<T>* src, cx<T>* dst, int n, int p, int lS, const cx<T>* tw,
+                                          int tid, int nth) {
+  typedef cx<T> C;
+  const int nb = n / R, items = nb << lS, S1 = (1 << lS) - 1;
+  if (p == 1) {
+    for (int i = tid; i < items; i += nth) {
+      const int s = i & S1, j = i >> lS;
+      C v[R];
+#pragma unroll
+      for (int t = 0; t < R; ++t) v[t] = src[sp(i + ((t * nb) << lS))];
+      tile_bf<T, R, true>(v, tw, 0, 0);
+#pragma unroll
+      for (int t = 0; t < R; ++t) dst[sp(((j * R + t) << lS) + s)] = v[t];
+    }
+  } else {
+    const int step = nb / p;
+    const bool p2 = (p & (p - 1)) == 0;
+    const int lp = __ffs(p) - 1;
+    const float rp = 1.0f / (float)p;
+    for (int i = tid; i < items; i += nth) {
+      const int s = i & S1, j = i >> lS;
+      const int q = p2 ? j >> lp : fdiv(j, rp), k = j - q * p;
+      C v[R];
+#pragma unroll
+      for (int t = 0; t < R; ++t) v[t] = src[sp(i + ((t * nb) << lS))];
+      tile_bf<T, R, false>(v, tw, k * step, n >> 3);
+      const int base = q * p * R + k;
+#pragma unroll
+      for (int t = 0; t < R; ++t) dst[sp(((base + t * p) << lS) + s)] = v[t];
+    }
+  }
+  __syncthreads();
+}
+
+// Forward DFT of length n of every sequence in cur; the result is in cur after an even number
+// of passes, in alt after an odd one.  The caller has synchronised; on return the tile is
+// complete.  Radices are packed four bits each, the first pass lowest.  One copy of the code
+// per kernel: a kernel runs two to six transforms, and inlined copies cost more in instruction
+// fetches than the passes themselves on small tiles.
+template <typename T>
+__device__ __noinline__ void tile_dft(cx<T>* cur, cx<T>* alt, int n, unsigned long long rad, int lS, const cx<T>* tw,
+                                      int tid, int nth) {
+  for (int p = 1; rad != 0; rad >>= 4) {
+    const int r = (int)(rad & 15);
+    if (r == 8) tile_pass<T, 8>(cur, alt, n, p, lS, tw, tid, nth);
+    else if (r == 4) tile_pass<T, 4>(cur, alt, n, p, lS, tw, tid, nth);
+    else if (r == 5) tile_pass<T, 5>(cur, alt, n, p, lS, tw, tid, nth);
+    else if (r == 3) tile_pass<T, 3>(cur, alt, n, p, lS, tw, tid, nth);
+    else tile_pass<T, 2>(cur, alt, n, p, lS, tw, tid, nth);
+    cx<T>* t = cur;
+    cur = alt;
+    alt = t;
+    p *= r;
+  }
+}
+
+// packed radices of a power of two 2^l: eights, the rest as fours (or one two); *passes their count
+inline unsigned long long tile_pow2_radices(int l, int* passes) {
+  unsigned long long rad = 0;
+  int k = 0, eights = l / 3, rest = l % 3;
+  auto put = [&](int r) { rad |= (unsigned long long)r << (4 * k++); };
+  if (rest == 1 && eights > 0) { --eights; rest = 4; }  // 2^(3a+1) = 8^(a-1) 4 4
+  for (int i = 0; i < eights; ++i) put(8);
+  for (; rest >= 2; rest -= 2) put(4);
+  if (rest == 1) put(2);
+  *passes = k;
+  return rad;
+}
+
+}  // namespace mjx

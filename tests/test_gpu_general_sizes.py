@@ -164,3 +164,29 @@ def test_etd_general_sizes_vs_oracle(cuda, method):
         ru, rv = OE.etdrk4_gray_scott(ui, vi, lam, 2e-5, 1e-5, 0.035, 0.065, 1.0, 4, 1.0)
         assert float(np.max(np.abs(mol.interior(out["u"].cpu().numpy(), og) - ru))) < 1e-12
         assert float(np.max(np.abs(mol.interior(out["v"].cpu().numpy(), og) - rv))) < 1e-12
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float64, 1e-12), (torch.float32, 2e-5)])
+@pytest.mark.parametrize("shape", [(1, 7), (7, 1), (3, 4096), (4096, 3), (2047, 3), (6, 1999), (1024, 30), (45, 250),
+                                   (8, 5, 3), (1, 9, 2048), (31, 16, 12)])
+def test_general_steps_vs_numpy(cuda, shape, dtype, tol):
+    """Several steps in one call (rows go from spectrum to spectrum, the multiplier comes from a
+    table) at the edges of the tile transform: single points, odd and prime lengths, the longest
+    lengths of each kind (whose tables stay in global memory), odd row counts, 2D and 3D."""
+    import moljax_gb300 as M
+    rng = np.random.default_rng(sum(shape))
+    u = rng.standard_normal(shape)
+    d = [0.7 / n for n in shape]
+    lam = sum(np.expand_dims(spectral_symbol_1d(n, h), [j for j in range(len(shape)) if j != i])
+              for i, (n, h) in enumerate(zip(shape, d)))
+    x = 0.5 * 1e-4 * 0.1 * lam
+    ref = u
+    for _ in range(3):
+        ref = np.real(np.fft.ifftn(np.fft.fftn(ref) * (1 + x) / (1 - x)))
+    ut = torch.tensor(u, dtype=dtype, device=cuda)
+    if len(shape) == 2:
+        got = M.fft_cn_step(ut, 0.1, d[1], 1e-4, 3, dy=d[0])
+    else:
+        got = M.fft_cn_step_3d(ut, 0.1, d[2], 1e-4, 3, dy=d[1], dz=d[0])
+    err = np.linalg.norm(got.double().cpu().numpy() - ref) / np.linalg.norm(ref)
+    assert err < tol, err
