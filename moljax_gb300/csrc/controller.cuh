@@ -1,45 +1,50 @@
 // The accept/reject and PI step-size update of one adaptive attempt, shared by
 // the single-solve controller kernel (csrc/imex.cu) and the batched controller
-// (csrc/imex_batch.cu).  One thread applies it to one DevState.
+// (csrc/imex_batch.cu).
 #pragma once
 
 #include "spectral.cuh"
 
 namespace mjx {
 
-// NaN-propagating min/max (jnp.minimum/maximum semantics).
-__device__ __forceinline__ double jmax(double a, double b) { return (a != a || b != b) ? (a + b) : (a > b ? a : b); }
-__device__ __forceinline__ double jmin(double a, double b) { return (a != a || b != b) ? (a + b) : (a < b ? a : b); }
+// What bounds the update: one dependent chain of FP64 instructions of a single warp, ~64 cycles
+// each whatever its active lanes.  With two pow calls, six divisions and three-comparison
+// min/max the controller took 15 us of a 139 us attempt at 1024^2.  The step factor
+//   (1/e)^kI (e_prev/e)^kP = exp(kP log e_prev - (kI + kP) log e)
+// now takes one log and one exp, both on the size of a rounding error in dt, log e_prev is kept
+// from the attempt that set it, the quotients that do not change are formed on the host, and
+// the square root runs beside the logarithm: 15.1 -> 7.1 us.
+
+// NaN test on the bits: an FP64 comparison would take an FP64 issue slot
+__device__ __forceinline__ bool jnan(double a) {
+  const unsigned hi = (unsigned)__double2hiint(a) & 0x7fffffffu;
+  return hi > 0x7ff00000u || (hi == 0x7ff00000u && __double2loint(a) != 0);
+}
+// NaN-propagating min/max (jnp.minimum/maximum semantics)
+__device__ __forceinline__ double jmax(double a, double b) { return (jnan(a) || a > b) ? a : b; }
+__device__ __forceinline__ double jmin(double a, double b) { return (jnan(a) || a < b) ? a : b; }
 __device__ __forceinline__ double jclip(double x, double lo, double hi) { return jmin(jmax(x, lo), hi); }
 
-// tot: sum over every degree of freedom of (err / (atol + rtol |y_new|))^2; bad: any
-// non-finite value.  Applies moljax/core/stepping.py:1246-1359 (scaled_error_norm,
-// propose_dt_imex, the accept and reject branches, the loop stop and final status) to
-// st and returns whether the run continues.  hist_t / hist_dt may be null.
-__device__ __forceinline__ bool ctl_update(DevState* st, double tot, int bad, double n_dof,
-                                           const mjx_pid_params& P, double* hist_t, double* hist_dt) {
-  const double order = (double)st->order;
+// log max(e, 1e-10) of the error norm e = sqrt(q), and the step factor before the safety
+// factor: propose_dt_imex (dt_policy.py:544-610) over pid_controller_dt (178-227) for e <= 1
+// and handle_rejected_step (230-268) above
+__device__ __forceinline__ double ctl_log(double q) { return jmax(0.5 * log(q), -23.025850929940456840); }
+__device__ __forceinline__ double ctl_factor(const CtlGain& G, bool small, double le, double lprev) {
+  return exp(small ? G.kP * lprev - (G.kI + G.kP) * le : -G.kI * jmax(le, 0.0));
+}
+
+// e = max(sqrt(tot / n_dof), 1e-10) with tot the sum over every degree of freedom of
+// (err / (atol + rtol |y_new|))^2, le = ctl_log, fac = ctl_factor; bad: any non-finite value.
+// Applies moljax/core/stepping.py:1246-1359 (the accept and reject branches, the loop stop and
+// final status) to st and returns whether the run continues.  hist_t / hist_dt may be null.
+__device__ __forceinline__ bool ctl_apply(DevState* st, double e, double le, double fac, int bad,
+                                          const mjx_pid_params& P, double* hist_t, double* hist_dt) {
   const double dtc = st->dtc;
-  // stepping.py:1246-1247
-  const double e = jmax(sqrt(tot / n_dof), 1e-10);
   const int finite = !bad;
-  const bool accept = (e <= 1.0) && finite;
-  // dt_policy.py:544-610 (propose_dt_imex)
-  double dt_a, pe_new;
-  if (e <= 1.0) {  // pid_controller_dt (178-227)
-    const double kI = P.kI / order, kP = P.kP / order;
-    const double es = jmax(e, 1e-10), pes = jmax(st->prev_err, 1e-10);
-    double fac = pow(1.0 / es, kI) * pow(pes / es, kP);
-    fac = jclip(fac * P.safety, P.min_factor, P.max_factor);
-    dt_a = jclip(dtc * fac, P.dt_min, P.dt_max);
-    pe_new = e;
-  } else {  // handle_rejected_step (230-268)
-    const double kI = P.kI / order;
-    double fac = P.safety * pow(1.0 / jmax(e, 1.0), kI);
-    fac = jclip(fac, P.min_factor, 1.0);
-    dt_a = jclip(dtc * fac, P.dt_min, P.dt_max);
-    pe_new = st->prev_err;
-  }
+  const bool small = e <= 1.0;
+  const bool accept = small && finite;
+  fac = jclip(P.safety * fac, P.min_factor, small ? P.max_factor : 1.0);
+  const double dt_a = jclip(dtc * fac, P.dt_min, P.dt_max);
   const double dt_new = jclip(jmin(dt_a, st->dt_cfl), P.dt_min, P.dt_max);
   st->err_last = e;
   st->save_slot = -1;
@@ -53,7 +58,8 @@ __device__ __forceinline__ bool ctl_update(DevState* st, double tot, int bad, do
     st->t = st->t + dtc;
     st->cur = 1 - st->cur;
     st->dt = dt_new;
-    st->prev_err = pe_new;
+    st->prev_err = e;
+    st->lprev = le;
     st->dt_last_accepted = dtc;
     st->n_acc += 1;
   } else {  // stepping.py:1311-1334
@@ -75,6 +81,13 @@ __device__ __forceinline__ bool ctl_update(DevState* st, double tot, int bad, do
     else if (st->status == MJX_STATUS_RUNNING_CODE) st->status = MJX_STATUS_MAX_STEPS_CODE;
   }
   return running;
+}
+
+// the whole update by one thread
+__device__ __forceinline__ bool ctl_update(DevState* st, double tot, int bad, const CtlGain& G,
+                                           const mjx_pid_params& P, double* hist_t, double* hist_dt) {
+  const double q = tot * G.inv_n, e = jmax(sqrt(q), 1e-10), le = ctl_log(q);
+  return ctl_apply(st, e, le, ctl_factor(G, e <= 1.0, le, st->lprev), bad, P, hist_t, hist_dt);
 }
 
 }  // namespace mjx

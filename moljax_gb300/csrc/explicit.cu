@@ -1412,7 +1412,7 @@ static mjx_status x_adaptive(const XModel& m, const mjx_explicit_problem* pb, co
   DevState h;
   memset(&h, 0, sizeof(h));
   const double dt_init = (dt0 < pb->dt_cfl || dt0 != dt0) ? dt0 : pb->dt_cfl;  // explicit: min(dt0, dt_cfl)
-  h.t = t0; h.dt = dt_init; h.t_end = t_end; h.prev_err = 1.0; h.dt_cfl = pb->dt_cfl;
+  h.t = t0; h.dt = dt_init; h.t_end = t_end; h.prev_err = 1.0; h.lprev = 0.0; h.dt_cfl = pb->dt_cfl;
   h.cur = 0; h.status = MJX_STATUS_RUNNING_CODE; h.write_idx = 1; h.finite = 1;
   h.max_saves = max_saves; h.save_every = save_every; h.order = order_of[pb->method];
   h.save_slot = -1;
@@ -1436,7 +1436,7 @@ static mjx_status x_adaptive(const XModel& m, const mjx_explicit_problem* pb, co
   CtlArgs ca;
   memset(&ca, 0, sizeof(ca));
   ca.st = st; ca.partial = (const double*)(ws + L.part); ca.nonfinite = (const int*)(ws + L.bad);
-  ca.nparts = XNPARTS; ca.n_dof = (double)nelem; ca.pid = *pid; ca.hist_t = hist_t; ca.hist_dt = hist_dt;
+  ca.nparts = XNPARTS; ca.gain = ctl_gain(*pid, h.order, (double)nelem); ca.pid = *pid; ca.hist_t = hist_t; ca.hist_dt = hist_dt;
   auto body = [&](cudaStream_t ls) -> cudaError_t {
     cudaError_t le = launch_x_attempt<T>(A, ls);
     if (le == cudaSuccess) le = launch_controller(ca, ls);

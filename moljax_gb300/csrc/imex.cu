@@ -70,17 +70,28 @@ static ImexLayout imex_layout(int ny, int nx, int nf, int elem, int nrows, int n
 // ------------------------------------------------------------------ controller
 
 
-__global__ void __launch_bounds__(256) controller_kernel(CtlArgs a) {
-  DevState* st = a.st;
-  if (st->done) {
+// Four warps, one on each FP64 sub-partition: they sum the partials, then one takes the
+// logarithm and the exponential of the step factor and another the square root.
+enum { CTL_THREADS = 128 };
+
+__global__ void __launch_bounds__(CTL_THREADS) controller_kernel(CtlArgs a) {
+  __shared__ double red[CTL_THREADS / 32];
+  __shared__ int redbad[CTL_THREADS / 32];
+  __shared__ double s_e;
+  const int w = threadIdx.x >> 5;
+  // the state and the first partials in one round trip to L2
+  DevState S = *a.st;
+  double s = 0.0, c = 0.0;
+  int bad = 0, i = threadIdx.x;
+  if (i < a.nparts) {  // Kahan per thread (the first value needs no compensation)
+    s = a.partial[i];
+    bad = a.nonfinite[i];
+  }
+  if (S.done) {
     if (threadIdx.x == 0 && a.use_handle) cudaGraphSetConditional(a.handle, 0u);
     return;
   }
-  __shared__ double red[8];
-  __shared__ int redbad[8];
-  double s = 0.0, c = 0.0;
-  int bad = 0;
-  for (int i = threadIdx.x; i < a.nparts; i += blockDim.x) {  // Kahan per thread
+  for (i += CTL_THREADS; i < a.nparts; i += CTL_THREADS) {
     const double yv = a.partial[i] - c;
     const double tv = s + yv;
     c = (tv - s) - yv;
@@ -92,13 +103,20 @@ __global__ void __launch_bounds__(256) controller_kernel(CtlArgs a) {
     s += __shfl_xor_sync(0xffffffffu, s, o);
     bad |= __shfl_xor_sync(0xffffffffu, bad, o);
   }
-  if ((threadIdx.x & 31) == 0) { red[threadIdx.x >> 5] = s; redbad[threadIdx.x >> 5] = bad; }
+  if ((threadIdx.x & 31) == 0) { red[w] = s; redbad[w] = bad; }
   __syncthreads();
+  if (w > 1) return;
+  const double q = ((red[0] + red[1]) + (red[2] + red[3])) * a.gain.inv_n;
+  double le = 0.0;
+  if (w == 1) s_e = jmax(sqrt(q), 1e-10);
+  else le = ctl_log(q);
+  asm volatile("bar.sync 1, 64;" ::: "memory");
   if (threadIdx.x != 0) return;
-  double tot = 0.0;
-  for (int i = 0; i < (int)(blockDim.x >> 5); ++i) { tot += red[i]; bad |= redbad[i]; }
-
-  const bool running = ctl_update(st, tot, bad, a.n_dof, a.pid, a.hist_t, a.hist_dt);
+  bad = redbad[0] | redbad[1] | redbad[2] | redbad[3];
+  const double e = s_e;
+  const double fac = ctl_factor(a.gain, e <= 1.0, le, S.lprev);
+  const bool running = ctl_apply(&S, e, le, fac, bad, a.pid, a.hist_t, a.hist_dt);
+  *a.st = S;
   if (a.use_handle) cudaGraphSetConditional(a.handle, running ? 1u : 0u);
 }
 
@@ -114,7 +132,7 @@ bool host_loop_mode() {
 }
 
 cudaError_t launch_controller(const CtlArgs& a, cudaStream_t s) {
-  controller_kernel<<<1, 256, 0, s>>>(a);
+  controller_kernel<<<1, CTL_THREADS, 0, s>>>(a);
   return cudaGetLastError();
 }
 
@@ -358,7 +376,7 @@ static mjx_status adaptive_run(const void* plan, const mjx_grid2d* g, const mjx_
   DevState h;
   memset(&h, 0, sizeof(h));
   const double dt_init = (dt0 < pb->dt_cfl || dt0 != dt0) ? dt0 : pb->dt_cfl;  // jnp.minimum
-  h.t = t0; h.dt = dt_init; h.t_end = t_end; h.prev_err = 1.0; h.dt_cfl = pb->dt_cfl;
+  h.t = t0; h.dt = dt_init; h.t_end = t_end; h.prev_err = 1.0; h.lprev = 0.0; h.dt_cfl = pb->dt_cfl;
   h.cur = 0; h.status = MJX_STATUS_RUNNING_CODE; h.write_idx = 1; h.finite = 1;
   h.max_saves = max_saves; h.save_every = save_every; h.order = pb->use_strang ? 2 : 1;  // stepping.py:1193
   h.save_slot = -1;
@@ -385,7 +403,7 @@ static mjx_status adaptive_run(const void* plan, const mjx_grid2d* g, const mjx_
   CtlArgs ca;
   memset(&ca, 0, sizeof(ca));
   ca.st = st; ca.partial = (const double*)(ws + L.part); ca.nonfinite = (const int*)(ws + L.bad);
-  ca.nparts = L.nparts; ca.n_dof = (double)nelem; ca.pid = *pid; ca.hist_t = hist_t; ca.hist_dt = hist_dt;
+  ca.nparts = L.nparts; ca.gain = ctl_gain(*pid, h.order, (double)nelem); ca.pid = *pid; ca.hist_t = hist_t; ca.hist_dt = hist_dt;
 
   if (running && host_loop_mode()) {
     const cudaError_t e = run_host_loop([&](cudaStream_t ls) -> cudaError_t {
@@ -425,7 +443,7 @@ static mjx_status adaptive_run(const void* plan, const mjx_grid2d* g, const mjx_
       for (int u = 0; u < kCondUnroll && le == cudaSuccess; ++u) {
         le = launch_attempt<T>(A, cs);
         if (le == cudaSuccess) {
-          controller_kernel<<<1, 256, 0, cs>>>(ca);
+          controller_kernel<<<1, CTL_THREADS, 0, cs>>>(ca);
           le = cudaGetLastError();
         }
         if (le == cudaSuccess && hist_y) {
@@ -533,7 +551,7 @@ static mjx_status attempt_kernel(const void* plan, const mjx_grid2d* g, const mj
   if (which == 0) {
     DevState h;
     memset(&h, 0, sizeof(h));
-    h.t = 0.0; h.dt = dt; h.dtc = dt; h.t_end = 1e300; h.prev_err = 1.0; h.dt_cfl = pb->dt_cfl;
+    h.t = 0.0; h.dt = dt; h.dtc = dt; h.t_end = 1e300; h.prev_err = 1.0; h.lprev = 0.0; h.dt_cfl = pb->dt_cfl;
     h.status = MJX_STATUS_RUNNING_CODE; h.write_idx = 1; h.finite = 1; h.max_saves = 1 << 30;
     h.save_every = 1 << 30; h.max_attempts = 1 << 30; h.order = pb->use_strang ? 2 : 1; h.save_slot = -1;
     const long long nelem = (long long)pb->nfields * g->ny * g->nx;

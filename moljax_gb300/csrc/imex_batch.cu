@@ -64,7 +64,7 @@ struct BInst {
   double* hist_dt;
   double D[2];
   double F, k;
-  double n_dof;
+  CtlGain gain;
   float inv_norm;
   int pad;
   mjx_pid_params pid;
@@ -273,47 +273,63 @@ __global__ void __launch_bounds__(BT, 4) brow_kernel(const __grid_constant__ BAr
 }
 
 // ------------------------------------------------------------------ controller
-// One CTA: warp i handles instances i, i + 32, ...; thread 0 then decides whether the
-// epoch goes on and sets the conditional node.
+// One CTA: the warps sum the instances' partials (warp i those of instances i, i + 32, ...),
+// then lane t updates instance t, 32 instances to a warp: an FP64 instruction costs a warp the
+// same ~64 cycles for one lane as for 32, so one warp per instance would multiply the update's
+// time by the warps that share a sub-partition (18.9 us for eight instances, 8.4 us now).
+// Thread 0 then decides whether the epoch goes on and sets the conditional node.
 __global__ void __launch_bounds__(1024) bctl_kernel(const __grid_constant__ BArgs a,
                                                    cudaGraphConditionalHandle handle) {
   BEng* eng = a.eng;
   __shared__ int s_run, s_fin;
+  __shared__ double s_tot[1024];
+  __shared__ int s_bad[1024];
   if (eng->halt) {
     if (threadIdx.x == 0) cudaGraphSetConditional(handle, 0u);
     return;
   }
   if (threadIdx.x == 0) { s_run = 0; s_fin = 0; }
-  __syncthreads();
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  int run_local = 0, fin_local = 0;
-  for (int i = wid; i < eng->n_slots; i += nwarps) {
-    BInst* I = a.tab + i;
-    if (I->st.done) continue;
-    double s = 0.0, c = 0.0;
-    int bad = 0;
-    for (int p = lane; p < I->nparts; p += 32) {  // Kahan per lane
-      const double yv = I->partial[p] - c;
-      const double tv = s + yv;
-      c = (tv - s) - yv;
-      s = tv;
-      bad |= I->nonfinite[p];
-    }
+  const int nt = blockDim.x, n_slots = eng->n_slots;
+  for (int base = 0; base < n_slots; base += nt) {
+    const int top = n_slots - base < nt ? n_slots - base : nt;
+    for (int i = wid; i < top; i += nwarps) {
+      const BInst* I = a.tab + base + i;
+      if (I->st.done) continue;
+      double s = 0.0, c = 0.0;
+      int bad = 0, p = lane;
+      if (p < I->nparts) {  // Kahan per lane (the first value needs no compensation)
+        s = I->partial[p];
+        bad = I->nonfinite[p];
+      }
+      for (p += 32; p < I->nparts; p += 32) {
+        const double yv = I->partial[p] - c;
+        const double tv = s + yv;
+        c = (tv - s) - yv;
+        s = tv;
+        bad |= I->nonfinite[p];
+      }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      s += __shfl_xor_sync(0xffffffffu, s, o);
-      bad |= __shfl_xor_sync(0xffffffffu, bad, o);
+      for (int o = 16; o > 0; o >>= 1) {
+        s += __shfl_xor_sync(0xffffffffu, s, o);
+        bad |= __shfl_xor_sync(0xffffffffu, bad, o);
+      }
+      if (lane == 0) { s_tot[i] = s; s_bad[i] = bad; }
     }
-    if (lane == 0) {
-      const bool running = ctl_update(&I->st, s, bad, I->n_dof, I->pid, I->hist_t, I->hist_dt);
-      if (running) ++run_local; else ++fin_local;
+    __syncthreads();
+    if ((int)threadIdx.x < top) {
+      BInst* I = a.tab + base + threadIdx.x;
+      DevState S = I->st;  // one round trip to L2
+      if (!S.done) {
+        const CtlGain G = I->gain;
+        const mjx_pid_params P = I->pid;
+        const bool running = ctl_update(&S, s_tot[threadIdx.x], s_bad[threadIdx.x], G, P, I->hist_t, I->hist_dt);
+        I->st = S;
+        atomicAdd(running ? &s_run : &s_fin, 1);
+      }
     }
+    __syncthreads();
   }
-  if (lane == 0) {
-    if (run_local) atomicAdd(&s_run, run_local);
-    if (fin_local) atomicAdd(&s_fin, fin_local);
-  }
-  __syncthreads();
   if (threadIdx.x != 0) return;
   eng->attempts += 1;
   eng->finished += s_fin;
@@ -615,12 +631,12 @@ mjx_status mjx_gsbatch_admit(void* batch, const mjx_gs_instance* d, int io_dtype
   I.D[0] = d->Du > 1e-14 ? d->Du : 0.0;
   I.D[1] = d->Dv > 1e-14 ? d->Dv : 0.0;
   I.F = d->F; I.k = d->k;
-  I.n_dof = 2.0 * g.ny * g.nx;
   I.inv_norm = (float)(1.0 / ((double)g.nx * (double)g.ny));
   I.pid = d->pid;
+  I.gain = ctl_gain(d->pid, 2, 2.0 * g.ny * g.nx);
   DevState& h = I.st;
   const double dt_init = (d->dt0 < d->dt_cfl || d->dt0 != d->dt0) ? d->dt0 : d->dt_cfl;
-  h.t = d->t0; h.dt = dt_init; h.t_end = d->t_end; h.prev_err = 1.0; h.dt_cfl = d->dt_cfl;
+  h.t = d->t0; h.dt = dt_init; h.t_end = d->t_end; h.prev_err = 1.0; h.lprev = 0.0; h.dt_cfl = d->dt_cfl;
   h.status = MJX_STATUS_RUNNING_CODE; h.write_idx = 1; h.finite = 1;
   h.max_saves = max_saves; h.save_every = d->save_every; h.order = 2; h.save_slot = -1;
   h.max_attempts = d->max_attempts > 0 ? d->max_attempts : 20 * d->max_steps + 1000;

@@ -391,7 +391,7 @@ mjx_status mjx_imex_mixed_attempt_kernel2d(const void* plan32, const void* plan6
     MJX_CUDA_TRY(cudaMemcpyAsync(w + L.ys1, w + L.ys0, (size_t)nf * L.fs * 16, cudaMemcpyDeviceToDevice, s));
     DevState h;
     memset(&h, 0, sizeof(h));
-    h.dt = dt; h.dtc = dt; h.t_end = 1e300; h.prev_err = 1.0; h.status = MJX_STATUS_RUNNING_CODE;
+    h.dt = dt; h.dtc = dt; h.t_end = 1e300; h.prev_err = 1.0; h.lprev = 0.0; h.status = MJX_STATUS_RUNNING_CODE;
     h.order = 2; h.save_slot = -1; h.max_saves = 1 << 30; h.save_every = 1 << 30; h.max_attempts = 1 << 30;
     MJX_CUDA_TRY(cudaMemcpyAsync(st, &h, sizeof(h), cudaMemcpyHostToDevice, s));
     MJX_CUDA_TRY(cudaStreamSynchronize(s));
@@ -410,7 +410,7 @@ mjx_status mjx_imex_mixed_attempt_kernel2d(const void* plan32, const void* plan6
       CtlArgs ca;
       memset(&ca, 0, sizeof(ca));
       ca.st = st; ca.partial = (const double*)(w + L.part); ca.nonfinite = (const int*)(w + L.bad);
-      ca.nparts = L.nparts; ca.n_dof = (double)nf * g->ny * g->nx; ca.pid = *pid;
+      ca.nparts = L.nparts; ca.gain = ctl_gain(*pid, 2, (double)nf * g->ny * g->nx); ca.pid = *pid;
       e = launch_controller(ca, s);
       break;
     }
@@ -476,7 +476,7 @@ static mjx_status capture_mixed(ImexMixedPlan& P) {
   CtlArgs ca;
   memset(&ca, 0, sizeof(ca));
   ca.st = st; ca.partial = (const double*)(P.ws + P.L.part); ca.nonfinite = (const int*)(P.ws + P.L.bad);
-  ca.nparts = P.L.nparts; ca.n_dof = (double)P.pb.nfields * P.g.ny * P.g.nx; ca.pid = P.pid;
+  ca.nparts = P.L.nparts; ca.gain = ctl_gain(P.pid, 2, (double)P.pb.nfields * P.g.ny * P.g.nx); ca.pid = P.pid;
   ca.hist_t = P.ht; ca.hist_dt = P.hdt;
   cudaError_t ce = cudaSuccess;
   do {
@@ -526,7 +526,7 @@ static mjx_status run_mixed(ImexMixedPlan& P, int io_dtype, double t0, double t_
   DevState h;
   memset(&h, 0, sizeof(h));
   const double dt_init = (dt0 < P.pb.dt_cfl || dt0 != dt0) ? dt0 : P.pb.dt_cfl;
-  h.t = t0; h.dt = dt_init; h.t_end = t_end; h.prev_err = 1.0; h.dt_cfl = P.pb.dt_cfl;
+  h.t = t0; h.dt = dt_init; h.t_end = t_end; h.prev_err = 1.0; h.lprev = 0.0; h.dt_cfl = P.pb.dt_cfl;
   h.status = MJX_STATUS_RUNNING_CODE; h.write_idx = 1; h.finite = 1;
   h.max_saves = max_saves; h.save_every = P.save_every; h.order = 2; h.save_slot = -1;
   h.max_attempts = P.pb.max_attempts > 0 ? P.pb.max_attempts : 20 * P.max_steps + 1000;
@@ -545,7 +545,8 @@ static mjx_status run_mixed(ImexMixedPlan& P, int io_dtype, double t0, double t_
     CtlArgs ca;
     memset(&ca, 0, sizeof(ca));
     ca.st = st; ca.partial = (const double*)(w + P.L.part); ca.nonfinite = (const int*)(w + P.L.bad);
-    ca.nparts = P.L.nparts; ca.n_dof = (double)nf * P.g.ny * P.g.nx; ca.pid = P.pid; ca.hist_t = ht; ca.hist_dt = hdt;
+    ca.nparts = P.L.nparts; ca.gain = ctl_gain(P.pid, 2, (double)nf * P.g.ny * P.g.nx); ca.pid = P.pid;
+    ca.hist_t = ht; ca.hist_dt = hdt;
     const cudaError_t he = run_host_loop([&](cudaStream_t ls) -> cudaError_t {
       const cudaError_t le = launch_mix_attempt(A, ls);
       return le == cudaSuccess ? launch_controller(ca, ls) : le;

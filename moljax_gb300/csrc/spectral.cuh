@@ -15,6 +15,7 @@ namespace mjx {
 // Device-resident state of an adaptive run (lives in the caller's workspace).
 struct DevState {
   double t, dt, dtc, t_end, prev_err, err_last, dt_cfl, dt_last_accepted;
+  double lprev;  // log max(prev_err, 1e-10)
   int cur, status, n_acc, n_rej, write_idx, attempts, done, finite;
   int max_saves, save_every, max_attempts, order;
   int save_slot, pad0, pad1, pad2;
@@ -161,12 +162,22 @@ template <typename T>
 cudaError_t launch_col(const ColArgs<T>& a, cudaStream_t s);
 
 // Arguments of the adaptive controller kernel (csrc/imex.cu).
+struct CtlGain {
+  double kI, kP;    // the controller's gains over the error order
+  double inv_n;     // 1 / degrees of freedom
+};
+inline CtlGain ctl_gain(const mjx_pid_params& p, int order, double n_dof) {
+  CtlGain g;
+  g.kI = p.kI / order; g.kP = p.kP / order; g.inv_n = 1.0 / n_dof;
+  return g;
+}
+
 struct CtlArgs {
   DevState* st;
   const double* partial;
   const int* nonfinite;
   int nparts;
-  double n_dof;
+  CtlGain gain;
   mjx_pid_params pid;
   double* hist_t;
   double* hist_dt;
