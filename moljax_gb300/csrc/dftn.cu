@@ -108,80 +108,6 @@ static void host_fft2(std::vector<double>& re, std::vector<double>& im) {
       }
 }
 
-template <typename T>
-struct Dft {
-  const cx<T>* tw;    // length-L twiddles in the form of tile_dft
-  const cx<T>* chirp; // length n
-  const cx<T>* bhat;  // length L, FFT_L(b) / L
-  int n, L, bluestein;
-  int odd;            // an odd number of passes: the buffers swap
-  int tps;            // threads per sequence
-  int staged;         // the tables are copied to shared memory first
-  unsigned long long rad;
-};
-
-// A tile's two buffers and its tables.  Small tiles copy the tables to shared memory while
-// their data loads are in flight: a pass whose twiddles come from a cold L1 waits ~700 cycles
-// for L2, several times the pass itself.
-template <typename T>
-struct Tile {
-  cx<T>* cur;
-  cx<T>* alt;
-  const cx<T>* tw;
-  const cx<T>* chirp;
-  const cx<T>* bhat;
-  int lS, tid, nth;
-};
-
-template <typename T>
-__device__ __forceinline__ Tile<T> tile_begin(const Dft<T>& d, unsigned char* smem, int lS) {
-  typedef cx<T> C;
-  Tile<T> t;
-  const int m = sp_size(d.L << lS);
-  t.cur = reinterpret_cast<C*>(smem);
-  t.alt = t.cur + m;
-  t.lS = lS; t.tid = threadIdx.x; t.nth = blockDim.x;
-  t.tw = d.tw; t.chirp = d.chirp; t.bhat = d.bhat;
-  if (d.staged) {
-    C* w = t.alt + m;
-    for (int i = t.tid; i < d.L; i += t.nth) w[i] = __ldg(&d.tw[i]);
-    t.tw = w;
-    if (d.bluestein) {
-      C* b = w + d.L;
-      C* c = b + d.L;
-      for (int i = t.tid; i < d.L; i += t.nth) b[i] = __ldg(&d.bhat[i]);
-      for (int i = t.tid; i < d.n; i += t.nth) c[i] = __ldg(&d.chirp[i]);
-      t.bhat = b; t.chirp = c;
-    }
-  }
-  return t;
-}
-
-// Forward DFT of the tile's sequences (elements 0 .. n - 1 of each), left in t.cur.  The caller
-// has synchronised.
-template <typename T>
-__device__ __forceinline__ void dft_tile(const Dft<T>& d, Tile<T>& t) {
-  typedef cx<T> C;
-  const int lS = t.lS, L = d.L, n = d.n;
-  if (d.bluestein) {
-    for (int e = t.tid; e < (L << lS); e += t.nth) {
-      const int j = e >> lS;
-      t.cur[sp(e)] = j < n ? cmul(t.cur[sp(e)], t.chirp[j]) : mk<C>((T)0, (T)0);
-    }
-    __syncthreads();
-  }
-  tile_dft<T>(t.cur, t.alt, L, d.rad, lS, t.tw, t.tid, t.nth);
-  if (d.odd) { C* x = t.cur; t.cur = t.alt; t.alt = x; }
-  if (!d.bluestein) return;
-  // the inverse transform of the product by conjugation
-  for (int e = t.tid; e < (L << lS); e += t.nth) t.cur[sp(e)] = cconj(cmul(t.cur[sp(e)], t.bhat[e >> lS]));
-  __syncthreads();
-  tile_dft<T>(t.cur, t.alt, L, d.rad, lS, t.tw, t.tid, t.nth);
-  if (d.odd) { C* x = t.cur; t.cur = t.alt; t.alt = x; }
-  for (int e = t.tid; e < (n << lS); e += t.nth) t.cur[sp(e)] = cmul(cconj(t.cur[sp(e)]), t.chirp[e >> lS]);
-  __syncthreads();
-}
-
 // ------------------------------------------------------------------ row pass
 enum { GROW_LOAD_SPEC = 1, GROW_STORE_REAL = 2, GROW_STORE_SPEC = 4 };
 
@@ -428,43 +354,12 @@ static Dft<T> dft_desc(const void* plan, int n) {
     DftTune t;
     d.tps = (tune_dft_get(n, (int)sizeof(T), &t) && t.tpsm > 0) ? t.tpsm : n / 8;
   } else {
-    int passes = 0;
-    d.rad = tile_pow2_radices(g.log2L, &passes);
-    d.odd = passes & 1;
+    d.log2L = g.log2L;
     d.tps = g.L / 8;
   }
   if (d.tps < 1) d.tps = 1;
   if (d.tps > 256) d.tps = 256;
   return d;
-}
-
-template <typename T>
-static size_t tile_smem(const Dft<T>& d, int l) {
-  size_t e = 2 * (size_t)sp_size(d.L << l);
-  if (d.staged) e += (size_t)d.L + (d.bluestein ? (size_t)d.L + d.n : 0);
-  return e * sizeof(cx<T>);
-}
-
-// Sequences per CTA (log2) for `total` sequences: up to `want`, within 512 threads and 96 KB of
-// shared memory (one sequence may take more), halved until the pass has about one CTA per SM;
-// tables in shared memory where the whole stays under 96 KB.  A pass with few sequences doubles
-// the threads of each (n/4 instead of n/8): its time is a chain of passes, not throughput.
-template <typename T>
-static int tile_log(Dft<T>& d, long long total, int want) {
-  const size_t cap = 96 * 1024;
-  int l = 0;
-  while ((2 << l) <= want && (2 << l) * d.tps <= 512 && tile_smem<T>(d, l + 1) <= cap) ++l;
-  while (l > 0 && (total + (1 << l) - 1) >> l < 128) --l;
-  if (((d.tps << l) + 31) / 32 * ((total + (1 << l) - 1) >> l) < 152 * 8 && (2 * d.tps << l) <= 512) d.tps *= 2;
-  d.staged = 1;
-  if (tile_smem<T>(d, l) > cap) d.staged = 0;
-  return l;
-}
-
-template <typename T>
-static int tile_threads(const Dft<T>& d, int l) {
-  const int t = ((d.tps << l) + 31) & ~31;
-  return t < 64 ? 64 : (t > 512 ? 512 : t);
 }
 
 template <typename T>
