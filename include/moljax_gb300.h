@@ -129,7 +129,9 @@ const char* mjx_last_error(void);
 size_t mjx_spec2d_plan_bytes(int ny, int nx, int dtype);
 mjx_status mjx_spec2d_plan_init(void* plan, const mjx_grid2d* grid, int symbol, int dtype,
                                 void* stream);
-/* Spectrum workspace for nfields fields: nfields * ny * (nx/2+1 padded) complex. */
+/* Spectrum workspace for nfields fields: nfields * ny * (nx/2+1 padded) complex; in FP64 also
+ * that many doubles for the multipliers of fixed steps (a workspace without them is accepted:
+ * the steps then form the multipliers each time). */
 size_t mjx_spec2d_ws_bytes(int ny, int nx, int nfields, int dtype);
 
 /* out_f = IFFT2( m(h, D_f, lam) * FFT2(in_f) ) for each of nfields fields.
@@ -177,7 +179,8 @@ mjx_status mjx_spectral_apply_general3d(const void* plan_z, const void* plan_y, 
 /* Plan: x / y / z twiddles and 1D symbols (FD or spectral) of an [nz][ny][nx] box. */
 size_t mjx_spec3d_plan_bytes(int nz, int ny, int nx, int dtype);
 mjx_status mjx_spec3d_plan_init(void* plan, const mjx_grid3d* grid, int symbol, int dtype, void* stream);
-/* Spectrum workspace: nz * ny * (nx/2+1 padded) complex. */
+/* Spectrum workspace: nz * ny * (nx/2+1 padded) complex; in FP64 also that many doubles (as
+ * mjx_spec2d_ws_bytes). */
 size_t mjx_spec3d_ws_bytes(int nz, int ny, int nx, int dtype);
 /* n_steps times u <- real(IFFTN( m(h, D, lam_x + lam_y + lam_z) FFTN(u) )), each a full
  * forward and inverse transform: with MJX_MULT_CN the 3D FFT-CN loop of
@@ -240,7 +243,8 @@ mjx_status mjx_gs_cn_newton2d(const void* plan, const mjx_grid2d* grid, int dtyp
                               void* y_out, int* iters, int* iters_total, double* last_res, void* ws,
                               size_t ws_bytes, void* stream);
 
-/* Workspace of mjx_gs_strang_exp2d: the two fields' half spectra. */
+/* Workspace of mjx_gs_strang_exp2d: the two fields' half spectra; in FP64 also as many doubles
+ * (as mjx_spec2d_ws_bytes). */
 size_t mjx_gs_strang_exp_ws_bytes(int ny, int nx, int dtype);
 /* n_steps fixed Strang steps of periodic Gray-Scott (imex_step / imex_solve of
  * benchmarks/benchmark_gray_scott.py:268-296): explicit Euler half step of the reaction,
@@ -271,7 +275,7 @@ mjx_status mjx_gs_rk4_spectral2d(const void* plan, const mjx_grid2d* grid, int d
  * run FFT-CN steps with only its input and output buffers.  The spectrum
  * scratch is a fixed 8 MiB array inside the library (held by every GPU that
  * loads the library until process exit), so the grid must satisfy
- * mjx_spec2d_ws_bytes(ny, nx, 1, dtype) <= MJX_NOALLOC_SCRATCH_BYTES (e.g.
+ * its half spectrum ny * (nx/2+1 padded) complex <= MJX_NOALLOC_SCRATCH_BYTES (e.g.
  * 1024^2 FP32, 512^2 FP64); larger grids return MJX_WORKSPACE.  The first call
  * in each CUDA context looks up the scratch address of that context (make that
  * call before any stream capture): the array has its own address in the

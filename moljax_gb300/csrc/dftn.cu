@@ -128,6 +128,7 @@ __global__ void __launch_bounds__(512) grow_kernel(const __grid_constant__ GRowA
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int n = a.d.n, hx = n / 2 + 1, lS = a.lS, S = 1 << lS, tid = threadIdx.x, nth = blockDim.x;
   Tile<T> t = tile_begin<T>(a.d, smem_raw, lS);
+  pdl_wait();
   const long long r0 = ((long long)blockIdx.x << lS) * 2;  // first row of this CTA
   const float rn = 1.0f / (float)n, rh = 1.0f / (float)hx;
   if (a.flags & GROW_LOAD_SPEC) {
@@ -265,6 +266,7 @@ __global__ void __launch_bounds__(512) gcol_kernel(const __grid_constant__ GColA
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int n = a.d.n, lC = a.lC, Cn = 1 << lC, tid = threadIdx.x, nth = blockDim.x;
   Tile<T> t = tile_begin<T>(a.d, smem_raw, lC);
+  pdl_wait();
   const int c0 = blockIdx.x << lC, b = blockIdx.y;
   C* g = a.spec + (long long)b * a.bstride + c0;
   const bool inv_first = (a.dirs & 1) == 0;
@@ -364,15 +366,15 @@ static Dft<T> dft_desc(const void* plan, int n) {
 
 template <typename T>
 static cudaError_t grow(const Dft<T>& d0, const T* in, T* out, cx<T>* spec, long long nrows, int ld, int flags,
-                        cudaStream_t s) {
+                        int pdl, cudaStream_t s) {
   GRowArgs<T> a;
   memset(&a, 0, sizeof(a));
   a.d = d0; a.in = in; a.out = out; a.spec = spec; a.nrows = nrows; a.ld = ld; a.flags = flags;
   const long long pairs = (nrows + 1) / 2;
   a.lS = tile_log<T>(a.d, pairs, 8);
   const long long grid = (pairs + (1 << a.lS) - 1) >> a.lS;
-  grow_kernel<T><<<(unsigned)grid, tile_threads<T>(a.d, a.lS), tile_smem<T>(a.d, a.lS), s>>>(a);
-  return cudaGetLastError();
+  return launch_chain(grow_kernel<T>, dim3((unsigned)grid), tile_threads<T>(a.d, a.lS), tile_smem<T>(a.d, a.lS), s, pdl,
+                      a);
 }
 
 template <typename T>
@@ -380,8 +382,7 @@ static cudaError_t gcol(GColArgs<T> a, int batch, cudaStream_t s) {
   // 4 FP32 or 2 FP64 columns fill a 32-byte sector of each row; twice that where the grid is large
   a.lC = tile_log<T>(a.d, (long long)a.ncols * batch, sizeof(T) == 4 ? 8 : 4);
   dim3 grid((a.ncols + (1 << a.lC) - 1) >> a.lC, batch);
-  gcol_kernel<T><<<grid, tile_threads<T>(a.d, a.lC), tile_smem<T>(a.d, a.lC), s>>>(a);
-  return cudaGetLastError();
+  return launch_chain(gcol_kernel<T>, grid, tile_threads<T>(a.d, a.lC), tile_smem<T>(a.d, a.lC), s, 1, a);
 }
 
 static const double* plan_symbol(const void* plan, int n, int elem, int symbol) {
@@ -422,7 +423,7 @@ static mjx_status general_apply(const void* plan_y, const void* plan_x, const mj
   c.mode = mult == MJX_MULT_TABLE ? GCOL_USER : GCOL_VALUE;
   c.tab = table;
   const long long rows = (long long)nf * ny;
-  MJX_CUDA_TRY(grow<T>(dx, in, nullptr, spec, rows, ld, GROW_STORE_SPEC, s));
+  MJX_CUDA_TRY(grow<T>(dx, in, nullptr, spec, rows, ld, GROW_STORE_SPEC, 0, s));
   if (n_steps > 1 && mult < MJX_MULT_ADV_SOLVE) {
     gtab_kernel<T><<<152 * 4, 256, 0, s>>>(tab, m, nf, ny, ld, ld, hx);
     MJX_CUDA_TRY(cudaGetLastError());
@@ -433,7 +434,7 @@ static mjx_status general_apply(const void* plan_y, const void* plan_x, const mj
     MJX_CUDA_TRY(gcol<T>(c, nf, s));
     const bool last = i == n_steps - 1;
     MJX_CUDA_TRY(grow<T>(dx, nullptr, out, spec, rows, ld,
-                         GROW_LOAD_SPEC | (last ? GROW_STORE_REAL : GROW_STORE_SPEC), s));
+                         GROW_LOAD_SPEC | (last ? GROW_STORE_REAL : GROW_STORE_SPEC), 1, s));
   }
   return MJX_OK;
 }
@@ -469,14 +470,14 @@ static mjx_status general_apply3(const void* pz, const void* py, const void* px,
     z.tab = tab;
   }
   const long long rows = (long long)nz * ny;
-  MJX_CUDA_TRY(grow<T>(dx, in, nullptr, spec, rows, ld, GROW_STORE_SPEC, s));
+  MJX_CUDA_TRY(grow<T>(dx, in, nullptr, spec, rows, ld, GROW_STORE_SPEC, 0, s));
   for (int i = 0; i < n_steps; ++i) {
     MJX_CUDA_TRY(gcol<T>(y, nz, s));
     MJX_CUDA_TRY(gcol<T>(z, 1, s));
     MJX_CUDA_TRY(gcol<T>(yb, nz, s));
     const bool last = i == n_steps - 1;
     MJX_CUDA_TRY(grow<T>(dx, nullptr, out, spec, rows, ld,
-                         GROW_LOAD_SPEC | (last ? GROW_STORE_REAL : GROW_STORE_SPEC), s));
+                         GROW_LOAD_SPEC | (last ? GROW_STORE_REAL : GROW_STORE_SPEC), 1, s));
   }
   return MJX_OK;
 }
@@ -676,7 +677,7 @@ static mjx_status tune_dft(const void* plan, int n, long long nrows, cx<T>* data
       d.odd = sched[17 * i] & 1;
       d.tps = uniq[j];
       auto pass = [&]() {
-        return grow<T>(d, nullptr, nullptr, data, rows, ld, GROW_LOAD_SPEC | GROW_STORE_SPEC, s);
+        return grow<T>(d, nullptr, nullptr, data, rows, ld, GROW_LOAD_SPEC | GROW_STORE_SPEC, 0, s);
       };
       cudaError_t ce = pass();
       if (ce == cudaSuccess) ce = cudaEventRecord(e0, s);

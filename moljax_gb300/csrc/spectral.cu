@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "spectral.cuh"
+#include "tfft.cuh"
 #include "tma.cuh"
 #include "wfft.cuh"
 
@@ -23,11 +24,13 @@ int spec_ldc(int nx) { return ((nx / 2 + 1) + 3) & ~3; }
 // transposed for the one-warp transform (entry 1024 + 32 k1 + l holds w^(l k1)), so that
 // the 32 lanes of a warp read one contiguous 256-byte run per twiddle instead of 32 rows
 // of the table.
-static int twx_count(int nx, int elem) { return (nx == 1024 && elem == 4) ? 2048 : nx; }
+static int twx_count(int nx, int elem) { return elem == 8 ? 2 * nx : (nx == 1024 ? 2048 : nx); }
+// FP64 tables are followed by their (cos, tan) form (tfft.cuh)
+static int twy_count(int ny, int elem) { return elem == 8 ? 2 * ny : ny; }
 
 size_t plan_bytes(int ny, int nx, int elem) {
   const size_t c = 2 * (size_t)elem;
-  return align256(twx_count(nx, elem) * c) + align256(ny * c) + align256(spec_ldc(nx) * (size_t)elem) +
+  return align256(twx_count(nx, elem) * c) + align256(twy_count(ny, elem) * c) + align256(spec_ldc(nx) * (size_t)elem) +
          align256(ny * (size_t)elem);
 }
 
@@ -36,7 +39,7 @@ PlanView plan_view(const void* plan, int ny, int nx, int elem) {
   const char* p = (const char*)plan;
   PlanView v;
   v.twx = p; p += align256(twx_count(nx, elem) * c);
-  v.twy = p; p += align256(ny * c);
+  v.twy = p; p += align256(twy_count(ny, elem) * c);
   v.lamx = p; p += align256(spec_ldc(nx) * (size_t)elem);
   v.lamy = p;
   return v;
@@ -54,46 +57,6 @@ int row_nseq(int n, int nrows) {
 
 int row_ctas(int n, int nrows, int npairs) { return npairs * nrows / row_nseq(n, nrows); }
 
-// ------------------------------------------------------------------ reactions
-template <typename T, int RX>
-__device__ __forceinline__ void react_heun(T& a, T& b, T h, T F, T k, T r) {
-  if (RX == RX_GRAY_SCOTT) {
-    // moljax/core/stepping.py:402-415 with operators.py:655-667
-    const T uvv = a * b * b;
-    const T fu = -uvv + F * ((T)1 - a);
-    const T fv = uvv - (F + k) * b;
-    const T ua = a + h * fu, va = b + h * fv;
-    const T uvv2 = ua * va * va;
-    const T gu = -uvv2 + F * ((T)1 - ua);
-    const T gv = uvv2 - (F + k) * va;
-    const T hh = (T)0.5 * h;
-    a = a + hh * (fu + gu);
-    b = b + hh * (fv + gv);
-  } else if (RX == RX_FISHER) {
-    const T fa = r * a * ((T)1 - a), fb = r * b * ((T)1 - b);
-    const T ta = a + h * fa, tb = b + h * fb;
-    const T hh = (T)0.5 * h;
-    a = a + hh * (fa + r * ta * ((T)1 - ta));
-    b = b + hh * (fb + r * tb * ((T)1 - tb));
-  }
-}
-
-// Explicit Euler reaction step y + h N(y) (imex_euler_step, stepping.py:349-359).
-template <typename T, int RX>
-__device__ __forceinline__ void react_euler(T& a, T& b, T h, T F, T k, T r) {
-  if (RX == RX_GRAY_SCOTT) {
-    const T uvv = a * b * b;
-    const T fu = -uvv + F * ((T)1 - a);
-    const T fv = uvv - (F + k) * b;
-    a = a + h * fu;
-    b = b + h * fv;
-  } else if (RX == RX_FISHER) {
-    const T fa = r * a * ((T)1 - a), fb = r * b * ((T)1 - b);
-    a = a + h * fa;
-    b = b + h * fb;
-  }
-}
-
 template <typename T> __device__ __forceinline__ bool finite_(T v) { return isfinite(v); }
 
 // ------------------------------------------------------------------ row pass
@@ -102,18 +65,18 @@ template <typename T> struct Occ { static constexpr int row = sizeof(T) == 4 ? 4
 // LOG2N > 0: the row length 2^LOG2N and one sequence per CTA are compile-time constants
 // (FP32 rows of 2048 and 4096 points), so that the transform's index arithmetic and radix
 // schedule fold into the code; LOG2N = 0 reads both from the arguments.
-// R4: radix-4 transforms with n/4 threads per sequence (short FP64 rows, fft_smem_r4).
-template <typename T, int RX, int LOG2N = 0, bool R4 = false>
+template <typename T, int RX, int LOG2N = 0>
 __global__ void __launch_bounds__(256, Occ<T>::row) row_kernel(const __grid_constant__ RowArgs<T> a) {
   typedef cx<T> C;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* buf = reinterpret_cast<C*>(smem_raw);
   const DevState* st = a.st;
+  pdl_wait();
   if (st != nullptr && st->done) return;
 
   const int n = LOG2N ? (1 << LOG2N) : a.n, half = n >> 1;
   const int log2n = LOG2N ? LOG2N : a.log2n, nseq = LOG2N ? 1 : a.nseq;
-  const int tps = R4 ? (n >= 4 ? n / 4 : 1) : (n >= 16 ? n / 16 : 1);
+  const int tps = n >= 16 ? n / 16 : 1;
   const int tid = threadIdx.x;
   const int s_loc = tid / tps, lt = tid % tps;
   const int seq0 = blockIdx.x * nseq;
@@ -147,8 +110,7 @@ __global__ void __launch_bounds__(256, Occ<T>::row) row_kernel(const __grid_cons
       }
     }
     __syncthreads();
-    if (R4) fft_smem_r4<T, true, false>(buf, n, log2n, nseq, n, 1, a.tw, tid);
-    else if (LOG2N) fft_smem_inl<T, true, false>(buf, n, log2n, nseq, n, 1, a.tw, tid);
+    if (LOG2N) fft_smem_inl<T, true, false>(buf, n, log2n, nseq, n, 1, a.tw, tid);
     else fft_smem<T, true, false>(buf, n, log2n, nseq, n, 1, a.tw, tid);
   } else {
     const T* ra = rin + pr.ra + y * a.rstride;
@@ -233,8 +195,7 @@ __global__ void __launch_bounds__(256, Occ<T>::row) row_kernel(const __grid_cons
   // 3. r2c and split into the two half spectra
   if (flags & ROW_STORE_SPEC) {
     __syncthreads();
-    if (R4) fft_smem_r4<T, false, false>(buf, n, log2n, nseq, n, 1, a.tw, tid);
-    else if (LOG2N) fft_smem_inl<T, false, false>(buf, n, log2n, nseq, n, 1, a.tw, tid);
+    if (LOG2N) fft_smem_inl<T, false, false>(buf, n, log2n, nseq, n, 1, a.tw, tid);
     else fft_smem<T, false, false>(buf, n, log2n, nseq, n, 1, a.tw, tid);
     C* A = a.spec + ((flags & ROW_SPEC_ALT) ? pr.oa : pr.sa) + y * a.ldc;
     C* B = a.spec + ((flags & ROW_SPEC_ALT) ? pr.ob : pr.sb) + y * a.ldc;
@@ -279,34 +240,14 @@ __global__ void __launch_bounds__(256, Occ<T>::row) row_kernel(const __grid_cons
 }
 
 // ------------------------------------------------------------------ column pass
-template <typename T>
-__device__ __forceinline__ T multiplier(int mul, T hD, T lam, int pw) {
-  T m;
-  if (mul == MUL_HELMHOLTZ) {
-    T den = (T)1 - hD * lam;  // moljax/core/fft_solvers.py:281-285
-    if (fabs(den) < (T)1e-14) den = (T)1e-14;
-    m = (T)1 / den;
-  } else if (mul == MUL_CN) {
-    const T x = (T)0.5 * hD * lam;
-    m = ((T)1 + x) / ((T)1 - x);
-  } else if (mul == MUL_EXP) {
-    m = exp(hD * lam);
-  } else if (mul == MUL_LAP) {
-    m = hD * lam;
-  } else {
-    m = (T)1;
-  }
-  return pw == 2 ? m * m : m;
-}
-
 template <typename T> struct ColThreads { static constexpr int v = sizeof(T) == 4 ? 1024 : 512; };
 
-// R4: radix-4 column transforms with ny/4 threads per column (short FP64 columns).
-template <typename T, bool R4 = false>
+template <typename T>
 __global__ void __launch_bounds__(ColThreads<T>::v, 1) col_kernel(const __grid_constant__ ColArgs<T> a) {
   typedef cx<T> C;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* buf = reinterpret_cast<C*>(smem_raw);
+  pdl_wait();
   if (a.st != nullptr && a.st->done) return;
   const ColJob jb = a.job[blockIdx.y];
   const int Cn = a.C, nout = jb.nout, W = Cn * nout;
@@ -339,8 +280,7 @@ __global__ void __launch_bounds__(ColThreads<T>::v, 1) col_kernel(const __grid_c
   __syncthreads();
   const int dirs = jb.dirs ? jb.dirs : 3;
   if (dirs & 1) {
-    if (R4) fft_smem_r4<T, false, true>(buf, ny, a.log2ny, Cn, 1, W, a.tw, tid);
-    else fft_smem<T, false, true>(buf, ny, a.log2ny, Cn, 1, W, a.tw, tid);
+    fft_smem<T, false, true>(buf, ny, a.log2ny, Cn, 1, W, a.tw, tid);
   }
   const T jscale = jb.scale != 0.0 ? (T)jb.scale : a.scale;
 
@@ -353,51 +293,13 @@ __global__ void __launch_bounds__(ColThreads<T>::v, 1) col_kernel(const __grid_c
     const T lam = lxy + a.lamy[ky];
     const C v = buf[sp(ky * W + c)];
     if (jb.mul == MUL_ADVDIFF || jb.mul == MUL_ADV_LAP || jb.mul == MUL_ADV_EXP || jb.mul == MUL_ADV_CN) {
-      // z = h (D lam - i (vx kx + vy ky)), kx, ky = 2 pi fftfreq (the Nyquist index
-      // negative); m = 1/(1 - z) with |1 - z| < 1e-14 -> 1e-14 (the solve of
-      // FFTAdvectionDiffusionPreconditioner, moljax/core/preconditioners.py:297-420, and of
-      // AdvectionDiffusionOperator, fft_operators.py:179-260), z itself (matvec) or exp(z)
-      // (exp_matvec), or the Crank-Nicolson factor (1 + z/2)/(1 - z/2) of the 1D advective
-      // FFT-CN (benchmarks/benchmark_solver_comparison.py:152-163).  The reference keeps
-      // real(ifft(.)); on the half spectrum that is the
-      // multiplier (m(k) + conj(m(-k)))/2, which equals m(k) except on the Nyquist lines,
-      // where fftfreq breaks the oddness of the advection term.
-      const int nxl = 2 * (a.ncols - 1);
-      const int mx = kx < nxl / 2 ? kx : kx - nxl, my = ky < ny / 2 ? ky : ky - ny;
-      const int nmx = mx == -nxl / 2 ? mx : -mx, nmy = my == -ny / 2 ? my : -my;
-      const double hh = h * jb.hfac[0];
-      const double zr = (double)hD0 * (double)lam;
-      double mre = 0.0, mim = 0.0;
-      for (int side = 0; side < 2; ++side) {
-        const int qx = side ? nmx : mx, qy = side ? nmy : my;
-        const double zi = -hh * (jb.vx * a.kxs * qx + jb.vy * a.kys * qy);
-        double fr, fi;
-        if (jb.mul == MUL_ADVDIFF) {
-          double dr = 1.0 - zr, di = -zi;
-          if (sqrt(dr * dr + di * di) < 1e-14) { dr = 1e-14; di = 0.0; }
-          const double den = dr * dr + di * di;
-          fr = dr / den;
-          fi = -di / den;
-        } else if (jb.mul == MUL_ADV_LAP) {
-          fr = zr;
-          fi = zi;
-        } else if (jb.mul == MUL_ADV_CN) {
-          const double nr = 1.0 + 0.5 * zr, ni = 0.5 * zi, dr = 1.0 - 0.5 * zr, di = -0.5 * zi;
-          const double den = dr * dr + di * di;
-          fr = (nr * dr + ni * di) / den;
-          fi = (ni * dr - nr * di) / den;
-        } else {
-          double sn, cs;
-          sincos(zi, &sn, &cs);
-          const double ez = exp(zr);
-          fr = ez * cs;
-          fi = ez * sn;
-        }
-        mre += 0.5 * fr;
-        mim += side ? -0.5 * fi : 0.5 * fi;  // conj(m(-k)) on the second side
-      }
-      const T mr = (T)mre, mi = (T)mim;
+      const double2 f = adv_multiplier<T>(a, jb, (double)hD0, h * jb.hfac[0], (double)lam, kx, ky);
+      const T mr = (T)f.x, mi = (T)f.y;
       buf[sp(ky * W + c)] = cscale(mk<C>(v.x * mr - v.y * mi, v.x * mi + v.y * mr), jscale);
+      continue;
+    }
+    if (jb.mul == MUL_TABLED) {
+      buf[sp(ky * W + c)] = cscale(v, kx < a.ncols ? a.mtab[jb.sin + ky * ldc + kx] : (T)0);
       continue;
     }
     if (jb.mul == MUL_TABLE) {
@@ -409,8 +311,7 @@ __global__ void __launch_bounds__(ColThreads<T>::v, 1) col_kernel(const __grid_c
   }
   __syncthreads();
   if (dirs & 2) {
-    if (R4) fft_smem_r4<T, true, true>(buf, ny, a.log2ny, W, 1, W, a.tw, tid);
-    else fft_smem<T, true, true>(buf, ny, a.log2ny, W, 1, W, a.tw, tid);
+    fft_smem<T, true, true>(buf, ny, a.log2ny, W, 1, W, a.tw, tid);
   }
 
   const int lw = __ffs(W) - 1;  // W = Cn or 2 Cn
@@ -429,6 +330,7 @@ __global__ void __launch_bounds__(128) row_kernel_w32(const __grid_constant__ Ro
   typedef float2 C;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const DevState* st = a.st;
+  pdl_wait();
   if (st != nullptr && st->done) return;
   const int lane = threadIdx.x & 31, s_loc = threadIdx.x >> 5;
   C* tile = reinterpret_cast<C*>(smem_raw) + s_loc * (32 * 33);
@@ -568,6 +470,8 @@ static size_t row_smem(int n, int nseq, int elem) { return (size_t)sp_size(nseq 
 
 template <typename T, int RX>
 cudaError_t launch_row(const RowArgs<T>& a0, cudaStream_t s) {
+  if constexpr (sizeof(T) == 8)
+    if (row64_takes(a0.n)) return launch_row64<RX>(a0, s);
   // Small grids: fewer row pairs per CTA until the pass covers every SM (the partial-sum
   // passes keep their CTA count, which sizes the controller's reduction).  FP64 transforms
   // are bound by the FP64 units, so a pass on a few SMs is a few times slower.
@@ -581,42 +485,26 @@ cudaError_t launch_row(const RowArgs<T>& a0, cudaStream_t s) {
   const int grid = a.npairs * a.nrows / a.nseq;
   if constexpr (sizeof(T) == 4) {
     if (a.n == 1024 && a.nseq <= 4) {  // one warp per 1024-point row
-      row_kernel_w32<RX><<<grid, 32 * a.nseq, (size_t)a.nseq * 32 * 33 * sizeof(float2), s>>>(a);
-      return cudaGetLastError();
-    }
-  }
-  if constexpr (sizeof(T) == 8) {
-    // short FP64 rows on a small grid (no error partials, whose CTA count is fixed): radix-4
-    // transforms, n/4 threads per sequence, at most 256 threads per CTA, every SM covered
-    // where possible.  Only when the radix-16 pass would run fewer than four warps per SM:
-    // with more rows the extra passes of radix 4 cost more than the threads gain.
-    if (!partials && a.n >= 4 && a.n <= 256 && (long long)a.npairs * a.nrows * tps < 152LL * 128) {
-      RowArgs<T> b = a;
-      const int tps4 = a.n / 4;
-      while (b.nseq > 1 && b.nseq * tps4 > 256) b.nseq >>= 1;
-      while (b.nseq > 1 && b.npairs * b.nrows / b.nseq < 152) b.nseq >>= 1;
-      const int grid4 = b.npairs * b.nrows / b.nseq;
-      row_kernel<T, RX, 0, true><<<grid4, b.nseq * tps4, row_smem(b.n, b.nseq, sizeof(T)), s>>>(b);
-      return cudaGetLastError();
+      return launch_chain(row_kernel_w32<RX>, dim3(grid), 32 * a.nseq, (size_t)a.nseq * 32 * 33 * sizeof(float2), s,
+                          a.pdl, a);
     }
   }
   const size_t smem = row_smem(a.n, a.nseq, sizeof(T));
   if constexpr (sizeof(T) == 4) {
     if (a.n == 4096 && a.nseq == 1) {
-      row_kernel<T, RX, 12><<<grid, tps, smem, s>>>(a);
-      return cudaGetLastError();
+      return launch_chain(row_kernel<T, RX, 12>, dim3(grid), tps, smem, s, a.pdl, a);
     }
     if (a.n == 2048 && a.nseq == 1) {
-      row_kernel<T, RX, 11><<<grid, tps, smem, s>>>(a);
-      return cudaGetLastError();
+      return launch_chain(row_kernel<T, RX, 11>, dim3(grid), tps, smem, s, a.pdl, a);
     }
   }
-  row_kernel<T, RX><<<grid, a.nseq * tps, smem, s>>>(a);
-  return cudaGetLastError();
+  return launch_chain(row_kernel<T, RX>, dim3(grid), a.nseq * tps, smem, s, a.pdl, a);
 }
 
 template <typename T>
 cudaError_t launch_col(const ColArgs<T>& a0, cudaStream_t s) {
+  if constexpr (sizeof(T) == 8)
+    if (col64_takes(a0.ny)) return launch_col64(a0, s);
   ColArgs<T> a = a0;
   int maxout = 1;
   for (int j = 0; j < a.njobs; ++j) maxout = a.job[j].nout > maxout ? a.job[j].nout : maxout;
@@ -624,23 +512,9 @@ cudaError_t launch_col(const ColArgs<T>& a0, cudaStream_t s) {
   // small grids: narrower tiles until the pass covers every SM (as launch_row)
   const long long planes = a.nplanes > 1 ? a.nplanes : 1;
   while (a.C > 1 && (long long)((a.ncols + a.C - 1) / a.C) * a.njobs * planes < 152) a.C >>= 1;
-  if constexpr (sizeof(T) == 8) {
-    // short FP64 columns on a small grid (fewer than four warps per SM at radix 16): radix-4
-    // transforms, ny/4 threads per column, narrower tiles to stay within the thread cap
-    if (a.ny >= 4 && a.ny <= 256 && (long long)a.ncols * a.njobs * planes * tps < 152LL * 128) {
-      ColArgs<T> b = a;
-      const int tps4 = a.ny / 4;
-      while (b.C > 1 && b.C * maxout * tps4 > ColThreads<T>::v) b.C >>= 1;
-      dim3 g4((b.ncols + b.C - 1) / b.C, b.njobs, b.nplanes > 1 ? b.nplanes : 1);
-      const size_t sm4 = (size_t)sp_size(b.ny * b.C * maxout) * sizeof(cx<T>);
-      col_kernel<T, true><<<g4, b.C * maxout * tps4, sm4, s>>>(b);
-      return cudaGetLastError();
-    }
-  }
   dim3 grid((a.ncols + a.C - 1) / a.C, a.njobs, a.nplanes > 1 ? a.nplanes : 1);
   const size_t smem = (size_t)sp_size(a.ny * a.C * maxout) * sizeof(cx<T>);
-  col_kernel<T><<<grid, a.C * maxout * tps, smem, s>>>(a);
-  return cudaGetLastError();
+  return launch_chain(col_kernel<T>, grid, a.C * maxout * tps, smem, s, a.pdl, a);
 }
 
 #define MJX_INST_ROW(T, RX) template cudaError_t launch_row<T, RX>(const RowArgs<T>&, cudaStream_t);
@@ -700,12 +574,12 @@ mjx_status ensure_kernel_attrs() {
     MJX_TRY(raise_smem(row_kernel<float, RX_GRAY_SCOTT, 12>, optin));
     MJX_TRY(raise_smem(row_kernel<float, RX_FISHER, 12>, optin));
 
+    MJX_TRY(raise_smem(row_kernel_w32<RX_NONE>, optin));
+    MJX_TRY(raise_smem(row_kernel_w32<RX_GRAY_SCOTT>, optin));
+    MJX_TRY(raise_smem(row_kernel_w32<RX_FISHER>, optin));
     MJX_TRY(raise_smem(col_kernel<float>, optin));
     MJX_TRY(raise_smem(col_kernel<double>, optin));
-    MJX_TRY(raise_smem(col_kernel<double, true>, optin));
-    MJX_TRY(raise_smem(row_kernel<double, RX_NONE, 0, true>, optin));
-    MJX_TRY(raise_smem(row_kernel<double, RX_GRAY_SCOTT, 0, true>, optin));
-    MJX_TRY(raise_smem(row_kernel<double, RX_FISHER, 0, true>, optin));
+    MJX_TRY(spectral64_attrs(optin));
     return MJX_OK;
   });
 }
@@ -891,14 +765,24 @@ mjx_status spectral_apply(const void* plan, const mjx_grid2d* g, int nfields, co
   return MJX_OK;
 }
 
+// Bytes of nfields half spectra; FP64 workspaces hold their multiplier table after them.
+static size_t spec_bytes(int ny, int nx, int nfields, int elem) {
+  return (size_t)nfields * ny * spec_ldc(nx) * 2 * elem;
+}
+
+// A step is one column pass and one row pass: the rows go from spectrum to spectrum (c2r, then
+// r2c of the same registers and shared memory; the real field of a step that is not the last
+// is not stored), and FP64 steps read their multipliers from a table formed once.
 template <typename T>
 mjx_status fft_cn(const void* plan, const mjx_grid2d* g, double D, double dt, int n_steps,
-                  const T* u_in, T* u_out, void* ws, cudaStream_t s) {
+                  const T* u_in, T* u_out, void* ws, size_t ws_bytes, cudaStream_t s) {
   const PlanView pv = plan_view(plan, g->ny, g->nx, sizeof(T));
   cx<T>* spec = (cx<T>*)ws;
   RowArgs<T> fwd = field_rows<T>(g, 1, pv, spec);
-  RowArgs<T> inv = fwd;
+  RowArgs<T> inv = fwd, both = fwd;
   fwd.pr[0].flags = ROW_STORE_SPEC;
+  fwd.rin[0] = u_in;
+  both.pr[0].flags = ROW_LOAD_SPEC | ROW_STORE_SPEC;
   inv.pr[0].flags = ROW_LOAD_SPEC | ROW_STORE_REAL;
   inv.rout[0] = u_out;
   ColArgs<T> c = field_cols<T>(g, pv, spec, 1);
@@ -910,11 +794,15 @@ mjx_status fft_cn(const void* plan, const mjx_grid2d* g, double D, double dt, in
       MJX_CUDA_TRY(cudaMemcpyAsync(u_out, u_in, sizeof(T) * g->ny * g->nx, cudaMemcpyDeviceToDevice, s));
     return MJX_OK;
   }
+  if constexpr (sizeof(T) == 8) {
+    const size_t sb = spec_bytes(g->ny, g->nx, 1, 8);
+    if (n_steps > 1 && ws_bytes >= sb + sb / 2) MJX_CUDA_TRY(tabulate_cols(c, (double*)ws + sb / 8, s));
+  }
+  MJX_CUDA_TRY((launch_row<T, RX_NONE>(fwd, s)));
+  both.pdl = inv.pdl = c.pdl = 1;
   for (int i = 0; i < n_steps; ++i) {
-    fwd.rin[0] = i == 0 ? u_in : u_out;
-    MJX_CUDA_TRY((launch_row<T, RX_NONE>(fwd, s)));
     MJX_CUDA_TRY(launch_col<T>(c, s));
-    MJX_CUDA_TRY((launch_row<T, RX_NONE>(inv, s)));
+    MJX_CUDA_TRY((launch_row<T, RX_NONE>(i < n_steps - 1 ? both : inv, s)));
   }
   return MJX_OK;
 }
@@ -990,7 +878,8 @@ size_t mjx_spec2d_plan_bytes(int ny, int nx, int dtype) {
 size_t mjx_spec2d_ws_bytes(int ny, int nx, int nfields, int dtype) {
   const int e = elem_size(dtype);
   if (!e || ilog2_exact(nx) < 1 || ilog2_exact(ny) < 1 || nfields < 1) return 0;
-  return (size_t)nfields * ny * spec_ldc(nx) * 2 * e;
+  const size_t sb = spec_bytes(ny, nx, nfields, e);
+  return e == 8 ? sb + sb / 2 : sb;
 }
 
 mjx_status mjx_spec2d_plan_init(void* plan, const mjx_grid2d* g, int symbol, int dtype,
@@ -1010,7 +899,11 @@ mjx_status mjx_spec2d_plan_init(void* plan, const mjx_grid2d* g, int symbol, int
       const double ang = twopi * (double)j / (double)n;
       const double c = cos(ang), s = -sin(ang);
       if (e == 4) { float* p = (float*)dst; p[2 * j] = (float)c; p[2 * j + 1] = (float)s; }
-      else { double* p = (double*)dst; p[2 * j] = c; p[2 * j + 1] = s; }
+      else {
+        double* p = (double*)dst;
+        p[2 * j] = c; p[2 * j + 1] = s;
+        tile_twiddle(j, n, 8, &p[2 * (n + j)], &p[2 * (n + j) + 1]);
+      }
     }
   };
   // eigenvalue of the 1D periodic Laplacian for integer frequency m on n points of spacing d
@@ -1020,7 +913,7 @@ mjx_status mjx_spec2d_plan_init(void* plan, const mjx_grid2d* g, int symbol, int
     return -k * k;
   };
   put_tw(pv.twx, nx);
-  if (twx_count(nx, e) != nx) {  // the transposed copy for the one-warp 1024-point transform
+  if (e == 4 && twx_count(nx, e) != nx) {  // the transposed copy for the one-warp 1024-point transform
     float* p = (float*)pv.twx;
     for (int k1 = 0; k1 < 32; ++k1)
       for (int l = 0; l < 32; ++l) {
@@ -1052,7 +945,7 @@ mjx_status mjx_spectral_apply2d(const void* plan, const mjx_grid2d* g, int dtype
   if ((mult < MJX_MULT_SCALE || mult > MJX_MULT_EXP) && mult != MJX_MULT_LAP) return MJX_BAD_ARG;
   const int e = elem_size(dtype);
   if (!e) return MJX_BAD_DTYPE;
-  if (ws == nullptr || ws_bytes < mjx_spec2d_ws_bytes(g->ny, g->nx, nfields, dtype)) return MJX_WORKSPACE;
+  if (ws == nullptr || ws_bytes < spec_bytes(g->ny, g->nx, nfields, e)) return MJX_WORKSPACE;
   MJX_TRY(ensure_kernel_attrs());
   cudaStream_t s = (cudaStream_t)stream;
   if (e == 4) return spectral_apply<float>(plan, g, nfields, D, h, mult, (const float*)in, (float*)out, ws, s);
@@ -1068,7 +961,7 @@ mjx_status mjx_advdiff_op2d(const void* plan, const mjx_grid2d* g, int dtype, in
     return MJX_BAD_ARG;
   const int e = elem_size(dtype);
   if (!e) return MJX_BAD_DTYPE;
-  if (ws == nullptr || ws_bytes < mjx_spec2d_ws_bytes(g->ny, g->nx, nfields, dtype)) return MJX_WORKSPACE;
+  if (ws == nullptr || ws_bytes < spec_bytes(g->ny, g->nx, nfields, e)) return MJX_WORKSPACE;
   MJX_TRY(ensure_kernel_attrs());
   cudaStream_t s = (cudaStream_t)stream;
   const int mul = op == 0 ? MUL_ADVDIFF : (op == 1 ? MUL_ADV_LAP : (op == 2 ? MUL_ADV_EXP : MUL_ADV_CN));
@@ -1085,7 +978,7 @@ mjx_status mjx_spectral_filter2d(const void* plan, const mjx_grid2d* g, int dtyp
     return MJX_BAD_ARG;
   const int e = elem_size(dtype);
   if (!e) return MJX_BAD_DTYPE;
-  if (ws == nullptr || ws_bytes < mjx_spec2d_ws_bytes(g->ny, g->nx, nfields, dtype)) return MJX_WORKSPACE;
+  if (ws == nullptr || ws_bytes < spec_bytes(g->ny, g->nx, nfields, e)) return MJX_WORKSPACE;
   MJX_TRY(ensure_kernel_attrs());
   cudaStream_t s = (cudaStream_t)stream;
   const double D[4] = {1.0, 1.0, 1.0, 1.0};
@@ -1105,7 +998,7 @@ mjx_status mjx_advdiff_apply2d(const void* plan, const mjx_grid2d* g, int dtype,
     return MJX_BAD_ARG;
   const int e = elem_size(dtype);
   if (!e) return MJX_BAD_DTYPE;
-  if (ws == nullptr || ws_bytes < mjx_spec2d_ws_bytes(g->ny, g->nx, nfields, dtype)) return MJX_WORKSPACE;
+  if (ws == nullptr || ws_bytes < spec_bytes(g->ny, g->nx, nfields, e)) return MJX_WORKSPACE;
   MJX_TRY(ensure_kernel_attrs());
   cudaStream_t s = (cudaStream_t)stream;
   if (e == 4)
@@ -1120,11 +1013,11 @@ mjx_status mjx_fft_cn2d(const void* plan, const mjx_grid2d* g, int dtype, double
   if (plan == nullptr || u_in == nullptr || u_out == nullptr || n_steps < 0) return MJX_BAD_ARG;
   const int e = elem_size(dtype);
   if (!e) return MJX_BAD_DTYPE;
-  if (ws == nullptr || ws_bytes < mjx_spec2d_ws_bytes(g->ny, g->nx, 1, dtype)) return MJX_WORKSPACE;
+  if (ws == nullptr || ws_bytes < spec_bytes(g->ny, g->nx, 1, e)) return MJX_WORKSPACE;
   MJX_TRY(ensure_kernel_attrs());
   cudaStream_t s = (cudaStream_t)stream;
-  if (e == 4) return fft_cn<float>(plan, g, D, dt, n_steps, (const float*)u_in, (float*)u_out, ws, s);
-  return fft_cn<double>(plan, g, D, dt, n_steps, (const double*)u_in, (double*)u_out, ws, s);
+  if (e == 4) return fft_cn<float>(plan, g, D, dt, n_steps, (const float*)u_in, (float*)u_out, ws, ws_bytes, s);
+  return fft_cn<double>(plan, g, D, dt, n_steps, (const double*)u_in, (double*)u_out, ws, ws_bytes, s);
 }
 
 // FFT-CN stepping for callers that cannot allocate device memory: the
@@ -1136,13 +1029,13 @@ mjx_status mjx_fft_cn2d_noalloc(const void* plan, const mjx_grid2d* g, int dtype
   const int e = elem_size(dtype);
   if (!e) return MJX_BAD_DTYPE;
   // the spectrum of one field must fit the fixed scratch
-  if (mjx_spec2d_ws_bytes(g->ny, g->nx, 1, dtype) > (size_t)MJX_NOALLOC_SCRATCH_BYTES) return MJX_WORKSPACE;
+  if (spec_bytes(g->ny, g->nx, 1, e) > (size_t)MJX_NOALLOC_SCRATCH_BYTES) return MJX_WORKSPACE;
   void* ws = nullptr;
   MJX_TRY(noalloc_scratch(&ws));  // first call on a device: symbol lookup (no allocation)
   MJX_TRY(ensure_kernel_attrs());
   cudaStream_t s = (cudaStream_t)stream;
-  if (e == 4) return fft_cn<float>(plan, g, D, dt, n_steps, (const float*)u_in, (float*)u_out, ws, s);
-  return fft_cn<double>(plan, g, D, dt, n_steps, (const double*)u_in, (double*)u_out, ws, s);
+  if (e == 4) return fft_cn<float>(plan, g, D, dt, n_steps, (const float*)u_in, (float*)u_out, ws, MJX_NOALLOC_SCRATCH_BYTES, s);
+  return fft_cn<double>(plan, g, D, dt, n_steps, (const double*)u_in, (double*)u_out, ws, MJX_NOALLOC_SCRATCH_BYTES, s);
 }
 
 }  // extern "C"

@@ -76,6 +76,59 @@ __device__ __forceinline__ void react_delta(T& a, T& b, T h, T F, T k, T r) {
   }
 }
 
+template <typename T, int RX>
+__device__ __forceinline__ void react_heun(T& a, T& b, T h, T F, T k, T r) {
+  if (RX == RX_GRAY_SCOTT) {
+    // moljax/core/stepping.py:402-415 with operators.py:655-667
+    const T uvv = a * b * b;
+    const T fu = -uvv + F * ((T)1 - a);
+    const T fv = uvv - (F + k) * b;
+    const T ua = a + h * fu, va = b + h * fv;
+    const T uvv2 = ua * va * va;
+    const T gu = -uvv2 + F * ((T)1 - ua);
+    const T gv = uvv2 - (F + k) * va;
+    const T hh = (T)0.5 * h;
+    a = a + hh * (fu + gu);
+    b = b + hh * (fv + gv);
+  } else if (RX == RX_FISHER) {
+    const T fa = r * a * ((T)1 - a), fb = r * b * ((T)1 - b);
+    const T ta = a + h * fa, tb = b + h * fb;
+    const T hh = (T)0.5 * h;
+    a = a + hh * (fa + r * ta * ((T)1 - ta));
+    b = b + hh * (fb + r * tb * ((T)1 - tb));
+  }
+}
+
+// Explicit Euler reaction step y + h N(y) (imex_euler_step, stepping.py:349-359).
+template <typename T, int RX>
+__device__ __forceinline__ void react_euler(T& a, T& b, T h, T F, T k, T r) {
+  if (RX == RX_GRAY_SCOTT) {
+    const T uvv = a * b * b;
+    const T fu = -uvv + F * ((T)1 - a);
+    const T fv = uvv - (F + k) * b;
+    a = a + h * fu;
+    b = b + h * fv;
+  } else if (RX == RX_FISHER) {
+    const T fa = r * a * ((T)1 - a), fb = r * b * ((T)1 - b);
+    a = a + h * fa;
+    b = b + h * fb;
+  }
+}
+
+// N(a, b): the reaction terms themselves (operators.py:655-667; Fisher-KPP r u (1-u))
+template <typename T, int RX>
+__device__ __forceinline__ void nonlin_terms(T& a, T& b, T F, T FK, T r) {
+  if (RX == RX_GRAY_SCOTT) {
+    const T uvv = a * b * b;
+    const T nu = -uvv + F * ((T)1 - a), nv = uvv - FK * b;
+    a = nu; b = nv;
+  } else if (RX == RX_FISHER) {
+    a = r * a * ((T)1 - a); b = r * b * ((T)1 - b);
+  } else {
+    a = (T)0; b = (T)0;
+  }
+}
+
 struct RowPair {
   long long ra, rb;    // real row offsets (elements) of rows a and b at y = 0
   long long sa, sb;    // spectrum offsets (complex elements) at ky = 0
@@ -101,6 +154,7 @@ template <typename T> struct RowArgs {
   double* partial;     // per-CTA error partial sums (ROW_ERRNORM)
   int* nonfinite;      // per-CTA non-finite flags (ROW_ERRNORM)
   const DevState* st;
+  int pdl;             // launched in a chain (launch_chain)
   RowPair pr[MJX_MAXPAIR];
 };
 
@@ -108,7 +162,8 @@ enum { MUL_SCALE = 0, MUL_HELMHOLTZ = 1, MUL_CN = 2, MUL_EXP = 3, MUL_ADVDIFF = 
        MUL_ADV_LAP = 6,   // h (D lam - i v.k): the advection-diffusion operator itself
        MUL_ADV_EXP = 7,   // exp(h (D lam - i v.k))
        MUL_TABLE = 8,     // a real multiplier per half-spectrum point (ColArgs::mtab)
-       MUL_ADV_CN = 9 };  // (1 + z/2)/(1 - z/2), z = h (D lam - i v.k): one Crank-Nicolson step
+       MUL_ADV_CN = 9,    // (1 + z/2)/(1 - z/2), z = h (D lam - i v.k): one Crank-Nicolson step
+       MUL_TABLED = 10 };  // FP64: the formed multiplier with its scale, at the job's offset in mtab
 
 struct ColJob {
   long long sin;         // spectrum offset of the input column block (ky=0, kx=0)
@@ -144,11 +199,82 @@ template <typename T> struct ColArgs {
   // the negated mirror -row(ny-1-ky) and only rows ky < ny/2 are written back (the
   // cell-centred odd extension of a Dirichlet DST-II solve)
   int oddy;
+  int pdl;               // launched in a chain (launch_chain)
   ColJob job[MJX_MAXJOB];
 };
 
+template <typename T>
+__device__ __forceinline__ T multiplier(int mul, T hD, T lam, int pw) {
+  T m;
+  if (mul == MUL_HELMHOLTZ) {
+    T den = (T)1 - hD * lam;  // moljax/core/fft_solvers.py:281-285
+    if (fabs(den) < (T)1e-14) den = (T)1e-14;
+    m = (T)1 / den;
+  } else if (mul == MUL_CN) {
+    const T x = (T)0.5 * hD * lam;
+    m = ((T)1 + x) / ((T)1 - x);
+  } else if (mul == MUL_EXP) {
+    m = exp(hD * lam);
+  } else if (mul == MUL_LAP) {
+    m = hD * lam;
+  } else {
+    m = (T)1;
+  }
+  return pw == 2 ? m * m : m;
+}
+
+// The complex multipliers of the advection forms at half-spectrum point (ky, kx).
+template <typename T>
+__device__ __forceinline__ double2 adv_multiplier(const ColArgs<T>& a, const ColJob& jb, double hD, double hh,
+                                                  double lam, int kx, int ky) {
+  // z = h (D lam - i (vx kx + vy ky)), kx, ky = 2 pi fftfreq (the Nyquist index
+  // negative); m = 1/(1 - z) with |1 - z| < 1e-14 -> 1e-14 (the solve of
+  // FFTAdvectionDiffusionPreconditioner, moljax/core/preconditioners.py:297-420, and of
+  // AdvectionDiffusionOperator, fft_operators.py:179-260), z itself (matvec) or exp(z)
+  // (exp_matvec), or the Crank-Nicolson factor (1 + z/2)/(1 - z/2) of the 1D advective
+  // FFT-CN (benchmarks/benchmark_solver_comparison.py:152-163).  The reference keeps
+  // real(ifft(.)); on the half spectrum that is the
+  // multiplier (m(k) + conj(m(-k)))/2, which equals m(k) except on the Nyquist lines,
+  // where fftfreq breaks the oddness of the advection term.
+  const int nxl = 2 * (a.ncols - 1), ny = a.ny;
+  const int mx = kx < nxl / 2 ? kx : kx - nxl, my = ky < ny / 2 ? ky : ky - ny;
+  const int nmx = mx == -nxl / 2 ? mx : -mx, nmy = my == -ny / 2 ? my : -my;
+    const double zr = hD * lam;
+  double mre = 0.0, mim = 0.0;
+  for (int side = 0; side < 2; ++side) {
+    const int qx = side ? nmx : mx, qy = side ? nmy : my;
+    const double zi = -hh * (jb.vx * a.kxs * qx + jb.vy * a.kys * qy);
+    double fr, fi;
+    if (jb.mul == MUL_ADVDIFF) {
+      double dr = 1.0 - zr, di = -zi;
+      if (sqrt(dr * dr + di * di) < 1e-14) { dr = 1e-14; di = 0.0; }
+      const double den = dr * dr + di * di;
+      fr = dr / den;
+      fi = -di / den;
+    } else if (jb.mul == MUL_ADV_LAP) {
+      fr = zr;
+      fi = zi;
+    } else if (jb.mul == MUL_ADV_CN) {
+      const double nr = 1.0 + 0.5 * zr, ni = 0.5 * zi, dr = 1.0 - 0.5 * zr, di = -0.5 * zi;
+      const double den = dr * dr + di * di;
+      fr = (nr * dr + ni * di) / den;
+      fi = (ni * dr - nr * di) / den;
+    } else {
+      double sn, cs;
+      sincos(zi, &sn, &cs);
+      const double ez = exp(zr);
+      fr = ez * cs;
+      fi = ez * sn;
+    }
+    mre += 0.5 * fr;
+    mim += side ? -0.5 * fi : 0.5 * fi;  // conj(m(-k)) on the second side
+  }
+  return make_double2(mre, mim);
+}
+
 // Plan layout (device bytes): twx[nx] twy[ny] lamx[ldc] lamy[ny], 256-byte aligned parts;
-// FP32 plans of 1024-point rows hold 2048 x twiddles (the second half transposed, wfft.cuh).
+// FP32 plans of 1024-point rows hold 2048 x twiddles (the second half transposed, wfft.cuh);
+// FP64 plans hold each twiddle table twice, the second in the (cos, tan) form of tfft.cuh.
 struct PlanView {
   const void* twx; const void* twy; const void* lamx; const void* lamy;
 };
@@ -160,6 +286,16 @@ template <typename T, int RX>
 cudaError_t launch_row(const RowArgs<T>& a, cudaStream_t s);
 template <typename T>
 cudaError_t launch_col(const ColArgs<T>& a, cudaStream_t s);
+
+// FP64 passes of spectral64.cu (launch_row / launch_col go there for the lengths they take)
+bool row64_takes(int n);
+bool col64_takes(int ny);
+template <int RX> cudaError_t launch_row64(const RowArgs<double>& a, cudaStream_t s);
+cudaError_t launch_col64(const ColArgs<double>& a, cudaStream_t s);
+mjx_status spectral64_attrs(int optin);
+// forms the multipliers of a's jobs in tab (as many doubles as the spectra have entries) and
+// makes the jobs read them
+cudaError_t tabulate_cols(ColArgs<double>& a, double* tab, cudaStream_t s);
 
 // Arguments of the adaptive controller kernel (csrc/imex.cu).
 struct CtlGain {

@@ -3,7 +3,7 @@
 // benchmarks/sisc/bench_3d_feasibility.py:71-87 (cn_step_3d inside a fori_loop).
 //
 // Layout: real u[nz][ny][nx]; half spectrum S[nz][ny][ldc] (ldc = spec_ldc(nx)).
-// One application is five passes over HBM:
+// One application is five passes over HBM, several in a row four each (X' and the next X fused):
 //   X   r2c of every (z, y) row (rows r and r + nz*ny/2 share one complex FFT)
 //   Y   forward FFT along y, one plane per gridDim.z
 //   Z   forward FFT along z -> m(lamx + lamy + lamz) / (nx ny nz) -> inverse FFT along z;
@@ -36,7 +36,7 @@ static mjx_status check_grid3(const mjx_grid3d* g) {
 
 template <typename T>
 static mjx_status apply3d(const void* plan, const mjx_grid3d* g, double D, double h, int mult, int n_steps,
-                          const T* in, T* out, void* ws, cudaStream_t s) {
+                          const T* in, T* out, void* ws, size_t ws_bytes, cudaStream_t s) {
   const int nx = g->nx, ny = g->ny, nz = g->nz, ldc = spec_ldc(nx);
   const PlanView pa = plan_view(plan, ny, nx, sizeof(T));
   const PlanView pz = plan_view((const char*)plan + al256(plan_bytes(ny, nx, sizeof(T))), nz, nx, sizeof(T));
@@ -78,38 +78,25 @@ static mjx_status apply3d(const void* plan, const mjx_grid3d* g, double D, doubl
   cz.job[0].nout = 1; cz.job[0].mul = mult; cz.job[0].D = D; cz.job[0].hfac[0] = 1.0; cz.job[0].pow[0] = 1;
   cz.job[0].dirs = 3;
 
-  auto one = [&](const RowArgs<T>& first, cudaStream_t st) -> cudaError_t {
+  // A step is Y, Z, Y' and one row pass: the rows of a step that is not the last go from
+  // spectrum to spectrum (c2r, then r2c without storing the real box).  FP64 steps read their
+  // z-pass multipliers from a table formed once.
+  if constexpr (sizeof(T) == 8) {
+    const size_t sb = (size_t)nz * plane * 16;
+    if (n_steps > 1 && ws_bytes >= sb + sb / 2) MJX_CUDA_TRY(tabulate_cols(cz, (double*)ws + sb / 8, s));
+  }
+  RowArgs<T> rr = rb;
+  rr.pr[0].flags = ROW_LOAD_SPEC | ROW_STORE_SPEC;
+  rr.pdl = rb.pdl = cyf.pdl = cz.pdl = cyb.pdl = 1;
+  auto one = [&](bool last, cudaStream_t st) -> cudaError_t {
     cudaError_t e;
-    if ((e = launch_row<T, RX_NONE>(first, st)) != cudaSuccess) return e;
     if ((e = launch_col<T>(cyf, st)) != cudaSuccess) return e;
     if ((e = launch_col<T>(cz, st)) != cudaSuccess) return e;
     if ((e = launch_col<T>(cyb, st)) != cudaSuccess) return e;
-    return launch_row<T, RX_NONE>(rb, st);
+    return launch_row<T, RX_NONE>(last ? rb : rr, st);
   };
-  MJX_CUDA_TRY(one(rf, s));
-  if (n_steps > 1) {
-    // later applications read the previous output: captured once, replayed
-    RowArgs<T> rf2 = rf;
-    rf2.rin[0] = out;
-    cudaStream_t cs = nullptr;
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
-    cudaError_t ce = cudaSuccess;
-    do {
-      if ((ce = cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking)) != cudaSuccess) break;
-      if ((ce = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal)) != cudaSuccess) break;
-      const cudaError_t le = one(rf2, cs);
-      ce = cudaStreamEndCapture(cs, &graph);
-      if (le != cudaSuccess) { ce = le; break; }
-      if (ce != cudaSuccess) break;
-      if ((ce = cudaGraphInstantiate(&exec, graph, 0)) != cudaSuccess) break;
-      for (int i = 1; i < n_steps && ce == cudaSuccess; ++i) ce = cudaGraphLaunch(exec, s);
-    } while (0);
-    if (exec) cudaGraphExecDestroy(exec);
-    if (graph) cudaGraphDestroy(graph);
-    if (cs) cudaStreamDestroy(cs);
-    if (ce != cudaSuccess) { set_last_error(ce, __FILE__, __LINE__); return MJX_CUDA_ERROR; }
-  }
+  MJX_CUDA_TRY((launch_row<T, RX_NONE>(rf, s)));
+  for (int i = 0; i < n_steps; ++i) MJX_CUDA_TRY(one(i == n_steps - 1, s));
   return MJX_OK;
 }
 
@@ -139,7 +126,8 @@ mjx_status mjx_spec3d_plan_init(void* plan, const mjx_grid3d* g, int symbol, int
 size_t mjx_spec3d_ws_bytes(int nz, int ny, int nx, int dtype) {
   const int e = elem_size(dtype);
   if (!e || ilog2_exact(nx) < 1 || ilog2_exact(ny) < 1 || ilog2_exact(nz) < 1) return 0;
-  return (size_t)nz * ny * spec_ldc(nx) * 2 * e;
+  const size_t sb = (size_t)nz * ny * spec_ldc(nx) * 2 * e;
+  return e == 8 ? sb + sb / 2 : sb;
 }
 
 mjx_status mjx_spectral_apply3d(const void* plan, const mjx_grid3d* g, int dtype, double D, double h, int mult,
@@ -150,12 +138,12 @@ mjx_status mjx_spectral_apply3d(const void* plan, const mjx_grid3d* g, int dtype
   if (!e) return MJX_BAD_DTYPE;
   if (!plan || !in || !out || n_steps < 1) return MJX_BAD_ARG;
   if ((mult < MJX_MULT_SCALE || mult > MJX_MULT_EXP) && mult != MJX_MULT_LAP) return MJX_BAD_ARG;
-  if (!ws || ws_bytes < mjx_spec3d_ws_bytes(g->nz, g->ny, g->nx, dtype)) return MJX_WORKSPACE;
+  if (!ws || ws_bytes < (size_t)g->nz * g->ny * spec_ldc(g->nx) * 2 * e) return MJX_WORKSPACE;
   MJX_TRY(ensure_kernel_attrs());
   cudaStream_t s = (cudaStream_t)stream;
   if (e == 4)
-    return apply3d<float>(plan, g, D, h, mult, n_steps, (const float*)in, (float*)out, ws, s);
-  return apply3d<double>(plan, g, D, h, mult, n_steps, (const double*)in, (double*)out, ws, s);
+    return apply3d<float>(plan, g, D, h, mult, n_steps, (const float*)in, (float*)out, ws, ws_bytes, s);
+  return apply3d<double>(plan, g, D, h, mult, n_steps, (const double*)in, (double*)out, ws, ws_bytes, s);
 }
 
 }  // extern "C"

@@ -151,38 +151,85 @@ __device__ __forceinline__ void tile_bf(cx<T>* v, const cx<T>* tw, int i, int ne
 __device__ __forceinline__ int fdiv(int a, float rb) { return (int)(((float)a + 0.5f) * rb); }
 
 // One pass: butterfly j (k = j mod p) of each sequence from src[j + t n/R] to
-// dst[(j - k) R + k + t p], after the twiddles w^(k t), w = exp(-2 pi i / (p R)).
+// dst[(j - k) R + k + t p], after the twiddles w^(k t), w = exp(-2 pi i / (p R)).  A stride that
+// is a multiple of 16 points keeps the padding's phase, so the R addresses are one base and
+// multiples of a constant; on small tiles, with a warp or two on each sub-partition, the index
+// arithmetic is as long as the FP64 arithmetic.
+template <typename T, int R>
+__device__ __forceinline__ void tile_load(cx<T>* v, const cx<T>* src, int i, int stride) {
+  if ((stride & 15) == 0) {
+    const cx<T>* q = src + sp(i);
+    const int d = sp(stride);
+#pragma unroll
+    for (int t = 0; t < R; ++t) v[t] = q[t * d];
+  } else {
+#pragma unroll
+    for (int t = 0; t < R; ++t) v[t] = src[sp(i + t * stride)];
+  }
+}
+template <typename T, int R>
+__device__ __forceinline__ void tile_store(const cx<T>* v, cx<T>* dst, int i, int stride) {
+  if ((stride & 15) == 0) {
+    cx<T>* q = dst + sp(i);
+    const int d = sp(stride);
+#pragma unroll
+    for (int t = 0; t < R; ++t) q[t * d] = v[t];
+  } else {
+#pragma unroll
+    for (int t = 0; t < R; ++t) dst[sp(i + t * stride)] = v[t];
+  }
+}
+
 template <typename T, int R>
 __device__ __forceinline__ void tile_pass(const cx<T>* src, cx<T>* dst, int n, int p, int lS, const cx<T>* tw,
                                           int tid, int nth) {
   typedef cx<T> C;
   const int nb = n / R, items = nb << lS, S1 = (1 << lS) - 1;
   if (p == 1) {
+#pragma unroll 1
     for (int i = tid; i < items; i += nth) {
-      const int s = i & S1, j = i >> lS;
+      const int s = i & S1;
       C v[R];
-#pragma unroll
-      for (int t = 0; t < R; ++t) v[t] = src[sp(i + ((t * nb) << lS))];
+      tile_load<T, R>(v, src, i, items);
       tile_bf<T, R, true>(v, tw, 0, 0);
-#pragma unroll
-      for (int t = 0; t < R; ++t) dst[sp(((j * R + t) << lS) + s)] = v[t];
+      tile_store<T, R>(v, dst, (i - s) * R + s, 1 << lS);
     }
   } else {
-    const int step = nb / p;
+    const int step = nb / p, pS = p << lS;
     const bool p2 = (p & (p - 1)) == 0;
-    const int lp = __ffs(p) - 1;
     const float rp = 1.0f / (float)p;
+#pragma unroll 1
     for (int i = tid; i < items; i += nth) {
-      const int s = i & S1, j = i >> lS;
-      const int q = p2 ? j >> lp : fdiv(j, rp), k = j - q * p;
+      // ks = k 2^lS + s: the place within the block of p butterflies of every sequence
+      const int ks = p2 ? i & (pS - 1) : i - fdiv(i >> lS, rp) * pS, k = ks >> lS;
       C v[R];
-#pragma unroll
-      for (int t = 0; t < R; ++t) v[t] = src[sp(i + ((t * nb) << lS))];
+      tile_load<T, R>(v, src, i, items);
       tile_bf<T, R, false>(v, tw, k * step, n >> 3);
-      const int base = q * p * R + k;
-#pragma unroll
-      for (int t = 0; t < R; ++t) dst[sp(((base + t * p) << lS) + s)] = v[t];
+      tile_store<T, R>(v, dst, (i - ks) * R + ks, pS);
     }
+  }
+  __syncthreads();
+}
+
+// A radix-2 FP64 pass with the two components of each butterfly on neighbouring lanes: each needs
+// one of the products u, v and two sums, so a tile of fewer than 128 butterflies fills twice the
+// warps with half the FP64 instructions each (a 128-point row: 128 lanes, three instructions).
+static __device__ __forceinline__ void tile_pass2_split(const double2* src, double2* dst, int n, int p, int lS,
+                                                 const double2* tw, int tid, int nth) {
+  const int items = (n >> 1) << lS, pS = p << lS, step = (n >> 1) / p;
+  const double* sr = reinterpret_cast<const double*>(src);
+  double* ds = reinterpret_cast<double*>(dst);
+#pragma unroll 1
+  for (int e = tid; e < 2 * items; e += nth) {
+    const int i = e >> 1, y = e & 1;
+    const int ks = (p & (p - 1)) == 0 ? i & (pS - 1) : i % pS;
+    const double2 w = tw[(ks >> lS) * step];
+    const double2 b = src[sp(i + items)];
+    const double a = sr[2 * sp(i) + y];
+    const double u = fma(w.y, y ? -b.x : b.y, y ? b.y : b.x);
+    const int o = (i - ks) * 2 + ks;
+    ds[2 * sp(o) + y] = fma(w.x, u, a);
+    ds[2 * sp(o + pS) + y] = fma(-w.x, u, a);
   }
   __syncthreads();
 }
@@ -192,16 +239,24 @@ __device__ __forceinline__ void tile_pass(const cx<T>* src, cx<T>* dst, int n, i
 // complete.  Radices are packed four bits each, the first pass lowest.  One copy of the code
 // per kernel: a kernel runs two to six transforms, and inlined copies cost more in instruction
 // fetches than the passes themselves on small tiles.
-template <typename T>
+// POW2: only the passes of powers of two (the less code, the fewer fetches).
+template <typename T, bool POW2>
 __device__ __noinline__ void tile_dft(cx<T>* cur, cx<T>* alt, int n, unsigned long long rad, int lS, const cx<T>* tw,
                                       int tid, int nth) {
   for (int p = 1; rad != 0; rad >>= 4) {
     const int r = (int)(rad & 15);
     if (r == 8) tile_pass<T, 8>(cur, alt, n, p, lS, tw, tid, nth);
     else if (r == 4) tile_pass<T, 4>(cur, alt, n, p, lS, tw, tid, nth);
-    else if (r == 5) tile_pass<T, 5>(cur, alt, n, p, lS, tw, tid, nth);
-    else if (r == 3) tile_pass<T, 3>(cur, alt, n, p, lS, tw, tid, nth);
-    else tile_pass<T, 2>(cur, alt, n, p, lS, tw, tid, nth);
+    else if (!POW2 && r == 5) tile_pass<T, 5>(cur, alt, n, p, lS, tw, tid, nth);
+    else if (!POW2 && r == 3) tile_pass<T, 3>(cur, alt, n, p, lS, tw, tid, nth);
+    else {
+      bool split = false;
+      if constexpr (sizeof(T) == 8) {
+        split = (n >> 1) << lS < 128;
+        if (split) tile_pass2_split(cur, alt, n, p, lS, tw, tid, nth);
+      }
+      if (!split) tile_pass<T, 2>(cur, alt, n, p, lS, tw, tid, nth);
+    }
     cx<T>* t = cur;
     cur = alt;
     alt = t;
@@ -289,13 +344,13 @@ __device__ __forceinline__ void dft_tile(const Dft<T>& d, Tile<T>& t) {
     }
     __syncthreads();
   }
-  tile_dft<T>(t.cur, t.alt, L, d.rad, lS, t.tw, t.tid, t.nth);
+  tile_dft<T, false>(t.cur, t.alt, L, d.rad, lS, t.tw, t.tid, t.nth);
   if (d.odd) { C* x = t.cur; t.cur = t.alt; t.alt = x; }
   if (!d.bluestein) return;
   // the inverse transform of the product by conjugation
   for (int e = t.tid; e < (L << lS); e += t.nth) t.cur[sp(e)] = cconj(cmul(t.cur[sp(e)], t.bhat[e >> lS]));
   __syncthreads();
-  tile_dft<T>(t.cur, t.alt, L, d.rad, lS, t.tw, t.tid, t.nth);
+  tile_dft<T, false>(t.cur, t.alt, L, d.rad, lS, t.tw, t.tid, t.nth);
   if (d.odd) { C* x = t.cur; t.cur = t.alt; t.alt = x; }
   for (int e = t.tid; e < (n << lS); e += t.nth) t.cur[sp(e)] = cmul(cconj(t.cur[sp(e)]), t.chirp[e >> lS]);
   __syncthreads();

@@ -117,3 +117,37 @@ def test_solver_comparison_1d_published(cuda):
     assert float(np.max(np.abs(w - fftcn.fft_cn_1d(w0, D, 1.0 / m, 1e-3, 200, "spectral", v=v)))) < 1e-12
     w = M.imex_advdiff_1d(torch.tensor(w0, device=cuda), D, v, 1.0 / m, 5e-3, 100).cpu().numpy()
     assert float(np.max(np.abs(w - fftcn.strang_exp_1d(w0, D, v, 1.0 / m, 5e-3, 100)))) < 1e-12
+
+
+@pytest.mark.parametrize("shape", [(2, 2), (2, 16), (4, 8), (16, 2), (64, 64), (128, 256), (1024, 4), (2048, 16), (8, 2048),
+                                   (4096, 4), (2, 4096)])
+def test_fp64_passes_at_tile_edges(cuda, shape):
+    """The FP64 row and column passes at the edges of their tiles (one to 32 sequences, radix 2, 4
+    and 8, single sequences of 2048, and 4096 on the FP32-style passes), one step against several
+    in a row (fused rows, tabulated multipliers), with a workspace that holds only the spectra, and
+    two-output column passes (an IMEX attempt), against NumPy FFTs."""
+    import ctypes as C
+    from moljax_gb300 import _native as N
+    from moljax_gb300.core.fft_solvers import get_plan
+    ny, nx = shape
+    rng = np.random.default_rng(ny + 3 * nx)
+    u = rng.standard_normal((ny, nx))
+    dy, dx, D, dt = 1.0 / ny, 1.0 / nx, 0.1, 1e-4
+    ky, kx = 2 * np.pi * np.fft.fftfreq(ny, dy), 2 * np.pi * np.fft.fftfreq(nx, dx)
+    x = -0.5 * dt * D * (ky[:, None] ** 2 + kx[None, :] ** 2)
+    plan = get_plan(ny, nx, dy, dx, "spectral", torch.float64, cuda)
+    ut = torch.tensor(u, device=cuda)
+    out = torch.empty_like(ut)
+    full = N.lib().mjx_spec2d_ws_bytes(ny, nx, 1, plan.code)
+    for steps in (1, 3):
+        ref = u
+        for _ in range(steps):
+            ref = np.real(np.fft.ifft2(np.fft.fft2(ref) * (1 + x) / (1 - x)))
+        for nbytes in (full, ny * ((nx // 2 + 1 + 3) // 4 * 4) * 16):
+            ws = torch.empty(nbytes, dtype=torch.uint8, device=cuda)
+            N.check("mjx_fft_cn2d", N.lib().mjx_fft_cn2d(
+                N.ptr(plan.buf), C.byref(plan.cgrid), plan.code, D, dt, steps, N.ptr(ut), N.ptr(out), N.ptr(ws),
+                ws.numel(), N.stream_ptr(cuda)))
+            assert float(np.max(np.abs(out.cpu().numpy() - ref))) < 1e-13 * max(1.0, float(np.max(np.abs(u))))
+    assert N.lib().mjx_fft_cn2d(N.ptr(plan.buf), C.byref(plan.cgrid), plan.code, D, dt, 1, N.ptr(ut), N.ptr(out),
+                                N.ptr(ws), ws.numel() - 16, N.stream_ptr(cuda)) == 10  # MJX_WORKSPACE
