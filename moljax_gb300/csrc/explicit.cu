@@ -1061,6 +1061,16 @@ struct XFused {
   T* out;
   int nst;     // 3: SSPRK3, 4: RK4 (the stage formulas are compiled in per method)
   int any_bc;  // some field is Dirichlet or Neumann
+  // adaptive attempts: the step of one branch, with dt and the current buffer from the device
+  // state (in / out of buffer `cur`, in2 / out2 of the other) and, for the last half step, the
+  // scaled error against the full step yf
+  const DevState* st;
+  const T* in2;
+  T* out2;
+  T hfac;
+  const T* yf;
+  double* partial;
+  int* nonfinite;
 };
 
 // periodic index: one add or subtract within a halo of the domain, a remainder beyond
@@ -1086,10 +1096,13 @@ __device__ __forceinline__ long long fcell_src(int gy, int gx, const XModel& m, 
   return -1;
 }
 
-template <typename T, int RX, int NF, int NST>
+// ERR: accumulate the scaled error of the output against yf (persistent blocks, so that the
+// partials stay few: the controller sums them with FP64 instructions).
+template <typename T, int RX, int NF, int NST, bool ERR>
 __global__ void __launch_bounds__(FTHREADS, (sizeof(T) * NF <= 8) ? 2 : 1)
 fused_step_kernel(const __grid_constant__ XFused<T> a) {
   extern __shared__ __align__(16) unsigned char fsm_raw[];
+  if (a.st != nullptr && a.st->done) return;
   T* sm = reinterpret_cast<T*>(fsm_raw);
   const XModel& m = a.m;
   const XCoef<T>& k = a.k;
@@ -1097,11 +1110,20 @@ fused_step_kernel(const __grid_constant__ XFused<T> a) {
   constexpr int NL = (RS + FTHREADS - 1) / FTHREADS;
   const int nf = m.nf, ny = m.ny, nx = m.nx, adv = m.advection;
   const long long per = (long long)ny * nx;
-  const int ntx = (nx + FTX - 1) / FTX;
-  const int ty = blockIdx.x / ntx, tx = blockIdx.x - ty * ntx;
-  const int X0 = tx * FTX - R, Y0 = ty * FTY - R;  // domain coordinates of region cell (0, 0)
+  const int ntx = (nx + FTX - 1) / FTX, ntiles = ntx * ((ny + FTY - 1) / FTY);
   const int tid = threadIdx.x;
-  const T h = k.hfixed;
+  const int cur = a.st != nullptr ? a.st->cur : 0;
+  const T* in = cur ? a.in2 : a.in;
+  T* out = cur ? a.out2 : a.out;
+  const T h = a.st != nullptr ? (T)a.st->dtc * a.hfac : k.hfixed;
+  T esum = (T)0;
+  int bad = 0;
+  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+  const int ty = tile / ntx, tx = tile - ty * ntx;
+  const int X0 = tx * FTX - R, Y0 = ty * FTY - R;  // domain coordinates of region cell (0, 0)
+  if (ERR) __syncthreads();  // the previous tile's last reads
+  // a region inside the domain needs no wrapping and has no ghosts (most tiles of a large grid)
+  const bool inside = X0 >= 0 && Y0 >= 0 && X0 + RW <= nx && Y0 + RH <= ny;
   const T idx2 = k.idx2, idy2 = k.idy2, idx = k.idx, idy = k.idy, vx = k.vx, vy = k.vy;
   const bool vxpos = k.vxpos != 0, vypos = k.vypos != 0;
   auto buf = [&](int b, int f) -> T* { return sm + (size_t)(b * NF + f) * RS; };
@@ -1117,9 +1139,13 @@ fused_step_kernel(const __grid_constant__ XFused<T> a) {
       for (int f = 0; f < NF; ++f) {
         v[j][f] = (T)0;
         if (f >= nf || i >= RS) continue;
+        if (inside) {
+          v[j][f] = in[f * per + (long long)(Y0 + ry) * nx + (X0 + rx)];
+          continue;
+        }
         int side;
         const long long si = fcell_src<T>(Y0 + ry, X0 + rx, m, m.kind[f], &side);
-        if (si >= 0) v[j][f] = a.in[f * per + si];
+        if (si >= 0) v[j][f] = in[f * per + si];
       }
     }
 #pragma unroll
@@ -1130,9 +1156,9 @@ fused_step_kernel(const __grid_constant__ XFused<T> a) {
 #pragma unroll
       for (int f = 0; f < NF; ++f) {
         if (f >= nf) break;
-        int side;
+        int side = -1;
         const int kind = m.kind[f];
-        (void)fcell_src<T>(Y0 + ry, X0 + rx, m, kind, &side);
+        if (!inside) (void)fcell_src<T>(Y0 + ry, X0 + rx, m, kind, &side);
         T x = v[j][f];
         if (side >= 0 && side < 4) x = xghost(x, kind, k.gv[f][side], side == 0 || side == 2);
         buf(0, f)[i] = x;
@@ -1250,10 +1276,18 @@ fused_step_kernel(const __grid_constant__ XFused<T> a) {
                                      : c13 * ys[q] + c23 * c[f][q] + h23 * Fv[f][q]);
         }
         if (o1b == FOUT) {
-          T* orow = a.out + f * per + (long long)gy * nx;
+          const long long ro = f * per + (long long)gy * nx;
           if (gy < ny) {
-            if (t0 && gx < nx) orow[gx] = o1[0];
-            if (t1 && gx + 1 < nx) orow[gx + 1] = o1[1];
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+              if (!(q ? t1 : t0) || gx + q >= nx) continue;
+              out[ro + gx + q] = o1[q];
+              if (ERR) {  // moljax/core/state.py:335-339
+                const T er = (o1[q] - a.yf[ro + gx + q]) / (k.atol + k.rtol * (o1[q] < (T)0 ? -o1[q] : o1[q]));
+                esum += er * er;
+                bad |= !isfinite(o1[q]);
+              }
+            }
           }
         } else {
           T2 w2;
@@ -1265,29 +1299,56 @@ fused_step_kernel(const __grid_constant__ XFused<T> a) {
     }
     if (s + 1 < NST) {
       __syncthreads();
-      if (a.any_bc) {  // the ghost ring of the new stage values
-        for (int i = tid; i < SW * SH; i += FTHREADS) {
-          const int sy = i / SW, sx = i - sy * SW;
-          const int ry = sy + lo, rx = sx + lo;
-          const int gy = Y0 + ry, gx = X0 + rx;
-          const bool iny = gy >= 0 && gy < ny, inx = gx >= 0 && gx < nx;
-          const bool gxr = iny && (gx == -1 || gx == nx), gyr = inx && (gy == -1 || gy == ny);
-          if (!gxr && !gyr) continue;
+      if (a.any_bc && !inside) {  // the ghost ring of the new stage values: two columns, two rows
+        for (int i = tid; i < 2 * (SW + SH); i += FTHREADS) {
+          const bool col = i < 2 * SH;
+          const int q = col ? i : i - 2 * SH, len = col ? SH : SW;
+          const bool second = q >= len;
+          const int along = (second ? q - len : q) + lo;
+          const int gy = col ? Y0 + along : (second ? ny : -1), gx = col ? (second ? nx : -1) : X0 + along;
+          const int ry = gy - Y0, rx = gx - X0;
+          // inside this stage's region, beside a domain cell
+          if (ry < lo || ry >= lo + SH || rx < lo || rx >= lo + SW) continue;
+          if (col ? (gy < 0 || gy >= ny) : (gx < 0 || gx >= nx)) continue;
           const int c0 = ry * RW + rx;
           // the adjacent domain cell lies one step inward, inside this stage's region
-          const int cin = gxr ? (gx < 0 ? c0 + 1 : c0 - 1) : (gy < 0 ? c0 + RW : c0 - RW);
+          const int cin = col ? (second ? c0 - 1 : c0 + 1) : (second ? c0 - RW : c0 + RW);
+          const int side = (col ? 0 : 2) + (second ? 1 : 0);
 #pragma unroll
           for (int f = 0; f < NF; ++f) {
             if (f >= nf) break;
             const int kind = m.kind[f];
             if (kind == MJX_BC_PERIODIC) continue;
             T* ob = buf(o1b, f);
-            ob[c0] = gxr ? xghost(ob[cin], kind, gx < 0 ? k.gv[f][0] : k.gv[f][1], gx < 0)
-                         : xghost(ob[cin], kind, gy < 0 ? k.gv[f][2] : k.gv[f][3], gy < 0);
+            ob[c0] = xghost(ob[cin], kind, k.gv[f][side], !second);
           }
         }
         __syncthreads();
       }
+    }
+  }
+  }  // tiles
+  if (ERR) {
+    __shared__ double red[FTHREADS / 32];
+    __shared__ int redb[FTHREADS / 32];
+    double esd = (double)esum;
+    for (int o = 16; o > 0; o >>= 1) {
+      esd += __shfl_xor_sync(0xffffffffu, esd, o);
+      bad |= __shfl_xor_sync(0xffffffffu, bad, o);
+    }
+    if ((tid & 31) == 0) { red[tid >> 5] = esd; redb[tid >> 5] = bad; }
+    __syncthreads();
+    if (tid == 0) {
+      double sum = 0.0, cc = 0.0;
+      int b = 0;
+      for (int w = 0; w < FTHREADS / 32; ++w) {  // Kahan
+        const double yv = red[w] - cc, tv = sum + yv;
+        cc = (tv - sum) - yv;
+        sum = tv;
+        b |= redb[w];
+      }
+      a.partial[blockIdx.x] = sum;
+      a.nonfinite[blockIdx.x] = b;
     }
   }
 }
@@ -1307,19 +1368,25 @@ static bool fused_ok(const XModel& m, int method) {
   return fused_smem<T>(method == 2 ? 4 : 3, nfa) <= 200 * 1024;
 }
 
-template <typename T, int RX, int NF, int NST>
+template <typename T, int RX, int NF, int NST, bool ERR = false>
 static cudaError_t launch_fused_t(const XFused<T>& f, size_t smem, unsigned blocks, cudaStream_t s) {
   // the dynamic shared-memory limit is a function attribute of the CUDA context: set it
   // once for each context this instantiation runs in
   static ContextOnce attr;
   cudaError_t e = cudaSuccess;
   const mjx_status st = attr.run([&]() -> mjx_status {
-    e = cudaFuncSetAttribute(fused_step_kernel<T, RX, NF, NST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = cudaFuncSetAttribute(fused_step_kernel<T, RX, NF, NST, ERR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     return e == cudaSuccess ? MJX_OK : MJX_CUDA_ERROR;
   });
   if (st != MJX_OK) return e != cudaSuccess ? e : cudaErrorDeviceUninitialized;
-  fused_step_kernel<T, RX, NF, NST><<<blocks, FTHREADS, smem, s>>>(f);
+  fused_step_kernel<T, RX, NF, NST, ERR><<<blocks, FTHREADS, smem, s>>>(f);
   return cudaGetLastError();
+}
+
+// blocks (= partials) of the fused error pass
+static int fused_err_blocks(const XModel& m) {
+  const int tiles = ((m.nx + FTX - 1) / FTX) * ((m.ny + FTY - 1) / FTY);
+  return tiles < 304 ? tiles : 304;
 }
 
 template <typename T, int RX>
@@ -1327,6 +1394,13 @@ static cudaError_t launch_fused_rx(const XFused<T>& f, cudaStream_t s) {
   const int nfa = f.m.nf <= 2 ? 2 : 4;
   const size_t smem = fused_smem<T>(f.nst, nfa);
   const unsigned blocks = (unsigned)(((f.m.nx + FTX - 1) / FTX) * ((f.m.ny + FTY - 1) / FTY));
+  if constexpr (sizeof(T) == 4) {
+    if (f.yf != nullptr) {  // the error pass (two fields at most): two persistent blocks per SM
+      const unsigned eb = (unsigned)fused_err_blocks(f.m);
+      return f.nst == 4 ? launch_fused_t<T, RX, 2, 4, true>(f, smem, eb, s)
+                        : launch_fused_t<T, RX, 2, 3, true>(f, smem, eb, s);
+    }
+  }
   if constexpr (RX == RX_GRAY_SCOTT) {  // two fields only
     return f.nst == 4 ? launch_fused_t<T, RX, 2, 4>(f, smem, blocks, s) : launch_fused_t<T, RX, 2, 3>(f, smem, blocks, s);
   } else {
@@ -1433,12 +1507,37 @@ static mjx_status x_adaptive(const XModel& m, const mjx_explicit_problem* pb, co
   MJX_CUDA_TRY(cudaStreamSynchronize(s));  // the host copies above read host memory
 
   const XAttempt<T> A = build_x<T>(m, pb->method, ws, L, st, pid->atol, pid->rtol);
+  // SSPRK3 and RK4 of up to two FP32 fields take the three steps of an attempt (full, half, half
+  // with the error) as three fused kernels instead of 9 or 12 stage kernels: 24 B of memory
+  // traffic a point and field instead of 192 B for RK4.  Two fields, 1500 x 2000 with walls, an
+  // attempt: 12 x 20 us -> 3 x 69 us.  More fields leave one block per SM, FP64 is bound by its
+  // arithmetic, which the halo rings increase, and kinetics networks run in the stage kernels.
+  XFused<T> fs[3];
+  const bool fused = sizeof(T) == 4 && m.nf <= 2 && fused_ok<T>(m, pb->method);
+  if (fused) {
+    T* const YF = (T*)(ws + L.b[XB_YF]);
+    T* const YH = (T*)(ws + L.b[XB_YH]);
+    for (int q = 0; q < 3; ++q) {
+      fs[q] = make_fused<T>(m, pb->method, 0.0);
+      fs[q].st = st;
+      fs[q].hfac = (T)(q == 0 ? 1.0 : 0.5);
+      fs[q].k.atol = (T)pid->atol; fs[q].k.rtol = (T)pid->rtol;
+      fs[q].in = q < 2 ? Y0 : YH; fs[q].in2 = q < 2 ? Y1 : YH;
+      fs[q].out = q == 0 ? YF : (q == 1 ? YH : Y1); fs[q].out2 = q == 0 ? YF : (q == 1 ? YH : Y0);
+    }
+    fs[2].yf = YF;
+    fs[2].partial = (double*)(ws + L.part); fs[2].nonfinite = (int*)(ws + L.bad);
+  }
   CtlArgs ca;
   memset(&ca, 0, sizeof(ca));
   ca.st = st; ca.partial = (const double*)(ws + L.part); ca.nonfinite = (const int*)(ws + L.bad);
-  ca.nparts = XNPARTS; ca.gain = ctl_gain(*pid, h.order, (double)nelem); ca.pid = *pid; ca.hist_t = hist_t; ca.hist_dt = hist_dt;
+  ca.nparts = fused ? fused_err_blocks(m) : XNPARTS; ca.gain = ctl_gain(*pid, h.order, (double)nelem); ca.pid = *pid; ca.hist_t = hist_t; ca.hist_dt = hist_dt;
   auto body = [&](cudaStream_t ls) -> cudaError_t {
-    cudaError_t le = launch_x_attempt<T>(A, ls);
+    cudaError_t le = cudaSuccess;
+    if (fused)
+      for (int q = 0; q < 3 && le == cudaSuccess; ++q) le = launch_fused<T>(fs[q], ls);
+    else
+      le = launch_x_attempt<T>(A, ls);
     if (le == cudaSuccess) le = launch_controller(ca, ls);
     if (le == cudaSuccess && hist_y) {
       xhist_copy_kernel<T><<<304, 256, 0, ls>>>(st, Y0, Y1, hist_y, nelem);
