@@ -53,7 +53,7 @@ static Dst1Geom dst1_geom(int N, int elem, int kind = 0) {
   g.log2L = ilog2_exact(g.L);
   const size_t c = 2 * (size_t)elem;
   size_t o = 0;
-  g.tw = o; o += a256(g.L * c);
+  g.tw = o; o += a256((g.L + (elem == 4 ? fft_pass_entries(g.L) : 0)) * c);
   g.chirp = o; o += a256(g.M * c);
   g.bhat = o; o += a256(g.L * c);
   g.shift = o; o += kind == 0 ? 0 : a256(N * c);
@@ -591,6 +591,7 @@ static void trig_tables(std::vector<unsigned char>& host, const Dst1Geom& g, int
     tile_twiddle(j, g.L, e, &re, &im);
     put(g.tw, j, re, im);
   }
+  if (e == 4) fft_pass_table((float*)(host.data() + g.tw), g.L);
   if (g.bluestein) {
     // c[n] = exp(-i pi n^2 / M), with n^2 reduced mod 2M to keep the angle exact
     std::vector<double> cre(g.M), cim(g.M);

@@ -102,29 +102,50 @@ __device__ __forceinline__ void dft_r(C* x) {
   else dft16<INV>(x);
 }
 
-// Twiddle w^r (r = 1..R-1) for a butterfly whose base index is t (w^r = tw[r t]),
-// rebuilt from at most six table reads: w^(4a+b) = w^(4a) * w^b.
-template <typename T, int R, bool INV>
-__device__ __forceinline__ void apply_twiddles(cx<T>* x, int t, const cx<T>* __restrict__ tw) {
+// Twiddle w^r (r = 1..R-1) for butterfly k of a pass of sub-length p, rebuilt from at most six
+// table reads: w^(4a+b) = w^(4a) * w^b.  PT reads the pass's own table (fft_pass_table: entry
+// [slot][k], so that the lanes of a warp read one run per slot); otherwise w^r = tw[r k twstep]
+// of the length's plain table, whose strided reads take a memory wavefront for nearly every
+// lane (4096-point FP32 rows: 156 of a transform's 348 shared and L1 wavefronts a warp; their
+// fused pass of 4096 row pairs takes 125 us with the pass tables, 149 us without, the 2048-point
+// one 63 against 71 us).
+template <typename T, int R, bool INV, bool PT>
+__device__ __forceinline__ void apply_twiddles(cx<T>* x, int k, int p, int twstep, const cx<T>* __restrict__ tw) {
   typedef cx<T> C;
-  const C w1 = __ldg(&tw[t]);
+  const int t = k * twstep;
+  auto w = [&](int r) { return PT ? __ldg(&tw[(r < 4 ? r - 1 : 2 + r / 4) * p + k]) : __ldg(&tw[r * t]); };
+  const C w1 = w(1);
   if constexpr (R == 2) { x[1] = INV ? cmulc(x[1], w1) : cmul(x[1], w1); return; }
-  const C w2 = __ldg(&tw[2 * t]), w3 = __ldg(&tw[3 * t]);
   C wb[4];
-  wb[1] = w1; wb[2] = w2; wb[3] = w3;
+  wb[1] = w1; wb[2] = w(2); wb[3] = w(3);
 #pragma unroll
   for (int b = 1; b < 4; ++b) x[b] = INV ? cmulc(x[b], wb[b]) : cmul(x[b], wb[b]);
   if constexpr (R > 4) {
 #pragma unroll
   for (int a4 = 1; a4 < R / 4; ++a4) {
-    const C wa = __ldg(&tw[4 * a4 * t]);
+    const C wa = w(4 * a4);
     x[4 * a4] = INV ? cmulc(x[4 * a4], wa) : cmul(x[4 * a4], wa);
 #pragma unroll
     for (int b = 1; b < 4; ++b) {
-      const C w = cmul(wa, wb[b]);
-      x[4 * a4 + b] = INV ? cmulc(x[4 * a4 + b], w) : cmul(x[4 * a4 + b], w);
+      const C wr = cmul(wa, wb[b]);
+      x[4 * a4 + b] = INV ? cmulc(x[4 * a4 + b], wr) : cmul(x[4 * a4 + b], wr);
     }
   }
+  }
+}
+
+// The pass tables of a length-n FP32 transform follow the n entries of its plain table: for
+// the passes of sub-length p = 16 and 256 six slots of p entries, w^(r k) with r = 1, 2, 3, 4,
+// 8, 12 and w = exp(-2 pi i / (p R)).  A last pass of radix 2, 4 or 8 uses the first 1, 3 or 4.
+__host__ __device__ constexpr int fft_pass_entries(int n) { return n <= 16 ? 0 : (n <= 256 ? 96 : 96 + 1536); }
+// host: fills them (re, im interleaved) from the plain table that precedes them
+inline void fft_pass_table(float* tab, int n) {
+  const int rs[6] = {1, 2, 3, 4, 8, 12};
+  for (int p = 16, o = n; p < n; o += 6 * p, p *= 16) {
+    const int R = n / p >= 16 ? 16 : n / p, step = n / (p * R);
+    for (int i = 0; i < 6; ++i)
+      for (int k = 0; k < p && rs[i] < R; ++k)
+        for (int c = 0; c < 2; ++c) tab[2 * (o + i * p + k) + c] = tab[2 * (rs[i] * k * step) + c];
   }
 }
 
@@ -135,7 +156,11 @@ __device__ __forceinline__ int pmod(int a, int b) { return (b & (b - 1)) == 0 ? 
 
 // One Stockham pass of radix R with current sub-length p (p*R divides n).
 // Element j of this thread's sequence is buf[base + j * es]; ES1 fixes es = 1.
-template <typename T, int R, bool INV, bool ES1>
+// n, R, p, tps and es are powers of two, base < es or a multiple of n: the parts of an index
+// (sequence, butterfly, r) occupy disjoint bits, and sp() of their sum is the sum of their
+// sp().  So a thread forms one padded address per pass and adds offsets that are uniform over
+// the block (constants where n is one), instead of padding each of its 32 indices.
+template <typename T, int R, bool INV, bool ES1, bool PT>
 __device__ __forceinline__ void stockham_pass(cx<T>* buf, int n, int p, int tps, int lt, int base,
                                               int es_rt, bool active,
                                               const cx<T>* __restrict__ tw) {
@@ -146,12 +171,12 @@ __device__ __forceinline__ void stockham_pass(cx<T>* buf, int n, int p, int tps,
   constexpr int NBMAX = 16 / R;
   C x[16];
   if (active) {
+    const C* in = buf + sp(base + lt * es);
 #pragma unroll
     for (int m = 0; m < NBMAX; ++m) {
       if (m < nb) {
-        const int i = lt + m * tps;
 #pragma unroll
-        for (int r = 0; r < R; ++r) x[m * R + r] = buf[sp(base + (i + r * Tn) * es)];
+        for (int r = 0; r < R; ++r) x[m * R + r] = in[sp(m * tps * es) + sp(r * Tn * es)];
       }
     }
   }
@@ -163,11 +188,12 @@ __device__ __forceinline__ void stockham_pass(cx<T>* buf, int n, int p, int tps,
       if (m < nb) {
         const int i = lt + m * tps;
         const int k = i & (p - 1);
-        if (p > 1) apply_twiddles<T, R, INV>(&x[m * R], k * twstep, tw);
+        if (p > 1)
+          apply_twiddles<T, R, INV, PT>(&x[m * R], k, p, twstep, PT ? tw + n + (p == 16 ? 0 : 96) : tw);
         dft_r<R, INV>(&x[m * R]);
-        const int j = (i - k) * R + k;
+        C* out = buf + sp(base + ((i - k) * R + k) * es);
 #pragma unroll
-        for (int r = 0; r < R; ++r) buf[sp(base + (j + r * p) * es)] = x[m * R + r];
+        for (int r = 0; r < R; ++r) out[sp(r * p * es)] = x[m * R + r];
       }
     }
   }
@@ -177,7 +203,8 @@ __device__ __forceinline__ void stockham_pass(cx<T>* buf, int n, int p, int tps,
 // In-place FFT of nseq sequences (see file comment), sequences s0 .. s0 + nseq - 1.
 // All threads of the block must call it; threads with tid >= nseq*tps only join the
 // barriers.  The caller must __syncthreads() after filling buf; on return buf is complete.
-template <typename T, bool INV, bool COLMAJOR>
+// PT: tw is followed by the pass tables of fft_pass_table.
+template <typename T, bool INV, bool COLMAJOR, bool PT = (sizeof(T) == 4)>
 __device__ __forceinline__ void fft_smem_inl(cx<T>* buf, int n, int log2n, int nseq, int ss, int es,
                          const cx<T>* __restrict__ tw, int tid, int s0 = 0) {
   const int tps = n >= 16 ? pdiv(n, 16) : 1;
@@ -191,23 +218,23 @@ __device__ __forceinline__ void fft_smem_inl(cx<T>* buf, int n, int log2n, int n
 #pragma unroll
   for (int k16 = 0; k16 < 3; ++k16) {
     if (rem >= 4) {
-      stockham_pass<T, 16, INV, !COLMAJOR>(buf, n, p, tps, lt, base, es, active, tw);
+      stockham_pass<T, 16, INV, !COLMAJOR, PT>(buf, n, p, tps, lt, base, es, active, tw);
       p <<= 4;
       rem -= 4;
     }
   }
-  if (rem == 3) stockham_pass<T, 8, INV, !COLMAJOR>(buf, n, p, tps, lt, base, es, active, tw);
-  else if (rem == 2) stockham_pass<T, 4, INV, !COLMAJOR>(buf, n, p, tps, lt, base, es, active, tw);
-  else if (rem == 1) stockham_pass<T, 2, INV, !COLMAJOR>(buf, n, p, tps, lt, base, es, active, tw);
+  if (rem == 3) stockham_pass<T, 8, INV, !COLMAJOR, PT>(buf, n, p, tps, lt, base, es, active, tw);
+  else if (rem == 2) stockham_pass<T, 4, INV, !COLMAJOR, PT>(buf, n, p, tps, lt, base, es, active, tw);
+  else if (rem == 1) stockham_pass<T, 2, INV, !COLMAJOR, PT>(buf, n, p, tps, lt, base, es, active, tw);
 }
 
 
 // fft_smem_inl is always inlined, so that a caller passing compile-time lengths gets the
 // index arithmetic and the radix schedule folded; fft_smem leaves the choice to the compiler.
-template <typename T, bool INV, bool COLMAJOR>
+template <typename T, bool INV, bool COLMAJOR, bool PT = (sizeof(T) == 4)>
 __device__ void fft_smem(cx<T>* buf, int n, int log2n, int nseq, int ss, int es, const cx<T>* __restrict__ tw,
                          int tid, int s0 = 0) {
-  fft_smem_inl<T, INV, COLMAJOR>(buf, n, log2n, nseq, ss, es, tw, tid, s0);
+  fft_smem_inl<T, INV, COLMAJOR, PT>(buf, n, log2n, nseq, ss, es, tw, tid, s0);
 }
 
 // The same transform in radix-4 passes (a final radix-2 pass when log2 n is odd), n/4
@@ -226,9 +253,9 @@ __device__ void fft_smem_r4(cx<T>* buf, int n, int log2n, int nseq, int ss, int 
   const int base = (s + s0) * ss;
   int p = 1;
   for (int rem = log2n; rem >= 2; rem -= 2) {
-    stockham_pass<T, 4, INV, !COLMAJOR>(buf, n, p, tps, lt, base, es, active, tw);
+    stockham_pass<T, 4, INV, !COLMAJOR, false>(buf, n, p, tps, lt, base, es, active, tw);
     p <<= 2;
   }
-  if (log2n & 1) stockham_pass<T, 2, INV, !COLMAJOR>(buf, n, p, tps, lt, base, es, active, tw);
+  if (log2n & 1) stockham_pass<T, 2, INV, !COLMAJOR, false>(buf, n, p, tps, lt, base, es, active, tw);
 }
 }  // namespace mjx

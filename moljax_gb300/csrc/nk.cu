@@ -752,7 +752,7 @@ __device__ __forceinline__ int dst_tps(int n) { return R4 ? (n >= 4 ? n >> 2 : 1
 template <bool R4, bool INV, bool COLMAJOR>
 __device__ __forceinline__ void dst_fft(float2* buf, const NkaArgs& a, int nseq, int ss, int es, int tid) {
   if (R4) fft_smem_r4<float, INV, COLMAJOR>(buf, a.n, a.log2n, nseq, ss, es, a.twn, tid);
-  else fft_smem<float, INV, COLMAJOR>(buf, a.n, a.log2n, nseq, ss, es, a.twn, tid);
+  else fft_smem<float, INV, COLMAJOR, false>(buf, a.n, a.log2n, nseq, ss, es, a.twn, tid);
 }
 
 // forward DST-II along x of the row pairs (y, y + n/2) of a.src into a.S

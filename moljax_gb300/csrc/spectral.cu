@@ -21,12 +21,14 @@ static inline size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 int spec_ldc(int nx) { return ((nx / 2 + 1) + 3) & ~3; }
 
 // Entries of the x twiddle table: FP32 plans of 1024-point rows append the same 1024 values
-// transposed for the one-warp transform (entry 1024 + 32 k1 + l holds w^(l k1)), so that
+// transposed for the one-warp transform (entry kW1024 + 32 k1 + l holds w^(l k1)), so that
 // the 32 lanes of a warp read one contiguous 256-byte run per twiddle instead of 32 rows
 // of the table.
-static int twx_count(int nx, int elem) { return elem == 8 ? 2 * nx : (nx == 1024 ? 2048 : nx); }
+static int twx_count(int nx, int elem) {
+  return elem == 8 ? 2 * nx : nx + fft_pass_entries(nx) + (nx == 1024 ? 1024 : 0);
+}
 // FP64 tables are followed by their (cos, tan) form (tfft.cuh)
-static int twy_count(int ny, int elem) { return elem == 8 ? 2 * ny : ny; }
+static int twy_count(int ny, int elem) { return elem == 8 ? 2 * ny : ny + fft_pass_entries(ny); }
 
 size_t plan_bytes(int ny, int nx, int elem) {
   const size_t c = 2 * (size_t)elem;
@@ -905,6 +907,7 @@ mjx_status mjx_spec2d_plan_init(void* plan, const mjx_grid2d* g, int symbol, int
         tile_twiddle(j, n, 8, &p[2 * (n + j)], &p[2 * (n + j) + 1]);
       }
     }
+    if (e == 4) fft_pass_table((float*)dst, n);
   };
   // eigenvalue of the 1D periodic Laplacian for integer frequency m on n points of spacing d
   auto lam1 = [&](int m, int n, double d) {
@@ -913,12 +916,12 @@ mjx_status mjx_spec2d_plan_init(void* plan, const mjx_grid2d* g, int symbol, int
     return -k * k;
   };
   put_tw(pv.twx, nx);
-  if (e == 4 && twx_count(nx, e) != nx) {  // the transposed copy for the one-warp 1024-point transform
+  if (e == 4 && nx == 1024) {  // the transposed copy for the one-warp 1024-point transform
     float* p = (float*)pv.twx;
     for (int k1 = 0; k1 < 32; ++k1)
       for (int l = 0; l < 32; ++l) {
-        p[2 * (1024 + 32 * k1 + l)] = p[2 * (l * k1)];
-        p[2 * (1024 + 32 * k1 + l) + 1] = p[2 * (l * k1) + 1];
+        p[2 * (kW1024 + 32 * k1 + l)] = p[2 * (l * k1)];
+        p[2 * (kW1024 + 32 * k1 + l) + 1] = p[2 * (l * k1) + 1];
       }
   }
   put_tw(pv.twy, ny);

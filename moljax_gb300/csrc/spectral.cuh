@@ -273,7 +273,8 @@ __device__ __forceinline__ double2 adv_multiplier(const ColArgs<T>& a, const Col
 }
 
 // Plan layout (device bytes): twx[nx] twy[ny] lamx[ldc] lamy[ny], 256-byte aligned parts;
-// FP32 plans of 1024-point rows hold 2048 x twiddles (the second half transposed, wfft.cuh);
+// FP32 plans follow each twiddle table by its pass tables (fft.cuh), and that of 1024-point rows
+// by the 1024 twiddles transposed (wfft.cuh);
 // FP64 plans hold each twiddle table twice, the second in the (cos, tan) form of tfft.cuh.
 struct PlanView {
   const void* twx; const void* twy; const void* lamx; const void* lamy;

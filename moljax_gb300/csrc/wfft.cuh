@@ -46,14 +46,17 @@ __device__ __forceinline__ void dft32(float2 (&a)[32]) {
   }
 }
 
+// first entry of the transposed part: after the plain table and the pass tables
+constexpr int kW1024 = 1024 + fft_pass_entries(1024);
+
 template <bool INV>
 __device__ __forceinline__ void wfft1024(float2 (&z)[32], float2* tile, const float2* __restrict__ tw, int lane) {
   dft32<INV>(z);
   // w^(lane k1) from the transposed copy that FP32 plans of 1024-point rows append to
-  // their twiddle table (tw[1024 + 32 k1 + lane] == tw[lane k1]): one contiguous run per k1
+  // their twiddle table (tw[kW1024 + 32 k1 + lane] == tw[lane k1]): one contiguous run per k1
 #pragma unroll
   for (int k1 = 1; k1 < 32; ++k1) {
-    const float2 w = __ldg(&tw[1024 + 32 * k1 + lane]);
+    const float2 w = __ldg(&tw[kW1024 + 32 * k1 + lane]);
     z[k1] = INV ? cmulc(z[k1], w) : cmul(z[k1], w);
   }
 #pragma unroll

@@ -151,3 +151,20 @@ def test_fp64_passes_at_tile_edges(cuda, shape):
             assert float(np.max(np.abs(out.cpu().numpy() - ref))) < 1e-13 * max(1.0, float(np.max(np.abs(u))))
     assert N.lib().mjx_fft_cn2d(N.ptr(plan.buf), C.byref(plan.cgrid), plan.code, D, dt, 1, N.ptr(ut), N.ptr(out),
                                 N.ptr(ws), ws.numel() - 16, N.stream_ptr(cuda)) == 10  # MJX_WORKSPACE
+
+
+@pytest.mark.parametrize("n,m", [(8, 32), (64, 128), (128, 512), (256, 2048), (1024, 256), (2048, 1024)])
+def test_fp32_passes_each_last_radix(cuda, n, m):
+    """FP32 row and column transforms of every length class of the pass tables (no second pass, a
+    last pass of radix 2, 4, 8 or 16 at sub-length 16 or 256), both ways round,
+    against the FP64 oracle.  Tolerance: 1.2e-7 a radix-2 level and direction, 24 levels at
+    most, rounded up; a misplaced twiddle gives an error of order one."""
+    from moljax_gb300.core import fft_solvers
+    rng = np.random.default_rng(n + 5 * m)
+    for ny, nx in ((n, m), (m, n)):
+        plan = fft_solvers.get_plan(ny, nx, 1.0 / ny, 1.0 / nx, "fd", torch.float32, cuda)
+        rhs = rng.standard_normal((2, ny, nx))
+        out = plan.apply(torch.tensor(rhs, dtype=torch.float32, device=cuda), [1e-4, 2e-4], 0.5, 1).cpu().numpy()
+        lam = mol.fd_symbol_2d(ny, nx, 1.0 / ny, 1.0 / nx)
+        for f in range(2):
+            assert _rel(out[f], mol.solve_helmholtz_2d(rhs[f], lam, 0.5, [1e-4, 2e-4][f])) < 3e-6
