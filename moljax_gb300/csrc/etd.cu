@@ -82,19 +82,21 @@ __device__ __forceinline__ double phi3_ref(double z) {
 
 enum { FORM_CONTOUR_RK4 = 0, FORM_PHI_RK4 = 1, FORM_PHI_ETD12 = 2 };
 
-// tab layout: [field][coef 0..5][ky][ldc]
+// tab layout: [field][coef 0..5], ny * ldc entries each, of which the rows ky = 0 .. ny/2 are
+// filled (the symbol is even in ky), in the tile order of the column passes (EArgs)
 //   RK4 forms: E, E2, Q, f1, f2, f3;   ETD1/ETD2: E, dt phi1, dt phi2
 // xonly: the symbol has no y part (each row an independent 1D problem).
 template <typename T>
 __global__ void etd_coeff_kernel(T* tab, int ny, int nx, int ldc, int symbol, int xonly, double dy,
                                  double dx, double D0, double D1, int nf, double dt, int M,
-                                 double f2_factor, int form) {
-  const long long per = (long long)ny * ldc;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < per * nf;
+                                 double f2_factor, int form, int tile) {
+  const long long per = (long long)ny * ldc, cnt = (long long)(ny / 2 + 1) * ldc;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < cnt * nf;
        i += (long long)gridDim.x * blockDim.x) {
-    const int f = (int)(i / per);
-    const long long r = i - f * per;
-    const int ky = (int)(r / ldc), kx = (int)(r - (long long)ky * ldc);
+    const int f = (int)(i / cnt);
+    const int ky = (int)((i - f * cnt) / ldc), kx = (int)(i - f * cnt - (long long)ky * ldc);
+    const int t0 = kx & ~(tile - 1), tw = min(tile, ldc - t0);
+    const long long r = (long long)t0 * (ny / 2 + 1) + (long long)ky * tw + (kx - t0);
     const int my = xonly ? 0 : (ky < ny / 2 ? ky : ky - ny);
     double lam;
     if (kx > nx / 2) {
@@ -153,6 +155,12 @@ __global__ void etd_coeff_kernel(T* tab, int ny, int nx, int ldc, int symbol, in
 // ------------------------------------------------------------------ stage column pass
 enum { E0 = 0, E1 = 1, E2S = 2, E3 = 3, E4 = 4, E5 = 5, E6 = 6, E7 = 7 };  // E5 ETD1, E6 ETD1 + keep N^, E7 ETD2
 
+// The row spectra zu, zn, zx are row-major, as the row passes want them.  The full spectra uh,
+// nu, ah, ss and the coefficient tables are touched by the column passes alone and lie in their
+// tile order: tile of `tile` columns after tile, [ky][column] inside (the last tile is as wide as
+// ldc leaves it), so that a CTA's operands are one contiguous run each.  Row-major, a CTA of four
+// FP32 columns reads 32-byte pieces, and L2 answers half a request's worth a lookup (the
+// stages of 4096^2 FP32: 283 to 382 us row-major, 241 to 280 us tiled).
 template <typename T> struct EArgs {
   int ny, log2ny, ncols, ldc, C, njobs;
   cx<T>* zu; cx<T>* zn; cx<T>* zx;
@@ -162,7 +170,7 @@ template <typename T> struct EArgs {
   const cx<T>* tw;
   T scale;
   int type;
-  int pad;
+  int tile;
 };
 
 // One CTA: C adjacent kx columns of one field (E1 transforms two inputs per column).
@@ -171,125 +179,169 @@ template <typename T> struct EArgs {
 // FP64 keeps 512 threads (its butterflies need the registers).
 template <typename T> struct EThreads { static constexpr int v = sizeof(T) == 4 ? 1024 : 512; };
 
+// A full spectrum's or table's share of one column tile (EArgs).
+template <typename T> struct ETile {
+  int wt, ny;       // row pitch of the tile, rows
+  long long go;     // first element of the CTA's columns in a full spectrum
+  int to;           // and in a coefficient table
+  __device__ __forceinline__ ETile(const EArgs<T>& a, int f, int kx0) : ny(a.ny) {
+    const int t0 = kx0 & ~(a.tile - 1);
+    wt = min(a.tile, a.ldc - t0);
+    go = (long long)f * a.fs + (long long)t0 * ny + (kx0 - t0);
+    to = t0 * (ny / 2 + 1) + (kx0 - t0);
+  }
+};
+
+// Operands and coefficients of one element of a stage.
+template <typename T, int TYPE> struct EOper {
+  cx<T> u, nu, s3;
+  T c0, c1, c2, c3;
+  __device__ __forceinline__ void load(const EArgs<T>& a, const T* tab, long long g, int tg) {
+    const long long per = a.fs;
+    if (TYPE == E1 || TYPE == E2S) {
+      c0 = tab[per + tg]; c1 = tab[2 * per + tg];
+      u = a.uh[g];
+    } else if (TYPE == E3) {  // u = a^, nu = N^u, s3 = S
+      c0 = tab[per + tg]; c1 = tab[2 * per + tg];
+      u = a.ah[g]; nu = a.nu[g]; s3 = a.ss[g];
+    } else if (TYPE == E4) {  // c0 = E, c1 = f1, c2 = f2, c3 = f3
+      c0 = tab[tg]; c1 = tab[3 * per + tg]; c2 = tab[4 * per + tg]; c3 = tab[5 * per + tg];
+      u = a.uh[g]; nu = a.nu[g]; s3 = a.ss[g];
+    } else if (TYPE >= E5) {  // c0 = E, c1 = phi1, c2 = phi2
+      c0 = tab[tg]; c1 = tab[per + tg];
+      u = a.uh[g];
+      if (TYPE == E7) { c2 = tab[2 * per + tg]; nu = a.nu[g]; }
+    }
+  }
+  // the stage's output for the transformed element xv, its side results stored
+  __device__ __forceinline__ cx<T> apply(const EArgs<T>& a, long long g, cx<T> xv) const {
+    typedef cx<T> Cx;
+    Cx out = xv;
+    if (TYPE == E0) {  // the initial U^ (later steps get it from E4)
+      a.uh[g] = xv;
+    } else if (TYPE == E1) {
+      a.nu[g] = xv;
+      out = mk<Cx>(c0 * u.x + c1 * xv.x, c0 * u.y + c1 * xv.y);
+      a.ah[g] = out;
+    } else if (TYPE == E2S) {
+      a.ss[g] = xv;
+      out = mk<Cx>(c0 * u.x + c1 * xv.x, c0 * u.y + c1 * xv.y);
+    } else if (TYPE == E3) {
+      a.ss[g] = cadd(s3, xv);
+      out = mk<Cx>(c0 * u.x + c1 * ((T)2 * xv.x - nu.x), c0 * u.y + c1 * ((T)2 * xv.y - nu.y));
+    } else if (TYPE >= E5) {
+      // ETD1 (fft_integrators.py:165-166) / ETD2 (234-236)
+      T ox = c0 * u.x + c1 * xv.x, oy = c0 * u.y + c1 * xv.y;
+      if (TYPE == E7) {
+        ox += c2 * (xv.x - nu.x);
+        oy += c2 * (xv.y - nu.y);
+      }
+      if (TYPE != E5) a.nu[g] = xv;
+      out = mk<Cx>(ox, oy);
+      a.uh[g] = out;
+    } else {
+      // next step's U^ (unnormalised, as the forward transform leaves it)
+      out = mk<Cx>(c0 * u.x + c1 * nu.x + c2 * s3.x + c3 * xv.x, c0 * u.y + c1 * nu.y + c2 * s3.y + c3 * xv.y);
+      a.uh[g] = out;
+    }
+    return out;
+  }
+};
+
+// The row spectra of a stage: E0 ZU, E1 and E5-E7 ZN, E2-E4 ZX in; ZU from E4 on, else ZX, out.
+template <typename T, int TYPE> __device__ __forceinline__ const cx<T>* etd_in(const EArgs<T>& a) {
+  return TYPE == E0 ? a.zu : ((TYPE == E1 || TYPE >= E5) ? a.zn : a.zx);
+}
+template <typename T, int TYPE> __device__ __forceinline__ cx<T>* etd_out(const EArgs<T>& a) {
+  return TYPE >= E4 ? a.zu : a.zx;
+}
+
 // The stage type is a template argument, so that each instance holds only its own operands.
-// R4: radix-4 column transforms with ny/4 threads per column (short FP64 columns).
-template <typename T, int TYPE, bool R4 = false>
+// Columns of at least 16 rows: ny/16 threads a column keep their 16 elements in registers from
+// the load to the store, and shared memory carries only the exchanges inside the transforms (8
+// trips and 8 barriers instead of 16 and 14: 4096^2 FP32 181 to 245 us a stage against 241 to 280,
+// 256^2 5.4 to 7.7 against 10 to 12).  What is left is the row spectra's 32-byte pieces and the
+// transforms, which one CTA per SM cannot overlap.
+template <typename T, int TYPE>
 __global__ void __launch_bounds__(EThreads<T>::v, 1) etd_col_kernel(const __grid_constant__ EArgs<T> a) {
   typedef cx<T> Cx;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Cx* buf = reinterpret_cast<Cx*>(smem_raw);
-  const int f = blockIdx.y;
-  constexpr int type = TYPE;
-  const int Cn = a.C, W = Cn;
-  const int lc = __ffs(Cn) - 1;  // the tile width is a power of two (halved from 16)
+  const int f = blockIdx.y, Cn = a.C;  // the tile width is a power of two (halved from 16)
+  const int kx0 = blockIdx.x * Cn;
+  const int ny = a.ny, tps = ny >> 4, c = threadIdx.x & (Cn - 1), lt = threadIdx.x >> (__ffs(Cn) - 1);
+  const bool in = kx0 + c < a.ncols;
+  const Cx zero = mk<Cx>((T)0, (T)0);
+  const T* tab = a.tab + (long long)f * 6 * a.fs;
+  const long long zo = (long long)f * a.fs + (long long)lt * a.ldc + kx0 + c, zs = (long long)tps * a.ldc;
+  const ETile<T> t(a, f, kx0);
+
+  Cx x[16];
+  const Cx* src = etd_in<T, TYPE>(a) + zo;
+#pragma unroll
+  for (int q = 0; q < 16; ++q) x[q] = in ? src[q * zs] : zero;
+  fft_regs<T, false, false>(x, buf, ny, a.log2ny, lt, c, Cn, a.tw);
+  // NB elements at a time: the operands are read and written in place, so the compiler cannot
+  // issue a later element's loads before an earlier element's stores
+  constexpr int NB = 2;
+  if (in) {
+#pragma unroll
+    for (int q0 = 0; q0 < 16; q0 += NB) {
+      EOper<T, TYPE> o[NB];
+#pragma unroll
+      for (int h = 0; h < NB; ++h) {
+        const int ky = lt + (q0 + h) * tps;
+        o[h].load(a, tab, t.go + ky * t.wt + c, t.to + (2 * ky > ny ? ny - ky : ky) * t.wt + c);
+      }
+#pragma unroll
+      for (int h = 0; h < NB; ++h)
+        x[q0 + h] = cscale(o[h].apply(a, t.go + (lt + (q0 + h) * tps) * t.wt + c, x[q0 + h]), a.scale);
+    }
+  }
+  if (TYPE == E0) return;
+  __syncthreads();
+  fft_regs<T, true, false>(x, buf, ny, a.log2ny, lt, c, Cn, a.tw);
+  Cx* dst = etd_out<T, TYPE>(a) + zo;
+  if (in) {
+#pragma unroll
+    for (int q = 0; q < 16; ++q) dst[q * zs] = x[q];
+  }
+}
+
+// The same stage with the tile in shared memory and radix-4 transforms, ny/4 threads per column:
+// columns of fewer than 16 rows, and short FP64 columns.
+template <typename T, int TYPE>
+__global__ void __launch_bounds__(EThreads<T>::v, 1) etd_col4_kernel(const __grid_constant__ EArgs<T> a) {
+  typedef cx<T> Cx;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Cx* buf = reinterpret_cast<Cx*>(smem_raw);
+  const int f = blockIdx.y, Cn = a.C, lc = __ffs(Cn) - 1;
   const int kx0 = blockIdx.x * Cn;
   const int ny = a.ny, tid = threadIdx.x, nth = blockDim.x;
-  const long long ldc = a.ldc, fo = (long long)f * a.fs, per = a.fs;
-  const T* tab = a.tab + (long long)f * 6 * per;
-
-  // load the row-spectrum tile: E0 ZU, E1 and E5-E7 ZN, E2-E4 ZX
-  const Cx* in0 = type == E0 ? a.zu : ((type == E1 || type >= E5) ? a.zn : a.zx);
+  const long long ldc = a.ldc, fo = (long long)f * a.fs;
+  const T* tab = a.tab + (long long)f * 6 * a.fs;
+  const Cx* src = etd_in<T, TYPE>(a);
+  const ETile<T> t(a, f, kx0);
   for (int e = tid; e < ny * Cn; e += nth) {
     const int ky = e >> lc, c = e & (Cn - 1), kx = kx0 + c;
-    buf[sp(ky * W + c)] = kx < a.ncols ? in0[fo + ky * ldc + kx] : mk<Cx>((T)0, (T)0);
+    buf[sp(e)] = kx < a.ncols ? src[fo + ky * ldc + kx] : mk<Cx>((T)0, (T)0);
   }
   __syncthreads();
-  if (R4) fft_smem_r4<T, false, true>(buf, ny, a.log2ny, Cn, 1, W, a.tw, tid);
-  else fft_smem<T, false, true>(buf, ny, a.log2ny, Cn, 1, W, a.tw, tid);
-
-  // The stage combination, two elements per thread at a time: the operands are read and
-  // written in place, so the compiler cannot issue a later element's loads before an
-  // earlier element's stores; loading both elements' operands first doubles the loads in
-  // flight of the one CTA per SM (the 4096-row passes wait on DRAM).
-  const T* tb0 = tab + 0 * per;
-  const T* tb1 = tab + 1 * per;
-  const T* tb2 = tab + 2 * per;
-  const T* tb3 = tab + 3 * per;
-  const T* tb4 = tab + 4 * per;
-  const T* tb5 = tab + 5 * per;
-  const Cx zero = mk<Cx>((T)0, (T)0);
-  for (int e0 = tid; e0 < ny * Cn; e0 += 2 * nth) {
-    Cx x[2], u[2], nu[2], s3[2];
-    T c0[2], c1[2], c2[2], c3[2];
-    long long g[2];
-    int sidx[2];
-    bool ok[2];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int e = e0 + h * nth;
-      const int ky = e >> lc, c = e & (Cn - 1), kx = kx0 + c;
-      ok[h] = e < ny * Cn && kx < a.ncols;
-      sidx[h] = e < ny * Cn ? sp(ky * W + c) : -1;
-      g[h] = fo + (long long)ky * ldc + kx;
-      const long long tg = (long long)ky * ldc + kx;
-      x[h] = u[h] = nu[h] = s3[h] = zero;
-      c0[h] = c1[h] = c2[h] = c3[h] = (T)0;
-      if (!ok[h]) continue;
-      x[h] = buf[sidx[h]];
-      if (type == E1 || type == E2S) {
-        c0[h] = tb1[tg]; c1[h] = tb2[tg];
-        u[h] = a.uh[g[h]];
-      } else if (type == E3) {
-        c0[h] = tb1[tg]; c1[h] = tb2[tg];
-        u[h] = a.ah[g[h]]; nu[h] = a.nu[g[h]]; s3[h] = a.ss[g[h]];
-      } else if (type >= E5) {
-        c0[h] = tb0[tg]; c1[h] = tb1[tg];
-        u[h] = a.uh[g[h]];
-        if (type == E7) { c2[h] = tb2[tg]; nu[h] = a.nu[g[h]]; }
-      } else if (type == E4) {
-        c0[h] = tb0[tg]; c1[h] = tb3[tg]; c2[h] = tb4[tg]; c3[h] = tb5[tg];
-        u[h] = a.uh[g[h]]; nu[h] = a.nu[g[h]]; s3[h] = a.ss[g[h]];
-      }
-    }
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      if (sidx[h] < 0) continue;
-      if (!ok[h]) { buf[sidx[h]] = zero; continue; }
-      const Cx xv = x[h];
-      Cx out;
-      if (type == E0) {  // the initial U^ (later steps get it from E4)
-        a.uh[g[h]] = xv;
-        continue;
-      } else if (type == E1) {
-        a.nu[g[h]] = xv;
-        out = mk<Cx>(c0[h] * u[h].x + c1[h] * xv.x, c0[h] * u[h].y + c1[h] * xv.y);
-        a.ah[g[h]] = out;
-      } else if (type == E2S) {
-        a.ss[g[h]] = xv;
-        out = mk<Cx>(c0[h] * u[h].x + c1[h] * xv.x, c0[h] * u[h].y + c1[h] * xv.y);
-      } else if (type == E3) {
-        // u = a^, nu = N^u, s3 = S
-        a.ss[g[h]] = cadd(s3[h], xv);
-        out = mk<Cx>(c0[h] * u[h].x + c1[h] * ((T)2 * xv.x - nu[h].x),
-                     c0[h] * u[h].y + c1[h] * ((T)2 * xv.y - nu[h].y));
-      } else if (type >= E5) {
-        // ETD1 (fft_integrators.py:165-166) / ETD2 (234-236): c0 = E, c1 = phi1, c2 = phi2
-        T ox = c0[h] * u[h].x + c1[h] * xv.x, oy = c0[h] * u[h].y + c1[h] * xv.y;
-        if (type == E7) {
-          ox += c2[h] * (xv.x - nu[h].x);
-          oy += c2[h] * (xv.y - nu[h].y);
-        }
-        if (type != E5) a.nu[g[h]] = xv;
-        out = mk<Cx>(ox, oy);
-        a.uh[g[h]] = out;
-      } else {
-        // E4: c0 = E, c1 = f1, c2 = f2, c3 = f3; next step's U^ (unnormalised, as the forward
-        // transform leaves it)
-        out = mk<Cx>(c0[h] * u[h].x + c1[h] * nu[h].x + c2[h] * s3[h].x + c3[h] * xv.x,
-                     c0[h] * u[h].y + c1[h] * nu[h].y + c2[h] * s3[h].y + c3[h] * xv.y);
-        a.uh[g[h]] = out;
-      }
-      buf[sidx[h]] = cscale(out, a.scale);
-    }
+  fft_smem_r4<T, false, true>(buf, ny, a.log2ny, Cn, 1, Cn, a.tw, tid);
+  for (int e = tid; e < ny * Cn; e += nth) {
+    const int ky = e >> lc, c = e & (Cn - 1);
+    if (kx0 + c >= a.ncols) continue;
+    EOper<T, TYPE> o;
+    o.load(a, tab, t.go + ky * t.wt + c, t.to + (2 * ky > ny ? ny - ky : ky) * t.wt + c);
+    buf[sp(e)] = cscale(o.apply(a, t.go + ky * t.wt + c, buf[sp(e)]), a.scale);
   }
-  if (type == E0) return;
+  if (TYPE == E0) return;
   __syncthreads();
-  if (R4) fft_smem_r4<T, true, true>(buf, ny, a.log2ny, Cn, 1, W, a.tw, tid);
-  else fft_smem<T, true, true>(buf, ny, a.log2ny, Cn, 1, W, a.tw, tid);
-  Cx* dst = type >= E4 ? a.zu : a.zx;
+  fft_smem_r4<T, true, true>(buf, ny, a.log2ny, Cn, 1, Cn, a.tw, tid);
+  Cx* dst = etd_out<T, TYPE>(a);
   for (int e = tid; e < ny * Cn; e += nth) {
     const int ky = e >> lc, c = e & (Cn - 1), kx = kx0 + c;
-    if (kx < a.ncols) dst[fo + ky * ldc + kx] = buf[sp(ky * W + c)];
+    if (kx < a.ncols) dst[fo + ky * ldc + kx] = buf[sp(e)];
   }
 }
 
@@ -318,6 +370,15 @@ static EtdLayout etd_layout(int ny, int nx, int elem) {
   return L;
 }
 
+// columns per CTA: the widest tile within the thread cap and ~200 KB of shared memory
+template <typename T>
+static int etd_tile(int ny) {
+  const int tps = ny >= 16 ? ny / 16 : 1;
+  int C = 16;
+  while (C > 1 && (C * tps > EThreads<T>::v || (size_t)sp_size(ny * C) * 2 * sizeof(T) > 200 * 1024)) C >>= 1;
+  return C;
+}
+
 template <typename T>
 struct EtdPlan {
   EArgs<T> c[8];
@@ -337,14 +398,6 @@ static EtdPlan<T> build_etd(const void* plan, const mjx_grid2d* g, int nf, doubl
   EArgs<T> e;
   memset(&e, 0, sizeof(e));
   e.ny = g->ny; e.log2ny = ilog2_exact(g->ny); e.ncols = g->nx / 2 + 1; e.ldc = ldc;
-  const int tps = g->ny >= 16 ? g->ny / 16 : 1;
-  // widest tile within the thread cap and ~200 KB of shared memory
-  auto tile = [&](int nin) {
-    int C = 16;
-    while (C > 1 && (C * nin * tps > EThreads<T>::v ||
-                     (size_t)sp_size(g->ny * nin * C) * 2 * sizeof(T) > 200 * 1024)) C >>= 1;
-    return C;
-  };
   e.njobs = nf;
   e.zu = (cx<T>*)(ws + L.zu); e.zn = (cx<T>*)(ws + L.zn); e.zx = (cx<T>*)(ws + L.zx);
   e.uh = (cx<T>*)(ws + L.uh); e.nu = (cx<T>*)(ws + L.nu); e.ah = (cx<T>*)(ws + L.ah); e.ss = (cx<T>*)(ws + L.ss);
@@ -356,7 +409,7 @@ static EtdPlan<T> build_etd(const void* plan, const mjx_grid2d* g, int nf, doubl
   for (int t = E0; t <= E7; ++t) {
     P.c[t] = e;
     P.c[t].type = t;
-    P.c[t].C = tile(1);
+    P.c[t].C = P.c[t].tile = etd_tile<T>(g->ny);
   }
   P.c0n = P.c[E0];
   P.c0n.zu = e.zx;
@@ -385,36 +438,36 @@ static EtdPlan<T> build_etd(const void* plan, const mjx_grid2d* g, int nf, doubl
   return P;
 }
 
-template <typename T, bool R4>
+template <typename T>
 static mjx_status etd_col_attrs(int optin) {
-  const void* k[8] = {(const void*)etd_col_kernel<T, E0, R4>, (const void*)etd_col_kernel<T, E1, R4>,
-                      (const void*)etd_col_kernel<T, E2S, R4>, (const void*)etd_col_kernel<T, E3, R4>,
-                      (const void*)etd_col_kernel<T, E4, R4>, (const void*)etd_col_kernel<T, E5, R4>,
-                      (const void*)etd_col_kernel<T, E6, R4>, (const void*)etd_col_kernel<T, E7, R4>};
-  for (int i = 0; i < 8; ++i)
+  const void* k[16] = {(const void*)etd_col_kernel<T, E0>,   (const void*)etd_col_kernel<T, E1>,
+                       (const void*)etd_col_kernel<T, E2S>,  (const void*)etd_col_kernel<T, E3>,
+                       (const void*)etd_col_kernel<T, E4>,   (const void*)etd_col_kernel<T, E5>,
+                       (const void*)etd_col_kernel<T, E6>,   (const void*)etd_col_kernel<T, E7>,
+                       (const void*)etd_col4_kernel<T, E0>,  (const void*)etd_col4_kernel<T, E1>,
+                       (const void*)etd_col4_kernel<T, E2S>, (const void*)etd_col4_kernel<T, E3>,
+                       (const void*)etd_col4_kernel<T, E4>,  (const void*)etd_col4_kernel<T, E5>,
+                       (const void*)etd_col4_kernel<T, E6>,  (const void*)etd_col4_kernel<T, E7>};
+  for (int i = 0; i < 16; ++i)
     MJX_CUDA_TRY(cudaFuncSetAttribute(k[i], cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
   return MJX_OK;
 }
 
 template <typename T, int TYPE>
 static void etd_col_launch(const EArgs<T>& e, cudaStream_t s) {
-  const int tps = e.ny >= 16 ? e.ny / 16 : 1;
-  if constexpr (sizeof(T) == 8) {
-    // FP64 columns of at most 256 points on a small grid (fewer than four warps per SM at
-    // radix 16): radix-4 transforms (ny/4 threads per column), narrower tiles within the cap
-    if (e.ny >= 4 && e.ny <= 256 && (long long)e.ncols * e.njobs * tps < 152LL * 128) {
-      EArgs<T> b = e;
-      const int tps4 = e.ny / 4;
-      while (b.C > 1 && b.C * tps4 > EThreads<T>::v) b.C >>= 1;
-      dim3 g4((b.ncols + b.C - 1) / b.C, b.njobs);
-      const size_t sm4 = (size_t)sp_size(b.ny * b.C) * 2 * sizeof(T);
-      etd_col_kernel<T, TYPE, true><<<g4, b.C * tps4, sm4, s>>>(b);
-      return;
-    }
+  const int tps = e.ny / 16;
+  // radix-4 columns (ny/4 threads each, narrower tiles within the cap): fewer than 16 rows, and
+  // FP64 columns of at most 256 points on a small grid (fewer than four warps per SM at radix 16)
+  if (e.ny < 16 || (sizeof(T) == 8 && e.ny <= 256 && (long long)e.ncols * e.njobs * tps < 152LL * 128)) {
+    EArgs<T> b = e;
+    const int tps4 = e.ny >= 4 ? e.ny / 4 : 1;
+    while (b.C > 1 && b.C * tps4 > EThreads<T>::v) b.C >>= 1;
+    dim3 g4((b.ncols + b.C - 1) / b.C, b.njobs);
+    etd_col4_kernel<T, TYPE><<<g4, b.C * tps4, (size_t)sp_size(b.ny * b.C) * 2 * sizeof(T), s>>>(b);
+    return;
   }
   dim3 grid((e.ncols + e.C - 1) / e.C, e.njobs);
-  const size_t smem = (size_t)sp_size(e.ny * e.C) * 2 * sizeof(T);
-  etd_col_kernel<T, TYPE><<<grid, e.C * tps, smem, s>>>(e);
+  etd_col_kernel<T, TYPE><<<grid, e.C * tps, (size_t)sp_size(e.ny * e.C) * 2 * sizeof(T), s>>>(e);
 }
 
 template <typename T>
@@ -493,9 +546,8 @@ static mjx_status etd_run(const void* plan, const mjx_grid2d* g, const mjx_etd_p
     int dev = 0, optin = 0;
     MJX_CUDA_TRY(cudaGetDevice(&dev));
     MJX_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    MJX_TRY((etd_col_attrs<float, false>(optin)));
-    MJX_TRY((etd_col_attrs<double, false>(optin)));
-    MJX_TRY((etd_col_attrs<double, true>(optin)));
+    MJX_TRY(etd_col_attrs<float>(optin));
+    MJX_TRY(etd_col_attrs<double>(optin));
     return MJX_OK;
   }));
   const int nf = pb->nfields, rx = pb->reaction;
@@ -503,7 +555,7 @@ static mjx_status etd_run(const void* plan, const mjx_grid2d* g, const mjx_etd_p
   if (recompute) {
     etd_coeff_kernel<T><<<152 * 8, 256, 0, s>>>((T*)(ws + L.tab), g->ny, g->nx, spec_ldc(g->nx), symbol, xonly,
                                                  g->dy, g->dx, pb->D[0], pb->D[1], nf, pb->dt, 32,
-                                                 pb->f2_factor, etd_form(pb));
+                                                 pb->f2_factor, etd_form(pb), etd_tile<T>(g->ny));
     MJX_CUDA_TRY(cudaGetLastError());
   }
   const EtdPlan<T> P = build_etd<T>(plan, g, nf, pb->F, pb->k, pb->r, ws, L, y_in, y_out, nprev_in, n_out);

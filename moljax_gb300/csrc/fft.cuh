@@ -229,6 +229,52 @@ __device__ __forceinline__ void fft_smem_inl(cx<T>* buf, int n, int log2n, int n
 }
 
 
+// The transform of 16 <= n <= 4096 points with both ends in registers: x[q] holds element
+// lt + q n/16 of the thread's sequence (thread mapping of fft_smem), on entry and on return, so
+// that a caller loads, combines and stores in registers; shared memory carries only the exchange
+// between passes.  The first pass reads exactly these elements and the last pass leaves them.
+// All n/16 threads of a sequence take part; buf is free for other data once every thread of
+// the block has returned and passed a barrier (the next call's first pass has none).
+template <typename T, int R, bool INV, bool PT>
+__device__ __forceinline__ void fft_last_pass(cx<T>* x, int n, int p, int tps, int lt, int es, const cx<T>* in,
+                                              const cx<T>* __restrict__ tw) {
+  typedef cx<T> C;
+  C z[16];
+#pragma unroll
+  for (int m = 0; m < 16 / R; ++m)
+#pragma unroll
+    for (int r = 0; r < R; ++r) z[m * R + r] = in[sp(m * tps * es) + sp(r * p * es)];
+  // p = n / R: butterfly i = lt + m n/16 has k = i, its outputs are i + r p
+#pragma unroll
+  for (int m = 0; m < 16 / R; ++m) {
+    apply_twiddles<T, R, INV, PT>(&z[m * R], lt + m * tps, p, 1, PT ? tw + n + (p == 16 ? 0 : 96) : tw);
+    dft_r<R, INV>(&z[m * R]);
+#pragma unroll
+    for (int r = 0; r < R; ++r) x[m + r * (16 / R)] = z[m * R + r];
+  }
+}
+
+template <typename T, bool INV, bool ES1, bool PT = (sizeof(T) == 4)>
+__device__ __forceinline__ void fft_regs(cx<T>* x, cx<T>* buf, int n, int log2n, int lt, int base, int es_rt,
+                                         const cx<T>* __restrict__ tw) {
+  const int es = ES1 ? 1 : es_rt, tps = n >> 4;
+  dft16<INV>(x);
+  if (log2n == 4) return;
+  cx<T>* out = buf + sp(base + lt * 16 * es);
+#pragma unroll
+  for (int r = 0; r < 16; ++r) out[sp(r * es)] = x[r];
+  __syncthreads();
+  if (log2n > 8) stockham_pass<T, 16, INV, ES1, PT>(buf, n, 16, tps, lt, base, es, true, tw);
+  const cx<T>* in = buf + sp(base + lt * es);
+  const int p = log2n > 8 ? 256 : 16;
+  switch (log2n & 3) {
+    case 0: fft_last_pass<T, 16, INV, PT>(x, n, p, tps, lt, es, in, tw); break;
+    case 1: fft_last_pass<T, 2, INV, PT>(x, n, p, tps, lt, es, in, tw); break;
+    case 2: fft_last_pass<T, 4, INV, PT>(x, n, p, tps, lt, es, in, tw); break;
+    default: fft_last_pass<T, 8, INV, PT>(x, n, p, tps, lt, es, in, tw); break;
+  }
+}
+
 // fft_smem_inl is always inlined, so that a caller passing compile-time lengths gets the
 // index arithmetic and the radix schedule folded; fft_smem leaves the choice to the compiler.
 template <typename T, bool INV, bool COLMAJOR, bool PT = (sizeof(T) == 4)>

@@ -81,3 +81,24 @@ def test_etdrk4_maximum_extent(cuda, ny, nx, dtype):
     tol = 1e-11 if dtype == torch.float64 else 3e-6
     assert _rel(mol.interior(out["u"].cpu().numpy(), og), ru) < tol
     assert _rel(mol.interior(out["v"].cpu().numpy(), og), rv) < tol
+
+
+@pytest.mark.parametrize("ny,nx", [(8, 64), (16, 256), (32, 16), (256, 32), (512, 64), (1024, 8), (2048, 32)])
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+def test_etdrk4_column_lengths(cuda, ny, nx, dtype):
+    """Every column length class (radix-4 columns below 16 rows, one to three passes, each last
+    radix) with full, narrow and single column tiles, against the oracle; tolerances as above (the
+    same stages, fewer transform levels)."""
+    import moljax_gb300 as M
+    L = 2.5
+    grid = M.Grid2D(nx, ny, 0.0, L, 0.0, L)
+    model = M.create_gray_scott_model(grid, 2e-5, 1e-5, 0.035, 0.065, dtype=dtype)
+    og = mol.Grid2D(nx, ny, 0, L, 0, L)
+    y0 = mol.gray_scott_ic(og, 5)
+    ym = {k: torch.tensor(v, dtype=dtype, device=cuda) for k, v in y0.items()}
+    out = M.etdrk4_gray_scott(model, ym, 0.5, 6)
+    ru, rv = OE.etdrk4_gray_scott(mol.interior(y0["u"], og), mol.interior(y0["v"], og),
+                                  mol.fd_symbol_2d(ny, nx, og.dy, og.dx), 2e-5, 1e-5, 0.035, 0.065, 0.5, 6, 2.0)
+    tol = 1e-11 if dtype == torch.float64 else 3e-6
+    assert _rel(mol.interior(out["u"].cpu().numpy(), og), ru) < tol
+    assert _rel(mol.interior(out["v"].cpu().numpy(), og), rv) < tol
