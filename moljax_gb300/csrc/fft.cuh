@@ -229,12 +229,12 @@ __device__ __forceinline__ void fft_smem_inl(cx<T>* buf, int n, int log2n, int n
 }
 
 
-// The transform of 16 <= n <= 4096 points with both ends in registers: x[q] holds element
-// lt + q n/16 of the thread's sequence (thread mapping of fft_smem), on entry and on return, so
-// that a caller loads, combines and stores in registers; shared memory carries only the exchange
-// between passes.  The first pass reads exactly these elements and the last pass leaves them.
-// All n/16 threads of a sequence take part; buf is free for other data once every thread of
-// the block has returned and passed a barrier (the next call's first pass has none).
+// The transform of n <= 4096 points with both ends in registers: x[q] holds element lt + q tps
+// of the thread's sequence (thread mapping of fft_smem, tps = n/16; a whole sequence below 16
+// points), on entry and on return, so that a caller loads, combines and stores in registers;
+// shared memory carries only the exchange between passes.  The first pass reads exactly these
+// elements and the last pass leaves them.  All threads of a sequence take part; the first pass
+// writes buf without a barrier before it, and the last one reads it without one after it.
 template <typename T, int R, bool INV, bool PT>
 __device__ __forceinline__ void fft_last_pass(cx<T>* x, int n, int p, int tps, int lt, int es, const cx<T>* in,
                                               const cx<T>* __restrict__ tw) {
@@ -258,8 +258,14 @@ template <typename T, bool INV, bool ES1, bool PT = (sizeof(T) == 4)>
 __device__ __forceinline__ void fft_regs(cx<T>* x, cx<T>* buf, int n, int log2n, int lt, int base, int es_rt,
                                          const cx<T>* __restrict__ tw) {
   const int es = ES1 ? 1 : es_rt, tps = n >> 4;
+  if (log2n <= 4) {
+    if (log2n == 4) dft16<INV>(x);
+    else if (log2n == 3) dft8<INV>(x);
+    else if (log2n == 2) dft4<INV>(x[0], x[1], x[2], x[3]);
+    else dft2<INV>(x[0], x[1]);
+    return;
+  }
   dft16<INV>(x);
-  if (log2n == 4) return;
   cx<T>* out = buf + sp(base + lt * 16 * es);
 #pragma unroll
   for (int r = 0; r < 16; ++r) out[sp(r * es)] = x[r];

@@ -64,9 +64,15 @@ template <typename T> __device__ __forceinline__ bool finite_(T v) { return isfi
 // ------------------------------------------------------------------ row pass
 template <typename T> struct Occ { static constexpr int row = sizeof(T) == 4 ? 4 : 2, col = sizeof(T) == 4 ? 2 : 1; };
 
-// LOG2N > 0: the row length 2^LOG2N and one sequence per CTA are compile-time constants
-// (FP32 rows of 2048 and 4096 points), so that the transform's index arithmetic and radix
-// schedule fold into the code; LOG2N = 0 reads both from the arguments.
+// LOG2N > 0: the row length 2^LOG2N (above 1024 one sequence per CTA) is a compile-time constant,
+// so that the transform's index arithmetic and radix schedule fold into the code; LOG2N = 0
+// (rows of at most 16 points) reads it from the arguments.  A thread keeps its elements
+// lt + m tps in registers from the load to the store (fft_regs); shared memory carries the
+// exchanges inside the transforms and the mirrored half of a spectrum, which the two-for-one
+// packing pairs with the other half.  FP32, fused (c2r, reaction, r2c), 256, 2048 and 4096 points:
+// 6.9, 58 and 100 us; through shared memory 14.7 (length at run time), 63 and 125 us.  The long
+// rows are bound by the SMs' issue and shared-memory bandwidth alike, the short ones by the
+// latency of one chain (load, five exchanges, store) on a few warps an SM.
 template <typename T, int RX, int LOG2N = 0>
 __global__ void __launch_bounds__(256, Occ<T>::row) row_kernel(const __grid_constant__ RowArgs<T> a) {
   typedef cx<T> C;
@@ -77,7 +83,7 @@ __global__ void __launch_bounds__(256, Occ<T>::row) row_kernel(const __grid_cons
   if (st != nullptr && st->done) return;
 
   const int n = LOG2N ? (1 << LOG2N) : a.n, half = n >> 1;
-  const int log2n = LOG2N ? LOG2N : a.log2n, nseq = LOG2N ? 1 : a.nseq;
+  const int log2n = LOG2N ? LOG2N : a.log2n, nseq = LOG2N > 10 ? 1 : a.nseq;
   const int tps = n >= 16 ? n / 16 : 1;
   const int tid = threadIdx.x;
   const int s_loc = tid / tps, lt = tid % tps;
@@ -90,13 +96,15 @@ __global__ void __launch_bounds__(256, Occ<T>::row) row_kernel(const __grid_cons
   const T* rin = a.rin_sel < 0 ? a.rin[0] : a.rin[a.rin_sel == 0 ? cur : 1 - cur];
   T* rout = a.rout_sel < 0 ? a.rout[0] : a.rout[a.rout_sel == 0 ? cur : 1 - cur];
   const int zb = s_loc * n;  // this sequence's first logical smem element
+  // element lt + m tps of the sequence, m < 16, is in x[m]; a mirrored index needs its own padding
 #define Z(x) buf[sp(zb + (x))]
+  C x[16];
 
   // 1. load: spectrum rows (c2r) or real rows
   if (flags & ROW_LOAD_SPEC) {
     const C* A = a.spec + pr.sa + y * a.ldc;
     const C* B = a.spec + pr.sb + y * a.ldc;
-    // every thread owns kk = lt + m*tps, m < 9 (n/2+1 <= 9*tps): issue all loads first
+    // every thread owns kk = lt + m*tps <= n/2, m < 9: issue all loads first
     C Ak[9], Bk[9];
 #pragma unroll
     for (int m = 0; m < 9; ++m) {
@@ -107,31 +115,30 @@ __global__ void __launch_bounds__(256, Occ<T>::row) row_kernel(const __grid_cons
     for (int m = 0; m < 9; ++m) {
       const int kk = lt + m * tps;
       if (kk <= half) {
-        Z(kk) = mk<C>(Ak[m].x - Bk[m].y, Ak[m].y + Bk[m].x);                    // A_k + i B_k
+        x[m] = mk<C>(Ak[m].x - Bk[m].y, Ak[m].y + Bk[m].x);                                  // A_k + i B_k
         if (kk > 0 && kk < half) Z(n - kk) = mk<C>(Ak[m].x + Bk[m].y, Bk[m].x - Ak[m].y);  // conj(A_k) + i conj(B_k)
       }
     }
     __syncthreads();
-    if (LOG2N) fft_smem_inl<T, true, false>(buf, n, log2n, nseq, n, 1, a.tw, tid);
-    else fft_smem<T, true, false>(buf, n, log2n, nseq, n, 1, a.tw, tid);
+    const C* zt = buf + sp(zb + lt);
+#pragma unroll
+    for (int m = 1; m < 16; ++m) {
+      const int kk = lt + m * tps;
+      if (kk > half && kk < n) x[m] = zt[sp(m * tps)];
+    }
+    __syncthreads();
+    fft_regs<T, true, true>(x, buf, n, log2n, lt, zb, 1, a.tw);
   } else {
     const T* ra = rin + pr.ra + y * a.rstride;
     const T* rb = rin + pr.rb + y * a.rstride;
-    T va[16], vb[16];
 #pragma unroll
     for (int m = 0; m < 16; ++m) {
-      const int x = lt + m * tps;
-      if (x < n) { va[m] = ra[x]; vb[m] = rb[x]; }
+      const int i = lt + m * tps;
+      if (i < n) x[m] = mk<C>(ra[i], rb[i]);
     }
-#pragma unroll
-    for (int m = 0; m < 16; ++m) {
-      const int x = lt + m * tps;
-      if (x < n) Z(x) = mk<C>(va[m], vb[m]);
-    }
-    __syncthreads();
   }
 
-  // 2. pointwise work on the real rows (each thread owns x = lt + m*tps)
+  // 2. pointwise work on the real rows
   const T sc = (flags & ROW_LOAD_SPEC) ? a.inv_scale : (T)1;
   T h = (T)0;
   if (flags & ROW_REACT) h = (T)((st != nullptr ? st->dtc : a.hfixed) * pr.hfac);
@@ -144,68 +151,78 @@ __global__ void __launch_bounds__(256, Occ<T>::row) row_kernel(const __grid_cons
   // parameters converted once (the per-element double arithmetic would occupy the FP64 pipe)
   const T pF = (T)a.F, pK = (T)a.k, pR = (T)a.r, pFK = (T)(a.F + a.k);
   const T pAtol = (T)a.atol, pRtol = (T)a.rtol;
-  T ra_[16], rb_[16];
-  if (flags & ROW_ERRNORM) {
 #pragma unroll
-    for (int m = 0; m < 16; ++m) {
-      const int x = lt + m * tps;
-      if (x < n) { ra_[m] = ea[x]; rb_[m] = eb[x]; }
-    }
-  }
-#pragma unroll
-  for (int m = 0; m < 16; ++m) {
-    const int x = lt + m * tps;
-    if (x >= n) continue;
-    const C v = Z(x);
-    T va = v.x * sc, vb = v.y * sc;
-    if (flags & ROW_NONLIN) {
-      // Gray-Scott reaction terms (operators.py:655-667); Fisher-KPP r u (1-u)
-      if (RX == RX_GRAY_SCOTT) {
-        const T uvv = va * vb * vb;
-        const T nu = -uvv + pF * ((T)1 - va), nv = uvv - pFK * vb;
-        va = nu; vb = nv;
-      } else if (RX == RX_FISHER) {
-        va = pR * va * ((T)1 - va); vb = pR * vb * ((T)1 - vb);
-      } else {
-        va = (T)0; vb = (T)0;
-      }
-    }
-    if (flags & ROW_REACT) {
-      if (flags & ROW_DELTA) react_delta<T, RX>(va, vb, h, pF, pK, pR);
-      else if (flags & ROW_EULER) {
-        react_euler<T, RX>(va, vb, h, pF, pK, pR);
-        if (flags & ROW_EULER2) react_euler<T, RX>(va, vb, h, pF, pK, pR);
-      }
-      else react_heun<T, RX>(va, vb, h, pF, pK, pR);
-    }
-    if (flags & ROW_STORE_REAL) { oa[x] = va; ob[x] = vb; }
+  for (int m0 = 0; m0 < 16; m0 += 4) {
+    T ra_[4], rb_[4];  // four references ahead of the stores, which may alias them for the compiler
     if (flags & ROW_ERRNORM) {
-      // moljax/core/state.py:335-339: (err / (atol + rtol |y_new|))^2
-      const T da = (va - ra_[m]) / (pAtol + pRtol * fabs(va));
-      const T db = (vb - rb_[m]) / (pAtol + pRtol * fabs(vb));
-      esum += da * da + db * db;
-      bad |= !(finite_(va) && finite_(vb));
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        const int i = lt + (m0 + m) * tps;
+        if (i < n) { ra_[m] = ea[i]; rb_[m] = eb[i]; }
+      }
     }
-    if (flags & ROW_ERRPAIR) {
-      const T da = va / (pAtol + pRtol * fabs(vb));
-      esum += da * da;
-      bad |= !(finite_(va) && finite_(vb));
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      const int i = lt + (m0 + m) * tps;
+      if (i >= n) continue;
+      const C v = x[m0 + m];
+      T va = v.x * sc, vb = v.y * sc;
+      if (flags & ROW_NONLIN) {
+        // Gray-Scott reaction terms (operators.py:655-667); Fisher-KPP r u (1-u)
+        if (RX == RX_GRAY_SCOTT) {
+          const T uvv = va * vb * vb;
+          const T nu = -uvv + pF * ((T)1 - va), nv = uvv - pFK * vb;
+          va = nu; vb = nv;
+        } else if (RX == RX_FISHER) {
+          va = pR * va * ((T)1 - va); vb = pR * vb * ((T)1 - vb);
+        } else {
+          va = (T)0; vb = (T)0;
+        }
+      }
+      if (flags & ROW_REACT) {
+        if (flags & ROW_DELTA) react_delta<T, RX>(va, vb, h, pF, pK, pR);
+        else if (flags & ROW_EULER) {
+          react_euler<T, RX>(va, vb, h, pF, pK, pR);
+          if (flags & ROW_EULER2) react_euler<T, RX>(va, vb, h, pF, pK, pR);
+        }
+        else react_heun<T, RX>(va, vb, h, pF, pK, pR);
+      }
+      if (flags & ROW_STORE_REAL) { oa[i] = va; ob[i] = vb; }
+      if (flags & ROW_ERRNORM) {
+        // moljax/core/state.py:335-339: (err / (atol + rtol |y_new|))^2
+        const T da = (va - ra_[m]) / (pAtol + pRtol * fabs(va));
+        const T db = (vb - rb_[m]) / (pAtol + pRtol * fabs(vb));
+        esum += da * da + db * db;
+        bad |= !(finite_(va) && finite_(vb));
+      }
+      if (flags & ROW_ERRPAIR) {
+        const T da = va / (pAtol + pRtol * fabs(vb));
+        esum += da * da;
+        bad |= !(finite_(va) && finite_(vb));
+      }
+      x[m0 + m] = mk<C>(va, vb);
     }
-    Z(x) = mk<C>(va, vb);
   }
 
   // 3. r2c and split into the two half spectra
   if (flags & ROW_STORE_SPEC) {
-    __syncthreads();
-    if (LOG2N) fft_smem_inl<T, false, false>(buf, n, log2n, nseq, n, 1, a.tw, tid);
-    else fft_smem<T, false, false>(buf, n, log2n, nseq, n, 1, a.tw, tid);
+    if (flags & ROW_LOAD_SPEC) __syncthreads();
+    fft_regs<T, false, true>(x, buf, n, log2n, lt, zb, 1, a.tw);
     C* A = a.spec + ((flags & ROW_SPEC_ALT) ? pr.oa : pr.sa) + y * a.ldc;
     C* B = a.spec + ((flags & ROW_SPEC_ALT) ? pr.ob : pr.sb) + y * a.ldc;
+    __syncthreads();
+    C* zt = buf + sp(zb + lt);
+#pragma unroll
+    for (int m = 1; m < 16; ++m) {
+      const int kk = lt + m * tps;
+      if (kk > half && kk < n) zt[sp(m * tps)] = x[m];
+    }
+    __syncthreads();
 #pragma unroll
     for (int m = 0; m < 9; ++m) {
       const int kk = lt + m * tps;
       if (kk > half) continue;
-      const C Zk = Z(kk), Zm = Z((n - kk) & (n - 1));
+      const C Zk = x[m], Zm = kk > 0 && kk < half ? Z(n - kk) : Zk;
       A[kk] = mk<C>((T)0.5 * (Zk.x + Zm.x), (T)0.5 * (Zk.y - Zm.y));
       B[kk] = mk<C>((T)0.5 * (Zk.y + Zm.y), (T)0.5 * (Zm.x - Zk.x));
     }
@@ -492,15 +509,17 @@ cudaError_t launch_row(const RowArgs<T>& a0, cudaStream_t s) {
     }
   }
   const size_t smem = row_smem(a.n, a.nseq, sizeof(T));
+  const int threads = a.nseq * tps;
+#define MJX_ROW(L) case L: return launch_chain(row_kernel<T, RX, L>, dim3(grid), threads, smem, s, a.pdl, a);
   if constexpr (sizeof(T) == 4) {
-    if (a.n == 4096 && a.nseq == 1) {
-      return launch_chain(row_kernel<T, RX, 12>, dim3(grid), tps, smem, s, a.pdl, a);
+    switch (a.log2n) {
+      MJX_ROW(5) MJX_ROW(6) MJX_ROW(7) MJX_ROW(8) MJX_ROW(9) MJX_ROW(11) MJX_ROW(12)
+      default: return launch_chain(row_kernel<T, RX>, dim3(grid), threads, smem, s, a.pdl, a);
     }
-    if (a.n == 2048 && a.nseq == 1) {
-      return launch_chain(row_kernel<T, RX, 11>, dim3(grid), tps, smem, s, a.pdl, a);
-    }
+  } else {
+    return launch_chain(row_kernel<T, RX, 12>, dim3(grid), threads, smem, s, a.pdl, a);  // the others: row64_takes
   }
-  return launch_chain(row_kernel<T, RX>, dim3(grid), a.nseq * tps, smem, s, a.pdl, a);
+#undef MJX_ROW
 }
 
 template <typename T>
@@ -555,6 +574,19 @@ static mjx_status raise_smem(K kernel, int optin) {
   return MJX_OK;
 }
 
+template <int RX>
+static mjx_status row_attrs(int optin) {
+  MJX_TRY(raise_smem(row_kernel<float, RX>, optin));
+  MJX_TRY(raise_smem(row_kernel<float, RX, 5>, optin));
+  MJX_TRY(raise_smem(row_kernel<float, RX, 6>, optin));
+  MJX_TRY(raise_smem(row_kernel<float, RX, 7>, optin));
+  MJX_TRY(raise_smem(row_kernel<float, RX, 8>, optin));
+  MJX_TRY(raise_smem(row_kernel<float, RX, 9>, optin));
+  MJX_TRY(raise_smem(row_kernel<float, RX, 11>, optin));
+  MJX_TRY(raise_smem(row_kernel<float, RX, 12>, optin));
+  return raise_smem(row_kernel<double, RX, 12>, optin);
+}
+
 // Raise the dynamic shared-memory limit of every kernel once per CUDA context
 // (function attributes belong to the context the kernels are loaded in).
 mjx_status ensure_kernel_attrs() {
@@ -563,19 +595,9 @@ mjx_status ensure_kernel_attrs() {
     int dev = 0, optin = 0;
     MJX_CUDA_TRY(cudaGetDevice(&dev));
     MJX_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    MJX_TRY(raise_smem(row_kernel<float, RX_NONE>, optin));
-    MJX_TRY(raise_smem(row_kernel<float, RX_GRAY_SCOTT>, optin));
-    MJX_TRY(raise_smem(row_kernel<float, RX_FISHER>, optin));
-    MJX_TRY(raise_smem(row_kernel<double, RX_NONE>, optin));
-    MJX_TRY(raise_smem(row_kernel<double, RX_GRAY_SCOTT>, optin));
-    MJX_TRY(raise_smem(row_kernel<double, RX_FISHER>, optin));
-    MJX_TRY(raise_smem(row_kernel<float, RX_NONE, 11>, optin));
-    MJX_TRY(raise_smem(row_kernel<float, RX_GRAY_SCOTT, 11>, optin));
-    MJX_TRY(raise_smem(row_kernel<float, RX_FISHER, 11>, optin));
-    MJX_TRY(raise_smem(row_kernel<float, RX_NONE, 12>, optin));
-    MJX_TRY(raise_smem(row_kernel<float, RX_GRAY_SCOTT, 12>, optin));
-    MJX_TRY(raise_smem(row_kernel<float, RX_FISHER, 12>, optin));
-
+    MJX_TRY(row_attrs<RX_NONE>(optin));
+    MJX_TRY(row_attrs<RX_GRAY_SCOTT>(optin));
+    MJX_TRY(row_attrs<RX_FISHER>(optin));
     MJX_TRY(raise_smem(row_kernel_w32<RX_NONE>, optin));
     MJX_TRY(raise_smem(row_kernel_w32<RX_GRAY_SCOTT>, optin));
     MJX_TRY(raise_smem(row_kernel_w32<RX_FISHER>, optin));
