@@ -233,8 +233,9 @@ __device__ __forceinline__ void fft_smem_inl(cx<T>* buf, int n, int log2n, int n
 // of the thread's sequence (thread mapping of fft_smem, tps = n/16; a whole sequence below 16
 // points), on entry and on return, so that a caller loads, combines and stores in registers;
 // shared memory carries only the exchange between passes.  The first pass reads exactly these
-// elements and the last pass leaves them.  All threads of a sequence take part; the first pass
-// writes buf without a barrier before it, and the last one reads it without one after it.
+// elements and the last pass leaves them.  All threads of the block call it, those of no
+// sequence with active = false; the first pass writes buf without a barrier before it, and the
+// last one reads it without one after it.
 template <typename T, int R, bool INV, bool PT>
 __device__ __forceinline__ void fft_last_pass(cx<T>* x, int n, int p, int tps, int lt, int es, const cx<T>* in,
                                               const cx<T>* __restrict__ tw) {
@@ -256,21 +257,25 @@ __device__ __forceinline__ void fft_last_pass(cx<T>* x, int n, int p, int tps, i
 
 template <typename T, bool INV, bool ES1, bool PT = (sizeof(T) == 4)>
 __device__ __forceinline__ void fft_regs(cx<T>* x, cx<T>* buf, int n, int log2n, int lt, int base, int es_rt,
-                                         const cx<T>* __restrict__ tw) {
+                                         const cx<T>* __restrict__ tw, bool active = true) {
   const int es = ES1 ? 1 : es_rt, tps = n >> 4;
   if (log2n <= 4) {
+    if (!active) return;
     if (log2n == 4) dft16<INV>(x);
     else if (log2n == 3) dft8<INV>(x);
     else if (log2n == 2) dft4<INV>(x[0], x[1], x[2], x[3]);
     else dft2<INV>(x[0], x[1]);
     return;
   }
-  dft16<INV>(x);
-  cx<T>* out = buf + sp(base + lt * 16 * es);
+  if (active) {
+    dft16<INV>(x);
+    cx<T>* out = buf + sp(base + lt * 16 * es);
 #pragma unroll
-  for (int r = 0; r < 16; ++r) out[sp(r * es)] = x[r];
+    for (int r = 0; r < 16; ++r) out[sp(r * es)] = x[r];
+  }
   __syncthreads();
-  if (log2n > 8) stockham_pass<T, 16, INV, ES1, PT>(buf, n, 16, tps, lt, base, es, true, tw);
+  if (log2n > 8) stockham_pass<T, 16, INV, ES1, PT>(buf, n, 16, tps, lt, base, es, active, tw);
+  if (!active) return;
   const cx<T>* in = buf + sp(base + lt * es);
   const int p = log2n > 8 ? 256 : 16;
   switch (log2n & 3) {

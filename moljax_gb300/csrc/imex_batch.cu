@@ -99,7 +99,10 @@ __host__ __device__ __forceinline__ unsigned witem(int inst, int job, int blk) {
 // One CTA per work item (the grid is the pass's work count, fixed when the engine's
 // graph is built for the current set of solves).  A grid-stride loop over the items
 // would keep the transforms from unrolling: their register arrays then go to local
-// memory (measured with -Xptxas -v: kilobytes of spills per thread, none this way).
+// memory.  Three CTAs per SM: 80 registers hold an item without the spills of 64
+// (eight solves of 64^2 to 512^2: C1 / C2 / C3 13 / 18 / 17 us against 15 / 21 / 23,
+// the rows 12 / 9.5 / 9.8 against 14 / 11.4 / 10.7; lengths at run time and elements in
+// shared memory between the transforms 16 / 24 / 19 and 17 / 13.8 / 12.9).
 template <int PASS>
 __device__ __forceinline__ void bcol_item(float2* buf, const BInst* I, unsigned it) {
   const int job = (it >> 16) & 15, tile = it & 0xffff;
@@ -108,18 +111,24 @@ __device__ __forceinline__ void bcol_item(float2* buf, const BInst* I, unsigned 
   const double h = I->st.dtc;
   MColTile t;
   t.ny = I->ny; t.log2ny = I->log2ny; t.ncols = I->ncols; t.C = I->colC;
-  t.type = PASS == BPASS_C1 ? MC_SPLIT : (PASS == BPASS_C3 ? MC_HALF_END : MC_MID_BOTH);
   t.kx0 = tile * I->colC;
   t.ldc = I->ldc; t.off = (long long)f * I->fs;
   t.ys_cur = I->ys[cur]; t.ys_next = I->ys[1 - cur];
   t.pa = I->pa; t.pb = I->pb; t.za = I->za; t.zb = I->zb;
   t.lamx = I->lamx; t.lamy = I->lamy; t.tw = I->twy;
   t.hA = (float)(0.5 * h * I->D[f]); t.hB = (float)(0.25 * h * I->D[f]); t.nrm = I->inv_norm;
-  mcol_tile(buf, t, threadIdx.x, BT);
+  constexpr int TYPE = PASS == BPASS_C1 ? MC_SPLIT : (PASS == BPASS_C3 ? MC_HALF_END : MC_MID);
+  switch (t.log2ny) {  // colC = 2048 / ny
+    case 6: mcol_tile<TYPE, 6, 32>(buf, t, threadIdx.x); break;
+    case 7: mcol_tile<TYPE, 7, 16>(buf, t, threadIdx.x); break;
+    case 8: mcol_tile<TYPE, 8, 8>(buf, t, threadIdx.x); break;
+    case 9: mcol_tile<TYPE, 9, 4>(buf, t, threadIdx.x); break;
+    default: mcol_tile<TYPE>(buf, t, threadIdx.x); break;
+  }
 }
 
 template <int PASS>
-__global__ void __launch_bounds__(BT, 4) bcol_kernel(const __grid_constant__ BArgs a) {
+__global__ void __launch_bounds__(BT, 3) bcol_kernel(const __grid_constant__ BArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float2* buf = reinterpret_cast<float2*>(smem_raw);
   const BEng* eng = a.eng;
@@ -139,12 +148,14 @@ __global__ void __launch_bounds__(BT, 4) bcol_kernel(const __grid_constant__ BAr
 // row spectrum (ZA or ZB) -> c2r -> Heun reaction increment of step hfac*dtc -> r2c.
 // R3: the pair (error row, solution row) of one field -> (e / (atol + rtol |y|))^2 summed
 // into the item's partial.
-template <int PASS>
+// A thread keeps its 16 elements in registers (fft_regs); shared memory holds the mirrored half of
+// the spectra besides the exchanges.  LOG2N > 0: compile-time row length.
+template <int PASS, int LOG2N = 0>
 __device__ __forceinline__ void brow_item(float2* buf, const BInst* I, unsigned it) {
   const int tid = threadIdx.x;
   {
     const int kind = (it >> 16) & 15, blk = it & 0xffff;
-    const int n = I->nx, half = n >> 1, log2n = I->log2nx;
+    const int n = LOG2N ? (1 << LOG2N) : I->nx, half = n >> 1, log2n = LOG2N ? LOG2N : I->log2nx;
     const int tps = n >> 4;
     const int nseq = I->rseq;
     const int s_loc = tid / tps, lt = tid - s_loc * tps;
@@ -165,6 +176,8 @@ __device__ __forceinline__ void brow_item(float2* buf, const BInst* I, unsigned 
     }
     const int zb0 = s_loc * n;
 #define Z(x) buf[sp(zb0 + (x))]
+    float2* zt = buf + sp(zb0 + lt);
+    float2 x[16];
     if (active) {
       const float2* A = base + sa + y * ldc;
       const float2* B = base + sb + y * ldc;
@@ -178,13 +191,19 @@ __device__ __forceinline__ void brow_item(float2* buf, const BInst* I, unsigned 
       for (int m = 0; m < 9; ++m) {
         const int kk = lt + m * tps;
         if (kk <= half) {
-          Z(kk) = fmk(Ak[m].x - Bk[m].y, Ak[m].y + Bk[m].x);                                  // A_k + i B_k
-          if (kk > 0 && kk < half) Z(n - kk) = fmk(Ak[m].x + Bk[m].y, Bk[m].x - Ak[m].y);    // conj(A_k) + i conj(B_k)
+          x[m] = fmk(Ak[m].x - Bk[m].y, Ak[m].y + Bk[m].x);                                // A_k + i B_k
+          if (kk > 0 && kk < half) Z(n - kk) = fmk(Ak[m].x + Bk[m].y, Bk[m].x - Ak[m].y);  // conj(A_k) + i conj(B_k)
         }
       }
     }
     __syncthreads();
-    fft_smem<float, true, false>(buf, n, log2n, nseq, n, 1, I->twx, tid);
+    if (active) {
+#pragma unroll
+      for (int m = 8; m < 16; ++m)
+        if (lt + m * tps > half) x[m] = zt[sp(m * tps)];
+    }
+    __syncthreads();
+    fft_regs<float, true, true>(x, buf, n, log2n, lt, zb0, 1, I->twx, active);
     if (PASS == BPASS_R3) {
       const float atol = (float)I->pid.atol, rtol = (float)I->pid.rtol;
       float esum = 0.f;
@@ -192,9 +211,7 @@ __device__ __forceinline__ void brow_item(float2* buf, const BInst* I, unsigned 
       if (active) {
 #pragma unroll
         for (int m = 0; m < 16; ++m) {
-          const int x = lt + m * tps;
-          if (x >= n) continue;
-          const float2 v = Z(x);
+          const float2 v = x[m];
           const float d = v.x / (atol + rtol * fabsf(v.y));
           esum += d * d;
           bad |= !(isfinite(v.x) && isfinite(v.y));
@@ -229,16 +246,20 @@ __device__ __forceinline__ void brow_item(float2* buf, const BInst* I, unsigned 
       if (active) {
 #pragma unroll
         for (int m = 0; m < 16; ++m) {
-          const int x = lt + m * tps;
-          if (x >= n) continue;
-          const float2 v = Z(x);
-          float va = v.x, vb = v.y;
+          float va = x[m].x, vb = x[m].y;
           react_delta<float, RX_GRAY_SCOTT>(va, vb, h, pF, pK, pR);
-          Z(x) = fmk(va, vb);
+          x[m] = fmk(va, vb);
         }
       }
       __syncthreads();
-      fft_smem<float, false, false>(buf, n, log2n, nseq, n, 1, I->twx, tid);
+      fft_regs<float, false, true>(x, buf, n, log2n, lt, zb0, 1, I->twx, active);
+      __syncthreads();
+      if (active) {
+#pragma unroll
+        for (int m = 8; m < 16; ++m)
+          if (lt + m * tps > half) zt[sp(m * tps)] = x[m];
+      }
+      __syncthreads();
       if (active) {
         float2* A = const_cast<float2*>(base) + sa + y * ldc;
         float2* B = const_cast<float2*>(base) + sb + y * ldc;
@@ -246,7 +267,7 @@ __device__ __forceinline__ void brow_item(float2* buf, const BInst* I, unsigned 
         for (int m = 0; m < 9; ++m) {
           const int kk = lt + m * tps;
           if (kk > half) continue;
-          const float2 Zk = Z(kk), Zm = Z((n - kk) & (n - 1));
+          const float2 Zk = x[m], Zm = kk > 0 && kk < half ? Z(n - kk) : Zk;
           A[kk] = fmk(0.5f * (Zk.x + Zm.x), 0.5f * (Zk.y - Zm.y));
           B[kk] = fmk(0.5f * (Zk.y + Zm.y), 0.5f * (Zm.x - Zk.x));
         }
@@ -257,7 +278,7 @@ __device__ __forceinline__ void brow_item(float2* buf, const BInst* I, unsigned 
 }
 
 template <int PASS>
-__global__ void __launch_bounds__(BT, 4) brow_kernel(const __grid_constant__ BArgs a) {
+__global__ void __launch_bounds__(BT, 3) brow_kernel(const __grid_constant__ BArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float2* buf = reinterpret_cast<float2*>(smem_raw);
   const BEng* eng = a.eng;
@@ -269,7 +290,13 @@ __global__ void __launch_bounds__(BT, 4) brow_kernel(const __grid_constant__ BAr
   const unsigned it = work[w];
   const BInst* I = a.tab + (it >> 20);
   if (I->st.done) return;  // uniform over the CTA
-  brow_item<PASS>(buf, I, it);
+  switch (I->log2nx) {
+    case 6: brow_item<PASS, 6>(buf, I, it); break;
+    case 7: brow_item<PASS, 7>(buf, I, it); break;
+    case 8: brow_item<PASS, 8>(buf, I, it); break;
+    case 9: brow_item<PASS, 9>(buf, I, it); break;
+    default: brow_item<PASS>(buf, I, it); break;
+  }
 }
 
 // ------------------------------------------------------------------ controller
@@ -571,7 +598,7 @@ mjx_status mjx_gsbatch_create(void** batch, int max_instances, int max_work, voi
   if (ce == cudaSuccess) { *B->h_stop = 0; ce = cudaHostGetDevicePointer((void**)&B->d_stop, B->h_stop, 0); }
   if (ce != cudaSuccess) { set_last_error(ce, __FILE__, __LINE__); free_batch(B); return MJX_CUDA_ERROR; }
   B->h_eng.host_stop = B->d_stop;
-  B->smem = (size_t)sp_size(4096) * sizeof(float2);
+  B->smem = mcol_smem(1, 2048);  // every column tile has ny C <= 2048, every row item 4096 points
   st = batch_attrs(B->smem);
   if (st == MJX_OK) {  // every slot of the device table starts free (done)
     ce = cudaMemcpy(B->args.tab, B->h_tab.data(), sizeof(BInst) * max_instances, cudaMemcpyHostToDevice);

@@ -58,8 +58,8 @@ struct MColArgs {
   MJob job[8];
 };
 
-// LOG2NY, CN: compile-time column length and tile width (mcol_tile), launched with NT threads
-template <int NT, int MINB, int LOG2NY = 0, int CN = 0>
+// LOG2NY, CN: compile-time column length and tile width (mcol_tile)
+template <int TYPE, int NT, int MINB, int LOG2NY = 0, int CN = 0>
 __global__ void __launch_bounds__(NT, MINB) mcol_kernel(const __grid_constant__ MColArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float2* buf = reinterpret_cast<float2*>(smem_raw);
@@ -69,14 +69,14 @@ __global__ void __launch_bounds__(NT, MINB) mcol_kernel(const __grid_constant__ 
   const int cur = st != nullptr ? st->cur : 0;
   const double h = st != nullptr ? st->dtc : a.hfixed;
   MColTile t;
-  t.ny = a.ny; t.log2ny = a.log2ny; t.ncols = a.ncols; t.C = a.C; t.type = jb.type;
+  t.ny = a.ny; t.log2ny = a.log2ny; t.ncols = a.ncols; t.C = a.C;
   t.kx0 = blockIdx.x * a.C;
   t.ldc = a.ldc; t.off = jb.off;
   t.ys_cur = a.ys[cur]; t.ys_next = a.ys[1 - cur];
   t.pa = a.pa; t.pb = a.pb; t.za = a.za; t.zb = a.zb;
   t.lamx = a.lamx; t.lamy = a.lamy; t.tw = a.tw;
   t.hA = (float)(0.5 * h * jb.D); t.hB = (float)(0.25 * h * jb.D); t.nrm = a.inv_norm;
-  mcol_tile<LOG2NY, CN, LOG2NY ? NT : 0>(buf, t, threadIdx.x, blockDim.x);
+  mcol_tile<TYPE, LOG2NY, CN>(buf, t, threadIdx.x);
 }
 
 __global__ void f32_to_f64(const float* in, double* out, long long n) {
@@ -161,7 +161,7 @@ static MixAttempt build_mix(const void* plan32, const mjx_grid2d* g, const mjx_i
   // column tile width: the widest C with 2 C ny/16 <= cap threads and <= 200 KB of smem
   auto tile = [&](int cap) {
     int C = 8;
-    while (C > 1 && (2 * C * tps > cap || (size_t)sp_size(g->ny * 2 * C) * 8 > 200 * 1024)) C >>= 1;
+    while (C > 1 && (2 * C * tps > cap || mcol_smem(g->ny, C) > 200 * 1024)) C >>= 1;
     return C;
   };
   c.C = tile(kColCap[1]);
@@ -179,9 +179,9 @@ static MixAttempt build_mix(const void* plan32, const mjx_grid2d* g, const mjx_i
     MJob j;
     memset(&j, 0, sizeof(j));
     j.off = (long long)f * L.fs; j.D = D;
-    j.type = MC_SPLIT; A.c1.job[A.c1.njobs++] = j;
-    j.type = MC_MID_BOTH; A.c2.job[A.c2.njobs++] = j;  // MC_FULL_END + MC_HALF_MID, one tile
-    j.type = MC_HALF_END; A.c3.job[A.c3.njobs++] = j;
+    A.c1.job[A.c1.njobs++] = j;
+    A.c2.job[A.c2.njobs++] = j;
+    A.c3.job[A.c3.njobs++] = j;
   }
   // row passes over the FP32 row spectra ZA/ZB (contiguous: ZB = ZA + zoff)
   const long long zoff = (long long)((L.zb - L.za) / sizeof(float2));
@@ -225,15 +225,34 @@ static MixAttempt build_mix(const void* plan32, const mjx_grid2d* g, const mjx_i
   return A;
 }
 
+template <int TYPE>
 static cudaError_t mcol(const MColArgs& c, cudaStream_t s) {
   const int tps = c.ny >= 16 ? c.ny / 16 : 1;
-  const size_t smem = (size_t)sp_size(c.ny * 2 * c.C) * sizeof(float2);
+  const size_t smem = mcol_smem(c.ny, c.C);
   dim3 grid((c.ncols + c.C - 1) / c.C, c.njobs);
   const int nt = 2 * c.C * tps;
-  if (c.ny == 1024 && c.C == 4 && nt == 512) mcol_kernel<512, 2, 10, 4><<<grid, nt, smem, s>>>(c);
-  else if (nt <= 256) mcol_kernel<256, 4><<<grid, nt, smem, s>>>(c);
-  else mcol_kernel<512, 2><<<grid, nt, smem, s>>>(c);
+  if (c.ny == 4096 && c.C == 1) mcol_kernel<TYPE, 512, 2, 12, 1><<<grid, nt, smem, s>>>(c);
+  else if (c.ny == 2048 && c.C == 2) mcol_kernel<TYPE, 512, 2, 11, 2><<<grid, nt, smem, s>>>(c);
+  else if (c.ny == 1024 && c.C == 4) mcol_kernel<TYPE, 512, 2, 10, 4><<<grid, nt, smem, s>>>(c);
+  else if (c.ny == 512 && c.C == 8) mcol_kernel<TYPE, 512, 2, 9, 8><<<grid, nt, smem, s>>>(c);
+  else if (c.ny == 256 && c.C == 8) mcol_kernel<TYPE, 256, 4, 8, 8><<<grid, nt, smem, s>>>(c);
+  else if (c.ny == 128 && c.C == 8) mcol_kernel<TYPE, 256, 4, 7, 8><<<grid, nt, smem, s>>>(c);
+  else if (c.ny == 64 && c.C == 8) mcol_kernel<TYPE, 256, 4, 6, 8><<<grid, nt, smem, s>>>(c);
+  else if (nt <= 256) mcol_kernel<TYPE, 256, 4><<<grid, nt, smem, s>>>(c);
+  else mcol_kernel<TYPE, 512, 2><<<grid, nt, smem, s>>>(c);
   return cudaGetLastError();
+}
+
+template <int TYPE>
+static mjx_status mcol_attrs(int optin) {
+  const void* k[9] = {(const void*)mcol_kernel<TYPE, 512, 2, 12, 1>, (const void*)mcol_kernel<TYPE, 512, 2, 11, 2>,
+                      (const void*)mcol_kernel<TYPE, 512, 2, 10, 4>, (const void*)mcol_kernel<TYPE, 512, 2, 9, 8>,
+                      (const void*)mcol_kernel<TYPE, 256, 4, 8, 8>, (const void*)mcol_kernel<TYPE, 256, 4, 7, 8>,
+                      (const void*)mcol_kernel<TYPE, 256, 4, 6, 8>, (const void*)mcol_kernel<TYPE, 256, 4>,
+                      (const void*)mcol_kernel<TYPE, 512, 2>};
+  for (int i = 0; i < 9; ++i)
+    MJX_CUDA_TRY(cudaFuncSetAttribute(k[i], cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+  return MJX_OK;
 }
 
 static cudaError_t mrow(const RowArgs<float>& r, int rx, cudaStream_t s) {
@@ -246,11 +265,11 @@ static constexpr int kCondUnroll = 4;
 
 static cudaError_t launch_mix_attempt(const MixAttempt& A, cudaStream_t s) {
   cudaError_t e;
-  if ((e = mcol(A.c1, s)) != cudaSuccess) return e;
+  if ((e = mcol<MC_SPLIT>(A.c1, s)) != cudaSuccess) return e;
   if ((e = mrow(A.r1, A.rx, s)) != cudaSuccess) return e;
-  if ((e = mcol(A.c2, s)) != cudaSuccess) return e;
+  if ((e = mcol<MC_MID>(A.c2, s)) != cudaSuccess) return e;
   if ((e = mrow(A.r2, A.rx, s)) != cudaSuccess) return e;
-  if ((e = mcol(A.c3, s)) != cudaSuccess) return e;
+  if ((e = mcol<MC_HALF_END>(A.c3, s)) != cudaSuccess) return e;
   return mrow(A.r3, RX_NONE, s);
 }
 
@@ -351,9 +370,9 @@ mjx_status ensure_mix_attrs() {
     int dev = 0, optin = 0;
     MJX_CUDA_TRY(cudaGetDevice(&dev));
     MJX_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    MJX_CUDA_TRY(cudaFuncSetAttribute(mcol_kernel<256, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
-    MJX_CUDA_TRY(cudaFuncSetAttribute(mcol_kernel<512, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
-    MJX_CUDA_TRY(cudaFuncSetAttribute(mcol_kernel<512, 2, 10, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+    MJX_TRY(mcol_attrs<MC_SPLIT>(optin));
+    MJX_TRY(mcol_attrs<MC_MID>(optin));
+    MJX_TRY(mcol_attrs<MC_HALF_END>(optin));
     return MJX_OK;
   });
 }
@@ -400,11 +419,11 @@ mjx_status mjx_imex_mixed_attempt_kernel2d(const void* plan32, const void* plan6
   const MixAttempt A = build_mix(plan32, g, pb, pid, w, L, st);
   cudaError_t e;
   switch (which) {
-    case 1: e = mcol(A.c1, s); break;
+    case 1: e = mcol<MC_SPLIT>(A.c1, s); break;
     case 2: e = mrow(A.r1, A.rx, s); break;
-    case 3: e = mcol(A.c2, s); break;
+    case 3: e = mcol<MC_MID>(A.c2, s); break;
     case 4: e = mrow(A.r2, A.rx, s); break;
-    case 5: e = mcol(A.c3, s); break;
+    case 5: e = mcol<MC_HALF_END>(A.c3, s); break;
     case 6: e = mrow(A.r3, RX_NONE, s); break;
     case 7: {  // the controller
       CtlArgs ca;

@@ -8,9 +8,9 @@
 
 namespace mjx {
 
-// MC_MID_BOTH is MC_FULL_END and MC_HALF_MID of the same columns in one tile (ZA in the
-// left half, ZB in the right half): the C2 pass then needs half the CTAs
-enum { MC_SPLIT = 0, MC_FULL_END = 1, MC_HALF_MID = 2, MC_HALF_END = 3, MC_MID_BOTH = 4 };
+// The three column passes of an attempt.  The two halves of a CTA's threads take the full step
+// (A) and the half steps (B) of the same columns.
+enum { MC_SPLIT = 0, MC_MID = 1, MC_HALF_END = 2 };
 
 __device__ __forceinline__ float2 fmk(float x, float y) { float2 r; r.x = x; r.y = y; return r; }
 
@@ -69,7 +69,7 @@ __device__ __forceinline__ float4 ff_add_c(float4 X, float2 d) {
 // fills it from MColArgs, the batched kernel (csrc/imex_batch.cu) from its
 // instance table.
 struct MColTile {
-  int ny, log2ny, ncols, C, type, kx0;
+  int ny, log2ny, ncols, C, kx0;
   long long ldc, off;       // row stride; field offset shared by every buffer
   const float4* ys_cur;     // state Y^[cur]
   float4* ys_next;          // state Y^[1-cur]
@@ -83,133 +83,93 @@ struct MColTile {
   float hA, hB, nrm;        // dt/2 D, dt/4 D, 1/(nx ny)
 };
 
-// One tile: C adjacent kx columns of one job over all ny rows.  Threads per CTA
-// = 2 C ny/16, so every thread combines exactly min(8, ny/2) elements.  The state
-// operands are read in the combine loop rather than held across the forward
-// transform: 64 registers, so four 256-thread CTAs share an SM and hide each
-// other's load latency (the column passes are latency-bound at 1024^2, where the
-// whole working set sits in L2).  Only ny = 4096 needs 512-thread CTAs.
-// The caller synchronises the block before buf is reused for another tile.
-// LOG2NY, CN, NTH > 0 fix the column length, the tile width and the thread count at compile
-// time (the 1024-row passes of the benchmark size), so that the index arithmetic and the
-// transforms' radix schedule fold into the code; 0 reads them at run time.
-__host__ __device__ constexpr int mc_log2(int v) { return v <= 1 ? 0 : 1 + mc_log2(v >> 1); }
+// shared memory of a tile: the two halves side by side
+inline size_t mcol_smem(int ny, int C) { return 2 * (size_t)sp_size(ny * C) * sizeof(float2); }
 
-template <int LOG2NY = 0, int CN = 0, int NTH = 0>
-__device__ __forceinline__ void mcol_tile(float2* buf, const MColTile& t, int tid, int nth_rt) {
-  // the tile holds two outputs side by side (W = 2C) where a job writes two transforms
-  // (C1 split, C3 end); the single-output jobs of C2 use a compact tile (W = C), whose
-  // column transforms then walk shared memory with half the stride
-  const int type = t.type;
-  const int nth = NTH ? NTH : nth_rt;
-  const int Cn = CN ? CN : t.C, W = (type == MC_FULL_END || type == MC_HALF_MID) ? Cn : 2 * Cn;
-  const int kx0 = t.kx0;
-  const int ny = LOG2NY ? (1 << LOG2NY) : t.ny;
-  const int log2ny = LOG2NY ? LOG2NY : t.log2ny;
-  const int total = ny * Cn;
-  const int lc = CN ? mc_log2(CN) : __ffs(Cn) - 1;  // the tile width is a power of two
-  const long long ldc = t.ldc;
-  const float hA = t.hA, hB = t.hB, nrm = t.nrm;
+// One tile: C adjacent kx columns of one field over all ny rows, C ny/16 threads (C below 16
+// rows) for each half.  A thread holds its 16 elements in registers from the load to the store
+// (fft_regs; 64 registers, so that four 256-thread or two 512-thread CTAs share an SM and hide
+// each other's L2 latency, which bounds these passes at 1024^2), the operands of NB elements at a
+// time.  C3 runs its forward transform and its update in both halves: the idle half would save
+// nothing and the exchange costs two barriers.
+//   C1 MC_SPLIT     PA = M_A Y, PB = M_B Y; ZA, ZB <- inverse of both
+//   C2 MC_MID       PA <- M_A (PA + F ZA);  PB <- M_B^2 (PB + F ZB), ZB <- its inverse
+//   C3 MC_HALF_END  Y' = M_B (PB + F ZB); ZA <- inverse of Y' - PA, ZB <- inverse of Y'
+// LOG2NY, CN > 0 fix the column length and the tile width at compile time (the lengths 64 to
+// 4096, in the batch 64 to 512), so that the index arithmetic and the radix schedule fold into
+// the code.  C1 / C2 / C3 at 1024^2: 14 / 20 / 21 us, against 24 us each with every element in
+// shared memory between the transforms; 256^2 1.8x a solve.  Four operands in flight beat two in
+// C1 (13.6 against 14.6 us) and lose in C2 and C3, where they spill (24 us).
+template <int TYPE, int LOG2NY = 0, int CN = 0>
+__device__ __forceinline__ void mcol_tile(float2* buf, const MColTile& t, int tid) {
+  const int ny = LOG2NY ? (1 << LOG2NY) : t.ny, log2ny = LOG2NY ? LOG2NY : t.log2ny;
+  const int Cn = CN ? CN : t.C;  // a power of two
+  const int tps = ny >= 16 ? ny >> 4 : 1, per = Cn * tps;
+  const bool right = tid >= per, active = tid < 2 * per;
+  const int r = right ? tid - per : tid, c = r & (Cn - 1), lt = r >> (__ffs(Cn) - 1);
+  const int kx = t.kx0 + c, ldc = (int)t.ldc;
+  const bool in = active && kx < t.ncols;
+  const long long g0 = t.off + (long long)lt * ldc + kx;
+  const int gs = tps * ldc;
+  float2* half = buf + (right ? sp_size(ny * Cn) : 0);
+  const float nrm = t.nrm, lx = in ? t.lamx[kx] : 0.f;
+  const float* lamy = t.lamy + lt;
+  float2 x[16];
+#pragma unroll
+  for (int q = 0; q < 16; ++q) x[q] = fmk(0.f, 0.f);
 
-  if (type != MC_SPLIT) {
-    // load the FP32 increment tile(s) and transform them forward along y
-    const int halves = type == MC_MID_BOTH ? 2 : 1;
-    for (int hf = 0; hf < halves; ++hf) {
-      const float2* zin = (type == MC_FULL_END || (type == MC_MID_BOTH && hf == 0)) ? t.za : t.zb;
-      float2 v[8];
+  if (TYPE != MC_SPLIT) {
+    const float2* z = ((TYPE == MC_MID && !right) ? t.za : t.zb) + g0;
+    if (in) {
 #pragma unroll
-      for (int m = 0; m < 8; ++m) {
-        const int e = tid + m * nth;
-        const int ky = e >> lc, c = e & (Cn - 1), kx = kx0 + c;
-        if (e < total) v[m] = kx < t.ncols ? zin[t.off + ky * ldc + kx] : fmk(0.f, 0.f);
-      }
-#pragma unroll
-      for (int m = 0; m < 8; ++m) {
-        const int e = tid + m * nth;
-        const int ky = e >> lc, c = e & (Cn - 1);
-        if (e < total) buf[sp(ky * W + hf * Cn + c)] = v[m];
-      }
+      for (int q = 0; q < 16; ++q)
+        if (q * tps < ny) x[q] = z[q * gs];
     }
-    __syncthreads();
-    if (LOG2NY) fft_smem_inl<float, false, true>(buf, ny, log2ny, type == MC_MID_BOTH ? W : Cn, 1, W, t.tw, tid);
-    else fft_smem<float, false, true>(buf, ny, log2ny, type == MC_MID_BOTH ? W : Cn, 1, W, t.tw, tid);
+    fft_regs<float, false, false>(x, half, ny, log2ny, lt, c, Cn, t.tw, active);
   }
 
-  // float-float combine, element by element
+  // float-float combine
+  const bool two = TYPE == MC_HALF_END && !right;  // two operands
+  const float4* op = (TYPE == MC_SPLIT ? t.ys_cur : ((TYPE == MC_MID && !right) ? t.pa : t.pb)) + g0;
+  const float4* oq = t.pa + g0;
+  float4* res = (TYPE == MC_HALF_END ? t.ys_next : (right ? t.pb : t.pa)) + g0;
+  const float hD = (TYPE == MC_HALF_END || right) ? t.hB : t.hA;
+  constexpr int NB = TYPE == MC_SPLIT ? 4 : 2;  // elements whose operands are in flight together
+  if (in) {
 #pragma unroll
-  for (int m = 0; m < 8; ++m) {
-    const int e = tid + m * nth;
-    if (e >= total) continue;
-    const int ky = e >> lc, c = e & (Cn - 1), kx = kx0 + c;
-    if (kx >= t.ncols) {
-      buf[sp(ky * W + c)] = fmk(0.f, 0.f);
-      if (W > Cn) buf[sp(ky * W + Cn + c)] = fmk(0.f, 0.f);
-      continue;
-    }
-    const long long g = t.off + ky * ldc + kx;
-    const float lam = t.lamx[kx] + t.lamy[ky];
-    float4 Pm, Qm;
-    if (type == MC_SPLIT) Pm = t.ys_cur[g];
-    else if (type == MC_FULL_END || type == MC_MID_BOTH) Pm = t.pa[g];
-    else Pm = t.pb[g];
-    if (type == MC_HALF_END) Qm = t.pa[g];
-    if (type == MC_MID_BOTH) Qm = t.pb[g];
-    if (type == MC_MID_BOTH) {  // MC_FULL_END on the left half, MC_HALF_MID on the right
-      const float2 d = buf[sp(ky * W + c)], d2 = buf[sp(ky * W + Cn + c)];
-      t.pa[g] = ff_mstep_c(ff_add_c(Pm, d), mu_of(hA, lam));
-      const float mu = mu_of(hB, lam);
-      const float4 X = ff_mstep_c(ff_mstep_c(ff_add_c(Qm, d2), mu), mu);
-      t.pb[g] = X;
-      buf[sp(ky * W + Cn + c)] = fmk(ff_scaled(ff_re(X), nrm), ff_scaled(ff_im(X), nrm));
-    } else if (type == MC_SPLIT) {
-      const float4 PA = ff_mstep_c(Pm, mu_of(hA, lam)), PB = ff_mstep_c(Pm, mu_of(hB, lam));
-      t.pa[g] = PA;
-      t.pb[g] = PB;
-      buf[sp(ky * W + c)] = fmk(ff_scaled(ff_re(PA), nrm), ff_scaled(ff_im(PA), nrm));
-      buf[sp(ky * W + Cn + c)] = fmk(ff_scaled(ff_re(PB), nrm), ff_scaled(ff_im(PB), nrm));
-    } else {
-      const float2 d = buf[sp(ky * W + c)];
-      if (type == MC_FULL_END) {
-        t.pa[g] = ff_mstep_c(ff_add_c(Pm, d), mu_of(hA, lam));
-      } else if (type == MC_HALF_MID) {
-        const float mu = mu_of(hB, lam);
-        const float4 X = ff_mstep_c(ff_mstep_c(ff_add_c(Pm, d), mu), mu);
-        t.pb[g] = X;
-        buf[sp(ky * W + c)] = fmk(ff_scaled(ff_re(X), nrm), ff_scaled(ff_im(X), nrm));
-      } else {  // MC_HALF_END
-        const float4 X = ff_mstep_c(ff_add_c(Pm, d), mu_of(hB, lam));
-        t.ys_next[g] = X;
-        const float4 Fa = Qm;
-        buf[sp(ky * W + c)] = fmk(ff_diff_scaled(ff_re(X), ff_re(Fa), nrm),
-                                  ff_diff_scaled(ff_im(X), ff_im(Fa), nrm));
-        buf[sp(ky * W + Cn + c)] = fmk(ff_scaled(ff_re(X), nrm), ff_scaled(ff_im(X), nrm));
+    for (int q0 = 0; q0 < 16; q0 += NB) {
+      float4 P[NB], Q[NB];
+      float lam[NB];
+#pragma unroll
+      for (int h = 0; h < NB; ++h) {
+        const int q = q0 + h;
+        if (q * tps >= ny) continue;
+        P[h] = op[q * gs];
+        if (two) Q[h] = oq[q * gs];
+        lam[h] = lx + lamy[q * tps];
+      }
+#pragma unroll
+      for (int h = 0; h < NB; ++h) {
+        const int q = q0 + h;
+        if (q * tps >= ny) continue;
+        const float mu = mu_of(hD, lam[h]);
+        float4 X = TYPE == MC_SPLIT ? P[h] : ff_add_c(P[h], x[q]);
+        X = ff_mstep_c(X, mu);
+        if (TYPE == MC_MID && right) X = ff_mstep_c(X, mu);
+        if (TYPE != MC_HALF_END || right) res[q * gs] = X;
+        x[q] = two ? fmk(ff_diff_scaled(ff_re(X), ff_re(Q[h]), nrm), ff_diff_scaled(ff_im(X), ff_im(Q[h]), nrm))
+                   : fmk(ff_scaled(ff_re(X), nrm), ff_scaled(ff_im(X), nrm));
       }
     }
   }
-  if (type == MC_FULL_END) return;
-  __syncthreads();
-  if (type == MC_MID_BOTH) {  // only the right (MC_HALF_MID) half goes back
-    if (LOG2NY) fft_smem_inl<float, true, true>(buf, ny, log2ny, Cn, 1, W, t.tw, tid, Cn);
-    else fft_smem<float, true, true>(buf, ny, log2ny, Cn, 1, W, t.tw, tid, Cn);
-    for (int e = tid; e < ny * Cn; e += nth) {
-      const int ky = e >> lc, c = e & (Cn - 1), kx = kx0 + c;
-      if (kx < t.ncols) t.zb[t.off + ky * ldc + kx] = buf[sp(ky * W + Cn + c)];
-    }
-    return;
-  }
-  const int nseq = (type == MC_HALF_MID) ? Cn : W;
-  if (LOG2NY) fft_smem_inl<float, true, true>(buf, ny, log2ny, nseq, 1, W, t.tw, tid);
-  else fft_smem<float, true, true>(buf, ny, log2ny, nseq, 1, W, t.tw, tid);
-  const int lns = __ffs(nseq) - 1;
-  for (int e = tid; e < ny * nseq; e += nth) {
-    const int ky = e >> lns, col = e & (nseq - 1);
-    const int half = col >> lc, c = col & (Cn - 1), kx = kx0 + c;
-    if (kx >= t.ncols) continue;
-    const long long g = t.off + ky * ldc + kx;
-    const float2 v = buf[sp(ky * W + col)];
-    if (type == MC_HALF_MID) t.zb[g] = v;
-    else if (half == 0) t.za[g] = v;
-    else t.zb[g] = v;
+  if (TYPE != MC_SPLIT) __syncthreads();
+  const bool back = active && (TYPE != MC_MID || right);  // C2 keeps PA in spectral space
+  fft_regs<float, true, false>(x, half, ny, log2ny, lt, c, Cn, t.tw, back);
+  float2* z = (right ? t.zb : t.za) + g0;
+  if (in && back) {
+#pragma unroll
+    for (int q = 0; q < 16; ++q)
+      if (q * tps < ny) z[q * gs] = x[q];
   }
 }
 

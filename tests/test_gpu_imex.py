@@ -267,3 +267,34 @@ def test_adaptive_mixed_maximum_extent(cuda, ny, nx):
     assert rf.status == 0
     for k in ("u", "v"):
         assert _rel(rf.y_final[k].cpu().numpy(), ro.y_final[k]) < 1e-4
+
+
+@pytest.mark.parametrize("ny,nx", [(4, 16), (16, 64), (64, 512), (128, 1024), (256, 128), (512, 32), (1024, 16), (2048, 64)])
+def test_mixed_and_batched_lengths(cuda, ny, nx):
+    """Every column and row length class of the mixed passes (fewer than 16 rows, lengths at run
+    and at compile time, one to three radix passes), alone and as a batch item, against the oracle:
+    the same step counts, and the tolerance of the mixed solves above."""
+    import moljax_gb300 as M
+    L = 2.5
+    grid = M.Grid2D(nx, ny, 0.0, L, 0.0, L)
+    model, cache, diff = M.create_gray_scott_periodic_fft(grid, 2e-5, 1e-5, 0.035, 0.065, torch.float32, cuda)
+    og = mol.Grid2D(nx, ny, 0, L, 0, L)
+    y0 = mol.gray_scott_ic(og, 3)
+    ym = {k: torch.tensor(v, dtype=torch.float32, device=cuda) for k, v in y0.items()}
+    om, lam, od = OI.gray_scott_periodic(og, 2e-5, 1e-5, 0.035, 0.065)
+    pid = M.PIDParams(atol=1e-7, rtol=1e-5)
+    r = M.adaptive_integrate_imex(model, ym, 0.0, 8.0, 1.0, cache, diff, pid_params=pid, save_every=100,
+                                  save_y_history=False, precision="mixed")
+    ro = OI.adaptive_integrate_imex(om, y0, 0.0, 8.0, 1.0, lam, od, pid=OI.PIDParams(atol=1e-7, rtol=1e-5),
+                                    save_every=100, keep_history=False)
+    assert r.status == ro.status == 0
+    assert (r.n_accepted, r.n_rejected) == (ro.n_accepted, ro.n_rejected)
+    for k in ("u", "v"):
+        assert _rel(r.y_final[k].cpu().numpy(), ro.y_final[k]) < 1e-6
+    if ny < 16:
+        return
+    p = M.GrayScottProblem(grid, 2e-5, 1e-5, 0.035, 0.065, ym, 0.0, 8.0, 1.0, pid=pid, max_steps=4000, save_every=100)
+    (out, rb), = M.adaptive_integrate_imex_batch([p], cuda)
+    assert (rb.status, rb.n_accepted, rb.n_rejected) == (0, ro.n_accepted, ro.n_rejected)
+    for i, k in enumerate(("u", "v")):
+        assert _rel(out[i].cpu().numpy(), mol.interior(ro.y_final[k], og)) < 1e-6
