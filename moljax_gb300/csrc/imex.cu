@@ -209,7 +209,7 @@ static Attempt<T> build_attempt(const void* plan, const mjx_grid2d* g, const mjx
   base.nseq = row_nseq(g->nx, pg.nrows); base.rstride = g->nx;
   base.rin[0] = Y0; base.rin[1] = Y1; base.rout[0] = Y0; base.rout[1] = Y1;
   base.rin_sel = 0; base.rout_sel = 1;
-  base.eref = YF; base.spec = S; base.tw = (const cx<T>*)pv.twx; base.inv_scale = (T)1;
+  base.eref = YF; base.spec = S; base.tw = (const cx<T>*)pv.twx; base.inv_scale = (T)1; base.warp = 1;
   base.F = pb->F; base.k = pb->k; base.r = pb->r;
   base.atol = pid->atol; base.rtol = pid->rtol;
   base.partial = (double*)(ws + L.part); base.nonfinite = (int*)(ws + L.bad);

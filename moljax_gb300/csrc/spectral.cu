@@ -70,7 +70,8 @@ template <typename T> struct Occ { static constexpr int row = sizeof(T) == 4 ? 4
 // lt + m tps in registers from the load to the store (fft_regs); shared memory carries the
 // exchanges inside the transforms and the mirrored half of a spectrum, which the two-for-one
 // packing pairs with the other half.  FP32, fused (c2r, reaction, r2c), 256, 2048 and 4096 points:
-// 6.9, 58 and 100 us; through shared memory 14.7 (length at run time), 63 and 125 us.  The long
+// 6.9, 58 and 100 us; through shared memory 14.7 (length at run time), 63 and 125 us.  1024 points:
+// 13.2 us (2048 row pairs), 18.0 with 32 points a lane of one warp a row (row_kernel_w32).  The long
 // rows are bound by the SMs' issue and shared-memory bandwidth alike, the short ones by the
 // latency of one chain (load, five exchanges, store) on a few warps an SM.
 template <typename T, int RX, int LOG2N = 0>
@@ -343,7 +344,10 @@ __global__ void __launch_bounds__(ColThreads<T>::v, 1) col_kernel(const __grid_c
 
 // ------------------------------------------------------------------ warp row pass (n = 1024)
 // The row pass of row_kernel (same flags, pair table, pointwise work and error partials) for
-// FP32 rows of 1024 points, one warp per sequence.
+// FP32 rows of 1024 points, one warp per sequence: the row transform of the FP32 adaptive IMEX
+// loop.  Its error estimate is a difference of FP32 solutions, so the step sizes and with them the
+// end state follow the transform's rounding (1024^2, t = 6: 2.8e-5 apart between this kernel and
+// row_kernel); that loop keeps the transform that its results were made with.
 template <int RX>
 __global__ void __launch_bounds__(128) row_kernel_w32(const __grid_constant__ RowArgs<float> a) {
   typedef float2 C;
@@ -503,7 +507,7 @@ cudaError_t launch_row(const RowArgs<T>& a0, cudaStream_t s) {
   const int tps = a.n >= 16 ? a.n / 16 : 1;
   const int grid = a.npairs * a.nrows / a.nseq;
   if constexpr (sizeof(T) == 4) {
-    if (a.n == 1024 && a.nseq <= 4) {  // one warp per 1024-point row
+    if (a.n == 1024 && a.warp && a.nseq <= 4) {  // one warp per 1024-point row
       return launch_chain(row_kernel_w32<RX>, dim3(grid), 32 * a.nseq, (size_t)a.nseq * 32 * 33 * sizeof(float2), s,
                           a.pdl, a);
     }
@@ -513,7 +517,7 @@ cudaError_t launch_row(const RowArgs<T>& a0, cudaStream_t s) {
 #define MJX_ROW(L) case L: return launch_chain(row_kernel<T, RX, L>, dim3(grid), threads, smem, s, a.pdl, a);
   if constexpr (sizeof(T) == 4) {
     switch (a.log2n) {
-      MJX_ROW(5) MJX_ROW(6) MJX_ROW(7) MJX_ROW(8) MJX_ROW(9) MJX_ROW(11) MJX_ROW(12)
+      MJX_ROW(5) MJX_ROW(6) MJX_ROW(7) MJX_ROW(8) MJX_ROW(9) MJX_ROW(10) MJX_ROW(11) MJX_ROW(12)
       default: return launch_chain(row_kernel<T, RX>, dim3(grid), threads, smem, s, a.pdl, a);
     }
   } else {
@@ -582,6 +586,7 @@ static mjx_status row_attrs(int optin) {
   MJX_TRY(raise_smem(row_kernel<float, RX, 7>, optin));
   MJX_TRY(raise_smem(row_kernel<float, RX, 8>, optin));
   MJX_TRY(raise_smem(row_kernel<float, RX, 9>, optin));
+  MJX_TRY(raise_smem(row_kernel<float, RX, 10>, optin));
   MJX_TRY(raise_smem(row_kernel<float, RX, 11>, optin));
   MJX_TRY(raise_smem(row_kernel<float, RX, 12>, optin));
   return raise_smem(row_kernel<double, RX, 12>, optin);

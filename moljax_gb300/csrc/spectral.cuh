@@ -147,6 +147,7 @@ template <typename T> struct RowArgs {
   const T* eref;       // error reference base (same offsets as the real output)
   cx<T>* spec;         // spectrum base (read and/or written in place)
   const cx<T>* tw;     // twiddles for n
+  int warp;            // FP32 rows of 1024 points: the one-warp transform (row_kernel_w32)
   T inv_scale;         // scale applied after the inverse transform
   double hfixed;       // reaction step when st == nullptr
   double F, k, r;      // reaction parameters
