@@ -264,7 +264,7 @@ __device__ __forceinline__ void fft_regs(cx<T>* x, cx<T>* buf, int n, int log2n,
     if (log2n == 4) dft16<INV>(x);
     else if (log2n == 3) dft8<INV>(x);
     else if (log2n == 2) dft4<INV>(x[0], x[1], x[2], x[3]);
-    else dft2<INV>(x[0], x[1]);
+    else if (log2n == 1) dft2<INV>(x[0], x[1]);
     return;
   }
   if (active) {

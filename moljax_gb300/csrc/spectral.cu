@@ -262,83 +262,95 @@ __global__ void __launch_bounds__(256, Occ<T>::row) row_kernel(const __grid_cons
 // ------------------------------------------------------------------ column pass
 template <typename T> struct ColThreads { static constexpr int v = sizeof(T) == 4 ? 1024 : 512; };
 
-template <typename T>
-__global__ void __launch_bounds__(ColThreads<T>::v, 1) col_kernel(const __grid_constant__ ColArgs<T> a) {
+// C ny/16 threads (C below 16 rows) per output of a tile of C columns; a thread keeps its 16
+// elements in registers from the load to the store (fft_regs).  A second output has its own threads
+// and its own half of the shared memory, and repeats the forward transform there: the threads would
+// be idle meanwhile.  LOG2NY > 0 fixes the length at compile time.  Chained with its rows, FFT-CN
+// FP32 takes 29 us a step at 256^2 (48 with the elements in shared memory between the transforms
+// and the length at run time), 38 at 1024^2 (61).  512 and 1024 rows get 128 registers a thread
+// (their CTAs have at most 512): 12.8 and 18.9 us against 14.8 and 21.6; shorter columns fit in 64,
+// and a box's passes want the CTAs (128 rows: 25.7 us against 29.6).
+template <typename T, int LOG2NY = 0>
+__global__ void __launch_bounds__(LOG2NY == 9 || LOG2NY == 10 ? 512 : ColThreads<T>::v, 1) col_kernel(const __grid_constant__ ColArgs<T> a) {
   typedef cx<T> C;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* buf = reinterpret_cast<C*>(smem_raw);
   pdl_wait();
   if (a.st != nullptr && a.st->done) return;
   const ColJob jb = a.job[blockIdx.y];
-  const int Cn = a.C, nout = jb.nout, W = Cn * nout;
-  const int kx0 = blockIdx.x * Cn;
-  const int ny = a.ny, tid = threadIdx.x, nth = blockDim.x;
-  const int lc = __ffs(Cn) - 1;  // the tile width is a power of two (col_tile / tile halve from one)
-  const long long ldc = a.ldc;
-  const long long po = (long long)blockIdx.z * a.pstride;
+  const int ny = LOG2NY ? (1 << LOG2NY) : a.ny, log2ny = LOG2NY ? LOG2NY : a.log2ny;
+  const int Cn = a.C, tps = ny >= 16 ? ny >> 4 : 1, per = Cn * tps;  // C: a power of two
+  const int o = threadIdx.x >= per ? 1 : 0, r = threadIdx.x - o * per, c = r & (Cn - 1), lt = r >> (__ffs(Cn) - 1);
+  const int kx = blockIdx.x * Cn + c;
+  const bool active = o < jb.nout, in = active && kx < a.ncols;
+  const long long ldc = a.ldc, po = (long long)blockIdx.z * a.pstride;
+  C* buf = reinterpret_cast<C*>(smem_raw) + o * sp_size(ny * Cn);
+  C x[16];
 
-  {
-    C v[16];
+  const C* src = a.spec + po + jb.sin + kx;
 #pragma unroll
-    for (int m = 0; m < 16; ++m) {
-      const int e = tid + m * nth;
-      const int ky = e >> lc, c = e & (Cn - 1), kx = kx0 + c;
-      const bool mir = a.oddy && ky >= (ny >> 1);
-      const int kyl = mir ? ny - 1 - ky : ky;
-      if (e < ny * Cn) {
-        v[m] = kx < a.ncols ? a.spec[po + jb.sin + kyl * ldc + kx] : mk<C>((T)0, (T)0);
-        if (mir) v[m] = mk<C>(-v[m].x, -v[m].y);
-      }
-    }
-#pragma unroll
-    for (int m = 0; m < 16; ++m) {
-      const int e = tid + m * nth;
-      const int ky = e >> lc, c = e & (Cn - 1);
-      if (e < ny * Cn) buf[sp(ky * W + c)] = v[m];
+  for (int q = 0; q < 16; ++q) {
+    const int ky = lt + q * tps;
+    x[q] = mk<C>((T)0, (T)0);
+    if (!in || ky >= ny) continue;
+    if (a.oddy && ky >= (ny >> 1)) {
+      const C v = src[(ny - 1 - ky) * ldc];
+      x[q] = mk<C>(-v.x, -v.y);
+    } else {
+      x[q] = src[ky * ldc];
     }
   }
-  __syncthreads();
   const int dirs = jb.dirs ? jb.dirs : 3;
-  if (dirs & 1) {
-    fft_smem<T, false, true>(buf, ny, a.log2ny, Cn, 1, W, a.tw, tid);
-  }
+  if (dirs & 1) fft_regs<T, false, false>(x, buf, ny, log2ny, lt, c, Cn, a.tw, active);
+
   const T jscale = jb.scale != 0.0 ? (T)jb.scale : a.scale;
-
   const double h = a.st != nullptr ? a.st->dtc : a.hfixed;
-  const T hD0 = (T)(h * jb.hfac[0] * jb.D), hD1 = (T)(h * jb.hfac[1] * jb.D);
-  for (int e = tid; e < ny * Cn; e += nth) {
-    const int ky = e >> lc, c = e & (Cn - 1), kx = kx0 + c;
-    T lxy = (T)0;
-    if (kx < a.ncols) lxy = a.ldc3 ? a.lamx[kx % a.ldc3] + a.lamy2[kx / a.ldc3] : a.lamx[kx];
-    const T lam = lxy + a.lamy[ky];
-    const C v = buf[sp(ky * W + c)];
-    if (jb.mul == MUL_ADVDIFF || jb.mul == MUL_ADV_LAP || jb.mul == MUL_ADV_EXP || jb.mul == MUL_ADV_CN) {
-      const double2 f = adv_multiplier<T>(a, jb, (double)hD0, h * jb.hfac[0], (double)lam, kx, ky);
-      const T mr = (T)f.x, mi = (T)f.y;
-      buf[sp(ky * W + c)] = cscale(mk<C>(v.x * mr - v.y * mi, v.x * mi + v.y * mr), jscale);
-      continue;
+  const T hD = (T)(h * jb.hfac[o] * jb.D);
+  T lxy = (T)0;
+  if (in) lxy = a.ldc3 ? a.lamx[kx % a.ldc3] + a.lamy2[kx / a.ldc3] : a.lamx[kx];
+  if (jb.mul == MUL_ADVDIFF || jb.mul == MUL_ADV_LAP || jb.mul == MUL_ADV_EXP || jb.mul == MUL_ADV_CN) {
+    // one copy of the complex multiplier's code: the elements pass through their places in shared memory
+    C* own = buf + sp(lt * Cn + c);
+    __syncthreads();
+    if (in) {
+#pragma unroll
+      for (int q = 0; q < 16; ++q)
+        if (q * tps < ny) own[sp(q * tps * Cn)] = x[q];
+#pragma unroll 1
+      for (int ky = lt, q = 0; ky < ny && q < 16; ky += tps, ++q) {
+        const double2 f = adv_multiplier<T>(a, jb, (double)hD, h * jb.hfac[0], (double)(lxy + a.lamy[ky]), kx, ky);
+        const T mr = (T)f.x, mi = (T)f.y;
+        C& e = own[sp(q * tps * Cn)];
+        e = cscale(mk<C>(e.x * mr - e.y * mi, e.x * mi + e.y * mr), jscale);
+      }
+#pragma unroll
+      for (int q = 0; q < 16; ++q)
+        if (q * tps < ny) x[q] = own[sp(q * tps * Cn)];
     }
-    if (jb.mul == MUL_TABLED) {
-      buf[sp(ky * W + c)] = cscale(v, kx < a.ncols ? a.mtab[jb.sin + ky * ldc + kx] : (T)0);
-      continue;
+  } else {
+    const int mul = jb.mul, pw = jb.pow[o];
+    const T* tab = mul == MUL_TABLED ? a.mtab + jb.sin + kx : a.mtab + kx;
+#pragma unroll
+    for (int q = 0; q < 16; ++q) {
+      const int ky = lt + q * tps;
+      if (!in || ky >= ny) continue;
+      T m;
+      if (mul == MUL_TABLED) m = tab[ky * ldc];
+      else if (mul == MUL_TABLE) m = jscale * tab[ky * ldc];
+      else m = jscale * multiplier<T>(mul, hD, lxy + a.lamy[ky], pw);
+      x[q] = cscale(x[q], m);
     }
-    if (jb.mul == MUL_TABLE) {
-      buf[sp(ky * W + c)] = cscale(v, jscale * a.mtab[(long long)ky * ldc + kx]);
-      continue;
-    }
-    buf[sp(ky * W + c)] = cscale(v, jscale * multiplier<T>(jb.mul, hD0, lam, jb.pow[0]));
-    if (nout > 1) buf[sp(ky * W + Cn + c)] = cscale(v, jscale * multiplier<T>(jb.mul, hD1, lam, jb.pow[1]));
   }
-  __syncthreads();
   if (dirs & 2) {
-    fft_smem<T, true, true>(buf, ny, a.log2ny, W, 1, W, a.tw, tid);
+    if (dirs & 1 || jb.mul >= MUL_ADVDIFF) __syncthreads();
+    fft_regs<T, true, false>(x, buf, ny, log2ny, lt, c, Cn, a.tw, active);
   }
 
-  const int lw = __ffs(W) - 1;  // W = Cn or 2 Cn
-  for (int e = tid; e < ny * W; e += nth) {
-    const int ky = e >> lw, col = e & (W - 1);
-    const int o = col >> lc, c = col & (Cn - 1), kx = kx0 + c;
-    if (kx < a.ncols && !(a.oddy && ky >= (ny >> 1))) a.spec[po + jb.sout[o] + ky * ldc + kx] = buf[sp(ky * W + col)];
+  if (!in) return;
+  C* dst = a.spec + po + jb.sout[o] + kx;
+#pragma unroll
+  for (int q = 0; q < 16; ++q) {
+    const int ky = lt + q * tps;
+    if (ky < ny && !(a.oddy && ky >= (ny >> 1))) dst[ky * ldc] = x[q];
   }
 }
 
@@ -538,8 +550,18 @@ cudaError_t launch_col(const ColArgs<T>& a0, cudaStream_t s) {
   const long long planes = a.nplanes > 1 ? a.nplanes : 1;
   while (a.C > 1 && (long long)((a.ncols + a.C - 1) / a.C) * a.njobs * planes < 152) a.C >>= 1;
   dim3 grid((a.ncols + a.C - 1) / a.C, a.njobs, a.nplanes > 1 ? a.nplanes : 1);
-  const size_t smem = (size_t)sp_size(a.ny * a.C * maxout) * sizeof(cx<T>);
-  return launch_chain(col_kernel<T>, grid, a.C * maxout * tps, smem, s, a.pdl, a);
+  const size_t smem = (size_t)sp_size(a.ny * a.C) * maxout * sizeof(cx<T>);
+  const int threads = a.C * maxout * tps;
+#define MJX_COL(L) case L: return launch_chain(col_kernel<T, L>, grid, threads, smem, s, a.pdl, a);
+  if constexpr (sizeof(T) == 4) {
+    switch (a.log2ny) {
+      MJX_COL(5) MJX_COL(6) MJX_COL(7) MJX_COL(8) MJX_COL(9) MJX_COL(10) MJX_COL(11) MJX_COL(12)
+      default: return launch_chain(col_kernel<T>, grid, threads, smem, s, a.pdl, a);
+    }
+  } else {
+    return launch_chain(col_kernel<T, 12>, grid, threads, smem, s, a.pdl, a);  // the others: col64_takes
+  }
+#undef MJX_COL
 }
 
 #define MJX_INST_ROW(T, RX) template cudaError_t launch_row<T, RX>(const RowArgs<T>&, cudaStream_t);
@@ -607,7 +629,15 @@ mjx_status ensure_kernel_attrs() {
     MJX_TRY(raise_smem(row_kernel_w32<RX_GRAY_SCOTT>, optin));
     MJX_TRY(raise_smem(row_kernel_w32<RX_FISHER>, optin));
     MJX_TRY(raise_smem(col_kernel<float>, optin));
-    MJX_TRY(raise_smem(col_kernel<double>, optin));
+    MJX_TRY(raise_smem(col_kernel<float, 5>, optin));
+    MJX_TRY(raise_smem(col_kernel<float, 6>, optin));
+    MJX_TRY(raise_smem(col_kernel<float, 7>, optin));
+    MJX_TRY(raise_smem(col_kernel<float, 8>, optin));
+    MJX_TRY(raise_smem(col_kernel<float, 9>, optin));
+    MJX_TRY(raise_smem(col_kernel<float, 10>, optin));
+    MJX_TRY(raise_smem(col_kernel<float, 11>, optin));
+    MJX_TRY(raise_smem(col_kernel<float, 12>, optin));
+    MJX_TRY(raise_smem(col_kernel<double, 12>, optin));
     MJX_TRY(spectral64_attrs(optin));
     return MJX_OK;
   });
