@@ -300,6 +300,26 @@ __device__ void fft_smem(cx<T>* buf, int n, int log2n, int nseq, int ss, int es,
 // where each warp of the radix-16 schedule would keep only n/16 lanes busy and wait on
 // GB300's narrow FP64 pipe.  Same layout, barriers and output order as fft_smem.
 template <typename T, bool INV, bool COLMAJOR>
+__device__ __forceinline__ void fft_smem_r4_inl(cx<T>* buf, int n, int log2n, int nseq, int ss, int es,
+                                                const cx<T>* __restrict__ tw, int tid, int s0 = 0) {
+  const int tps = n >= 4 ? pdiv(n, 4) : 1;
+  const bool active = tid < nseq * tps;
+  int lt, s;
+  if (COLMAJOR) { s = pmod(tid, nseq); lt = pdiv(tid, nseq); }
+  else { lt = pmod(tid, tps); s = pdiv(tid, tps); }
+  const int base = (s + s0) * ss;
+  int p = 1;
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+    if (2 * k + 2 <= log2n) {
+      stockham_pass<T, 4, INV, !COLMAJOR, false>(buf, n, p, tps, lt, base, es, active, tw);
+      p <<= 2;
+    }
+  }
+  if (log2n & 1) stockham_pass<T, 2, INV, !COLMAJOR, false>(buf, n, p, tps, lt, base, es, active, tw);
+}
+
+template <typename T, bool INV, bool COLMAJOR>
 __device__ void fft_smem_r4(cx<T>* buf, int n, int log2n, int nseq, int ss, int es, const cx<T>* __restrict__ tw,
                             int tid, int s0 = 0) {
   const int tps = n >= 4 ? pdiv(n, 4) : 1;

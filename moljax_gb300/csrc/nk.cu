@@ -749,21 +749,23 @@ __device__ __forceinline__ float2 dct_merge(float cak, float cam, float cbk, flo
 template <bool R4>
 __device__ __forceinline__ int dst_tps(int n) { return R4 ? (n >= 4 ? n >> 2 : 1) : (n >= 16 ? n >> 4 : 1); }
 
-template <bool R4, bool INV, bool COLMAJOR>
+// LOG2N > 0: the length as a compile-time constant, so that the index arithmetic and the passes fold
+template <bool R4, int LOG2N, bool INV, bool COLMAJOR>
 __device__ __forceinline__ void dst_fft(float2* buf, const NkaArgs& a, int nseq, int ss, int es, int tid) {
-  if (R4) fft_smem_r4<float, INV, COLMAJOR>(buf, a.n, a.log2n, nseq, ss, es, a.twn, tid);
+  if (LOG2N) fft_smem_r4_inl<float, INV, COLMAJOR>(buf, 1 << LOG2N, LOG2N, nseq, ss, es, a.twn, tid);
+  else if (R4) fft_smem_r4<float, INV, COLMAJOR>(buf, a.n, a.log2n, nseq, ss, es, a.twn, tid);
   else fft_smem<float, INV, COLMAJOR, false>(buf, a.n, a.log2n, nseq, ss, es, a.twn, tid);
 }
 
 // forward DST-II along x of the row pairs (y, y + n/2) of a.src into a.S
-template <bool R4>
+template <bool R4, int LOG2N>
 __global__ void __launch_bounds__(256) dst_row_fwd_kernel(const __grid_constant__ NkaArgs a) {
   typedef float2 C;
   constexpr int PTS = R4 ? 4 : 16;  // elements per thread
   if (a.skip_converged && a.gs->converged) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* buf = reinterpret_cast<C*>(smem_raw);
-  const int n = a.n, hn = n >> 1;
+  const int n = LOG2N ? 1 << LOG2N : a.n, hn = n >> 1;
   const int tps = dst_tps<R4>(n);
   const int tid = threadIdx.x, s_loc = pdiv(tid, tps), lt = tid - s_loc * tps;
   const bool active = s_loc < a.nseq;  // whole warps are launched
@@ -780,7 +782,7 @@ __global__ void __launch_bounds__(256) dst_row_fwd_kernel(const __grid_constant_
     }
   }
   __syncthreads();
-  dst_fft<R4, false, false>(buf, a, a.nseq, n, 1, tid);
+  dst_fft<R4, LOG2N, false, false>(buf, a, a.nseq, n, 1, tid);
   if (!active) return;
   float* Sa = a.S + (long long)y * n;
   float* Sb = a.S + (long long)(y + hn) * n;
@@ -798,13 +800,13 @@ __global__ void __launch_bounds__(256) dst_row_fwd_kernel(const __grid_constant_
 
 // columns kx0 .. kx0 + C - 1 of a.S: DST-II along y, the Helmholtz inverse (with the 1/n^2
 // of the two unnormalised inverse transforms), DST-III along y, in place
-template <bool R4>
+template <bool R4, int LOG2N>
 __global__ void __launch_bounds__(256) dst_col_kernel(const __grid_constant__ NkaArgs a) {
   typedef float2 C;
   if (a.skip_converged && a.gs->converged) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* buf = reinterpret_cast<C*>(smem_raw);
-  const int n = a.n, Cn = a.C, ns = Cn >> 1, lc = __ffs(Cn) - 1, ls = lc - 1;
+  const int n = LOG2N ? 1 << LOG2N : a.n, Cn = a.C, ns = Cn >> 1, lc = __ffs(Cn) - 1, ls = lc - 1;
   const int kx0 = blockIdx.x * Cn;
   const int tid = threadIdx.x, nth = blockDim.x;
   // load (sign and Makhoul position along y), columns 2q and 2q + 1 as sequence q
@@ -815,7 +817,7 @@ __global__ void __launch_bounds__(256) dst_col_kernel(const __grid_constant__ Nk
     *slot = (y & 1) ? -v : v;
   }
   __syncthreads();
-  dst_fft<R4, false, true>(buf, a, ns, 1, ns, tid);
+  dst_fft<R4, LOG2N, false, true>(buf, a, ns, 1, ns, tid);
   // per (sequence, k <= n/2): the coefficients of k and n - k, the multiplier, the inverse
   // inputs of k and n - k (each item owns its two slots)
   const float hD = (float)a.st->dtc, inv_n2 = 1.0f / ((float)n * (float)n);
@@ -843,7 +845,7 @@ __global__ void __launch_bounds__(256) dst_col_kernel(const __grid_constant__ Nk
     if (k > 0 && km != k) buf[sp(q + km * ns)] = dct_merge(cam, cak, cbm, cbk, a.ph[n - k]);
   }
   __syncthreads();
-  dst_fft<R4, true, true>(buf, a, ns, 1, ns, tid);
+  dst_fft<R4, LOG2N, true, true>(buf, a, ns, 1, ns, tid);
   for (int e = tid; e < n * Cn; e += nth) {
     const int y = e >> lc, c = e & (Cn - 1);
     const float v = reinterpret_cast<const float*>(&buf[sp((c >> 1) + mk_pos(y, n) * ns)])[c & 1];
@@ -852,14 +854,14 @@ __global__ void __launch_bounds__(256) dst_col_kernel(const __grid_constant__ Nk
 }
 
 // inverse DST-III along x of the row pairs (y, y + n/2) of a.S; w = (1/a0) result
-template <int MODE, bool R4>
+template <int MODE, bool R4, int LOG2N>
 __global__ void __launch_bounds__(256) dst_row_inv_kernel(const __grid_constant__ NkaArgs a) {
   typedef float2 C;
   constexpr int PTS = R4 ? 4 : 16, KPTS = PTS / 2 + 1;  // elements, coefficient pairs per thread
   if (a.skip_converged && a.gs->converged) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* buf = reinterpret_cast<C*>(smem_raw);
-  const int n = a.n, hn = n >> 1;
+  const int n = LOG2N ? 1 << LOG2N : a.n, hn = n >> 1;
   const int tps = dst_tps<R4>(n);
   const int tid = threadIdx.x, s_loc = pdiv(tid, tps), lt = tid - s_loc * tps;
   const bool active = s_loc < a.nseq;  // whole warps are launched
@@ -879,7 +881,7 @@ __global__ void __launch_bounds__(256) dst_row_inv_kernel(const __grid_constant_
     }
   }
   __syncthreads();
-  dst_fft<R4, true, false>(buf, a, a.nseq, n, 1, tid);
+  dst_fft<R4, LOG2N, true, false>(buf, a, a.nseq, n, 1, tid);
   const float sc = (float)a.K->inv_a0;
   float wa[PTS], wb[PTS];
 #pragma unroll
@@ -1284,24 +1286,29 @@ static DstGeom dst_geom(int n, bool r4) {
 // pass lasts one sequence's dependent work, a quarter as long with n/4 threads per sequence
 static bool dst_r4(int n) { return n <= 512; }
 
+template <int MODE, bool R4, int LOG2N>
+static cudaError_t nka_dst(NKRun& r, const NkaArgs& a, const DstGeom& g) {
+  dst_row_fwd_kernel<R4, LOG2N><<<g.ctas, g.threads, g.smem, r.s>>>(a);
+  dst_col_kernel<R4, LOG2N><<<r.n / g.C, g.col_threads, g.col_smem, r.s>>>(a);
+  dst_row_inv_kernel<MODE, R4, LOG2N><<<g.ctas, g.threads, g.smem, r.s>>>(a);
+  return cudaGetLastError();
+}
+
 // w = M^-1 a.src: DST-II along x, along y with the multiplier and DST-III along y, DST-III
-// along x (MODE: w into t, or the cycle start V_0 = w)
+// along x (MODE: w into t, or the cycle start V_0 = w).  Grids of 64^2 to 512^2 have instances of
+// their length: five BDF2 steps at 512^2, 138 solves, 9.4 ms with the length at run time, 8.6 ms.
 template <int MODE>
 static cudaError_t nka_precond(NKRun& r, NkaArgs a) {
-  const bool r4 = dst_r4(r.n);
-  const DstGeom g = dst_geom(r.n, r4);
+  const DstGeom g = dst_geom(r.n, dst_r4(r.n));
   a.nseq = g.nseq;
   a.C = g.C;
-  if (r4) {
-    dst_row_fwd_kernel<true><<<g.ctas, g.threads, g.smem, r.s>>>(a);
-    dst_col_kernel<true><<<r.n / g.C, g.col_threads, g.col_smem, r.s>>>(a);
-    dst_row_inv_kernel<MODE, true><<<g.ctas, g.threads, g.smem, r.s>>>(a);
-  } else {
-    dst_row_fwd_kernel<false><<<g.ctas, g.threads, g.smem, r.s>>>(a);
-    dst_col_kernel<false><<<r.n / g.C, g.col_threads, g.col_smem, r.s>>>(a);
-    dst_row_inv_kernel<MODE, false><<<g.ctas, g.threads, g.smem, r.s>>>(a);
+  switch (r.n) {
+    case 512: return nka_dst<MODE, true, 9>(r, a, g);
+    case 256: return nka_dst<MODE, true, 8>(r, a, g);
+    case 128: return nka_dst<MODE, true, 7>(r, a, g);
+    case 64: return nka_dst<MODE, true, 6>(r, a, g);
+    default: return dst_r4(r.n) ? nka_dst<MODE, true, 0>(r, a, g) : nka_dst<MODE, false, 0>(r, a, g);
   }
-  return cudaGetLastError();
 }
 
 // The cycle start: V_0 = M^-1 (b - A dx) (first: M^-1 b), |V_0|, the GMRES header and, with a
