@@ -574,8 +574,9 @@ def run_etdrk4(args, local):
 def run_fft3d(args, local):
     """3D FFT-CN diffusion (benchmarks/sisc/bench_3d_feasibility.py: D = 0.1, T = 0.01 in 10
     steps, spectral symbol) at n^3: the published case (10 steps) timed as the reference
-    times it, plus --etd-steps steps for throughput and the HBM roofline of a step (five
-    passes, each reading and writing the box: 80 B per point FP64, 40 B FP32)."""
+    times it, plus --etd-steps steps for throughput and the HBM roofline of a step (four
+    passes between the first r2c and the last c2r, each reading and writing the box: 64 B per
+    point FP64, 32 B FP32)."""
     import numpy as np
     import torch
     import moljax_gb300 as M
@@ -609,7 +610,7 @@ def run_fft3d(args, local):
     e1.record(s)
     e1.synchronize()
     t = e0.elapsed_time(e1) * 1e-3
-    per_pt = 80 if dt_ == torch.float64 else 40
+    per_pt = 64 if dt_ == torch.float64 else 32
     b = per_pt * n ** 3
     peak, peak_kind = peaks()
     gbs = b * S / t / 1e9
@@ -667,11 +668,10 @@ def run_explicit(args, local):
 
 def run_explicit_adaptive(args, model, y0, dt, n, S, dev):
     """adaptive_integrate with RK4 (step doubling: a full step and two half steps per
-    attempt, 12 stencil-stage launches, the error fused into the last; PI controller and
+    attempt, one fused step kernel each, the error in the last; PI controller and
     CFL limit on the device in a conditional graph) for S attempts from t = 0, no state
-    history.  Reports attempts/s, accepted pt-steps/s and the stage kernels' HBM rate
-    (12 stages x 16/4 accesses: 48 accesses = 192 B per point and field per attempt in
-    FP32)."""
+    history.  Reports attempts/s, accepted pt-steps/s and the step kernels' HBM rate
+    (2 + 2 + 3 accesses: 28 B per point and field per attempt in FP32)."""
     import torch
     import moljax_gb300 as M
     pid = M.PIDParams(atol=1e-7, rtol=1e-5)
@@ -687,7 +687,7 @@ def run_explicit_adaptive(args, model, y0, dt, n, S, dev):
     e1.synchronize()
     t = e0.elapsed_time(e1) * 1e-3
     att = r.n_accepted + r.n_rejected
-    b = 2 * n * n * 192
+    b = 2 * n * n * 28
     peak, peak_kind = peaks()
     return {"workload": f"advection-diffusion adaptive RK4 (step doubling) 2 fields {n}x{n} FP32, upwind, periodic, "
                         f"rtol=1e-5, atol=1e-7", "n": n, "attempts": att, "n_accepted": r.n_accepted,
@@ -825,7 +825,7 @@ def fftcn_leg(dev):
     rel = float(torch.linalg.norm(u - exact) / torch.linalg.norm(exact))
     return {"workload": "FFT-CN 2D periodic diffusion 128x128 FP64, D=0.1, dt=0.01, 100 steps (fft_cn_step)",
             "value": n * n * S / t, "unit": UNIT, "ms_per_solve": t * 1e3, "us_per_step": t / S * 1e6,
-            "rel_l2_vs_analytic_decay": rel, "gpu_launches_per_solve": 3 * S,
+            "rel_l2_vs_analytic_decay": rel, "gpu_launches_per_solve": 2 * S + 2,
             "roofline": "latency-bound (128^2 FP64 field, 128 KB, on chip): absolute throughput only"}
 
 

@@ -744,7 +744,7 @@ int mjx_gsbatch_work_items(int ny, int nx);
 /* Creates a batch engine in the caller's device workspace ws (mjx_gsbatch_bytes).
  * Every solve runs the mixed-precision attempt of mjx_imex_adaptive2d_mixed with
  * its own dt, controller state, accept mask and status; one persistent kernel per
- * attempt stage covers every solve in flight, and a batched controller (one warp per
+ * attempt stage covers every solve in flight, and a batched controller (one lane per
  * solve) applies the PI / accept-reject update of each.  The attempt loop is a CUDA
  * graph with a conditional while node, captured once here; admissions and retirements
  * change only device memory.  The engine also holds one mapped pinned host flag

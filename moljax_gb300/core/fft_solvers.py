@@ -102,8 +102,8 @@ def _pow2(n: int) -> bool:
 
 class GeneralSpectralPlan:
     """Periodic (ny, nx) grid of any supported size (powers of two up to 4096, other sizes up
-    to 2048): the full-spectrum path of ``mjx_spectral_apply_general2d`` (row DFTs by
-    Stockham or Bluestein, transposes, column DFTs and the multiplier).  Same ``apply`` as
+    to 2048): half-spectrum row and column passes of ``csrc/dftn.cu`` (mixed-radix Stockham or
+    Bluestein; complex multipliers and tables the full-spectrum path).  Same ``apply`` as
     ``SpectralPlan``; the fused device loops (IMEX, ETD) take powers of two, their
     host-driven forms run on this plan."""
 

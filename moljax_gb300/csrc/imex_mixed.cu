@@ -35,8 +35,6 @@ int elem_size(int dtype);
 void set_last_error(cudaError_t e, const char* file, int line);
 
 struct MJob {
-  int type;
-  int pad;
   long long off;  // field offset (complex elements) shared by every buffer
   double D;
 };
