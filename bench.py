@@ -458,19 +458,20 @@ def run_ours(args, rank, world, local):
 
 def etd_kernel_bytes(n):
     """Algorithmic bytes of the 8 ETDRK4 passes of one step (2 fields, FP32): per field and
-    half-spectrum element, complex 8 B / coefficient 4 B accesses (C1 5+2, R1 2, C2 4+2, R2 2,
-    C3 6+2, R3 2, C4 6+4, R4 2)."""
+    half-spectrum element, complex 8 B / coefficient 2 B accesses (FP32, even in ky: half of
+    them; C1 5+2, R1 2, C2 4+2, R2 2, C3 6+2, R3 2, C4 6+4, R4 2)."""
     nc = n * (n // 2 + 1)
-    per = {"C1": 5 * 8 + 2 * 4, "R1": 16, "C2": 4 * 8 + 2 * 4, "R2": 16, "C3": 6 * 8 + 2 * 4,
-           "R3": 16, "C4": 6 * 8 + 4 * 4, "R4": 16}
+    per = {"C1": 5 * 8 + 2 * 2, "R1": 16, "C2": 4 * 8 + 2 * 2, "R2": 16, "C3": 6 * 8 + 2 * 2,
+           "R3": 16, "C4": 6 * 8 + 4 * 2, "R4": 16}
     return {k: 2 * nc * v for k, v in per.items()}
 
 
 def etd12_step_bytes(n, method):
     """Algorithmic bytes of one ETD1 / ETD2 step (2 fields, FP32): per field and half-spectrum
-    element, column pass ETD1 4 complex + 2 coefficient accesses, ETD2 6 + 3; row pass 2."""
+    element, column pass ETD1 4 complex + 2 coefficient accesses (2 B each: even in ky), ETD2
+    6 + 3; row pass 2."""
     nc = n * (n // 2 + 1)
-    col = 4 * 8 + 2 * 4 if method == "etd1" else 6 * 8 + 3 * 4
+    col = 4 * 8 + 2 * 2 if method == "etd1" else 6 * 8 + 3 * 2
     return 2 * nc * (col + 16)
 
 

@@ -200,19 +200,19 @@ __device__ __forceinline__ void stockham_pass(cx<T>* buf, int n, int p, int tps,
   __syncthreads();
 }
 
-// In-place FFT of nseq sequences (see file comment), sequences s0 .. s0 + nseq - 1.
+// In-place FFT of nseq sequences (see file comment).
 // All threads of the block must call it; threads with tid >= nseq*tps only join the
 // barriers.  The caller must __syncthreads() after filling buf; on return buf is complete.
 // PT: tw is followed by the pass tables of fft_pass_table.
 template <typename T, bool INV, bool COLMAJOR, bool PT = (sizeof(T) == 4)>
-__device__ __forceinline__ void fft_smem_inl(cx<T>* buf, int n, int log2n, int nseq, int ss, int es,
-                         const cx<T>* __restrict__ tw, int tid, int s0 = 0) {
+__device__ void fft_smem(cx<T>* buf, int n, int log2n, int nseq, int ss, int es, const cx<T>* __restrict__ tw,
+                         int tid) {
   const int tps = n >= 16 ? pdiv(n, 16) : 1;
   const bool active = tid < nseq * tps;
   int lt, s;
   if (COLMAJOR) { s = pmod(tid, nseq); lt = pdiv(tid, nseq); }
   else { lt = pmod(tid, tps); s = pdiv(tid, tps); }
-  const int base = (s + s0) * ss;
+  const int base = s * ss;
   // straight-line schedule: up to three radix-16 passes (n <= 4096), then radix 2/4/8
   int p = 1, rem = log2n;
 #pragma unroll
@@ -286,14 +286,6 @@ __device__ __forceinline__ void fft_regs(cx<T>* x, cx<T>* buf, int n, int log2n,
   }
 }
 
-// fft_smem_inl is always inlined, so that a caller passing compile-time lengths gets the
-// index arithmetic and the radix schedule folded; fft_smem leaves the choice to the compiler.
-template <typename T, bool INV, bool COLMAJOR, bool PT = (sizeof(T) == 4)>
-__device__ void fft_smem(cx<T>* buf, int n, int log2n, int nseq, int ss, int es, const cx<T>* __restrict__ tw,
-                         int tid, int s0 = 0) {
-  fft_smem_inl<T, INV, COLMAJOR, PT>(buf, n, log2n, nseq, ss, es, tw, tid, s0);
-}
-
 // The same transform in radix-4 passes (a final radix-2 pass when log2 n is odd), n/4
 // threads per sequence with one butterfly each: four times the threads of the radix-16
 // schedule and about a third of the arithmetic per thread.  Used for short FP64 transforms,
@@ -301,13 +293,13 @@ __device__ void fft_smem(cx<T>* buf, int n, int log2n, int nseq, int ss, int es,
 // GB300's narrow FP64 pipe.  Same layout, barriers and output order as fft_smem.
 template <typename T, bool INV, bool COLMAJOR>
 __device__ __forceinline__ void fft_smem_r4_inl(cx<T>* buf, int n, int log2n, int nseq, int ss, int es,
-                                                const cx<T>* __restrict__ tw, int tid, int s0 = 0) {
+                                                const cx<T>* __restrict__ tw, int tid) {
   const int tps = n >= 4 ? pdiv(n, 4) : 1;
   const bool active = tid < nseq * tps;
   int lt, s;
   if (COLMAJOR) { s = pmod(tid, nseq); lt = pdiv(tid, nseq); }
   else { lt = pmod(tid, tps); s = pdiv(tid, tps); }
-  const int base = (s + s0) * ss;
+  const int base = s * ss;
   int p = 1;
 #pragma unroll
   for (int k = 0; k < 6; ++k) {
@@ -321,13 +313,13 @@ __device__ __forceinline__ void fft_smem_r4_inl(cx<T>* buf, int n, int log2n, in
 
 template <typename T, bool INV, bool COLMAJOR>
 __device__ void fft_smem_r4(cx<T>* buf, int n, int log2n, int nseq, int ss, int es, const cx<T>* __restrict__ tw,
-                            int tid, int s0 = 0) {
+                            int tid) {
   const int tps = n >= 4 ? pdiv(n, 4) : 1;
   const bool active = tid < nseq * tps;
   int lt, s;
   if (COLMAJOR) { s = pmod(tid, nseq); lt = pdiv(tid, nseq); }
   else { lt = pmod(tid, tps); s = pdiv(tid, tps); }
-  const int base = (s + s0) * ss;
+  const int base = s * ss;
   int p = 1;
   for (int rem = log2n; rem >= 2; rem -= 2) {
     stockham_pass<T, 4, INV, !COLMAJOR, false>(buf, n, p, tps, lt, base, es, active, tw);

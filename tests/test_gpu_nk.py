@@ -302,3 +302,18 @@ def test_device_newton_loop_matches_host_loop(cuda, tmp_path):
                                          nk_params=M.NKParams(gmres_restart=30), be_guess="previous")
     np.testing.assert_array_equal(st.cpu().numpy(), child["st"])
     assert _rel(u.cpu().numpy(), child["u"]) < 1e-12
+
+
+@pytest.mark.parametrize("n", [32, 64, 128, 256, 512])
+def test_nk_preconditioner_lengths(cuda, n):
+    """The DST passes of every length with an instance of its own, and one below them: one BDF2 step against the oracle, tolerance and Newton counts as above."""
+    import moljax_gb300 as M
+    dx = 1.0 / n
+    u0 = ONK.gaussians_ic(n)
+    dt = 100 * dx * dx
+    u, st = M.integrate_implicit_vardiff(torch.tensor(u0, device=cuda), dx, dt, 1, method="bdf2",
+                                         nk_params=M.NKParams(gmres_restart=30), be_guess="previous")
+    ref, rst = _oracle(u0, dx, dt, 1, "bdf2")
+    assert _rel(u.cpu().numpy(), ref) < 1e-7
+    assert bool(st[:, 2].all())
+    assert np.max(np.abs(st[:, 0].numpy() - np.array([s[0] for s in rst]))) <= 1
