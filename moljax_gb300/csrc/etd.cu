@@ -173,7 +173,7 @@ template <typename T> struct EArgs {
   int tile;
 };
 
-// One CTA: C adjacent kx columns of one field (E1 transforms two inputs per column).
+// One CTA: C adjacent kx columns of one field.
 // FP32 CTAs take up to 1024 threads, so that at ny = 4096 a CTA still covers 2-4
 // columns and each warp access reads whole 32-byte sectors of the row-major spectra;
 // FP64 keeps 512 threads (its butterflies need the registers).

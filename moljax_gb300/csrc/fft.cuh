@@ -6,7 +6,8 @@
 // (the last pass uses radix 2/4/8 with 16/R butterflies per thread), held in
 // registers, with one shared-memory exchange per pass (Stockham autosort, so
 // the output is in natural order).  Twiddles come from a per-length table
-// tw[j] = exp(-2 pi i j / n) computed on the host in FP64.
+// tw[j] = exp(-2 pi i j / n) computed on the host in FP64, FP32 ones through the pass tables that
+// follow it.  fft_regs is the same transform for callers that hold the elements in registers.
 //
 // COLMAJOR selects the thread mapping: false -> threads of one sequence are
 // consecutive (rows, es == 1); true -> consecutive threads walk across
@@ -106,9 +107,9 @@ __device__ __forceinline__ void dft_r(C* x) {
 // table reads: w^(4a+b) = w^(4a) * w^b.  PT reads the pass's own table (fft_pass_table: entry
 // [slot][k], so that the lanes of a warp read one run per slot); otherwise w^r = tw[r k twstep]
 // of the length's plain table, whose strided reads take a memory wavefront for nearly every
-// lane (4096-point FP32 rows: 156 of a transform's 348 shared and L1 wavefronts a warp; their
-// fused pass of 4096 row pairs takes 125 us with the pass tables, 149 us without, the 2048-point
-// one 63 against 71 us).
+// lane (4096-point FP32 rows: 156 of a transform's 348 shared and L1 wavefronts a warp; the
+// pass tables took their fused pass of 4096 row pairs from 149 to 125 us, the 2048-point one from
+// 71 to 63 us; 100 and 58 us with fft_regs).
 template <typename T, int R, bool INV, bool PT>
 __device__ __forceinline__ void apply_twiddles(cx<T>* x, int k, int p, int twstep, const cx<T>* __restrict__ tw) {
   typedef cx<T> C;

@@ -136,8 +136,8 @@ static int mix_nparts(int ny, int nx, int nf) { return row_ctas(nx, ny, nf); }
 
 // thread caps of the C1 / C2 / C3 column tiles: 512 -> four columns per CTA at 1024 rows
 // (whole 32-byte sectors of the FP32 tile; two 64-register CTAs per SM), 256 -> two columns
-// (four CTAs per SM).  Measured at 1024^2: 881 ms per solve with 512 for all three passes,
-// 901 ms with 256; mixed choices in between.
+// (four CTAs per SM).  Measured at 1024^2 with the tile in shared memory between the transforms:
+// 881 ms per solve with 512 for all three passes, 901 ms with 256; mixed choices in between.
 static constexpr int kColCap[3] = {512, 512, 512};
 
 struct MixAttempt {
