@@ -117,11 +117,11 @@ struct GRowArgs {
   const T* in;        // real rows of n values
   T* out;
   cx<T>* spec;        // half-spectrum rows, stride ld
-  long long nrows;    // real rows; pair q holds rows 2q and 2q + 1
+  long long nrows;    // real rows of a field; pair q holds rows 2q and 2q + 1
   int ld, lS, flags;
 };
 
-// S = 2^lS row pairs per CTA.
+// S = 2^lS row pairs per CTA; blockIdx.y is the field.
 template <typename T>
 __global__ void __launch_bounds__(512) grow_kernel(const __grid_constant__ GRowArgs<T> a) {
   typedef cx<T> C;
@@ -130,6 +130,9 @@ __global__ void __launch_bounds__(512) grow_kernel(const __grid_constant__ GRowA
   Tile<T> t = tile_begin<T>(a.d, smem_raw, lS);
   pdl_wait();
   const long long r0 = ((long long)blockIdx.x << lS) * 2;  // first row of this CTA
+  const T* in = a.in + blockIdx.y * a.nrows * n;
+  T* out = a.out + blockIdx.y * a.nrows * n;
+  C* spec = a.spec + blockIdx.y * a.nrows * a.ld;
   const float rn = 1.0f / (float)n, rh = 1.0f / (float)hx;
   if (a.flags & GROW_LOAD_SPEC) {
     // conj of Z_k = A_k + i B_k and Z_{n-k} = conj(A_k) + i conj(B_k)
@@ -137,8 +140,8 @@ __global__ void __launch_bounds__(512) grow_kernel(const __grid_constant__ GRowA
       const int s = fdiv(e, rh), k = e - s * hx;
       const long long ra = r0 + 2 * s, rb = ra + 1;
       C A = mk<C>((T)0, (T)0), B = A;
-      if (ra < a.nrows) A = a.spec[ra * a.ld + k];
-      if (rb < a.nrows) B = a.spec[rb * a.ld + k];
+      if (ra < a.nrows) A = spec[ra * a.ld + k];
+      if (rb < a.nrows) B = spec[rb * a.ld + k];
       t.cur[sp((k << lS) + s)] = mk<C>(A.x - B.y, -(A.y + B.x));
       if (k > 0 && 2 * k < n) t.cur[sp(((n - k) << lS) + s)] = mk<C>(A.x + B.y, A.y - B.x);
     }
@@ -149,8 +152,8 @@ __global__ void __launch_bounds__(512) grow_kernel(const __grid_constant__ GRowA
         const int s = fdiv(e, rn), x = e - s * n;
         const long long ra = r0 + 2 * s, rb = ra + 1;
         const C v = t.cur[sp((x << lS) + s)];
-        if (ra < a.nrows) a.out[ra * n + x] = v.x;
-        if (rb < a.nrows) a.out[rb * n + x] = -v.y;
+        if (ra < a.nrows) out[ra * n + x] = v.x;
+        if (rb < a.nrows) out[rb * n + x] = -v.y;
       }
       return;
     }
@@ -162,7 +165,7 @@ __global__ void __launch_bounds__(512) grow_kernel(const __grid_constant__ GRowA
     for (int e = tid; e < S * n; e += nth) {
       const int s = fdiv(e, rn), x = e - s * n;
       const long long ra = r0 + 2 * s, rb = ra + 1;
-      const T va = ra < a.nrows ? a.in[ra * n + x] : (T)0, vb = rb < a.nrows ? a.in[rb * n + x] : (T)0;
+      const T va = ra < a.nrows ? in[ra * n + x] : (T)0, vb = rb < a.nrows ? in[rb * n + x] : (T)0;
       t.cur[sp((x << lS) + s)] = mk<C>(va, vb);
     }
   }
@@ -172,8 +175,8 @@ __global__ void __launch_bounds__(512) grow_kernel(const __grid_constant__ GRowA
     const int s = fdiv(e, rh), k = e - s * hx;
     const long long ra = r0 + 2 * s, rb = ra + 1;
     const C Zk = t.cur[sp((k << lS) + s)], Zm = t.cur[sp(((k == 0 ? 0 : n - k) << lS) + s)];
-    if (ra < a.nrows) a.spec[ra * a.ld + k] = mk<C>((T)0.5 * (Zk.x + Zm.x), (T)0.5 * (Zk.y - Zm.y));
-    if (rb < a.nrows) a.spec[rb * a.ld + k] = mk<C>((T)0.5 * (Zk.y + Zm.y), (T)0.5 * (Zm.x - Zk.x));
+    if (ra < a.nrows) spec[ra * a.ld + k] = mk<C>((T)0.5 * (Zk.x + Zm.x), (T)0.5 * (Zk.y - Zm.y));
+    if (rb < a.nrows) spec[rb * a.ld + k] = mk<C>((T)0.5 * (Zk.y + Zm.y), (T)0.5 * (Zm.x - Zk.x));
   }
 }
 
@@ -364,17 +367,22 @@ static Dft<T> dft_desc(const void* plan, int n) {
   return d;
 }
 
+// nf fields of nrows rows.  The two rows of a pair are of one field: a pair of different fields
+// would give each the rounding errors, infinities and NaN of the other (a field of order 1 in FP32
+// behind one of order 1e6 was wrong in its second digit).  With an even number of rows the stack
+// is one run of pairs; with an odd one each field's last row is alone in its pair.
 template <typename T>
-static cudaError_t grow(const Dft<T>& d0, const T* in, T* out, cx<T>* spec, long long nrows, int ld, int flags,
+static cudaError_t grow(const Dft<T>& d0, const T* in, T* out, cx<T>* spec, long long nrows, int nf, int ld, int flags,
                         int pdl, cudaStream_t s) {
+  if (nrows % 2 == 0) { nrows *= nf; nf = 1; }
   GRowArgs<T> a;
   memset(&a, 0, sizeof(a));
   a.d = d0; a.in = in; a.out = out; a.spec = spec; a.nrows = nrows; a.ld = ld; a.flags = flags;
   const long long pairs = (nrows + 1) / 2;
-  a.lS = tile_log<T>(a.d, pairs, 8);
+  a.lS = tile_log<T>(a.d, pairs * nf, 8);
   const long long grid = (pairs + (1 << a.lS) - 1) >> a.lS;
-  return launch_chain(grow_kernel<T>, dim3((unsigned)grid), tile_threads<T>(a.d, a.lS), tile_smem<T>(a.d, a.lS), s, pdl,
-                      a);
+  return launch_chain(grow_kernel<T>, dim3((unsigned)grid, nf), tile_threads<T>(a.d, a.lS), tile_smem<T>(a.d, a.lS), s,
+                      pdl, a);
 }
 
 template <typename T>
@@ -422,8 +430,7 @@ static mjx_status general_apply(const void* plan_y, const void* plan_x, const mj
   }
   c.mode = mult == MJX_MULT_TABLE ? GCOL_USER : GCOL_VALUE;
   c.tab = table;
-  const long long rows = (long long)nf * ny;
-  MJX_CUDA_TRY(grow<T>(dx, in, nullptr, spec, rows, ld, GROW_STORE_SPEC, 0, s));
+  MJX_CUDA_TRY(grow<T>(dx, in, nullptr, spec, ny, nf, ld, GROW_STORE_SPEC, 0, s));
   if (n_steps > 1 && mult < MJX_MULT_ADV_SOLVE) {
     gtab_kernel<T><<<152 * 4, 256, 0, s>>>(tab, m, nf, ny, ld, ld, hx);
     MJX_CUDA_TRY(cudaGetLastError());
@@ -433,7 +440,7 @@ static mjx_status general_apply(const void* plan_y, const void* plan_x, const mj
   for (int i = 0; i < n_steps; ++i) {
     MJX_CUDA_TRY(gcol<T>(c, nf, s));
     const bool last = i == n_steps - 1;
-    MJX_CUDA_TRY(grow<T>(dx, nullptr, out, spec, rows, ld,
+    MJX_CUDA_TRY(grow<T>(dx, nullptr, out, spec, ny, nf, ld,
                          GROW_LOAD_SPEC | (last ? GROW_STORE_REAL : GROW_STORE_SPEC), 1, s));
   }
   return MJX_OK;
@@ -470,13 +477,13 @@ static mjx_status general_apply3(const void* pz, const void* py, const void* px,
     z.tab = tab;
   }
   const long long rows = (long long)nz * ny;
-  MJX_CUDA_TRY(grow<T>(dx, in, nullptr, spec, rows, ld, GROW_STORE_SPEC, 0, s));
+  MJX_CUDA_TRY(grow<T>(dx, in, nullptr, spec, rows, 1, ld, GROW_STORE_SPEC, 0, s));
   for (int i = 0; i < n_steps; ++i) {
     MJX_CUDA_TRY(gcol<T>(y, nz, s));
     MJX_CUDA_TRY(gcol<T>(z, 1, s));
     MJX_CUDA_TRY(gcol<T>(yb, nz, s));
     const bool last = i == n_steps - 1;
-    MJX_CUDA_TRY(grow<T>(dx, nullptr, out, spec, rows, ld,
+    MJX_CUDA_TRY(grow<T>(dx, nullptr, out, spec, rows, 1, ld,
                          GROW_LOAD_SPEC | (last ? GROW_STORE_REAL : GROW_STORE_SPEC), 1, s));
   }
   return MJX_OK;
@@ -677,7 +684,7 @@ static mjx_status tune_dft(const void* plan, int n, long long nrows, cx<T>* data
       d.odd = sched[17 * i] & 1;
       d.tps = uniq[j];
       auto pass = [&]() {
-        return grow<T>(d, nullptr, nullptr, data, rows, ld, GROW_LOAD_SPEC | GROW_STORE_SPEC, 0, s);
+        return grow<T>(d, nullptr, nullptr, data, rows, 1, ld, GROW_LOAD_SPEC | GROW_STORE_SPEC, 0, s);
       };
       cudaError_t ce = pass();
       if (ce == cudaSuccess) ce = cudaEventRecord(e0, s);

@@ -190,3 +190,33 @@ def test_general_steps_vs_numpy(cuda, shape, dtype, tol):
         got = M.fft_cn_step_3d(ut, 0.1, d[2], 1e-4, 3, dy=d[1], dz=d[0])
     err = np.linalg.norm(got.double().cpu().numpy() - ref) / np.linalg.norm(ref)
     assert err < tol, err
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float64, 1e-13), (torch.float32, 2e-5)])
+@pytest.mark.parametrize("shape", [(7, 6), (45, 30), (97, 64), (1, 12), (250, 15)])
+def test_stacked_fields_stay_apart(cuda, shape, dtype, tol):
+    """Each field of a stack is transformed by itself: with an odd number of rows no row of one
+    field shares a complex transform with a row of the next, so a field's error is set by its own
+    size and a field of NaN leaves the others as they are.  Tolerances relative to each field: those
+    of the single fields (test_general_steps_vs_numpy)."""
+    from moljax_gb300 import _native as N
+    from moljax_gb300.core.fft_solvers import get_plan
+    ny, nx = shape
+    dy, dx = 0.7 / ny, 1.3 / nx
+    plan = get_plan(ny, nx, dy, dx, "fd", dtype, cuda)
+    assert plan.general
+    lam = _lam(ny, nx, dy, dx, "fd")
+    u = np.random.default_rng(ny + nx).standard_normal((5, ny, nx))
+    D = [0.05, 0.02, 0.01, 0.03, 0.04]
+    ut = torch.tensor(u, dtype=dtype, device=cuda) * torch.tensor([1e6, 1.0, 1e-6, 1e3, 1e-3], dtype=dtype,
+                                                                  device=cuda)[:, None, None]
+    got = plan.apply(ut, D, 0.01, N.MULT_HELMHOLTZ)
+    for f in range(5):
+        ref = np.real(np.fft.ifft2(np.fft.fft2(ut[f].double().cpu().numpy()) / (1 - 0.01 * D[f] * lam)))
+        err = np.linalg.norm(got[f].double().cpu().numpy() - ref) / np.linalg.norm(ref)
+        assert err < tol, (f, err)
+    ut[1] = float("nan")
+    bad = plan.apply(ut, D, 0.01, N.MULT_HELMHOLTZ)
+    assert bool(torch.isnan(bad[1]).all())
+    for f in (0, 2, 3, 4):
+        assert torch.equal(bad[f], got[f])
