@@ -135,20 +135,26 @@ class GeneralSpectralPlan:
     def ws_bytes(self, nfields: int) -> int:
         return N.lib().mjx_spectral_general2d_ws_bytes(self.ny, self.nx, nfields, self.code)
 
-    def apply(self, x: torch.Tensor, D, h: float, mult: int, out: Optional[torch.Tensor] = None,
-              vx=None, vy=None, table: Optional[torch.Tensor] = None):
-        """out_f = real(IFFT2(m(h, D_f, ...) FFT2(x_f))) for x of shape (ny, nx) or (nf, ny, nx)."""
+    def _stack(self, x: torch.Tensor) -> torch.Tensor:
+        """x as contiguous (nf, ny, nx) fields of the plan's type on the GPU."""
         x3 = x.reshape(-1, self.ny, self.nx).contiguous()
         N.require_cuda(x3)
         if x3.dtype != self.dtype:
             raise TypeError(f"plan dtype {self.dtype} does not match {x3.dtype}")
-        nf = x3.shape[0]
+        return x3
 
-        def per_field(v):
-            if v is None:
-                return [0.0] * nf
-            return [float(v)] * nf if not isinstance(v, (list, tuple)) else [float(t) for t in v]
-        Ds, vxs, vys = per_field(D), per_field(vx), per_field(vy)
+    @staticmethod
+    def _per_field(v, nf: int):
+        if v is None:
+            return [0.0] * nf
+        return [float(v)] * nf if not isinstance(v, (list, tuple)) else [float(t) for t in v]
+
+    def apply(self, x: torch.Tensor, D, h: float, mult: int, out: Optional[torch.Tensor] = None,
+              vx=None, vy=None, table: Optional[torch.Tensor] = None):
+        """out_f = real(IFFT2(m(h, D_f, ...) FFT2(x_f))) for x of shape (ny, nx) or (nf, ny, nx)."""
+        x3 = self._stack(x)
+        nf = x3.shape[0]
+        Ds, vxs, vys = (self._per_field(v, nf) for v in (D, vx, vy))
         out3 = torch.empty_like(x3) if out is None else out.reshape(-1, self.ny, self.nx)
         sym = SYMBOLS[self.symbol]
         for i in range(0, nf, 4):
@@ -162,20 +168,20 @@ class GeneralSpectralPlan:
                 N.ptr(ws), ws.numel(), N.stream_ptr(self.device)))
         return out3.reshape(x.shape)
 
-    def steps(self, u: torch.Tensor, D: float, h: float, mult: int, n_steps: int) -> torch.Tensor:
-        """n_steps times u <- real(IFFT2(m(h, D) FFT2(u))) on one (ny, nx) field."""
-        x3 = u.reshape(-1, self.ny, self.nx)
+    def steps(self, u: torch.Tensor, D, h: float, mult: int, n_steps: int) -> torch.Tensor:
+        """n_steps times u <- real(IFFT2(m(h, D) FFT2(u))); u and D as in ``apply``."""
+        x3 = self._stack(u)
         if x3.shape[0] != 1 or n_steps < 1:  # stacked fields go step by step
             for _ in range(n_steps):
                 u = self.apply(u, D, h, mult)
             return u
-        out = torch.empty_like(u)
+        out = torch.empty_like(x3)
         ws = workspace(self.ws_bytes(1), self.device, "general")
         N.check("mjx_spectral_steps_general2d", N.lib().mjx_spectral_steps_general2d(
             N.ptr(self.buf_y), N.ptr(self.buf_x), C.byref(self.cgrid), SYMBOLS[self.symbol], self.code, 1,
-            (C.c_double * 1)(float(D)), float(h), int(mult), int(n_steps), N.ptr(u), N.ptr(out), N.ptr(ws),
-            ws.numel(), N.stream_ptr(self.device)))
-        return out
+            (C.c_double * 1)(self._per_field(D, 1)[0]), float(h), int(mult), int(n_steps), N.ptr(x3), N.ptr(out),
+            N.ptr(ws), ws.numel(), N.stream_ptr(self.device)))
+        return out.reshape(u.shape)
 
 
 def get_plan(ny, nx, dy, dx, symbol="fd", dtype=torch.float64, device=None):

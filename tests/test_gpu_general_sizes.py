@@ -220,3 +220,28 @@ def test_stacked_fields_stay_apart(cuda, shape, dtype, tol):
     assert bool(torch.isnan(bad[1]).all())
     for f in (0, 2, 3, 4):
         assert torch.equal(bad[f], got[f])
+
+
+def test_steps_take_what_apply_takes(cuda):
+    """Several steps in one call take the tensors and diffusivities that single steps take
+    (strided fields, a list of one diffusivity, a leading axis of one) and refuse what those refuse."""
+    import moljax_gb300 as M
+    from moljax_gb300 import _native as N
+    from moljax_gb300.core.fft_solvers import get_plan
+    ny, nx = 12, 20
+    plan = get_plan(ny, nx, 1.0 / ny, 1.0 / nx, "fd", torch.float64, cuda)
+    u = torch.tensor(np.random.default_rng(2).standard_normal((nx, ny)), device=cuda).T
+    assert not u.is_contiguous()
+    one = plan.apply(plan.apply(u, 0.1, 1e-3, N.MULT_CN), 0.1, 1e-3, N.MULT_CN)
+    got = plan.steps(u, 0.1, 1e-3, N.MULT_CN, 2)
+    assert got.shape == one.shape and float((got - one).abs().max()) < 1e-13
+    for D in ([0.1], (0.1,), torch.tensor(0.1, dtype=torch.float64)):
+        for v in (u, u[None]):
+            got = plan.steps(v, D, 1e-3, N.MULT_CN, 2)
+            assert got.shape == v.shape and float((got.reshape(ny, nx) - one).abs().max()) < 1e-13
+            step = M.fft_cn_step(v, D, 1.0 / nx, 1e-3, 2, symbol="fd", dy=1.0 / ny)
+            assert step.shape == v.shape and float((step.reshape(ny, nx) - one).abs().max()) < 1e-13
+    with pytest.raises(TypeError):
+        plan.steps(u.float(), 0.1, 1e-3, N.MULT_CN, 2)
+    with pytest.raises((TypeError, ValueError, RuntimeError)):
+        plan.steps(u.cpu(), 0.1, 1e-3, N.MULT_CN, 2)
