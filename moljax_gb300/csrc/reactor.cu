@@ -226,7 +226,8 @@ __device__ void reactor_steps(const mjx_reactor_instance& I, T* row, const doubl
     } else {
       T d0 = (T)0, dl = (T)0;
       if (!inner) {  // rows 0 and n - 1
-        const T r0 = fma(half_dt, fma(Ld, cv[1], mul_rn(Lp, cv[2])), cv[1]);
+        const T c1 = n > 1 ? cv[2] : (T)0;  // one node has no right-hand neighbour
+        const T r0 = fma(half_dt, fma(Ld, cv[1], mul_rn(Lp, c1)), cv[1]);
         d0 = mul_rn(dkcn ? r0 + mul_rn(dtt, idz) : cin, mi[0]);
         const int last = n - 1 + pad * ((n - 1) / P), prev = n - 2 + pad * ((n - 2) / P);
         const T cn = row[last], cm = row[max(prev, 0)];

@@ -127,3 +127,27 @@ def test_reactor_chunk_edges_vs_oracle(cuda, variant, dtype, tol):
         ref = fn(c.n, c.Pe, c.Da, c.dt, c.n_steps, c.c_init)
         err = np.linalg.norm(o.double().cpu().numpy() - ref) / np.linalg.norm(ref)
         assert err < tol, (c.n, err)
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float64, 1e-12), (torch.float32, 1e-5)])
+def test_reactor_single_node(cuda, dtype, tol):
+    """A reactor of one node beside longer ones: no right-hand neighbour, whatever an earlier launch
+    left in shared memory.  References: the closed scalar recurrences of the three variants."""
+    from moljax_gb300.core import reactor as R
+    Pe, Da, dt, steps, c0 = 20.0, 1.5, 0.05, 3, 0.25
+    q, kap = 1.0 / Pe, 0.5 * dt / Pe
+    Ld = -2.0 * q - 1.0 - Da
+    dk = cn = c0
+    for _ in range(steps):
+        dk = (dk + kap * (-2.0 * dk) + dt * (-(dk - 1.0) - Da * dk)) / (1.0 + 2.0 * kap)
+        cn = (cn + 0.5 * dt * Ld * cn + dt) / (1.0 - 0.5 * dt * Ld)
+    want = {R.DANCKWERTS: dk, R.DIRICHLET: 0.75, R.DANCKWERTS_CN: cn}
+    fill = [R.ReactorCase(300, Pe, Da, 1e-3, 1, R.DANCKWERTS_CN, 1e4) for _ in range(600)]
+    for _ in range(3):
+        R.solve_batch(fill, dtype)
+        for variant, ref in want.items():
+            cases = [R.ReactorCase(1, Pe, Da, dt, steps, variant, c0, 0.75) for _ in range(300)]
+            cases.append(R.ReactorCase(2, Pe, Da, dt, steps, variant, c0, 0.75))
+            outs = R.solve_batch(cases, dtype)
+            got = torch.cat(outs[:-1]).double()
+            assert float((got - ref).abs().max()) < tol, variant
