@@ -36,7 +36,7 @@ mjx_status ensure_kernel_attrs();
 mjx_status check_grid(const mjx_grid2d* g);
 int elem_size(int dtype);
 
-enum { BT = 256 };           // threads per CTA of the batched pass kernels
+enum { BT = 256, BTL = 512 };  // threads per CTA of the batched passes; of long columns
 enum { BPASS_C1 = 0, BPASS_R1 = 1, BPASS_C2 = 2, BPASS_R2 = 3, BPASS_C3 = 4, BPASS_R3 = 5, BNPASS = 6 };
 enum { SLOT_FREE = 0, SLOT_RUNNING = 1, SLOT_FINISHED = 2 };
 
@@ -44,7 +44,7 @@ enum { SLOT_FREE = 0, SLOT_RUNNING = 1, SLOT_FINISHED = 2 };
 struct BInst {
   DevState st;
   int ny, nx, log2ny, log2nx, ldc, ncols;
-  int colC;                  // columns per column work item (2048 / ny, at most 32)
+  int colC;                  // columns per column work item (b_colC)
   int rseq;                  // row pairs per row work item (min(4096 / nx, ny))
   int nblk;                  // row blocks per row kind (ny / rseq)
   int nparts;                // R3 work items = error partials (2 nblk)
@@ -95,15 +95,25 @@ __host__ __device__ __forceinline__ unsigned witem(int inst, int job, int blk) {
   return ((unsigned)inst << 20) | ((unsigned)job << 16) | (unsigned)blk;
 }
 
+// Columns of a column item, row pairs of a row item (16 <= ny <= 2048, 16 <= nx <= 4096).  Columns of
+// 1024 rows and more are long: 512 threads an item, so that its columns are whole 32-byte sectors
+// at 1024 rows and half ones at 2048.
+static __host__ __device__ constexpr bool b_long(int ny) { return ny >= 1024; }
+static __host__ __device__ constexpr int b_colC(int ny) {
+  return b_long(ny) ? 4096 / ny : (2048 / ny > 32 ? 32 : 2048 / ny);
+}
+static __host__ __device__ constexpr int b_rseq(int ny, int nx) { return 4096 / nx > ny ? ny : 4096 / nx; }
+
 // ------------------------------------------------------------------ column passes
 // One CTA per work item (the grid is the pass's work count, fixed when the engine's
 // graph is built for the current set of solves).  A grid-stride loop over the items
 // would keep the transforms from unrolling: their register arrays then go to local
-// memory.  Three CTAs per SM: 80 registers hold an item without the spills of 64
+// memory.  Three CTAs per SM: at 80 registers the instances of a pass spill little, at 64 much
 // (eight solves of 64^2 to 512^2: C1 / C2 / C3 13 / 18 / 17 us against 15 / 21 / 23,
 // the rows 12 / 9.5 / 9.8 against 14 / 11.4 / 10.7; lengths at run time and elements in
-// shared memory between the transforms 16 / 24 / 19 and 17 / 13.8 / 12.9).
-template <int PASS>
+// shared memory between the transforms 16 / 24 / 19 and 17 / 13.8 / 12.9).  Long columns have
+// their own launch, with the tile and the threads of the single solve (mcol_kernel).
+template <int PASS, bool LONG>
 __device__ __forceinline__ void bcol_item(float2* buf, const BInst* I, unsigned it) {
   const int job = (it >> 16) & 15, tile = it & 0xffff;
   const int f = job;
@@ -118,29 +128,30 @@ __device__ __forceinline__ void bcol_item(float2* buf, const BInst* I, unsigned 
   t.lamx = I->lamx; t.lamy = I->lamy; t.tw = I->twy;
   t.hA = (float)(0.5 * h * I->D[f]); t.hB = (float)(0.25 * h * I->D[f]); t.nrm = I->inv_norm;
   constexpr int TYPE = PASS == BPASS_C1 ? MC_SPLIT : (PASS == BPASS_C3 ? MC_HALF_END : MC_MID);
-  switch (t.log2ny) {  // colC = 2048 / ny
-    case 6: mcol_tile<TYPE, 6, 32>(buf, t, threadIdx.x); break;
-    case 7: mcol_tile<TYPE, 7, 16>(buf, t, threadIdx.x); break;
-    case 8: mcol_tile<TYPE, 8, 8>(buf, t, threadIdx.x); break;
-    case 9: mcol_tile<TYPE, 9, 4>(buf, t, threadIdx.x); break;
-    default: mcol_tile<TYPE>(buf, t, threadIdx.x); break;
+#define MJX_BCOL(L) case L: mcol_tile<TYPE, L, b_colC(1 << L)>(buf, t, threadIdx.x); break;
+  if constexpr (LONG) {
+    switch (t.log2ny) { MJX_BCOL(10) MJX_BCOL(11) }
+  } else {
+    switch (t.log2ny) { MJX_BCOL(4) MJX_BCOL(5) MJX_BCOL(6) MJX_BCOL(7) MJX_BCOL(8) MJX_BCOL(9) }
   }
+#undef MJX_BCOL
 }
 
-template <int PASS>
-__global__ void __launch_bounds__(BT, 3) bcol_kernel(const __grid_constant__ BArgs a) {
+// items first, first + 1, ... of the pass (the long ones come first in its list)
+template <int PASS, bool LONG>
+__global__ void __launch_bounds__(LONG ? BTL : BT, LONG ? 2 : 3) bcol_kernel(const __grid_constant__ BArgs a, int first) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float2* buf = reinterpret_cast<float2*>(smem_raw);
   const BEng* eng = a.eng;
   if (eng->halt) return;
   const int nw = eng->nwork[PASS];
   const unsigned* work = a.work[PASS];
-  const int w = blockIdx.x;
+  const int w = first + blockIdx.x;
   if (w >= nw) return;
   const unsigned it = work[w];
   const BInst* I = a.tab + (it >> 20);
   if (I->st.done) return;  // uniform over the CTA
-  bcol_item<PASS>(buf, I, it);
+  bcol_item<PASS, LONG>(buf, I, it);
 }
 
 // ------------------------------------------------------------------ row passes
@@ -149,14 +160,14 @@ __global__ void __launch_bounds__(BT, 3) bcol_kernel(const __grid_constant__ BAr
 // R3: the pair (error row, solution row) of one field -> (e / (atol + rtol |y|))^2 summed
 // into the item's partial.
 // A thread keeps its 16 elements in registers (fft_regs); shared memory holds the mirrored half of
-// the spectra besides the exchanges.  LOG2N > 0: compile-time row length.
-template <int PASS, int LOG2N = 0>
+// the spectra besides the exchanges.  LOG2N: the row length.
+template <int PASS, int LOG2N>
 __device__ __forceinline__ void brow_item(float2* buf, const BInst* I, unsigned it) {
   const int tid = threadIdx.x;
   {
     const int kind = (it >> 16) & 15, blk = it & 0xffff;
-    const int n = LOG2N ? (1 << LOG2N) : I->nx, half = n >> 1, log2n = LOG2N ? LOG2N : I->log2nx;
-    const int tps = n >> 4;
+    constexpr int n = 1 << LOG2N, half = n >> 1, log2n = LOG2N;
+    constexpr int tps = n >> 4;
     const int nseq = I->rseq;
     const int s_loc = tid / tps, lt = tid - s_loc * tps;
     const bool active = s_loc < nseq;
@@ -290,13 +301,11 @@ __global__ void __launch_bounds__(BT, 3) brow_kernel(const __grid_constant__ BAr
   const unsigned it = work[w];
   const BInst* I = a.tab + (it >> 20);
   if (I->st.done) return;  // uniform over the CTA
+#define MJX_BROW(L) case L: brow_item<PASS, L>(buf, I, it); break;
   switch (I->log2nx) {
-    case 6: brow_item<PASS, 6>(buf, I, it); break;
-    case 7: brow_item<PASS, 7>(buf, I, it); break;
-    case 8: brow_item<PASS, 8>(buf, I, it); break;
-    case 9: brow_item<PASS, 9>(buf, I, it); break;
-    default: brow_item<PASS>(buf, I, it); break;
+    MJX_BROW(4) MJX_BROW(5) MJX_BROW(6) MJX_BROW(7) MJX_BROW(8) MJX_BROW(9) MJX_BROW(10) MJX_BROW(11) MJX_BROW(12)
   }
+#undef MJX_BROW
 }
 
 // ------------------------------------------------------------------ controller
@@ -378,8 +387,6 @@ static inline size_t al256b(size_t b) { return (b + 255) & ~size_t(255); }
 static bool batch_size_ok(int ny, int nx) {
   return ilog2_exact(ny) >= 4 && ilog2_exact(nx) >= 4 && ny <= 2048 && nx <= 4096;
 }
-static int b_colC(int ny) { const int c = 2048 / ny; return c > 32 ? 32 : c; }
-static int b_rseq(int ny, int nx) { const int q = 4096 / nx; return q > ny ? ny : q; }
 
 static InstLayout inst_layout(int ny, int nx, int max_saves) {
   InstLayout L;
@@ -458,15 +465,27 @@ struct GsBatch {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   size_t smem = 0;
+  int nlong = 0;                    // long column items, the first of each column pass's list
   BEng h_eng;
 };
+
+// shared memory of a long column item (4096 points a half)
+static size_t long_smem() { return mcol_smem(1, 4096); }
+
+template <int PASS>
+static mjx_status bcol_attrs(size_t smem) {
+  MJX_CUDA_TRY(cudaFuncSetAttribute(bcol_kernel<PASS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  MJX_CUDA_TRY(cudaFuncSetAttribute(bcol_kernel<PASS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)long_smem()));
+  return MJX_OK;
+}
 
 static mjx_status batch_attrs(size_t smem) {
   static ContextOnce once;
   return once.run([&]() -> mjx_status {
-    MJX_CUDA_TRY(cudaFuncSetAttribute(bcol_kernel<BPASS_C1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    MJX_CUDA_TRY(cudaFuncSetAttribute(bcol_kernel<BPASS_C2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    MJX_CUDA_TRY(cudaFuncSetAttribute(bcol_kernel<BPASS_C3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    MJX_TRY(bcol_attrs<BPASS_C1>(smem));
+    MJX_TRY(bcol_attrs<BPASS_C2>(smem));
+    MJX_TRY(bcol_attrs<BPASS_C3>(smem));
     MJX_CUDA_TRY(cudaFuncSetAttribute(brow_kernel<BPASS_R1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     MJX_CUDA_TRY(cudaFuncSetAttribute(brow_kernel<BPASS_R2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     MJX_CUDA_TRY(cudaFuncSetAttribute(brow_kernel<BPASS_R3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -474,13 +493,20 @@ static mjx_status batch_attrs(size_t smem) {
   });
 }
 
+template <int PASS>
+static void launch_bcol(const GsBatch& B, cudaStream_t s) {
+  const int rest = B.h_eng.nwork[PASS] - B.nlong;
+  if (B.nlong > 0) bcol_kernel<PASS, true><<<B.nlong, BTL, long_smem(), s>>>(B.args, 0);
+  if (rest > 0) bcol_kernel<PASS, false><<<rest, BT, B.smem, s>>>(B.args, B.nlong);
+}
+
 static cudaError_t launch_batch_attempt(const GsBatch& B, cudaGraphConditionalHandle hdl, cudaStream_t s) {
   const int* nw = B.h_eng.nwork;
-  bcol_kernel<BPASS_C1><<<nw[BPASS_C1], BT, B.smem, s>>>(B.args);
+  launch_bcol<BPASS_C1>(B, s);
   brow_kernel<BPASS_R1><<<nw[BPASS_R1], BT, B.smem, s>>>(B.args);
-  bcol_kernel<BPASS_C2><<<nw[BPASS_C2], BT, B.smem, s>>>(B.args);
+  launch_bcol<BPASS_C2>(B, s);
   brow_kernel<BPASS_R2><<<nw[BPASS_R2], BT, B.smem, s>>>(B.args);
-  bcol_kernel<BPASS_C3><<<nw[BPASS_C3], BT, B.smem, s>>>(B.args);
+  launch_bcol<BPASS_C3>(B, s);
   brow_kernel<BPASS_R3><<<nw[BPASS_R3], BT, B.smem, s>>>(B.args);
   bctl_kernel<<<1, 1024, 0, s>>>(B.args, hdl);
   return cudaGetLastError();
@@ -533,9 +559,12 @@ static void free_batch(GsBatch* B) {
 static mjx_status upload_work(GsBatch& B, cudaStream_t s) {
   std::vector<unsigned> w[BNPASS];
   int n_slots = 0;
-  for (int i = 0; i < B.max_inst; ++i) {
-    if (B.state[i] != SLOT_FREE) n_slots = i + 1;
-    if (B.state[i] == SLOT_RUNNING) inst_items(B.h_tab[i], i, w);
+  for (int part = 0; part < 2; ++part) {  // long columns, then the others
+    for (int i = 0; i < B.max_inst; ++i) {
+      if (B.state[i] != SLOT_FREE) n_slots = i + 1 > n_slots ? i + 1 : n_slots;
+      if (B.state[i] == SLOT_RUNNING && b_long(B.h_tab[i].ny) == (part == 0)) inst_items(B.h_tab[i], i, w);
+    }
+    if (part == 0) B.nlong = (int)w[BPASS_C1].size();
   }
   for (int p = 0; p < BNPASS; ++p) {
     if ((int)w[p].size() > B.max_work) return MJX_BAD_SHAPE;
@@ -598,7 +627,7 @@ mjx_status mjx_gsbatch_create(void** batch, int max_instances, int max_work, voi
   if (ce == cudaSuccess) { *B->h_stop = 0; ce = cudaHostGetDevicePointer((void**)&B->d_stop, B->h_stop, 0); }
   if (ce != cudaSuccess) { set_last_error(ce, __FILE__, __LINE__); free_batch(B); return MJX_CUDA_ERROR; }
   B->h_eng.host_stop = B->d_stop;
-  B->smem = mcol_smem(1, 2048);  // every column tile has ny C <= 2048, every row item 4096 points
+  B->smem = mcol_smem(1, 2048);  // every column tile but the long ones has ny C <= 2048, every row item 4096 points
   st = batch_attrs(B->smem);
   if (st == MJX_OK) {  // every slot of the device table starts free (done)
     ce = cudaMemcpy(B->args.tab, B->h_tab.data(), sizeof(BInst) * max_instances, cudaMemcpyHostToDevice);

@@ -119,3 +119,18 @@ def test_batch_rejects_unsupported_sizes(cuda):
     with pytest.raises(ValueError):
         eng.admit(p)
     eng.close()
+
+
+def test_long_and_short_columns_share_a_batch(cuda):
+    """Items whose columns have their own launch (1024 rows and more) beside shorter ones, of row
+    lengths on both sides: each bitwise as alone, while items of either kind finish first."""
+    import moljax_gb300 as M
+    cases = [(64, 1024, 0.035, 0.065, 4.0, 1), (1024, 32, 0.03, 0.06, 5.0, 2), (16, 16, 0.045, 0.062, 9.0, 3),
+             (2048, 16, 0.05, 0.065, 3.0, 4), (512, 64, 0.025, 0.055, 6.0, 5), (1024, 2048, 0.04, 0.06, 2.0, 6)]
+    probs = [_problem(*c, cuda, max_steps=4000, save_every=50)[0] for c in cases]
+    together = M.adaptive_integrate_imex_batch(probs, cuda)
+    for p, (out, r), c in zip(probs, together, cases):
+        (alone, ra), = M.adaptive_integrate_imex_batch([p], cuda)
+        assert (r.status, r.n_accepted, r.n_rejected) == (0, ra.n_accepted, ra.n_rejected), c
+        for f in range(2):
+            assert torch.equal(out[f], alone[f]), c
