@@ -30,7 +30,9 @@ __device__ __forceinline__ double jclip(double x, double lo, double hi) { return
 // and handle_rejected_step (230-268) above
 __device__ __forceinline__ double ctl_log(double q) { return jmax(0.5 * log(q), -23.025850929940456840); }
 __device__ __forceinline__ double ctl_factor(const CtlGain& G, bool small, double le, double lprev) {
-  return exp(small ? G.kP * lprev - (G.kI + G.kP) * le : -G.kI * jmax(le, 0.0));
+  // x^0 is 1 for every x, also where the norm has overflowed or is NaN: without an integral gain a
+  // rejected step shrinks by the safety factor
+  return exp(small ? G.kP * lprev - (G.kI + G.kP) * le : (G.kI == 0.0 ? 0.0 : -G.kI * jmax(le, 0.0)));
 }
 
 // e = max(sqrt(tot / n_dof), 1e-10) with tot the sum over every degree of freedom of

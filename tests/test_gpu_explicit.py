@@ -384,3 +384,17 @@ def test_tma_stage_form(cuda, shape, kind):
     for k in names:
         F = t["rhs"][k].cpu().double().numpy()[c]
         assert _rel(F, R[k][c]) < 2e-5, k
+
+
+def test_adaptive_overflowing_error_norm_without_integral_gain(cuda):
+    """An error norm that overflows (a vanishing atol) rejects the attempt; without an integral gain
+    (1/e)^kI is 1 whatever e is, so the steps shrink by the safety factor until dt_min."""
+    n = 16
+    M, model, ym, om, y0 = _gs(n, mol.NEUMANN, cuda)
+    kw = dict(atol=1e-200, rtol=0.0, kI=0.0, kP=0.0, dt_min=0.01)
+    r = M.adaptive_integrate(model, ym, 0.0, 30.0, 1.0, M.IntegratorType.RK4, max_steps=4000,
+                             pid_params=M.PIDParams(**kw), save_y_history=False)
+    with np.errstate(over="ignore"):
+        ro = OX.adaptive_integrate_explicit(om, y0, 0.0, 30.0, 1.0, 2, max_steps=4000, pid=OI.PIDParams(**kw))
+    assert r.status == ro.status == M.StatusCode.DT_TOO_SMALL
+    assert (r.n_accepted, r.n_rejected) == (ro.n_accepted, ro.n_rejected)
