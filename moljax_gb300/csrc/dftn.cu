@@ -332,10 +332,11 @@ __global__ void gtab_kernel(T* tab, const __grid_constant__ GMul m, int nf, int 
 }
 
 // ------------------------------------------------------------------ launch geometry
-// half-spectrum row length, whole 32-byte sectors
+// half-spectrum row length: whole 32-byte sectors, but unpadded below four points, where a pad
+// would take the spectra beyond the workspace (general_ws) and a row beyond the tuner's scratch
 static int gen_ld(int nx, int elem) {
-  const int q = 32 / (2 * elem);
-  return (nx / 2 + 1 + q - 1) / q * q;
+  const int hx = nx / 2 + 1, q = 32 / (2 * elem);
+  return nx < 4 ? hx : (hx + q - 1) / q * q;
 }
 
 // radices (at most 16 of them, each below 16) as tile_dft takes them
@@ -489,12 +490,9 @@ static mjx_status general_apply3(const void* pz, const void* py, const void* px,
   return MJX_OK;
 }
 
-// workspace: the half spectra and the formed multipliers (at least the four reals per point of
-// a full complex spectrum and its transpose, which the query has always asked for)
-static size_t general_ws(size_t rows, int nx, int elem) {
-  const size_t need = rows * gen_ld(nx, elem) * 3 * elem, old = rows * nx * 4 * elem;
-  return need > old ? need : old;
-}
+// workspace: the half spectra (2 gen_ld reals a row) and the formed multipliers (gen_ld), within the
+// four reals a point that the query asks for: 3 gen_ld <= 4 nx for every nx
+static size_t general_ws(size_t rows, int nx, int elem) { return rows * nx * 4 * elem; }
 
 static mjx_status set_dft_attrs() {
   static ContextOnce once;
@@ -669,9 +667,6 @@ static mjx_status tune_dft(const void* plan, int n, long long nrows, cx<T>* data
   tune_dft_clear(n, (int)sizeof(T));
   Dft<T> d = dft_desc<T>(plan, n);
   const int ld = gen_ld(n, sizeof(T));
-  long long rows = nrows * n / ld;  // half-spectrum rows that fit the scratch
-  if (rows > nrows) rows = nrows;
-  if (rows < 1) return MJX_WORKSPACE;
   cudaEvent_t e0, e1;
   MJX_CUDA_TRY(cudaEventCreate(&e0));
   MJX_CUDA_TRY(cudaEventCreate(&e1));
@@ -684,7 +679,7 @@ static mjx_status tune_dft(const void* plan, int n, long long nrows, cx<T>* data
       d.odd = sched[17 * i] & 1;
       d.tps = uniq[j];
       auto pass = [&]() {
-        return grow<T>(d, nullptr, nullptr, data, rows, 1, ld, GROW_LOAD_SPEC | GROW_STORE_SPEC, 0, s);
+        return grow<T>(d, nullptr, nullptr, data, nrows, 1, ld, GROW_LOAD_SPEC | GROW_STORE_SPEC, 0, s);
       };
       cudaError_t ce = pass();
       if (ce == cudaSuccess) ce = cudaEventRecord(e0, s);

@@ -80,3 +80,13 @@ def test_dft_schedule_candidates_and_registry(native_lib, tmp_path):
     assert AT.stencil_rows(100, 70, 2, torch.float32) == 16
     AT.set_dft_schedule(48, torch.float64, ())
     AT.set_stencil_rows(100, 70, 2, torch.float32, 0)
+
+
+def test_general_workspace_sizes(native_lib):
+    """The workspace of the general periodic forms: two complex numbers a point, also for rows of
+    one or two points, whose half spectra are not padded."""
+    for dtype, e in ((0, 4), (1, 8)):
+        for ny in (1, 2, 3, 5, 64, 100, 2047):
+            for nx in (1, 2, 3, 4, 5, 6, 7, 9, 33, 100, 2047, 4096):
+                assert native_lib.mjx_spectral_general2d_ws_bytes(ny, nx, 2, dtype) == 2 * 2 * ny * nx * 2 * e
+                assert native_lib.mjx_spectral_general3d_ws_bytes(3, ny, nx, dtype) == 2 * 3 * ny * nx * 2 * e

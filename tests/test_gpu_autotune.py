@@ -103,3 +103,15 @@ def test_stencil_tile_heights_bit_identical(cuda, shape):
         assert torch.equal(torch.stack([F["c1"], F["c2"]]).cpu(), outs[0])
     finally:
         AT.set_stencil_rows(ny, nx, 2, torch.float32, 0)
+
+
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+def test_tunes_a_single_short_row(cuda, dtype):
+    """One row of any length that has schedules is enough to tune on."""
+    from moljax_gb300.core import autotune as AT
+    for n in (3, 5, 6, 9, 12, 15):
+        try:
+            res = AT.autotune_dft(n, dtype, cuda, nrows=1, reps=2)
+            assert res is not None and AT.dft_schedule(n, dtype) == (tuple(res.choice[0]), res.choice[1])
+        finally:
+            AT.set_dft_schedule(n, dtype, ())
