@@ -398,3 +398,110 @@ def test_adaptive_overflowing_error_norm_without_integral_gain(cuda):
         ro = OX.adaptive_integrate_explicit(om, y0, 0.0, 30.0, 1.0, 2, max_steps=4000, pid=OI.PIDParams(**kw))
     assert r.status == ro.status == M.StatusCode.DT_TOO_SMALL
     assert (r.n_accepted, r.n_rejected) == (ro.n_accepted, ro.n_rejected)
+
+
+def _two_field_case(case, shape, cuda):
+    """(model, padded FP32 state, oracle model, padded FP64 state) of an FP32 model of at most two
+    fields: Gray-Scott, Fisher-KPP, or advection-diffusion with upwind or central differences."""
+    import moljax_gb300 as M
+    from moljax_gb300.core.bc import FieldBCSpec, BCType
+    kind, bcs = case
+    ny, nx = shape
+    grid, og = M.Grid2D(nx, ny, 0.0, 2.5, 0.0, 2.0), mol.Grid2D(nx, ny, 0, 2.5, 0, 2.0)
+    rng = np.random.default_rng(7 * ny + nx)
+    if kind == "gs":
+        model = M.create_gray_scott_model(grid, 2e-3, 1e-3, 0.035, 0.065, BCType.PERIODIC, torch.float32)
+        names, D = ("u", "v"), {"u": 2e-3, "v": 1e-3}
+        ok = dict(reaction=lambda y: mol.gray_scott_reaction(y, 0.035, 0.065),
+                  params={"Du": 2e-3, "Dv": 1e-3, "F": 0.035, "k": 0.065})
+    elif kind == "fisher":
+        model = M.create_fisher_kpp_model(grid, 2e-3, 1.2, BCType.PERIODIC, torch.float32)
+        names, D = ("u",), {"u": 2e-3}
+        ok = dict(reaction=lambda y: mol.fisher_kpp_reaction(y, 1.2), params={"D": 2e-3, "r": 1.2})
+    else:
+        names = ("c1", "c2")[:len(bcs)]
+        model = M.create_advection_diffusion_model(grid, names, 2e-3, 0.3, -0.2, BCType.PERIODIC, kind == "upwind",
+                                                   torch.float32)
+        D = {k: 2e-3 for k in names}
+        ok = dict(advection=kind, vx=0.3, vy=-0.2, params={"D": 2e-3, "vx": 0.3, "vy": -0.2})
+    spec, vals = {}, {}
+    for i, (k, bc) in enumerate(zip(names, bcs)):
+        if bc == mol.PERIODIC:
+            spec[k] = FieldBCSpec(kind=BCType(bc))
+            continue
+        vals[k] = {s: v + 0.1 * i for s, v in SIDES.items()}
+        fn = (lambda X, Y, t, p, w=vals[k]: dict(w))
+        spec[k] = FieldBCSpec(kind=BCType(bc), value=fn) if bc == mol.DIRICHLET else FieldBCSpec(kind=BCType(bc), flux=fn)
+    model = M.MOLModel(model.grid, spec, model.params, model.linear_ops, model.nonlinear_ops, model.metadata)
+    om = OX.ExplicitModel(og, dict(zip(names, bcs)), D, vals, **ok)
+    # FP32 numbers, so that both sides start from the same state
+    y0 = {k: mol.pad(rng.uniform(0.1, 1.0, (ny, nx)).astype(np.float32).astype(np.float64), og) for k in names}
+    ym = {k: torch.tensor(v, dtype=torch.float32, device=cuda) for k, v in y0.items()}
+    return M, model, ym, om, y0, og
+
+
+P_, D_, N_ = mol.PERIODIC, mol.DIRICHLET, mol.NEUMANN
+
+
+@pytest.mark.parametrize("shape", [(1, 1), (3, 2), (2, 9), (33, 5), (32, 64), (37, 70), (130, 200)])
+@pytest.mark.parametrize("case", [("gs", (P_, P_)), ("gs", (N_, D_)), ("fisher", (P_,)), ("fisher", (D_,)),
+                                  ("upwind", (P_, D_)), ("central", (N_, P_)), ("upwind", (N_,))])
+@pytest.mark.parametrize("method", [1, 2])
+def test_adaptive_fp32_two_fields_vs_oracle(cuda, method, case, shape):
+    """The adaptive SSPRK3 and RK4 loops of up to two FP32 fields (three fused steps an attempt)
+    on grids below, at and above a tile and the halo, for every reaction, with boundary kinds that
+    differ between the fields.  With the step size pinned both sides take the same seven steps: the
+    oracle's saved times, and its state within FP32 rounding (an FP32 step leaves at most 2e-6 of
+    the state: four stages, a stencil whose weights sum to less than two at the diffusion limit;
+    fourteen half steps, 5e-5 with a factor of two).  The error norm e shows in the step that follows
+    a rejection, 0.45 dt / e^(kI / order): with atol set to a fifth of the oracle's error FP32 rounding
+    (4e-7 of the state in the difference of the two solutions) moves it by that share of the error."""
+    M, model, ym, om, y0, og = _two_field_case(case, shape, cuda)
+    itype = {1: M.IntegratorType.SSPRK3, 2: M.IntegratorType.RK4}[method]
+    lim = min(OX.heisenberg_cfl_dt(og, om.params, OI.CFLParams()), 0.5)
+    s = og.interior_slice
+    pid = dict(atol=1e30, rtol=0.0, safety=1.0, min_factor=1.0, max_factor=1.0)
+    r = M.adaptive_integrate(model, ym, 0.0, 3.2 * lim, 0.5 * lim, itype, max_steps=100, pid_params=M.PIDParams(**pid),
+                             save_every=1)
+    ro = OX.adaptive_integrate_explicit(om, y0, 0.0, 3.2 * lim, 0.5 * lim, method, max_steps=100,
+                                        pid=OI.PIDParams(**pid), save_every=1)
+    assert r.status == ro.status == 0
+    assert (r.n_accepted, r.n_rejected, r.n_steps) == (ro.n_accepted, ro.n_rejected, ro.n_steps) == (7, 0, 8)
+    np.testing.assert_allclose(r.t_history.cpu().numpy()[:8], ro.t_history[:8], rtol=1e-12)
+    for k in y0:
+        scale = float(np.max(np.abs(ro.y_final[k][s])))
+        np.testing.assert_allclose(r.y_final[k].double().cpu().numpy()[s], ro.y_final[k][s], rtol=0, atol=5e-5 * scale)
+        # the saved states: the start and the end
+        np.testing.assert_array_equal(r.y_history[k][0].double().cpu().numpy(), y0[k][s])
+        np.testing.assert_array_equal(r.y_history[k][7].cpu().numpy(), r.y_final[k].cpu().numpy()[s])
+    _, err = OX.step_explicit_with_error(om, y0, lim, method)
+    rms = mol.scaled_error_norm(err, y0, og, 1.0, 0.0)
+    tol = 4e-7 * max(float(np.max(np.abs(v[s]))) for v in y0.values()) / max(rms, 1e-30)
+    if tol > 0.1:  # the error is of the size of FP32 rounding
+        return
+    kI = float(OX.ORDER[method])
+    pid = dict(atol=rms / 5.0, rtol=0.0, kI=kI, kP=0.0, min_factor=1e-6)
+    r = M.adaptive_integrate(model, ym, 0.0, 10 * lim, lim, itype, max_steps=1, pid_params=M.PIDParams(**pid), save_every=1)
+    ro = OX.adaptive_integrate_explicit(om, y0, 0.0, 10 * lim, lim, method, max_steps=1, pid=OI.PIDParams(**pid),
+                                        save_every=1)
+    assert (r.n_accepted, r.n_rejected) == (ro.n_accepted, ro.n_rejected) == (1, 1)
+    assert float(r.dt_history[0]) == pytest.approx(ro.dt_history[0], rel=max(tol, 1e-4))
+
+
+@pytest.mark.parametrize("method", [1, 2])
+def test_adaptive_fp32_two_fields_rejections_and_nonfinite(cuda, method):
+    """The same loops with tolerances that reject steps (the error norm itself decides: FP32 counts
+    within one of the FP64 oracle's), and a NaN in the state, which ends the run at its first attempt."""
+    M, model, ym, om, y0, og = _two_field_case(("gs", (N_, D_)), (37, 70), cuda)
+    itype = {1: M.IntegratorType.SSPRK3, 2: M.IntegratorType.RK4}[method]
+    # a step doubling error of about 1e-3 of the state at the CFL limit, well above FP32 rounding
+    pid = dict(atol=1e-4, rtol=1e-4)
+    r = M.adaptive_integrate(model, ym, 0.0, 1.0, 0.4, itype, max_steps=400, pid_params=M.PIDParams(**pid))
+    ro = OX.adaptive_integrate_explicit(om, y0, 0.0, 1.0, 0.4, method, max_steps=400, pid=OI.PIDParams(**pid))
+    assert r.status == ro.status == 0
+    assert abs(r.n_accepted - ro.n_accepted) <= 1 and abs(r.n_rejected - ro.n_rejected) <= 1
+    bad = {k: v.clone() for k, v in ym.items()}
+    bad["v"][20, 33] = float("nan")
+    r = M.adaptive_integrate(model, bad, 0.0, 1.0, 0.1, itype, max_steps=400, pid_params=M.PIDParams(**pid))
+    assert r.status == M.StatusCode.NON_FINITE_VALUES
+    assert (r.n_accepted, r.n_rejected) == (0, 1)
