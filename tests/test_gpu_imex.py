@@ -298,3 +298,28 @@ def test_mixed_and_batched_lengths(cuda, ny, nx):
     assert (rb.status, rb.n_accepted, rb.n_rejected) == (0, ro.n_accepted, ro.n_rejected)
     for i, k in enumerate(("u", "v")):
         assert _rel(out[i].cpu().numpy(), mol.interior(ro.y_final[k], og)) < 1e-6
+
+
+@pytest.mark.parametrize("ny,nx", [(2, 2048), (16, 2048), (32, 512), (128, 16), (512, 32), (1024, 64), (2048, 16),
+                                   (2048, 256), (4096, 16)])
+def test_fp64_two_output_columns_vs_oracle(cuda, ny, nx):
+    """FP64 IMEX attempts, whose first column pass has two outputs, from sixteen columns a CTA to
+    one (2048 rows, where two outputs of two columns would not fit), and the 4096-row form: the
+    oracle's counts and state (the tolerance of test_adaptive_fp64_matches_oracle_counts)."""
+    import moljax_gb300 as M
+    L = 2.5
+    grid, og = M.Grid2D(nx, ny, 0.0, L, 0.0, L), mol.Grid2D(nx, ny, 0, L, 0, L)
+    model, cache, diff = M.create_gray_scott_periodic_fft(grid, 2e-5, 1e-5, 0.035, 0.065, torch.float64, cuda)
+    rng = np.random.default_rng(ny + nx)
+    y0 = {k: mol.bc_2d(mol.pad(b + 0.1 * rng.uniform(0, 1, (ny, nx)), og), og, mol.PERIODIC)
+          for k, b in (("u", 0.6), ("v", 0.2))}
+    ym = {k: torch.tensor(v, device=cuda) for k, v in y0.items()}
+    om, lam, od = OI.gray_scott_periodic(og, 2e-5, 1e-5, 0.035, 0.065)
+    r = M.adaptive_integrate_imex(model, ym, 0.0, 2.0, 1.0, cache, diff, pid_params=M.PIDParams(atol=1e-6, rtol=1e-4),
+                                  max_steps=500, save_every=100, save_y_history=False)
+    ro = OI.adaptive_integrate_imex(om, y0, 0.0, 2.0, 1.0, lam, od, pid=OI.PIDParams(atol=1e-6, rtol=1e-4),
+                                    max_steps=500, save_every=100, keep_history=False)
+    assert r.status == ro.status == 0
+    assert (r.n_accepted, r.n_rejected) == (ro.n_accepted, ro.n_rejected) and ro.n_accepted >= 2
+    for k in ("u", "v"):
+        assert _rel(r.y_final[k].cpu().numpy(), ro.y_final[k]) < 1e-11
