@@ -151,3 +151,25 @@ def test_reactor_single_node(cuda, dtype, tol):
             outs = R.solve_batch(cases, dtype)
             got = torch.cat(outs[:-1]).double()
             assert float((got - ref).abs().max()) < tol, variant
+
+
+@pytest.mark.parametrize("dtype,eps", [(torch.float64, 2.0 ** -53), (torch.float32, 2.0 ** -24)])
+@pytest.mark.parametrize("variant", ["danckwerts", "dirichlet", "danckwerts_cn"])
+def test_reactor_full_chunks_vs_oracle(cuda, variant, dtype, eps):
+    """Two nodes, and lengths whose 256 chunks are all full with more than one node each, up to the
+    register kernel's longest (4096).  Tolerance: a step rounds dt/2 times the row's diagonal
+    2/(Pe dz^2) + 1/dz + Da against a state of order one, which the solve does not amplify; eight
+    steps, a factor of four for the other terms, and the tolerances of the short reactors below it."""
+    from moljax_gb300.core import reactor as R
+    kind = {"danckwerts": R.DANCKWERTS, "dirichlet": R.DIRICHLET, "danckwerts_cn": R.DANCKWERTS_CN}[variant]
+    fn = {"danckwerts": OR.danckwerts_cn, "danckwerts_cn": OR.danckwerts_full_cn,
+          "dirichlet": lambda *a: OR.dirichlet_cn(*a[:5], 1.0, a[5])}[variant]
+    cases = []
+    for i, n in enumerate((2, 512, 768, 1024, 4096)):
+        dt = 0.5 / n if variant == "danckwerts" else R.served_dt(n)[0]
+        cases.append(R.ReactorCase(n, 15.0 + 17 * i, 0.5 + 0.4 * i, dt, 8, kind, 0.25))
+    for c, o in zip(cases, R.solve_batch(cases, dtype)):
+        ref = fn(c.n, c.Pe, c.Da, c.dt, c.n_steps, c.c_init)
+        err = np.linalg.norm(o.double().cpu().numpy() - ref) / np.linalg.norm(ref)
+        diag = 2.0 * c.n ** 2 / c.Pe + c.n + c.Da
+        assert err < max(4 * c.n_steps * 0.5 * c.dt * diag * eps, 1e-11 if eps < 1e-10 else 1e-4), (c.n, err)
