@@ -743,30 +743,33 @@ __device__ __forceinline__ float2 dct_merge(float cak, float cam, float cbk, flo
   return make_float2(vax - vby, vay + vbx);
 }
 
-// Threads per sequence of the shared-memory transforms of the DST passes: n/16 for the
-// radix-16 Stockham (fft_smem), n/4 for the radix-4 one (fft_smem_r4: a quarter of the
-// dependent work per thread, for passes with few sequences)
-template <bool R4>
-__device__ __forceinline__ int dst_tps(int n) { return R4 ? (n >= 4 ? n >> 2 : 1) : (n >= 16 ? n >> 4 : 1); }
+// Radix 4 for the DST passes up to n = 512: at most n/2 row pairs and n/2 column pairs per
+// pass, too few sequences for the radix-16 schedule's n/16 threads each to fill the SMs, so the
+// pass lasts one sequence's dependent work, a quarter as long with n/4 threads per sequence
+__host__ __device__ constexpr bool dst_r4(int log2n) { return log2n <= 9; }
+__host__ __device__ constexpr int dst_tps(int log2n) {
+  return dst_r4(log2n) ? (log2n >= 2 ? 1 << (log2n - 2) : 1) : 1 << (log2n - 4);
+}
 
-// LOG2N > 0: the length as a compile-time constant, so that the index arithmetic and the passes fold
-template <bool R4, int LOG2N, bool INV, bool COLMAJOR>
+// The length 2^LOG2N is a compile-time constant, so that the index arithmetic and the passes fold: two
+// BDF2 steps at 32^2, 512^2 and 2048^2 2.45, 4.2 and 14.5 ms, with the length at run time 2.8, 4.7 and
+// 15.5 ms.
+template <int LOG2N, bool INV, bool COLMAJOR>
 __device__ __forceinline__ void dst_fft(float2* buf, const NkaArgs& a, int nseq, int ss, int es, int tid) {
-  if (LOG2N) fft_smem_r4_inl<float, INV, COLMAJOR>(buf, 1 << LOG2N, LOG2N, nseq, ss, es, a.twn, tid);
-  else if (R4) fft_smem_r4<float, INV, COLMAJOR>(buf, a.n, a.log2n, nseq, ss, es, a.twn, tid);
-  else fft_smem<float, INV, COLMAJOR, false>(buf, a.n, a.log2n, nseq, ss, es, a.twn, tid);
+  if (dst_r4(LOG2N)) fft_smem_r4_inl<float, INV, COLMAJOR>(buf, 1 << LOG2N, LOG2N, nseq, ss, es, a.twn, tid);
+  else fft_smem<float, INV, COLMAJOR, false>(buf, 1 << LOG2N, LOG2N, nseq, ss, es, a.twn, tid);
 }
 
 // forward DST-II along x of the row pairs (y, y + n/2) of a.src into a.S
-template <bool R4, int LOG2N>
+template <int LOG2N>
 __global__ void __launch_bounds__(256) dst_row_fwd_kernel(const __grid_constant__ NkaArgs a) {
   typedef float2 C;
-  constexpr int PTS = R4 ? 4 : 16;  // elements per thread
+  constexpr int PTS = dst_r4(LOG2N) ? 4 : 16;  // elements per thread
   if (a.skip_converged && a.gs->converged) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* buf = reinterpret_cast<C*>(smem_raw);
-  const int n = LOG2N ? 1 << LOG2N : a.n, hn = n >> 1;
-  const int tps = dst_tps<R4>(n);
+  constexpr int n = 1 << LOG2N, hn = n >> 1;
+  constexpr int tps = dst_tps(LOG2N);
   const int tid = threadIdx.x, s_loc = pdiv(tid, tps), lt = tid - s_loc * tps;
   const bool active = s_loc < a.nseq;  // whole warps are launched
   const int y = blockIdx.x * a.nseq + s_loc;
@@ -782,7 +785,7 @@ __global__ void __launch_bounds__(256) dst_row_fwd_kernel(const __grid_constant_
     }
   }
   __syncthreads();
-  dst_fft<R4, LOG2N, false, false>(buf, a, a.nseq, n, 1, tid);
+  dst_fft<LOG2N, false, false>(buf, a, a.nseq, n, 1, tid);
   if (!active) return;
   float* Sa = a.S + (long long)y * n;
   float* Sb = a.S + (long long)(y + hn) * n;
@@ -800,13 +803,14 @@ __global__ void __launch_bounds__(256) dst_row_fwd_kernel(const __grid_constant_
 
 // columns kx0 .. kx0 + C - 1 of a.S: DST-II along y, the Helmholtz inverse (with the 1/n^2
 // of the two unnormalised inverse transforms), DST-III along y, in place
-template <bool R4, int LOG2N>
+template <int LOG2N>
 __global__ void __launch_bounds__(256) dst_col_kernel(const __grid_constant__ NkaArgs a) {
   typedef float2 C;
   if (a.skip_converged && a.gs->converged) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* buf = reinterpret_cast<C*>(smem_raw);
-  const int n = LOG2N ? 1 << LOG2N : a.n, Cn = a.C, ns = Cn >> 1, lc = __ffs(Cn) - 1, ls = lc - 1;
+  constexpr int n = 1 << LOG2N;
+  const int Cn = a.C, ns = Cn >> 1, lc = __ffs(Cn) - 1, ls = lc - 1;
   const int kx0 = blockIdx.x * Cn;
   const int tid = threadIdx.x, nth = blockDim.x;
   // load (sign and Makhoul position along y), columns 2q and 2q + 1 as sequence q
@@ -817,7 +821,7 @@ __global__ void __launch_bounds__(256) dst_col_kernel(const __grid_constant__ Nk
     *slot = (y & 1) ? -v : v;
   }
   __syncthreads();
-  dst_fft<R4, LOG2N, false, true>(buf, a, ns, 1, ns, tid);
+  dst_fft<LOG2N, false, true>(buf, a, ns, 1, ns, tid);
   // per (sequence, k <= n/2): the coefficients of k and n - k, the multiplier, the inverse
   // inputs of k and n - k (each item owns its two slots)
   const float hD = (float)a.st->dtc, inv_n2 = 1.0f / ((float)n * (float)n);
@@ -845,7 +849,7 @@ __global__ void __launch_bounds__(256) dst_col_kernel(const __grid_constant__ Nk
     if (k > 0 && km != k) buf[sp(q + km * ns)] = dct_merge(cam, cak, cbm, cbk, a.ph[n - k]);
   }
   __syncthreads();
-  dst_fft<R4, LOG2N, true, true>(buf, a, ns, 1, ns, tid);
+  dst_fft<LOG2N, true, true>(buf, a, ns, 1, ns, tid);
   for (int e = tid; e < n * Cn; e += nth) {
     const int y = e >> lc, c = e & (Cn - 1);
     const float v = reinterpret_cast<const float*>(&buf[sp((c >> 1) + mk_pos(y, n) * ns)])[c & 1];
@@ -854,15 +858,15 @@ __global__ void __launch_bounds__(256) dst_col_kernel(const __grid_constant__ Nk
 }
 
 // inverse DST-III along x of the row pairs (y, y + n/2) of a.S; w = (1/a0) result
-template <int MODE, bool R4, int LOG2N>
+template <int MODE, int LOG2N>
 __global__ void __launch_bounds__(256) dst_row_inv_kernel(const __grid_constant__ NkaArgs a) {
   typedef float2 C;
-  constexpr int PTS = R4 ? 4 : 16, KPTS = PTS / 2 + 1;  // elements, coefficient pairs per thread
+  constexpr int PTS = dst_r4(LOG2N) ? 4 : 16, KPTS = PTS / 2 + 1;  // elements, coefficient pairs per thread
   if (a.skip_converged && a.gs->converged) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* buf = reinterpret_cast<C*>(smem_raw);
-  const int n = LOG2N ? 1 << LOG2N : a.n, hn = n >> 1;
-  const int tps = dst_tps<R4>(n);
+  constexpr int n = 1 << LOG2N, hn = n >> 1;
+  constexpr int tps = dst_tps(LOG2N);
   const int tid = threadIdx.x, s_loc = pdiv(tid, tps), lt = tid - s_loc * tps;
   const bool active = s_loc < a.nseq;  // whole warps are launched
   const int y = blockIdx.x * a.nseq + s_loc;
@@ -881,7 +885,7 @@ __global__ void __launch_bounds__(256) dst_row_inv_kernel(const __grid_constant_
     }
   }
   __syncthreads();
-  dst_fft<R4, LOG2N, true, false>(buf, a, a.nseq, n, 1, tid);
+  dst_fft<LOG2N, true, false>(buf, a, a.nseq, n, 1, tid);
   const float sc = (float)a.K->inv_a0;
   float wa[PTS], wb[PTS];
 #pragma unroll
@@ -1261,9 +1265,9 @@ static NkaArgs nka_args(NKRun& r) {
 // columns, C/2 complex sequences, at least 152 tiles where n allows and within the default
 // 48 KB of shared memory
 struct DstGeom { int nseq, ctas, threads, C, col_threads; size_t smem, col_smem; };
-static DstGeom dst_geom(int n, bool r4) {
+static DstGeom dst_geom(int log2n) {
   DstGeom g;
-  const int hn = n / 2, tps = r4 ? (n >= 4 ? n / 4 : 1) : (n >= 16 ? n / 16 : 1);
+  const int n = 1 << log2n, hn = n / 2, tps = dst_tps(log2n);
   int ns = row_nseq(n, hn);
   if (ns > hn) ns = hn;
   while (ns > 1 && (hn / ns < 152 || ns * tps > 256)) ns >>= 1;
@@ -1281,33 +1285,27 @@ static DstGeom dst_geom(int n, bool r4) {
   return g;
 }
 
-// Radix 4 for the DST passes up to n = 512: at most n/2 row pairs and n/2 column pairs per
-// pass, too few sequences for the radix-16 schedule's n/16 threads each to fill the SMs, so the
-// pass lasts one sequence's dependent work, a quarter as long with n/4 threads per sequence
-static bool dst_r4(int n) { return n <= 512; }
-
-template <int MODE, bool R4, int LOG2N>
+template <int MODE, int LOG2N>
 static cudaError_t nka_dst(NKRun& r, const NkaArgs& a, const DstGeom& g) {
-  dst_row_fwd_kernel<R4, LOG2N><<<g.ctas, g.threads, g.smem, r.s>>>(a);
-  dst_col_kernel<R4, LOG2N><<<r.n / g.C, g.col_threads, g.col_smem, r.s>>>(a);
-  dst_row_inv_kernel<MODE, R4, LOG2N><<<g.ctas, g.threads, g.smem, r.s>>>(a);
+  dst_row_fwd_kernel<LOG2N><<<g.ctas, g.threads, g.smem, r.s>>>(a);
+  dst_col_kernel<LOG2N><<<r.n / g.C, g.col_threads, g.col_smem, r.s>>>(a);
+  dst_row_inv_kernel<MODE, LOG2N><<<g.ctas, g.threads, g.smem, r.s>>>(a);
   return cudaGetLastError();
 }
 
 // w = M^-1 a.src: DST-II along x, along y with the multiplier and DST-III along y, DST-III
-// along x (MODE: w into t, or the cycle start V_0 = w).  Grids of 64^2 to 512^2 have instances of
-// their length: five BDF2 steps at 512^2, 138 solves, 9.4 ms with the length at run time, 8.6 ms.
+// along x (MODE: w into t, or the cycle start V_0 = w)
 template <int MODE>
 static cudaError_t nka_precond(NKRun& r, NkaArgs a) {
-  const DstGeom g = dst_geom(r.n, dst_r4(r.n));
+  const DstGeom g = dst_geom(a.log2n);
   a.nseq = g.nseq;
   a.C = g.C;
-  switch (r.n) {
-    case 512: return nka_dst<MODE, true, 9>(r, a, g);
-    case 256: return nka_dst<MODE, true, 8>(r, a, g);
-    case 128: return nka_dst<MODE, true, 7>(r, a, g);
-    case 64: return nka_dst<MODE, true, 6>(r, a, g);
-    default: return dst_r4(r.n) ? nka_dst<MODE, true, 0>(r, a, g) : nka_dst<MODE, false, 0>(r, a, g);
+  switch (a.log2n) {
+#define MJX_DST(L) case L: return nka_dst<MODE, L>(r, a, g);
+    MJX_DST(1) MJX_DST(2) MJX_DST(3) MJX_DST(4) MJX_DST(5) MJX_DST(6) MJX_DST(7) MJX_DST(8) MJX_DST(9)
+    MJX_DST(10)
+    default: return nka_dst<MODE, 11>(r, a, g);
+#undef MJX_DST
   }
 }
 
