@@ -66,9 +66,19 @@ __device__ __forceinline__ void tw_bfr(double2& a, double2& b, double2 w) {
   a = mk<double2>(fma(w.x, v, a.x), fma(-w.x, u, a.y));
 }
 
-// v <- DFT_R(v_t w^t) in natural order, w^t the table entry at t * i; ne = n / 8 (radix 8)
+// v <- DFT_R(v_t w^t) in natural order, w^t the table entry at t * i; ne = n / 8 (radix 8).
+// FP64 folds the twiddles into the butterfly's sums.  FP32, which gains no operation by that,
+// multiplies each point by its own table entry: folded, a point of radix 4 and 8 goes through two or
+// three rounded twiddles.  Error of 50 steps against that of the separate full-spectrum passes, mean
+// over 40 grids of 5 to 400 points a side: 0.84, folded 1.10.  The longest Bluestein lengths, whose
+// tables stay in global memory, take 7 to 10 % longer for it (1600 x 1001: 254 -> 272 us, 3 steps).
 template <typename T, int R, bool FIRST>
 __device__ __forceinline__ void tile_bf(cx<T>* v, const cx<T>* tw, int i, int ne) {
+  if constexpr (sizeof(T) == 4 && R > 2 && !FIRST) {
+#pragma unroll
+    for (int t = 1; t < R; ++t) v[t] = cmul(v[t], tw[t * i]);
+    return tile_bf<T, R, true>(v, tw, 0, 0);
+  }
   typedef cx<T> C;
   if constexpr (R == 2) {
     if (FIRST) dft2<false>(v[0], v[1]);
