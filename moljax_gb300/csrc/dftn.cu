@@ -86,28 +86,6 @@ static bool dft_len_ok(int n) {
   return n <= 2048;
 }
 
-// in-place iterative radix-2 FFT on the host (FP64), for the Bluestein filter
-static void host_fft2(std::vector<double>& re, std::vector<double>& im) {
-  const int n = (int)re.size();
-  for (int i = 1, j = 0; i < n; ++i) {
-    int bit = n >> 1;
-    for (; j & bit; bit >>= 1) j ^= bit;
-    j ^= bit;
-    if (i < j) { std::swap(re[i], re[j]); std::swap(im[i], im[j]); }
-  }
-  const double twopi = 6.283185307179586476925286766559;
-  for (int len = 2; len <= n; len <<= 1)
-    for (int i = 0; i < n; i += len)
-      for (int k = 0; k < len / 2; ++k) {
-        const double ang = -twopi * k / len;
-        const double wr = cos(ang), wi = sin(ang);
-        const int u = i + k, v = i + k + len / 2;
-        const double xr = re[v] * wr - im[v] * wi, xi = re[v] * wi + im[v] * wr;
-        re[v] = re[u] - xr; im[v] = im[u] - xi;
-        re[u] += xr; im[u] += xi;
-      }
-}
-
 // ------------------------------------------------------------------ row pass
 enum { GROW_LOAD_SPEC = 1, GROW_STORE_REAL = 2, GROW_STORE_SPEC = 4 };
 
@@ -530,27 +508,18 @@ mjx_status mjx_dftn_plan_init(void* plan, int n, int dtype, void* stream) {
     if (e == 4) { float* q = (float*)(host.data() + off); q[2 * i] = (float)re; q[2 * i + 1] = (float)im; }
     else { double* q = (double*)(host.data() + off); q[2 * i] = re; q[2 * i + 1] = im; }
   };
-  const double twopi = 6.283185307179586476925286766559, pi = 0.5 * twopi;
-  for (int j = 0; j < g.L; ++j) {  // L = n unless Bluestein
+  const double twopi = 6.283185307179586476925286766559;
+  const Roots roots(g.L);  // L = n unless Bluestein
+  for (int j = 0; j < g.L; ++j) {
     double re, im;
-    tile_twiddle(j, g.L, e, &re, &im);
+    tile_twiddle(roots, j, e, &re, &im);
     put(g.tw, j, re, im);
   }
   if (g.bluestein) {
-    std::vector<double> cre(n), cim(n);
-    for (int j = 0; j < n; ++j) {  // exp(-i pi j^2 / n), j^2 reduced mod 2n to keep the angle exact
-      const long long r = ((long long)j * j) % (2LL * n);
-      cre[j] = cos(pi * (double)r / n);
-      cim[j] = -sin(pi * (double)r / n);
-      put(g.chirp, j, cre[j], cim[j]);
-    }
-    std::vector<double> bre(g.L, 0.0), bim(g.L, 0.0);
-    for (int j = 0; j < n; ++j) {
-      bre[j] = cre[j]; bim[j] = -cim[j];
-      if (j > 0) { bre[g.L - j] = cre[j]; bim[g.L - j] = -cim[j]; }
-    }
-    host_fft2(bre, bim);
-    for (int j = 0; j < g.L; ++j) put(g.bhat, j, bre[j] / g.L, bim[j] / g.L);
+    std::vector<double> chirp, bhat;
+    bluestein_tables(n, roots, e == 8, &chirp, &bhat);
+    for (int j = 0; j < n; ++j) put(g.chirp, j, chirp[2 * j], chirp[2 * j + 1]);
+    for (int j = 0; j < g.L; ++j) put(g.bhat, j, bhat[2 * j], bhat[2 * j + 1]);
   }
   double* sym = (double*)(host.data() + g.sym);
   for (int j = 0; j < n; ++j) {

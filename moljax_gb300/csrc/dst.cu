@@ -462,29 +462,6 @@ __global__ void __launch_bounds__(512) dct2_kernel(const __grid_constant__ Dst1A
   }
 }
 
-// In-place iterative radix-2 FFT on the host (FP64), for the Bluestein filter.
-static void host_fft(std::vector<double>& re, std::vector<double>& im) {
-  const int n = (int)re.size();
-  for (int i = 1, j = 0; i < n; ++i) {
-    int bit = n >> 1;
-    for (; j & bit; bit >>= 1) j ^= bit;
-    j ^= bit;
-    if (i < j) { std::swap(re[i], re[j]); std::swap(im[i], im[j]); }
-  }
-  const double twopi = 6.283185307179586476925286766559;
-  for (int len = 2; len <= n; len <<= 1) {
-    for (int i = 0; i < n; i += len)
-      for (int k = 0; k < len / 2; ++k) {
-        const double ang = -twopi * k / len;
-        const double wr = cos(ang), wi = sin(ang);
-        const int u = i + k, v = i + k + len / 2;
-        const double xr = re[v] * wr - im[v] * wi, xi = re[v] * wi + im[v] * wr;
-        re[v] = re[u] - xr; im[v] = im[u] - xi;
-        re[u] += xr; im[u] += xi;
-      }
-  }
-}
-
 // FP32 launch: sequences per CTA to 256 threads, fewer until every SM has a CTA
 static Dst32Args trig_args32(const Dst1Geom& g, const char* p, long long nrows, long long nseq_total, int mode,
                              const float* x, float* out, const float* lam, double h, double D, float scale) {
@@ -586,28 +563,18 @@ static void trig_tables(std::vector<unsigned char>& host, const Dst1Geom& g, int
     if (e == 4) { float* q = (float*)(host.data() + off); q[2 * i] = (float)re; q[2 * i + 1] = (float)im; }
     else { double* q = (double*)(host.data() + off); q[2 * i] = re; q[2 * i + 1] = im; }
   };
+  const Roots roots(g.L);
   for (int j = 0; j < g.L; ++j) {
     double re, im;
-    tile_twiddle(j, g.L, e, &re, &im);
+    tile_twiddle(roots, j, e, &re, &im);
     put(g.tw, j, re, im);
   }
   if (e == 4) fft_pass_table((float*)(host.data() + g.tw), g.L);
   if (g.bluestein) {
-    // c[n] = exp(-i pi n^2 / M), with n^2 reduced mod 2M to keep the angle exact
-    std::vector<double> cre(g.M), cim(g.M);
-    for (int j = 0; j < g.M; ++j) {
-      const long long r = ((long long)j * j) % (2LL * g.M);
-      cre[j] = cos(pi * (double)r / g.M);
-      cim[j] = -sin(pi * (double)r / g.M);
-      put(g.chirp, j, cre[j], cim[j]);
-    }
-    std::vector<double> bre(g.L, 0.0), bim(g.L, 0.0);
-    for (int j = 0; j < g.M; ++j) {
-      bre[j] = cre[j]; bim[j] = -cim[j];
-      if (j > 0) { bre[g.L - j] = cre[j]; bim[g.L - j] = -cim[j]; }
-    }
-    host_fft(bre, bim);
-    for (int j = 0; j < g.L; ++j) put(g.bhat, j, bre[j] / g.L, bim[j] / g.L);
+    std::vector<double> chirp, bhat;
+    bluestein_tables(g.M, roots, e == 8, &chirp, &bhat);
+    for (int j = 0; j < g.M; ++j) put(g.chirp, j, chirp[2 * j], chirp[2 * j + 1]);
+    for (int j = 0; j < g.L; ++j) put(g.bhat, j, bhat[2 * j], bhat[2 * j + 1]);
   }
   if (kind == 1)
     for (int k = 0; k < g.N; ++k) put(g.shift, k, cos(pi * k / (2.0 * g.N)), -sin(pi * k / (2.0 * g.N)));

@@ -958,13 +958,15 @@ mjx_status mjx_spec2d_plan_init(void* plan, const mjx_grid2d* g, int symbol, int
       const double ang = twopi * (double)j / (double)n;
       const double c = cos(ang), s = -sin(ang);
       if (e == 4) { float* p = (float*)dst; p[2 * j] = (float)c; p[2 * j + 1] = (float)s; }
-      else {
-        double* p = (double*)dst;
-        p[2 * j] = c; p[2 * j + 1] = s;
-        tile_twiddle(j, n, 8, &p[2 * (n + j)], &p[2 * (n + j) + 1]);
-      }
+      else { double* p = (double*)dst; p[2 * j] = c; p[2 * j + 1] = s; }
     }
-    if (e == 4) fft_pass_table((float*)dst, n);
+    if (e == 4) {
+      fft_pass_table((float*)dst, n);
+    } else {
+      double* p = (double*)dst + 2 * n;
+      const Roots roots(n);
+      for (int j = 0; j < n; ++j) tile_twiddle(roots, j, 8, &p[2 * j], &p[2 * j + 1]);
+    }
   };
   // eigenvalue of the 1D periodic Laplacian for integer frequency m on n points of spacing d
   auto lam1 = [&](int m, int n, double d) {
@@ -981,7 +983,8 @@ mjx_status mjx_spec2d_plan_init(void* plan, const mjx_grid2d* g, int symbol, int
         p[2 * (kW1024 + 32 * k1 + l) + 1] = p[2 * (l * k1) + 1];
       }
   }
-  put_tw(pv.twy, ny);
+  if (ny == nx && e == 8) memcpy((void*)pv.twy, pv.twx, (size_t)twy_count(ny, e) * 2 * e);
+  else put_tw(pv.twy, ny);
   for (int kx = 0; kx < ldc; ++kx) {
     const double v = kx <= nx / 2 ? lam1(kx, nx, g->dx) : 0.0;
     if (e == 4) ((float*)pv.lamx)[kx] = (float)v; else ((double*)pv.lamx)[kx] = v;

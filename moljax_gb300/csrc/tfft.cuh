@@ -19,22 +19,22 @@
 #include <math.h>
 
 #include "fft.cuh"
+#include "roots.cuh"
 
 namespace mjx {
 
-// host: entry j of n of a twiddle table in the form that tile_dft reads
-inline void tile_twiddle(int j, int n, int elem, double* re, double* im) {
+// host: entry j of a twiddle table in the form that tile_dft reads, from the roots of its length
+inline void tile_twiddle(const Roots& r, int j, int elem, double* re, double* im) {
+  const DD c = r.c[j], s = r.s[j];
   if (elem == 4) {
-    const double ang = 6.283185307179586476925286766559 * (double)j / (double)n;
-    *re = cos(ang);
-    *im = -sin(ang);
-  } else if (4LL * j == n || 4LL * j == 3LL * n) {
+    *re = c.h;
+    *im = -s.h;
+  } else if (c.h == 0.0) {  // pi / 2, 3 pi / 2
     *re = 0x1p-60;
-    *im = 4LL * j == n ? 0x1p60 : -0x1p60;
+    *im = s.h > 0.0 ? 0x1p60 : -0x1p60;
   } else {  // the tangent belongs to the rounded cosine, so that their product is the sine
-    const long double a = 6.283185307179586476925286766559005768L * (long double)j / (long double)n;
-    *re = (double)cosl(a);
-    *im = (double)(sinl(a) / (long double)*re);
+    *re = c.h;
+    *im = dd_div(s, c.h).h;
   }
 }
 

@@ -271,3 +271,11 @@ def test_fp32_rounding_of_repeated_transforms(cuda, shape):
     error grows with the steps.  Half a rounding (rms) a level when each point takes one rounded
     twiddle a butterfly; two or three in a row leave more."""
     assert _identity_error(shape, torch.float32, 50, cuda) < 0.52 * 50 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("shape", [(1999, 6), (97, 6), (17, 6), (1024, 7)])
+def test_fp64_rounding_with_bluestein_tables(cuda, shape):
+    """One FP64 transform pair through Bluestein lengths: chirp and filter are rounded once from their
+    exact values, so the error is that of the transforms' arithmetic, at most 0.65 of a rounding (rms)
+    a level; tables formed from rounded angles add as much again."""
+    assert _identity_error(shape, torch.float64, 1, cuda) < 0.65 * 2.0 ** -53
