@@ -161,7 +161,6 @@ __global__ void __launch_bounds__(512) grow_kernel(const __grid_constant__ GRowA
 // ------------------------------------------------------------------ multipliers
 struct GMul {
   int mult, nx, nb, ny;     // sizes along x, the batch axis of a box (0 in 2D), the column
-  int symbol;
   const double* sx;         // d^2 lambda along x, the batch axis and the column
   const double* sb;
   const double* sy;
@@ -396,7 +395,7 @@ static mjx_status general_apply(const void* plan_y, const void* plan_x, const mj
   c.d = dft_desc<T>(plan_y, ny);
   c.spec = spec; c.bstride = (long long)ny * ld; c.ld = c.ldx = ld; c.ncols = c.hx = hx; c.dirs = 3;
   GMul& m = c.m;
-  m.mult = mult; m.nx = nx; m.nb = 0; m.ny = ny; m.symbol = symbol; m.h = h;
+  m.mult = mult; m.nx = nx; m.nb = 0; m.ny = ny; m.h = h;
   symbol_axis(plan_x, nx, sizeof(T), symbol, g->dx, &m.sx, &m.ix);
   symbol_axis(plan_y, ny, sizeof(T), symbol, g->dy, &m.sy, &m.iy);
   m.kxs = twopi / (nx * g->dx);
@@ -444,7 +443,7 @@ static mjx_status general_apply3(const void* pz, const void* py, const void* px,
   z.d = dft_desc<T>(pz, nz);
   z.bstride = 0; z.ld = z.ncols = ny * ld; z.dirs = 3; z.mode = GCOL_VALUE;
   GMul& m = z.m;
-  m.mult = mult; m.nx = nx; m.nb = ny; m.ny = nz; m.symbol = symbol; m.h = h; m.D[0] = D;
+  m.mult = mult; m.nx = nx; m.nb = ny; m.ny = nz; m.h = h; m.D[0] = D;
   symbol_axis(px, nx, sizeof(T), symbol, g->dx, &m.sx, &m.ix);
   symbol_axis(py, ny, sizeof(T), symbol, g->dy, &m.sb, &m.ib);
   symbol_axis(pz, nz, sizeof(T), symbol, g->dz, &m.sy, &m.iy);

@@ -291,13 +291,7 @@ __global__ void __launch_bounds__(LOG2NY == 9 || LOG2NY == 10 ? 512 : ColThreads
   for (int q = 0; q < 16; ++q) {
     const int ky = lt + q * tps;
     x[q] = mk<C>((T)0, (T)0);
-    if (!in || ky >= ny) continue;
-    if (a.oddy && ky >= (ny >> 1)) {
-      const C v = src[(ny - 1 - ky) * ldc];
-      x[q] = mk<C>(-v.x, -v.y);
-    } else {
-      x[q] = src[ky * ldc];
-    }
+    if (in && ky < ny) x[q] = src[ky * ldc];
   }
   const int dirs = jb.dirs ? jb.dirs : 3;
   if (dirs & 1) fft_regs<T, false, false>(x, buf, ny, log2ny, lt, c, Cn, a.tw, active);
@@ -350,7 +344,7 @@ __global__ void __launch_bounds__(LOG2NY == 9 || LOG2NY == 10 ? 512 : ColThreads
 #pragma unroll
   for (int q = 0; q < 16; ++q) {
     const int ky = lt + q * tps;
-    if (ky < ny && !(a.oddy && ky >= (ny >> 1))) dst[ky * ldc] = x[q];
+    if (ky < ny) dst[ky * ldc] = x[q];
   }
 }
 
