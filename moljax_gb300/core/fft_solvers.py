@@ -103,7 +103,7 @@ def _pow2(n: int) -> bool:
 class GeneralSpectralPlan:
     """Periodic (ny, nx) grid of any supported size (powers of two up to 4096, other sizes up
     to 2048): half-spectrum row and column passes of ``csrc/dftn.cu`` (mixed-radix Stockham or
-    Bluestein; complex multipliers and tables the full-spectrum path).  Same ``apply`` as
+    Bluestein; complex multipliers and tables as their Hermitian part).  Same ``apply`` as
     ``SpectralPlan``; the fused device loops (IMEX, ETD) take powers of two, their
     host-driven forms run on this plan."""
 
@@ -186,7 +186,7 @@ class GeneralSpectralPlan:
 
 def get_plan(ny, nx, dy, dx, symbol="fd", dtype=torch.float64, device=None):
     """The spectral plan of a periodic (ny, nx) grid: the fused power-of-two passes, or the
-    general full-spectrum path for other sizes."""
+    general half-spectrum passes for other sizes."""
     dev = _device(device)
     key = (int(ny), int(nx), float(dy), float(dx), symbol, dtype, str(dev))
     p = _plans.get(key)

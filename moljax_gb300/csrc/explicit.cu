@@ -1508,8 +1508,8 @@ static mjx_status x_adaptive(const XModel& m, const mjx_explicit_problem* pb, co
 
   const XAttempt<T> A = build_x<T>(m, pb->method, ws, L, st, pid->atol, pid->rtol);
   // SSPRK3 and RK4 of up to two FP32 fields take the three steps of an attempt (full, half, half
-  // with the error) as three fused kernels instead of 9 or 12 stage kernels: 24 B of memory
-  // traffic a point and field instead of 192 B for RK4.  Two fields, 1500 x 2000 with walls, an
+  // with the error) as three fused kernels instead of 9 or 12 stage kernels: 28 B of memory
+  // traffic a point and field (the last one also reads the full step) instead of 192 B for RK4.  Two fields, 1500 x 2000 with walls, an
   // attempt: 12 x 20 us -> 3 x 69 us.  More fields leave one block per SM, FP64 is bound by its
   // arithmetic, which the halo rings increase, and kinetics networks run in the stage kernels.
   XFused<T> fs[3];

@@ -96,10 +96,12 @@ inline size_t mcol_smem(int ny, int C) { return 2 * (size_t)sp_size(ny * C) * si
 //   C2 MC_MID       PA <- M_A (PA + F ZA);  PB <- M_B^2 (PB + F ZB), ZB <- its inverse
 //   C3 MC_HALF_END  Y' = M_B (PB + F ZB); ZA <- inverse of Y' - PA, ZB <- inverse of Y'
 // LOG2NY, CN > 0 fix the column length and the tile width at compile time (the lengths 64 to
-// 4096, in the batch 64 to 512), so that the index arithmetic and the radix schedule fold into
-// the code.  C1 / C2 / C3 at 1024^2: 14 / 20 / 21 us, against 24 us each with every element in
+// 4096, in the batch every length), so that the index arithmetic and the radix schedule fold into
+// the code; shorter columns of a single solve read both (8 x 64 to 32 x 4096 a solve 1.4 to 1.6 times
+// as fast as with every element in shared memory).  C1 / C2 / C3 at 1024^2: 14 / 20 / 21 us, against 24 us each with every element in
 // shared memory between the transforms; 256^2 1.8x a solve.  Four operands in flight beat two in
-// C1 (13.6 against 14.6 us) and lose in C2 and C3, where they spill (24 us).
+// C1 (13.6 against 14.6 us) and lose in C2 and C3 (24 us), whose registers they overflow; with two
+// C2 spills 116 bytes a thread and C3 16 at 1024 rows.
 template <int TYPE, int LOG2NY = 0, int CN = 0>
 __device__ __forceinline__ void mcol_tile(float2* buf, const MColTile& t, int tid) {
   const int ny = LOG2NY ? (1 << LOG2NY) : t.ny, log2ny = LOG2NY ? LOG2NY : t.log2ny;

@@ -269,7 +269,8 @@ template <typename T> struct ColThreads { static constexpr int v = sizeof(T) == 
 // FP32 takes 29 us a step at 256^2 (48 with the elements in shared memory between the transforms
 // and the length at run time), 38 at 1024^2 (61).  512 and 1024 rows get 128 registers a thread
 // (their CTAs have at most 512): 12.8 and 18.9 us against 14.8 and 21.6; shorter columns fit in 64,
-// and a box's passes want the CTAs (128 rows: 25.7 us against 29.6).
+// and a box's passes want the CTAs (128 rows: 25.7 us against 29.6).  The other lengths, five steps:
+// 4 x 256 51 us (157), 16 x 4096 80 (167), 2048 x 256 103 (228), 4096 x 1024 235 (312).
 template <typename T, int LOG2NY = 0>
 __global__ void __launch_bounds__(LOG2NY == 9 || LOG2NY == 10 ? 512 : ColThreads<T>::v, 1) col_kernel(const __grid_constant__ ColArgs<T> a) {
   typedef cx<T> C;
@@ -353,7 +354,8 @@ __global__ void __launch_bounds__(LOG2NY == 9 || LOG2NY == 10 ? 512 : ColThreads
 // FP32 rows of 1024 points, one warp per sequence: the row transform of the FP32 adaptive IMEX
 // loop.  Its error estimate is a difference of FP32 solutions, so the step sizes and with them the
 // end state follow the transform's rounding (1024^2, t = 6: 2.8e-5 apart between this kernel and
-// row_kernel); that loop keeps the transform that its results were made with.
+// row_kernel; their errors against FP64 8.8e-5 and 6.7e-5).  That loop keeps the transform that its
+// results were made with, although row_kernel is nearer and faster (13.2 against 18.0 us).
 template <int RX>
 __global__ void __launch_bounds__(128) row_kernel_w32(const __grid_constant__ RowArgs<float> a) {
   typedef float2 C;

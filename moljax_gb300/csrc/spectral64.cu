@@ -12,8 +12,11 @@
 //   FFT-CN 128^2, 100 steps   4713 -> 1790 us
 //   FFT-CN 128^3, 10 steps    4754 -> 3060 us
 //   Strang 256^2, 100 steps   4665 -> 3015 us
-// What bounds them now: FP64 issue, 70 % of it in the 256^2 row pass (128 CTAs of four warps) and
-// 85 % in the box's passes; the 128^2 steps two chains of seven radix-2 passes.
+// What bounds them now: in the box's passes FP64 issue (82 to 86 % of the busy SMs' rate); at 256^2
+// (128 and 130 CTAs of four warps) it is 55 % of it in the rows and 43 % in the columns, the rest the
+// dependent chain of one warp a sub-partition; at 128^2 that chain (seven radix-2 passes, 23 %).
+// Columns of 4096 rows in col_kernel<double, 12>: a step at 4096 x 64 and 4096 x 1024 133 and 686 us
+// (164 and 820 with every element in shared memory between the transforms).
 // Longer transforms stay with spectral.cu: two buffers of 4096 FP64 points leave one CTA an SM
 // and no second phase to overlap with.
 #include <string.h>
