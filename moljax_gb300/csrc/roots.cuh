@@ -28,7 +28,7 @@ inline DD dd_add(DD a, DD b) {
 }
 inline DD dd_neg(DD a) { return {-a.h, -a.l}; }
 inline DD dd_mul(DD a, DD b) {
-  const double p = a.h * b.h;
+  const double p = fma(a.h, b.h, 0.0);  // rounded here: a host compiler may fuse a plain product into a sum
   return dd_fast(p, fma(a.h, b.h, -p) + (a.h * b.l + a.l * b.h));
 }
 inline DD dd_div(DD a, double d) {
